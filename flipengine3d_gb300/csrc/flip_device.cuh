@@ -114,41 +114,32 @@ void launch_mark_fast(const ParticleSoA &p, int n, const float *maxSpeedSq, unsi
 // outside the system hold zeros
 // Sweep layout: the vectors of the MIC(0) sweeps (factor rows, right-hand
 // side, result) are stored step-major.  The interior pencils along i are cut
-// into tiles of SWEEP_TJ x SWEEP_TK: SWEEP_TJ along the tile's lane axis a
-// and SWEEP_TK along its slot axis b, where (a, b) = (j, k), or (k, j) when
-// `swap` is set (the orientation is chosen per solve).  Pencil (l, w) of a
-// tile holds cell i at forward step tf = i - 1 + SWEEP_SL * l + SWEEP_SW * w:
-// a pencil runs SWEEP_SL steps behind its lane neighbour and SWEEP_SW steps
-// behind its slot neighbour, so a term crosses lanes SWEEP_SL steps and slots
-// SWEEP_SW steps after it is formed.  Entry (tile, tf, w, l) lives at
-// ((tile * T + tf) * SWEEP_NP + w * SWEEP_TJ + l),
-// T = I - 2 + SWEEP_SL * (SWEEP_TJ - 1) + SWEEP_SW * (SWEEP_TK - 1).  A chunk of
-// consecutive steps of a tile is one contiguous block, in either sweep
-// direction.  Entries that hold no interior cell stay zero.
-#ifndef SWEEP_SL
-#define SWEEP_SL 1
-#endif
-#ifndef SWEEP_SW
-#define SWEEP_SW 1
-#endif
-#ifndef SWEEP_SLOTS
-#define SWEEP_SLOTS 8   // pencils of a tile along its slot axis
-#endif
-constexpr int SWEEP_TJ = 32, SWEEP_TK = SWEEP_SLOTS, SWEEP_NP = SWEEP_TJ * SWEEP_TK;
-static_assert(SWEEP_SL >= 1 && SWEEP_SL <= 4 && SWEEP_SW >= 1 && SWEEP_SW <= 4, "sweep skews");
+// into tiles of SWEEP_WA x SWEEP_WB along axes (a, b) = (j, k), or (k, j) when
+// `swap` is set (the orientation is chosen per solve).  Pencil (A, B) of a tile
+// holds cell i at forward step tf = i - 1 + A + B: a pencil runs one step
+// behind each of its lower neighbours.  A tile is worked by warps of SWEEP_VA x
+// SWEEP_VB pencils, one per lane: warp wa + 2 wb, lane la + 8 lb holds pencil
+// (8 wa + la, 4 wb + lb), and its entry at step tf is
+// (tile * T + tf) * SWEEP_NP + warp * 32 + lane.
+// T = I - 2 + (SWEEP_WA - 1) + (SWEEP_WB - 1) up to a multiple of SWEEP_CH, so that
+// a chunk of SWEEP_CH steps is one contiguous block in either sweep direction.
+// Entries that hold no interior cell stay zero.
+constexpr int SWEEP_WA = 16, SWEEP_WB = 8, SWEEP_NP = SWEEP_WA * SWEEP_WB, SWEEP_CH = 8;
+constexpr int SWEEP_VA = 8, SWEEP_VB = 4;
+constexpr int SWEEP_CA = 2, SWEEP_CB = 4;   // tiles of a thread-block cluster along a and b
 struct SweepLayout {
-    int ntj, ntk, T;   // tiles along the lane and warp axes, steps per tile
-    int swap;          // 0: lanes along j, warps along k; 1: lanes along k, warps along j
-    int EA, EB;        // grid extents along the lane and warp axes
+    int nta, ntb, T;   // tiles along a and b, steps per tile
+    int swap;          // 0: (a, b) = (j, k); 1: (a, b) = (k, j)
+    int EA, EB;        // grid extents along a and b
 };
 inline SweepLayout sweep_layout(int I, int J, int K, int swap = 0) {
     SweepLayout g;
     g.swap = swap;
     g.EA = swap ? K : J;
     g.EB = swap ? J : K;
-    g.ntj = (g.EA - 2 + SWEEP_TJ - 1) / SWEEP_TJ;
-    g.ntk = (g.EB - 2 + SWEEP_TK - 1) / SWEEP_TK;
-    g.T = (I - 2) + SWEEP_SL * (SWEEP_TJ - 1) + SWEEP_SW * (SWEEP_TK - 1);
+    g.nta = (g.EA - 2 + SWEEP_WA - 1) / SWEEP_WA;
+    g.ntb = (g.EB - 2 + SWEEP_WB - 1) / SWEEP_WB;
+    g.T = ((I - 2) + (SWEEP_WA - 1) + (SWEEP_WB - 1) + SWEEP_CH - 1) / SWEEP_CH * SWEEP_CH;
     return g;
 }
 // entries of either orientation: the arrays are allocated for the larger
@@ -156,16 +147,17 @@ inline long long sweep_layout_size(int I, int J, int K) {
     long long best = 0;
     for (int sw = 0; sw < 2; sw++) {
         SweepLayout g = sweep_layout(I, J, K, sw);
-        best = std::max(best, (long long)g.ntj * g.ntk * g.T * SWEEP_NP);
+        best = std::max(best, (long long)g.nta * g.ntb * g.T * SWEEP_NP);
     }
     return best;
 }
 // entry of interior cell (i, j, k)
 __host__ __device__ __forceinline__ long long sweep_index(const SweepLayout &g, int i, int j, int k) {
     const int aa = (g.swap ? k : j) - 1, bb = (g.swap ? j : k) - 1;
-    const int l = aa % SWEEP_TJ, w = bb % SWEEP_TK;
-    const int tile = aa / SWEEP_TJ + g.ntj * (bb / SWEEP_TK);
-    return ((long long)tile * g.T + (i - 1 + SWEEP_SL * l + SWEEP_SW * w)) * SWEEP_NP + w * SWEEP_TJ + l;
+    const int A = aa % SWEEP_WA, B = bb % SWEEP_WB;
+    const int tile = aa / SWEEP_WA + g.nta * (bb / SWEEP_WB);
+    const int warp = A / SWEEP_VA + SWEEP_WA / SWEEP_VA * (B / SWEEP_VB), lane = A % SWEEP_VA + SWEEP_VA * (B % SWEEP_VB);
+    return ((long long)tile * g.T + (i - 1 + A + B)) * SWEEP_NP + warp * 32 + lane;
 }
 
 // Device-side control of the PCG loop: the convergence test runs on the

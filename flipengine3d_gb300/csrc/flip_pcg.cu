@@ -893,16 +893,18 @@ int pressure_project(const StepConsts &c, const PressureArgs &a, PressureBuffers
         return FLIP_E_RUNTIME;
     }
     // Sweep tile orientation for this solve: the one whose tiles the rows'
-    // extent crosses with the shorter chain of hops.  A hop across the lane
-    // axis delays the next tile by about SL TJ + chunk + handoff steps, across
-    // the warp axis by about SW TK + chunk + handoff.
+    // extent crosses with the shorter chain of hops.  A hop inside a cluster
+    // delays the next tile by about 8 steps (a group of edge terms and its way
+    // through shared memory), one between clusters by about 24.
     {
         const int jlo = mail->levelRange[3], jhi = mail->levelRange[4];
         const int klo = mail->levelRange[5], khi = mail->levelRange[6];
-        auto hops = [](int lo_, int hi_, int w) { return (hi_ - 1) / w - (lo_ - 1) / w; };
-        const int lagA = SWEEP_SL * SWEEP_TJ + 8 + 14, lagB = SWEEP_SW * SWEEP_TK + 8 + 14;
-        const long long cost0 = (long long)hops(jlo, jhi, SWEEP_TJ) * lagA + (long long)hops(klo, khi, SWEEP_TK) * lagB;
-        const long long cost1 = (long long)hops(klo, khi, SWEEP_TJ) * lagA + (long long)hops(jlo, jhi, SWEEP_TK) * lagB;
+        auto lag = [](int lo_, int hi_, int w, int tiles) {
+            const int hops = (hi_ - 1) / w - (lo_ - 1) / w, far = (hi_ - 1) / (w * tiles) - (lo_ - 1) / (w * tiles);
+            return 8 * (hops - far) + 24 * far;
+        };
+        const int cost0 = lag(jlo, jhi, SWEEP_WA, SWEEP_CA) + lag(klo, khi, SWEEP_WB, SWEEP_CB);
+        const int cost1 = lag(klo, khi, SWEEP_WA, SWEEP_CA) + lag(jlo, jhi, SWEEP_WB, SWEEP_CB);
         int want = cost1 < cost0 ? 1 : (cost0 < cost1 ? 0 : pb.sl.swap);
         if (a.sweepOrientation == 0 || a.sweepOrientation == 1) want = a.sweepOrientation;
         if (want != pb.sl.swap) {

@@ -9,56 +9,60 @@
 // (upper) neighbours only, so the cells of a plane i + j + k = const are
 // independent: the exact wavefront order.
 //
-// Mapping.  A CTA owns a tile of 32 (j) x 8 (k) pencils along i: lane l
-// of the tile holds the 8 pencils (l, w) of its column, the tile's "slots"
-// w = 0..7, and four compute warps take two slots each.  In the forward
-// sweep slot w of lane l processes i = 1 + t - l - w at step t, so a cell's
-// three lower neighbours (i-1 in the same slot, j-1 in lane l-1, k-1 in
-// slot w-1) were all formed at step t - 1: the j terms arrive by warp
-// shuffle, the i terms and the k terms between a warp's own slots stay in
-// registers, and the k term that crosses to the next warp goes through
-// shared memory around the one barrier per step of the compute warps (the
-// backward sweep is the mirror image).  A full chunk of steps runs as
-// straight-line code, with no test or vote between its steps.  In the
+// What bounds it: the dependency chain.  A sweep cannot take fewer steps than
+// the system's extent i + j + k; everything above that is time per step and
+// the delay with which one tile's edge terms reach the next.
+//
+// Mapping.  A tile is 16 (a) x 8 (b) pencils along i, worked by four warps of
+// 8 x 4 pencils, a pencil per lane.  In the forward sweep pencil (A, B) meets
+// cell i = 1 + t - A - B at step t, so a cell's three lower neighbours were
+// all formed at step t - 1: in the lane itself, or in the lane before it along
+// a or b (two shuffles a step).  The warps of a tile share the step numbers
+// and run on four schedulers without a barrier; each waits only for the terms
+// of its own edge pencils.  A step is bound by the latencies of one warp's
+// instructions (about 75 cycles, plus 60 for the group's and the chunk's
+// waits); bundles of 2 x 2 pencils per lane, one warp a tile, took 205 cycles
+// a step and saved fewer hops than that costs.  128 pencils
+// per CTA rather than more: a step reads 20 and writes 4 bytes per pencil, and
+// 3 KB a step is what one SM can draw from L2 in the time of a step.  In the
 // forward sweep a cell hands its neighbours the finished products L_c * y_c
 // rather than y_c: each product is rounded once, by whichever thread forms
 // it, so the bits are the reference's.
 //
+// Edges.  Every term that crosses to another warp has a word of its own in
+// the consumer's shared memory for the whole sweep (so no credit flows back),
+// laid out so that one 16-byte load takes a pencil's terms of EC = 4 steps.
+// The words start as a bit pattern that no product can have (a NaN payload;
+// FP32 products give the canonical NaN only), and the consumer looks at its
+// words until the pattern is gone.  Eight tiles (2 x 4: 32 x 32 pencils) form
+// a thread-block cluster, in which the edge lanes store straight into the
+// consumer's shared memory: a hop costs the group of steps and a few hundred
+// cycles.  Between clusters a term travels as one 64-bit word {sweep epoch,
+// value} in global memory, indexed by step; the consumer's four edge warps
+// poll the words of their groups of steps until the epoch is the current
+// sweep's.  Naturally aligned words are seen whole or not at all, so no fence
+// or flag sits between producer and consumer.
+//
 // Data movement.  The factor rows and the right-hand side live in the
 // step-major sweep layout (flip_device.cuh), so the 8 steps of a chunk of a
-// tile are one contiguous block in either direction.  A loader warp moves
-// whole chunks with bulk asynchronous copies into a ring of five
-// shared-memory slots as soon as a slot is free (an mbarrier per slot counts
-// the bytes in) and prefetches the chunk one ring further ahead into L2; an
-// edge warp fetches the terms that the neighbouring tiles publish for the
-// chunk's edge cells.  The two run independently, so a tile waiting for its
-// neighbours still has its operands on the way.  The compute warps read
-// the next step's operands from the slot while they compute the current
-// one and store each result straight to global memory (128 contiguous bytes
-// per slot and step); cells outside the grid read zero rows, so a step is
-// unpredicated.
+// tile are one contiguous block in either direction.  A loader thread moves
+// whole chunks with bulk asynchronous copies into a ring of shared-memory
+// slots, and prefetches the chunk one ring further ahead into L2.  Cells
+// outside the grid or the system have zero rows, so a step is unpredicated.
 //
-// Where a step's time goes (one warp, measured): the arithmetic and
-// shuffles of 8 slots take about 80 cycles, of 2 slots about 46; operands
-// from shared memory, result stores and a test or vote per step (which
-// splits the unrolled chunk into separate blocks) add 100-250 cycles at 8
-// slots.  Four warps of two slots each, in lockstep, with full chunks free
-// of tests, sweep the 128^3 dam region in 53 us per launch and a fully
-// liquid 128^3 box in 95 us (eight warps of one slot with tests per step:
-// 64 us and 95 us; the same in lockstep without tests: 55 us and 82 us).
+// Clusters take tickets in dependency order, so a tile only waits for tiles
+// that are already running (a cluster's own CTAs run together).  Every wait
+// is bounded: on timeout the tile raises the error flag and stops, and the
+// host reports FLIP_E_DEVICE_TIMEOUT; no wait can spin forever.  A CTA that
+// gives up stays until the other CTAs of its cluster are done, since they may
+// still store into its shared memory.
 //
-// Tile edges.  The threads on a tile's downstream edges publish each term
-// they form as one 64-bit word {sweep epoch, value}, indexed by step, in an
-// exchange array; the neighbour's edge warp polls exactly the words its
-// chunk needs until their epoch is the current sweep's.  A single naturally
-// aligned 64-bit store is seen whole or not at all, so no fence, flag or
-// progress counter sits between the producing step and the consuming one.
-// Cells that the producing tile does not compute contribute zero and are not
-// polled.  Tiles take tickets in dependency order, so a tile only waits for
-// tiles that are already running.  Every wait is bounded: on timeout the
-// tile raises the error flag and stops, and the host reports
-// FLIP_E_DEVICE_TIMEOUT; no wait can spin forever.
+// Measured per launch (events around a pair, one box): 128^3 dam break (518k
+// rows) 41.8 us, 64^3 19.6 us, 256 x 128 x 128 tank (1.8M rows) 56.6 us; the
+// form before it (tiles of 32 x 8 pencils, four warps in lockstep with a
+// barrier a step, every edge through L2) took 50.5, 23.0 and 71.3 us.
 #include <atomic>
+#include <type_traits>
 
 #include "flip_device.cuh"
 
@@ -66,28 +70,27 @@ namespace flip {
 
 namespace {
 
-#ifndef SWEEP_CH
-#define SWEEP_CH 8   // steps per chunk
-#endif
-constexpr int TJ = SWEEP_TJ, TK = SWEEP_TK, NP = SWEEP_NP, CH = SWEEP_CH, SL = SWEEP_SL, SW = SWEEP_SW;
-// one compute warp holds a tile's TK pencils of each lane in registers: a
-// cell's three lower neighbours are then all one step back
-static_assert(SL == 1 && SW == 1 && CH >= 1, "the compute warp expects skews of one step");
+constexpr int WA = SWEEP_WA, WB = SWEEP_WB, NP = SWEEP_NP, CH = SWEEP_CH;
+constexpr int VA = SWEEP_VA, VB = SWEEP_VB;                 // pencils of a warp along a and b
+constexpr int NWA = WA / VA, NWB = WB / VB, NWC = NWA * NWB;   // compute warps of a tile
+static_assert(VA == 8 && VB == 4 && NWA == 2 && NWB == 2 && CH == 8, "lane and warp mapping");
+constexpr int CA = SWEEP_CA, CB = SWEEP_CB, CL = CA * CB;   // tiles of a cluster along a and b
+constexpr int EC = 4;        // steps per group of edge words
 #ifndef SWEEP_NBUF
-#define SWEEP_NBUF 5   // ring slots that fit in shared memory
+#define SWEEP_NBUF 4   // operand slots in shared memory, 8 steps each
 #endif
 constexpr int NBUF = SWEEP_NBUF;
 static_assert(NBUF >= 2, "the ring needs a slot in flight beside the one in use");
-// the edge warp's lanes take the CH x TK j-edge words JQ at a time and the
-// CH x TJ k-edge words one step each
-constexpr int JQ = CH * TK / 32;
-static_assert((CH * TK) % 32 == 0 && TJ == 32 && JQ <= 32, "edge-word mapping of the edge warp");
-#ifndef SWEEP_SPW
-#define SWEEP_SPW 2   // slots (pencils along the warp axis) per compute warp
-#endif
-constexpr int SPW = SWEEP_SPW, NWC = TK / SPW;   // compute warps per tile
-static_assert(TK % SPW == 0, "a compute warp holds whole slots");
-constexpr int NCOMP = 32 * NWC, LOADER = NWC, EDGE = LOADER + 1, NTHREADS = NCOMP + 64;
+constexpr int NHELP = 4;     // edge warps: groups of steps polled at the same time
+constexpr int LOADER = NWC, EDGE = LOADER + 1, NTHREADS = 32 * (EDGE + NHELP);
+// The edge words of every step fit beside the operand slots up to this many
+// steps; longer grids (I above about 700) keep a ring of RC chunks of them
+// instead, and take every term of another tile from global memory.  A warp is
+// less than NBUF chunks ahead of the slowest warp of its tile (the operand
+// slots) and hands on terms of at most one chunk further.
+constexpr int WHOLE_STEPS = 720, RC = NBUF + 2;
+constexpr int GW = (VA + VB) * EC;   // edge words of a warp per group: VB a-edge pencils, then VA b-edge pencils
+constexpr unsigned ABSENT = 0xffffffffu;   // a word that has not come (the largest unsigned value)
 // Waiting for this CTA's own bulk copies in flight (they complete by
 // themselves) keeps the default limit, whatever limit the edge waits have.
 constexpr unsigned int DRAIN_SPIN_LIMIT = DEFAULT_SPIN_LIMIT;
@@ -96,11 +99,12 @@ struct SweepArgs {
     const float4 *L;               // factor rows, sweep layout
     const float *rin;              // right-hand side, sweep layout (backward: the forward result)
     float *out;                    // result, sweep layout (backward: in place over the forward result)
-    int J, K, NI, T;               // J, K: grid extents along the tile's lane and slot axes
-    int ntj, ntk;
+    int T;                         // steps per tile, a multiple of CH
+    int nta, ntb, nca;             // tiles along a and b, clusters along a
+    int nClusters;
     const int2 *range;             // per tile: first/last step (forward numbering) holding a system cell
-    unsigned long long *xchg;      // per tile: T x TK j-edge words, then T x TJ k-edge words
-    unsigned int *ticket;          // [0] forward tile tickets, [1] the pair's epoch, [2] backward tile tickets
+    unsigned long long *xchg;      // per tile: T x WB a-edge words, then T x WA b-edge words
+    unsigned int *ticket;          // [0] forward cluster tickets, [1] the pair's epoch, [2] backward cluster tickets
                                    // (set by sweep_prep before each pair)
     int *err;
     const int *skip;   // nonzero: return at once
@@ -111,22 +115,22 @@ struct SweepArgs {
 struct Slot {
     float4 L[CH][NP];   // rows in layout order: forward row q = step q, backward row q = step CH-1-q
     float r[CH][NP];
-    float eJ[CH][TK];   // by step: term from the neighbour tile along the lanes, for the edge lane of each slot
-    float eK[CH][TJ];   // by step: term from the neighbour tile along the slots, for each lane of the edge slot
 };
 struct SweepSmem {
     Slot slot[NBUF];
-    // per slot: operand bytes in (the loader), edge terms in (the edge warp),
-    // chunk done (the compute warps)
-    unsigned long long loaded[NBUF], edges[NBUF], done[NBUF];
-    // between compute warps g and g + 1, by step parity and lane: forward
-    // warp g's last slot's L_z y, backward warp g + 1's first slot's z
-    float hand[2][NWC > 1 ? NWC - 1 : 1][TJ];
+    unsigned long long loaded[NBUF], done[NBUF];   // per slot: operand bytes in; chunk done
     int abort;
-    int tile;
+    int cluster;
     unsigned int epoch;
+    int pad;
+    float unused[NWC][32 + 2 * GW];   // where lanes and steps without a taker store their terms
 };
-static_assert(sizeof(SweepSmem) <= 227 * 1024, "the sweep's shared memory fits one CTA");
+// after it: per warp, the edge words that come in, [group][pencil][step of the group]
+__host__ __device__ constexpr size_t sweep_smem_bytes(int edgeSteps) {
+    return sizeof(SweepSmem) + ((size_t)NWC * (edgeSteps / EC) + CH / EC) * GW * 4;   // a chunk more may be read
+}
+static_assert(sweep_smem_bytes(WHOLE_STEPS) <= 227 * 1024, "the sweep's shared memory fits one CTA");
+static_assert(sizeof(SweepSmem) % 16 == 0 && WHOLE_STEPS % CH == 0, "alignment of the edge words");
 
 __device__ __forceinline__ unsigned smem_addr(const void *p) { return (unsigned)__cvta_generic_to_shared(p); }
 __device__ __forceinline__ unsigned long long ld_word(const unsigned long long *p) {
@@ -134,153 +138,386 @@ __device__ __forceinline__ unsigned long long ld_word(const unsigned long long *
     asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
     return v;
 }
-__device__ __forceinline__ unsigned long long pack(unsigned int epoch, float v) {
-    return ((unsigned long long)epoch << 32) | __float_as_uint(v);
+__device__ __forceinline__ void mb_init(unsigned b, unsigned count) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(b), "r"(count) : "memory");
 }
-__device__ __forceinline__ void mb_init(unsigned long long *b, unsigned count) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_addr(b)), "r"(count) : "memory");
+__device__ __forceinline__ void mb_arrive_relaxed(unsigned on, unsigned b) {
+    asm volatile("{\n .reg .b64 st;\n .reg .pred q;\n setp.ne.u32 q, %1, 0;\n"
+                 " @q mbarrier.arrive.relaxed.cta.shared::cta.b64 st, [%0];\n}" ::"r"(b), "r"(on) : "memory");
 }
-__device__ __forceinline__ void mb_arrive(unsigned long long *b) {
-    asm volatile("{\n .reg .b64 st;\n mbarrier.arrive.shared::cta.b64 st, [%0];\n}" ::"r"(smem_addr(b)) : "memory");
+__device__ __forceinline__ void mb_arrive_expect_tx(unsigned b, unsigned bytes) {
+    asm volatile("{\n .reg .b64 st;\n mbarrier.arrive.expect_tx.relaxed.cta.shared::cta.b64 st, [%0], %1;\n}" ::"r"(b), "r"(bytes)
+                 : "memory");
 }
-__device__ __forceinline__ void mb_arrive_expect_tx(unsigned long long *b, unsigned bytes) {
-    asm volatile("{\n .reg .b64 st;\n mbarrier.arrive.expect_tx.shared::cta.b64 st, [%0], %1;\n}" ::"r"(smem_addr(b)),
-                 "r"(bytes) : "memory");
-}
-__device__ __forceinline__ bool mb_test(unsigned long long *b, unsigned parity) {
+__device__ __forceinline__ bool mb_test(unsigned b, unsigned parity) {
     unsigned ok;
     asm volatile("{\n .reg .pred p;\n mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}"
-                 : "=r"(ok) : "r"(smem_addr(b)), "r"(parity) : "memory");
+                 : "=r"(ok) : "r"(b), "r"(parity) : "memory");
     return ok != 0;
+}
+// A look ahead: the same without ordering anything.
+__device__ __forceinline__ unsigned mb_peek(unsigned b, unsigned parity) {
+    unsigned ok;
+    asm volatile("{\n .reg .pred p;\n mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}"
+                 : "=r"(ok) : "r"(b), "r"(parity));
+    return ok;
 }
 // One round of waiting for a phase: the thread is suspended until the phase
 // completes or about `ns` nanoseconds pass, so waiting warps take no issue
 // slots from the warps that compute on the same scheduler.
-__device__ __forceinline__ bool mb_try(unsigned long long *b, unsigned parity, unsigned ns) {
+__device__ __forceinline__ bool mb_try(unsigned b, unsigned parity, unsigned ns) {
     unsigned ok;
-    asm volatile("{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n selp.u32 %0, 1, 0, p;\n}"
-                 : "=r"(ok) : "r"(smem_addr(b)), "r"(parity), "r"(ns) : "memory");
+    asm volatile("{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n"
+                 " selp.u32 %0, 1, 0, p;\n}"
+                 : "=r"(ok) : "r"(b), "r"(parity), "r"(ns) : "memory");
     return ok != 0;
 }
 // Bounded wait for a phase of an mbarrier; false on abort or timeout (which
 // raises the abort and error flags).
-__device__ bool mb_wait(unsigned long long *b, unsigned parity, int *abortFlag, int *err, unsigned int limit) {
+__device__ __noinline__ bool mb_wait_slow(unsigned b, unsigned parity, int *abortFlag, int *err, unsigned int limit) {
     for (unsigned int spin = 0; spin < limit; spin++) {
         if (mb_try(b, parity, 256)) return true;
         if (*(volatile int *)abortFlag) return false;
+        if ((spin & 255u) == 255u && *(volatile int *)err) return false;   // another tile gave up
     }
     *(volatile int *)abortFlag = 1;
     atomicExch(err, 1);
     return false;
 }
+__device__ __forceinline__ bool mb_wait(unsigned b, unsigned parity, int *abortFlag, int *err, unsigned int limit) {
+    return mb_try(b, parity, 256) || mb_wait_slow(b, parity, abortFlag, err, limit);
+}
+// The same for a whole warp, which goes on or stops together.
+__device__ __forceinline__ bool warp_wait(unsigned b, unsigned parity, int *abortFlag, int *err, unsigned int limit) {
+    if (__all_sync(0xffffffffu, mb_try(b, parity, 256))) return true;
+    return __all_sync(0xffffffffu, mb_wait_slow(b, parity, abortFlag, err, limit));
+}
+// After `spin` looks at edge words that have not come: does the warp stop?
+// Looks are about a shared-memory round trip apart, then a suspension; the
+// limit counts the suspended ones, as mb_wait does.
+__device__ __noinline__ bool edge_gives_up(unsigned spin, int *abortFlag, int *err, unsigned int limit) {
+    if (spin < 64) return false;
+    __nanosleep(spin < 1024 ? 32 : 256);
+    const bool stop = *(volatile int *)abortFlag || ((spin & 255u) == 255u && *(volatile int *)err);
+    if (!__any_sync(0xffffffffu, stop || spin - 64 >= limit)) return false;
+    if (!__any_sync(0xffffffffu, stop)) atomicExch(err, 1);
+    return true;
+}
 // bulk copy global -> shared, completion counted in bytes on mbarrier b
-__device__ __forceinline__ void bulk_load(void *dst, const void *src, unsigned bytes, unsigned long long *b) {
+__device__ __forceinline__ void bulk_load(void *dst, const void *src, unsigned bytes, unsigned b) {
     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-                 ::"r"(smem_addr(dst)), "l"(src), "r"(bytes), "r"(smem_addr(b)) : "memory");
+                 ::"r"(smem_addr(dst)), "l"(src), "r"(bytes), "r"(b) : "memory");
 }
 __device__ __forceinline__ void prefetch_l2(const void *src, unsigned bytes) {
     asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(src), "r"(bytes) : "memory");
 }
-// named barrier of the compute warps, plain and with an OR vote
-__device__ __forceinline__ bool compute_sync_or(bool v) {
+__device__ __forceinline__ unsigned cluster_rank() {
     unsigned r;
-    asm volatile("{\n .reg .pred pi, po;\n setp.ne.u32 pi, %1, 0;\n bar.red.or.pred po, 1, %2, pi;\n selp.u32 %0, 1, 0, po;\n}"
-                 : "=r"(r) : "r"((unsigned)v), "n"(NCOMP) : "memory");
-    return r != 0;
+    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    return r;
 }
-__device__ __forceinline__ void compute_sync() { asm volatile("bar.sync 1, %0;" ::"n"(NCOMP) : "memory"); }
-// A published edge term, stored where `on` holds: a predicated store, not a
-// branch around one (only the tile's edge lanes publish), ordered against
-// nothing else (a consumer reads the word alone), so the compiler may move
-// the loads of later steps above it.
-__device__ __forceinline__ void st_term(bool on, unsigned long long *p, unsigned long long v) {
+__device__ __forceinline__ void cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\n barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ unsigned map_rank(unsigned addr, unsigned rank) {
+    unsigned r;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
+    return r;
+}
+__device__ __forceinline__ int ld_cluster(unsigned addr) {
+    int v;
+    asm volatile("ld.shared::cluster.s32 %0, [%1];" : "=r"(v) : "r"(addr) : "memory");
+    return v;
+}
+// An edge term stored into a CTA's shared memory (this one's or another of its
+// cluster); and, where `on` holds, as a word of the exchange array.  Ordered
+// against nothing else (the reader looks at the word itself), so the compiler
+// may move the loads of later steps above them.
+template <int OFF>
+__device__ __forceinline__ void hand_on(unsigned addr, float v) {
+    asm volatile("st.relaxed.cluster.shared::cluster.f32 [%0 + %2], %1;" ::"r"(addr), "f"(v), "n"(OFF));
+}
+__device__ __forceinline__ void publish(unsigned on, unsigned long long *p, unsigned epoch, float v) {
     asm volatile("{\n .reg .pred q;\n setp.ne.u32 q, %2, 0;\n @q st.relaxed.gpu.global.u64 [%0], %1;\n}"
-                 ::"l"(p), "l"(v), "r"((unsigned)on));
+                 ::"l"(p), "l"(((unsigned long long)epoch << 32) | __float_as_uint(v)), "r"(on));
 }
-// The j-edge terms of a lane's SPW slots at one step: consecutive words.
-template <int N>
-__device__ __forceinline__ void st_terms(bool on, unsigned long long *p, const float (&v)[N], unsigned int epoch) {
-#pragma unroll
-    for (int j = 0; j < N; j++) st_term(on, p + j, ((unsigned long long)epoch << 32) | __float_as_uint(v[j]));
+// A pencil's edge words of a group.
+__device__ __forceinline__ uint4 ld_edge(unsigned addr) {
+    uint4 v;
+    asm volatile("ld.volatile.shared::cta.v4.u32 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr));
+    return v;
+}
+__device__ __forceinline__ void clear_edge(unsigned addr) {
+    asm volatile("st.volatile.shared::cta.v4.u32 [%0], {%1, %1, %1, %1};" ::"r"(addr), "r"(ABSENT) : "memory");
+}
+__device__ __forceinline__ bool any_absent(uint4 a, uint4 b) {
+    return max(max(max(a.x, a.y), max(a.z, a.w)), max(max(b.x, b.y), max(b.z, b.w))) == ABSENT;
 }
 
-// SWAP: the tile's lanes run along k and its warps along j (else lanes along
-// j, warps along k).  The couplings that travel along each axis and the
-// order of the subtractions follow: forward -z, -y, -x; backward +x, +y, +z.
-template <bool FWD, bool SWAP>
-__global__ void __launch_bounds__(NTHREADS, 1) k_wavefront(SweepArgs a) {
+// What a compute warp works with (see k_wavefront).
+struct WarpJob {
+    SweepSmem *sm;
+    int *err;
+    unsigned spinLimit;
+    int c0, nChunks, lane;
+    const float4 *L;              // this lane's operands in slot 0, row 0
+    const float *r;
+    float *out;                   // result of this lane at the tile's step 0
+    int lastStep;                 // T - 1
+    bool inEdgeA, inEdgeB;
+    unsigned inA, inB;            // this lane's edge words (of chunk 0)
+    unsigned dstA, dstB;          // where it hands terms on: the consumer's words, moved to this warp's chunk 0
+    unsigned unused;              // and where to at other steps
+    // {first, count} of the chunks whose steps 0-6, and whose step 7, hand a term on
+    int2 kA, kA7, kB, kB7;
+    unsigned long long *xA, *xB;  // as words of the exchange array,
+    int2 pA, pA7, pB, pB7;        // in these
+    unsigned epoch;
+};
+
+// The steps of one warp.  PUB: it also publishes words for another cluster.
+template <bool FWD, bool SWAP, bool WHOLE, bool PUB>
+__device__ __forceinline__ bool run_steps(const WarpJob &w) {
+    constexpr unsigned CHB = (CH / EC) * GW * 4;   // edge bytes of a chunk
+    // forward: the products of the last cell, for the next one along i, a and
+    // b; backward: its z, which all three take
+    float tx = 0.0f, sA = 0.0f, sB = 0.0f;
+    // the edge words of the next group, read ahead
+    uint4 na = ld_edge(w.inA + (WHOLE ? w.c0 * CHB : 0)), nb = ld_edge(w.inB + (WHOLE ? w.c0 * CHB : 0));
+    unsigned ready = 0;   // the next chunk's operands were seen to be in
+    float *out = w.out + (ptrdiff_t)(FWD ? w.c0 * CH : w.lastStep - w.c0 * CH) * NP;
+    unsigned long long *xA = w.xA + (size_t)w.c0 * CH * WB, *xB = w.xB + (size_t)w.c0 * CH * WA;
+    unsigned cw = WHOLE ? w.c0 * CHB : 0;   // the chunk's edge words
+#pragma unroll 1
+    for (int n = 0; n < w.nChunks; n++) {
+        const int b = n % NBUF, c = w.c0 + n;
+        if (!__all_sync(0xffffffffu, ready) &&
+            !warp_wait(smem_addr(&w.sm->loaded[b]), (n / NBUF) & 1, &w.sm->abort, w.err, w.spinLimit))
+            return false;
+        asm volatile("" ::: "memory");
+        const float4 *L = reinterpret_cast<const float4 *>(reinterpret_cast<const char *>(w.L) + (size_t)b * sizeof(Slot));
+        const float *r = reinterpret_cast<const float *>(reinterpret_cast<const char *>(w.r) + (size_t)b * sizeof(Slot));
+        // a step's terms are taken one step later: step 7's fall into the next chunk
+        const unsigned cw1 = WHOLE ? cw + CHB : ((n + 1) % RC) * CHB;
+        // Chunks in which steps 0-6, and in which step 7, hand a term on (the
+        // windows start at step 0 or 7 of a chunk and end at its step 6 or 7:
+        // ranges are whole chunks, terms move by -1, 7 or 15).
+        auto in = [&](int2 k) { return (unsigned)(c - k.x) < (unsigned)k.y; };
+        const unsigned dA = in(w.kA) ? w.dstA + cw : w.unused, dA7 = in(w.kA7) ? w.dstA + cw1 : w.unused;
+        const unsigned dB = in(w.kB) ? w.dstB + cw : w.unused, dB7 = in(w.kB7) ? w.dstB + cw1 : w.unused;
+        const unsigned puA = PUB ? in(w.pA) : 0, puA7 = PUB ? in(w.pA7) : 0;
+        const unsigned puB = PUB ? in(w.pB) : 0, puB7 = PUB ? in(w.pB7) : 0;
+        // operands of the next step, loaded while the current one computes
+        float4 Ln = L[(FWD ? 0 : CH - 1) * NP];
+        float rn = r[(FWD ? 0 : CH - 1) * NP];
+        float xa[EC], xb[EC];
+        bool fine = true;
+        // the group's edge words, read ahead or awaited
+        auto take_edges = [&](unsigned off) {
+            while (__any_sync(0xffffffffu, any_absent(na, nb))) {
+                for (unsigned spin = 0;;) {
+                    na = ld_edge(w.inA + off);
+                    nb = ld_edge(w.inB + off);
+                    if (!__any_sync(0xffffffffu, any_absent(na, nb))) break;
+                    if (edge_gives_up(++spin, &w.sm->abort, w.err, w.spinLimit)) { fine = false; return; }
+                }
+            }
+            if (!WHOLE) {   // the ring's words are free again once all warps are done with the chunk
+                __syncwarp();
+                if (w.inEdgeA) clear_edge(w.inA + off);
+                if (w.inEdgeB) clear_edge(w.inB + off);
+            }
+            xa[0] = __uint_as_float(na.x); xa[1] = __uint_as_float(na.y); xa[2] = __uint_as_float(na.z); xa[3] = __uint_as_float(na.w);
+            xb[0] = __uint_as_float(nb.x); xb[1] = __uint_as_float(nb.y); xb[2] = __uint_as_float(nb.z); xb[3] = __uint_as_float(nb.w);
+        };
+        auto step = [&](auto U) {
+            constexpr int u = decltype(U)::value, s = u % EC;
+            const float4 Lc = Ln;
+            const float rr = rn;
+            if (u + 1 < CH) {
+                constexpr int q = FWD ? u + 1 : CH - 2 - u;
+                Ln = L[q * NP];
+                rn = r[q * NP];
+            }
+            float vA = FWD ? __shfl_up_sync(0xffffffffu, sA, 1) : __shfl_down_sync(0xffffffffu, sA, 1);
+            float vB = FWD ? __shfl_up_sync(0xffffffffu, sB, VA) : __shfl_down_sync(0xffffffffu, sB, VA);
+            if (w.inEdgeA) vA = xa[s];
+            if (w.inEdgeB) vB = xb[s];
+            float acc, res;
+            if (FWD) {
+                acc = __fsub_rn(rr, SWAP ? vA : vB);    // -z
+                acc = __fsub_rn(acc, SWAP ? vB : vA);   // -y
+                acc = __fsub_rn(acc, tx);               // -x
+                res = __fmul_rn(acc, Lc.x);
+                tx = __fmul_rn(Lc.y, res);
+                sA = __fmul_rn(SWAP ? Lc.w : Lc.z, res);
+                sB = __fmul_rn(SWAP ? Lc.z : Lc.w, res);
+            } else {
+                acc = __fsub_rn(rr, __fmul_rn(Lc.y, tx));                // +x
+                acc = __fsub_rn(acc, __fmul_rn(Lc.z, SWAP ? vB : vA));   // +y
+                acc = __fsub_rn(acc, __fmul_rn(Lc.w, SWAP ? vA : vB));   // +z
+                res = __fmul_rn(acc, Lc.x);
+                tx = sA = sB = res;
+            }
+            __stcg(out + (FWD ? u : -u) * NP, res);
+            constexpr int off = ((u + 1) / EC % (CH / EC)) * GW * 4 + (u + 1) % EC * 4;
+            hand_on<off>(u < 7 ? dA : dA7, sA);
+            hand_on<off>(u < 7 ? dB : dB7, sB);
+            if (PUB) {
+                publish(u < 7 ? puA : puA7, xA + u * WB, w.epoch, sA);
+                publish(u < 7 ? puB : puB7, xB + u * WA, w.epoch, sB);
+            }
+        };
+        using std::integral_constant;
+        take_edges(cw);
+        if (!fine) return false;
+        step(integral_constant<int, 0>{});
+        step(integral_constant<int, 1>{});
+        step(integral_constant<int, 2>{});
+        na = ld_edge(w.inA + cw + GW * 4);
+        nb = ld_edge(w.inB + cw + GW * 4);
+        step(integral_constant<int, 3>{});
+        take_edges(cw + GW * 4);
+        if (!fine) return false;
+        step(integral_constant<int, 4>{});
+        step(integral_constant<int, 5>{});
+        step(integral_constant<int, 6>{});
+        na = ld_edge(w.inA + cw1);   // past the last chunk: a place that is not used
+        nb = ld_edge(w.inB + cw1);
+        ready = mb_peek(smem_addr(&w.sm->loaded[(n + 1) % NBUF]), ((n + 1) / NBUF) & 1);
+        step(integral_constant<int, 7>{});
+        out += (FWD ? CH : -CH) * NP;
+        cw = cw1;
+        if (PUB) { xA += CH * WB; xB += CH * WA; }
+        // The slot may be refilled: every value read from it has been used.  A
+        // relaxed arrival, since a releasing one waits for the results' stores
+        // to reach L2.
+        __syncwarp();
+        mb_arrive_relaxed(w.lane == 0, smem_addr(&w.sm->done[b]));
+    }
+    return true;
+}
+
+// SWAP: the tiles' a axis is k and b is j (else a = j, b = k).  The couplings
+// that travel along each axis and the order of the subtractions follow:
+// forward -z, -y, -x; backward +x, +y, +z.  WHOLE: every step's edge words have
+// their own place (and terms inside a cluster are stored there); else a ring.
+template <bool FWD, bool SWAP, bool WHOLE>
+__global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(NTHREADS) k_wavefront(SweepArgs a) {
     extern __shared__ __align__(128) unsigned char smemRaw[];
     SweepSmem &sm = *reinterpret_cast<SweepSmem *>(smemRaw);
-    const int ntiles = a.ntj * a.ntk;
+    if (*(volatile const int *)a.skip) return;   // converged: nothing to do (all CTAs see the same)
+    const int T = a.T;
+    const int edgeGroups = (WHOLE ? T : RC * CH) / EC;   // groups of edge words per warp
+    float *edge = reinterpret_cast<float *>(smemRaw + sizeof(SweepSmem));   // [warp][group][GW]
+    const unsigned rank = cluster_rank();
     if (threadIdx.x == 0) {
-        if (*(volatile const int *)a.skip || *(volatile int *)a.err) {
-            sm.tile = -1;   // converged, or an earlier sweep gave up: nothing to do
-        } else {
-            int t = (int)atomicAdd(&a.ticket[FWD ? 0 : 2], 1u);
-            sm.tile = FWD ? t : ntiles - 1 - t;
-        }
+        if (rank == 0)
+            sm.cluster = *(volatile int *)a.err ? -1 : (int)atomicAdd(&a.ticket[FWD ? 0 : 2], 1u);
         sm.abort = 0;
         sm.epoch = *(volatile unsigned int *)&a.ticket[1] + (FWD ? 0u : 1u);   // forward e, backward e + 1
         for (int b = 0; b < NBUF; b++) {
-            mb_init(&sm.loaded[b], 1);      // the loader's arrival, plus the bytes of the chunk
-            mb_init(&sm.edges[b], 32);      // the edge warp's lanes
-            mb_init(&sm.done[b], NCOMP);
+            mb_init(smem_addr(&sm.loaded[b]), 1);   // the loader's arrival, plus the bytes of the chunk
+            mb_init(smem_addr(&sm.done[b]), NWC);
         }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    __syncthreads();
-    const int tile = sm.tile;
-    if (tile < 0 || tile >= ntiles) return;
-    const int tj = tile % a.ntj, tk = tile / a.ntj;
-    const int NI = a.NI, T = a.T;
-    auto steps_of = [&](int tl) {   // [first, last] step of a tile in this sweep's numbering
+    cluster_sync();
+    const int ticket = ld_cluster(map_rank(smem_addr(&sm.cluster), 0));
+    // The cluster and the tile of this CTA; clusters in dependency order.
+    const bool live = ticket >= 0 && ticket < a.nClusters;
+    const int cl = FWD ? ticket : a.nClusters - 1 - ticket;
+    const int ta = live ? (cl % a.nca) * CA + (int)rank % CA : a.nta, tb = live ? (cl / a.nca) * CB + (int)rank / CA : 0;
+    const bool exists = live && ta < a.nta && tb < a.ntb;
+    const int tile = ta + a.nta * tb;
+    // First and last step of a tile in this sweep's numbering, out to whole
+    // chunks (the steps added hold zero rows); hi < lo where it holds no cell.
+    auto steps_of = [&](int tl) {
         const int2 rg = a.range[tl];
-        return FWD ? rg : make_int2((T - 1) - rg.y, (T - 1) - rg.x);
+        if (rg.y < rg.x) return make_int2(T, -1);
+        const int lo = rg.x & ~(CH - 1), hi = rg.y | (CH - 1);
+        return FWD ? make_int2(lo, hi) : make_int2((T - 1) - hi, (T - 1) - lo);
     };
-    const int2 own = steps_of(tile);
-    const int tlo = own.x, thi = own.y;
-    if (thi < tlo) return;   // no system cell in the tile: nothing to compute or publish
-    const int nChunks = (thi - tlo) / CH + 1;
-    const int j0 = 1 + tj * TJ, k0 = 1 + tk * TK;
-    auto pencil_in = [&](int lr, int ww) { return j0 + lr <= a.J - 2 && k0 + ww <= a.K - 2; };
-    const size_t wordsPerTile = (size_t)T * (TJ + TK);
-    const unsigned int ep = sm.epoch;          // published with this sweep's terms
-    const unsigned int epWait = ep + a.epochSkew;   // awaited in the neighbours' words
-    // the chunk of steps [tb, tb + rows) as one block of the layout
-    auto chunk_rows = [&](int n) { return min(CH, thi + 1 - (tlo + n * CH)); };
-    auto chunk_row0 = [&](int rows) { return FWD ? 0 : CH - rows; };
-    auto chunk_tf0 = [&](int tb, int rows) { return FWD ? tb : T - tb - rows; };
+    // The tiles this one takes terms from (up) and hands terms to (down), by
+    // axis, and whether they are in the same cluster.  Consumer step te takes
+    // the a-edge term of the producer's step te + WA - 1 and the b-edge term
+    // of te + WB - 1, in the tiles' own step numbers; between warps of a tile
+    // it takes the term of step te - 1.
+    const int dir = FWD ? 1 : -1;
+    const int2 none = make_int2(T, -1);
+    const bool mute = a.epochSkew != 0;   // fault injection: nothing is handed on
+    auto range_at = [&](bool in, int tl) { return exists && in ? steps_of(tl) : none; };
+    const int2 own = range_at(true, tile);
+    const int2 rUA = range_at(ta - dir >= 0 && ta - dir < a.nta, tile - dir);
+    const int2 rUB = range_at(tb - dir >= 0 && tb - dir < a.ntb, tile - dir * a.nta);
+    const int2 rDA = range_at(ta + dir >= 0 && ta + dir < a.nta && !mute, tile + dir);
+    const int2 rDB = range_at(tb + dir >= 0 && tb + dir < a.ntb && !mute, tile + dir * a.nta);
+    const int lo = own.x, hi = own.y;
+    const bool work = hi >= lo;
+    const bool upAcl = WHOLE && (ta - dir) / CA == ta / CA && ta - dir >= 0;
+    const bool upBcl = WHOLE && (tb - dir) / CB == tb / CB && tb - dir >= 0;
+    const bool dnAcl = WHOLE && (ta + dir) / CA == ta / CA && ta + dir >= 0;
+    const bool dnBcl = WHOLE && (tb + dir) / CB == tb / CB && tb + dir >= 0;
+    // consumer steps that receive a term of another tile, along each axis
+    const int iA0 = max(lo, rUA.x - (WA - 1)), iA1 = min(hi, rUA.y - (WA - 1));
+    const int iB0 = max(lo, rUB.x - (WB - 1)), iB1 = min(hi, rUB.y - (WB - 1));
+    const bool pollA = iA1 >= iA0 && !upAcl, pollB = iB1 >= iB0 && !upBcl;
+    const bool helpers = work && (!WHOLE || pollA || pollB);
+    // the first warp along an axis (0 forward) takes the other tiles' terms
+    constexpr int W0 = FWD ? 0 : 1;
+    const int g0 = lo / EC, c0 = lo / CH, nChunks = (hi + 1) / CH - c0;
     const size_t tileBase = (size_t)tile * T * NP;
-    const int warp = threadIdx.x >> 5;
+    // chunk n into its slot: its 8 steps are one block of the layout
+    constexpr unsigned bl = CH * NP * sizeof(float4), br = CH * NP * sizeof(float);
+    auto chunk_entry = [&](int n) { return tileBase + (size_t)(FWD ? (c0 + n) * CH : T - (c0 + n + 1) * CH) * NP; };
+    auto issue = [&](int n) {
+        const int b = n % NBUF;
+        const unsigned bar = smem_addr(&sm.loaded[b]);
+        mb_arrive_expect_tx(bar, bl + br);
+        bulk_load(&sm.slot[b].L, a.L + chunk_entry(n), bl, bar);
+        bulk_load(&sm.slot[b].r, a.rin + chunk_entry(n), br, bar);
+    };
+    auto prefetch = [&](int n) {   // into L2, for its copy one ring later
+        if (n >= nChunks) return;
+        prefetch_l2(a.L + chunk_entry(n), bl);
+        prefetch_l2(a.rin + chunk_entry(n), br);
+    };
+    if (work && threadIdx.x == LOADER * 32) issue(0);   // comes while the edge words are set up
+    if (work) {
+        // Words that will come are ABSENT, the others are zero terms.  In the
+        // ring everything comes, the other tiles' zero terms too, except a
+        // warp's first term from the warp before it.
+        const int first = WHOLE ? g0 : 0, count = WHOLE ? (hi + 1) / EC - g0 : edgeGroups;
+        for (int q = threadIdx.x; q < NWC * count * (VA + VB); q += NTHREADS) {
+            const int pencil = q % (VA + VB), rest = q / (VA + VB), g = first + rest % count, wi = rest / count;
+            const bool isA = pencil < VB;
+            const bool outside = (isA ? wi % NWA : wi / NWA) == W0;   // its terms come from another tile
+            const int w0 = outside ? (isA ? iA0 : iB0) : lo + 1, w1 = outside ? (isA ? iA1 : iB1) : hi;
+            unsigned v[EC];
+            for (int s = 0; s < EC; s++) {
+                const int te = g * EC + s;
+                const bool comes = WHOLE ? te >= w0 && te <= w1 : outside || te != 0;
+                v[s] = comes ? ABSENT : 0u;
+            }
+            reinterpret_cast<uint4 *>(edge)[((size_t)wi * edgeGroups + g) * (VA + VB) + pencil] =
+                make_uint4(v[0], v[1], v[2], v[3]);
+        }
+    }
+    cluster_sync();   // also keeps rank 0 until every CTA has read its ticket
+    if (!work) return;
+    const size_t wordsPerTile = (size_t)T * (WA + WB);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
     if (warp == LOADER) {
-        // ================================================== loader warp
-        const int lane = threadIdx.x & 31;
+        // ================================================== loader thread
         if (lane != 0) return;
-        auto issue = [&](int m, int b) {   // operands of chunk m into slot b
-            Slot &sl = sm.slot[b];
-            const int tb = tlo + m * CH, rows = chunk_rows(m);
-            const unsigned bl = (unsigned)(rows * NP * sizeof(float4)), br = (unsigned)(rows * NP * sizeof(float));
-            const size_t e0 = tileBase + (size_t)chunk_tf0(tb, rows) * NP;
-            const int r0 = chunk_row0(rows);
-            mb_arrive_expect_tx(&sm.loaded[b], bl + br);
-            bulk_load(&sl.L[r0][0], a.L + e0, bl, &sm.loaded[b]);
-            bulk_load(&sl.r[r0][0], a.rin + e0, br, &sm.loaded[b]);
-        };
-        auto prefetch = [&](int m) {   // chunk m into L2, for its copy one ring later
-            if (m >= nChunks) return;
-            const int tb = tlo + m * CH, rows = chunk_rows(m);
-            const size_t e0 = tileBase + (size_t)chunk_tf0(tb, rows) * NP;
-            prefetch_l2(a.L + e0, (unsigned)(rows * NP * sizeof(float4)));
-            prefetch_l2(a.rin + e0, (unsigned)(rows * NP * sizeof(float)));
-        };
-        int issued = 0;
+        prefetch(NBUF);
+        int issued = 1;
         for (; issued < nChunks; issued++) {
-            const int b = issued % NBUF;
-            if (issued >= NBUF &&
-                !mb_wait(&sm.done[b], ((issued - NBUF) / NBUF) & 1, &sm.abort, a.err, a.spinLimit))
-                break;
-            issue(issued, b);
+            const int before = issued - NBUF;
+            if (before >= 0 && !mb_wait(smem_addr(&sm.done[before % NBUF]), (before / NBUF) & 1, &sm.abort, a.err, a.spinLimit)) break;
+            issue(issued);
             prefetch(issued + NBUF);
         }
         // The copies started must land before the CTA's shared memory is
@@ -288,255 +525,129 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_wavefront(SweepArgs a) {
         // phase completes once its bytes are in.
         for (int m = max(0, issued - NBUF); m < issued; m++)
             for (unsigned int spin = 0;
-                 spin < DRAIN_SPIN_LIMIT && !mb_test(&sm.loaded[m % NBUF], (m / NBUF) & 1); spin++)
+                 spin < DRAIN_SPIN_LIMIT && !mb_test(smem_addr(&sm.loaded[m % NBUF]), (m / NBUF) & 1); spin++)
                 __nanosleep(32);
         return;
     }
 
-    if (warp == EDGE) {
-        // ==================================================== edge warp
-        const int lane = threadIdx.x & 31;
-        const int srcJ = FWD ? (tj > 0 ? tile - 1 : -1) : (tj < a.ntj - 1 ? tile + 1 : -1);
-        const int srcK = FWD ? (tk > 0 ? tile - a.ntj : -1) : (tk < a.ntk - 1 ? tile + a.ntj : -1);
-        const int2 rgJ = srcJ >= 0 ? steps_of(srcJ) : make_int2(1, 0);
-        const int2 rgK = srcK >= 0 ? steps_of(srcK) : make_int2(1, 0);
-        const int laneJ = FWD ? 0 : TJ - 1, warpK = FWD ? 0 : TK - 1;
-        // Each lane's words: for the k edge, the one of its own lane of the
-        // upstream tile's edge warp at each step; for the j edge, JQ (step,
-        // warp) pairs of each chunk.  A word is needed at step te when the
-        // consumer cell is interior (te in [base, base + NI - 1]) and the
-        // producer tile computes its cell (te + skew in the producer's
-        // range): a window of steps fixed per lane, computed once.
-        auto base_of = [&](int lr, int ww) {
-            return FWD ? SL * lr + SW * ww : SL * (TJ - 1 - lr) + SW * (TK - 1 - ww);
-        };
-        int kLo = 1, kHi = 0;
-        if (srcK >= 0 && pencil_in(lane, warpK)) {
-            const int bs = base_of(lane, warpK);
-            kLo = max(bs, rgK.x - SW * (TK - 1));
-            kHi = min(min(bs + NI - 1, rgK.y - SW * (TK - 1)), thi);
-        }
-        const unsigned long long *pK = a.xchg + (srcK >= 0 ? srcK : 0) * wordsPerTile + (size_t)T * TK +
-                                       (size_t)SW * (TK - 1) * TJ + lane;   // + te * TJ
-        int jLo[JQ], jHi[JQ], jes[JQ];
-        const unsigned long long *pJ[JQ];
-#pragma unroll
-        for (int q = 0; q < JQ; q++) {
-            const int e = lane + 32 * q, es = e / TK, ew = e % TK;
-            jes[q] = es;
-            jLo[q] = 1;
-            jHi[q] = 0;
-            if (srcJ >= 0 && pencil_in(laneJ, ew)) {
-                const int bs = base_of(laneJ, ew);
-                jLo[q] = max(bs, rgJ.x - SL * (TJ - 1));
-                jHi[q] = min(min(bs + NI - 1, rgJ.y - SL * (TJ - 1)), thi);
+    if (warp >= EDGE) {
+        // ==================================================== edge warps
+        // Warp h polls the words of every NHELP-th group of steps: lane e one
+        // a-edge word (step e / WB, pencil e % WB) and two b-edge words.
+        if (!helpers) return;
+        const unsigned int epWait = sm.epoch + a.epochSkew;   // awaited in the neighbours' words
+        const unsigned long long *xA = a.xchg + (size_t)(tile - dir) * wordsPerTile + (WA - 1) * WB;
+        const unsigned long long *xB =
+            a.xchg + (size_t)(tile - dir * a.nta) * wordsPerTile + (size_t)T * WB + (WB - 1) * WA;
+        const int nGroups = nChunks * (CH / EC);
+        const int s4 = lane / WB, pA = lane % WB, sB0 = lane / WA, pB = lane % WA;
+        // the warps whose words these are
+        float *wA = edge + (size_t)(W0 + NWA * (pA / VB)) * edgeGroups * GW + (pA % VB) * EC + s4;
+        float *wB = edge + (size_t)(pB / VA + NWA * W0) * edgeGroups * GW + (VB + pB % VA) * EC + sB0;
+        for (int m = warp - EDGE; m < nGroups; m += NHELP) {
+            const int g = WHOLE ? g0 + m : m % edgeGroups;
+            if (!WHOLE && m >= 2 * NBUF) {   // the words' last group is done
+                const int prev = m / 2 - NBUF;
+                if (!mb_wait(smem_addr(&sm.done[prev % NBUF]), (prev / NBUF) & 1, &sm.abort, a.err, a.spinLimit)) return;
             }
-            pJ[q] = a.xchg + (srcJ >= 0 ? srcJ : 0) * wordsPerTile + (size_t)SL * (TJ - 1) * TK + ew;   // + te * TK
-        }
-        bool mine = kLo <= kHi;
-#pragma unroll
-        for (int q = 0; q < JQ; q++) mine = mine || jLo[q] <= jHi[q];
-        const bool anyEdge = __any_sync(0xffffffffu, mine);
-        for (int m = 0; m < nChunks; m++) {
-            const int b = m % NBUF;
-            Slot &sl = sm.slot[b];
-            if (m >= NBUF && !mb_wait(&sm.done[b], ((m - NBUF) / NBUF) & 1, &sm.abort, a.err, a.spinLimit))
-                return;   // aborting
-            const int tb = tlo + m * CH;
-            if (!anyEdge) {   // no upstream tile: the edge terms are zero
-                if (m < NBUF) {
-#pragma unroll
-                    for (int q2 = 0; q2 < CH; q2++) sl.eK[q2][lane] = 0.0f;
-#pragma unroll
-                    for (int q = 0; q < JQ; q++) sl.eJ[jes[q]][(lane + 32 * q) % TK] = 0.0f;
-                }
-                __syncwarp();
-                mb_arrive(&sm.edges[b]);
-                continue;
-            }
-            float vK[CH], vJ[JQ];
-            unsigned long long wK[CH], wJ[JQ];
-            unsigned int needK = 0, needJ = 0;
-#pragma unroll
-            for (int s2 = 0; s2 < CH; s2++) {
-                const int te = tb + s2;
-                const bool need = te >= kLo && te <= kHi;
-                wK[s2] = need ? ld_word(pK + (size_t)te * TJ) : 0ull;
-                needK |= need ? 1u << s2 : 0u;
-            }
-#pragma unroll
-            for (int q = 0; q < JQ; q++) {
-                const int te = tb + jes[q];
-                const bool need = te >= jLo[q] && te <= jHi[q];
-                wJ[q] = need ? ld_word(pJ[q] + (size_t)te * TK) : 0ull;
-                needJ |= need ? 1u << q : 0u;
-            }
+            const int t = (g0 + m) * EC, tA = t + s4, tB0 = t + sB0, tB1 = tB0 + EC / 2;
+            bool needA = pollA && tA >= iA0 && tA <= iA1;
+            bool needB0 = pollB && tB0 >= iB0 && tB0 <= iB1, needB1 = pollB && tB1 >= iB0 && tB1 <= iB1;
+            float vA = 0.f, vB0 = 0.f, vB1 = 0.f;
             bool ok = true;
-            for (unsigned int spin = 0;; spin++) {
-                unsigned int missK = 0, missJ = 0;
-#pragma unroll
-                for (int s2 = 0; s2 < CH; s2++)
-                    missK |= ((needK >> s2) & 1u) && (unsigned int)(wK[s2] >> 32) != epWait ? 1u << s2 : 0u;
-#pragma unroll
-                for (int q = 0; q < JQ; q++)
-                    missJ |= ((needJ >> q) & 1u) && (unsigned int)(wJ[q] >> 32) != epWait ? 1u << q : 0u;
-                if (!(missK | missJ)) break;
+            for (unsigned int spin = 0; needA || needB0 || needB1; spin++) {
                 if (spin >= a.spinLimit) {
                     atomicExch(a.err, 1);
                     ok = false;
                     break;
                 }
-                if (*(volatile int *)&sm.abort || *(volatile int *)a.err) { ok = false; break; }
-                if (spin > 64) __nanosleep(32);
-#pragma unroll
-                for (int s2 = 0; s2 < CH; s2++)
-                    if ((missK >> s2) & 1u) wK[s2] = ld_word(pK + (size_t)(tb + s2) * TJ);
-#pragma unroll
-                for (int q = 0; q < JQ; q++)
-                    if ((missJ >> q) & 1u) wJ[q] = ld_word(pJ[q] + (size_t)(tb + jes[q]) * TK);
+                if (spin > 8) {
+                    if (*(volatile int *)&sm.abort || ((spin & 63) == 63 && *(volatile int *)a.err)) { ok = false; break; }
+                    if (spin > 64) __nanosleep(32);
+                }
+                const unsigned long long w2 = needA ? ld_word(xA + (size_t)tA * WB + pA) : 0ull,
+                                         w0 = needB0 ? ld_word(xB + (size_t)tB0 * WA + pB) : 0ull,
+                                         w1 = needB1 ? ld_word(xB + (size_t)tB1 * WA + pB) : 0ull;
+                if (needA && (unsigned)(w2 >> 32) == epWait) { vA = __uint_as_float((unsigned)w2); needA = false; }
+                if (needB0 && (unsigned)(w0 >> 32) == epWait) { vB0 = __uint_as_float((unsigned)w0); needB0 = false; }
+                if (needB1 && (unsigned)(w1 >> 32) == epWait) { vB1 = __uint_as_float((unsigned)w1); needB1 = false; }
             }
             if (!__all_sync(0xffffffffu, ok)) {
                 // the compute warps and the loader see the flag in their waits
                 *(volatile int *)&sm.abort = 1;
                 return;
             }
-#pragma unroll
-            for (int s2 = 0; s2 < CH; s2++) vK[s2] = __uint_as_float((unsigned int)wK[s2]);
-#pragma unroll
-            for (int q = 0; q < JQ; q++) vJ[q] = __uint_as_float((unsigned int)wJ[q]);
-#pragma unroll
-            for (int s2 = 0; s2 < CH; s2++) sl.eK[s2][lane] = vK[s2];
-#pragma unroll
-            for (int q = 0; q < JQ; q++) sl.eJ[jes[q]][(lane + 32 * q) % TK] = vJ[q];
-            __syncwarp();
-            mb_arrive(&sm.edges[b]);
+            if (!WHOLE || pollA) *(volatile float *)(wA + g * GW) = vA;
+            if (!WHOLE || pollB) {
+                *(volatile float *)(wB + g * GW) = vB0;
+                *(volatile float *)(wB + g * GW + EC / 2) = vB1;
+            }
         }
         return;
     }
 
     // ====================================================== compute warps
-    // Slot w of lane l is pencil (l, w) of the tile; in the forward sweep it
-    // meets cell i = 1 + t - l - w at step t.  The three lower neighbours of
-    // a cell (i-1 in the same slot, j-1 in lane l-1, k-1 in slot w-1) were
-    // all formed at step t - 1, so the slots of a step are independent: the
-    // x term stays in the slot's register, the y term comes from lane l-1 by
-    // shuffle, the z term from slot w-1.  Compute warp g holds the SPW slots
-    // g*SPW.. of every lane and the warps run in lockstep, one barrier per
-    // step: the z term that crosses from warp g-1 to warp g is written to
-    // shared memory before the barrier and read after it (the backward sweep
-    // is the mirror image, its terms handed from warp g+1 to warp g).  Full
-    // chunks run without a test per step; only a tile's last chunk checks
-    // for its end.
-    const int l = threadIdx.x & 31, g = warp;
-    const int w0 = g * SPW;   // first slot of this warp
-    const bool takes = FWD ? g > 0 : g < NWC - 1;    // receives the z term from a neighbouring warp
-    const bool hands = FWD ? g < NWC - 1 : g > 0;    // hands its edge slot's term on
-    const bool slotEdgeIn = FWD ? g == 0 : g == NWC - 1;   // reads the upstream tile's k-edge terms
-    constexpr int NB = NWC > 1 ? NWC - 1 : 1;
-    const int bIn = min(max(FWD ? g - 1 : g, 0), NB - 1), bOut = min(max(FWD ? g : g - 1, 0), NB - 1);
-    const bool pubJ = FWD ? (l == TJ - 1 && tj < a.ntj - 1) : (l == 0 && tj > 0);
-    // the tile's k-edge slot (TK-1 forward, 0 backward) publishes for its lane
-    const bool pubK = (FWD ? tk < a.ntk - 1 && g == NWC - 1 : tk > 0 && g == 0);
-    unsigned long long *pubJw = a.xchg + tile * wordsPerTile + w0;                    // [t][TK]
-    unsigned long long *pubKw = a.xchg + tile * wordsPerTile + (size_t)T * TK + l;    // [t][TJ]
-    // forward: per slot the L_x y (own next cell), L_y y (lane l+1) and
-    // L_z y (slot w+1) terms of its last cell, in the tile's orientation;
-    // backward: per slot the z of its last cell, which all three take
-    float tx[SPW], tl[SPW], tw[SPW];
-#pragma unroll
-    for (int j = 0; j < SPW; j++) tx[j] = tl[j] = tw[j] = 0.0f;
-    float upNext = 0.0f;   // the neighbouring warp's term for the next step (none before the first)
-    for (int n = 0; n < nChunks; n++) {
-        const int b = n % NBUF;
-        const unsigned par = (n / NBUF) & 1;
-        const bool fine = mb_wait(&sm.loaded[b], par, &sm.abort, a.err, a.spinLimit) &&
-                          mb_wait(&sm.edges[b], par, &sm.abort, a.err, a.spinLimit);
-        if (compute_sync_or(!fine)) {   // every compute warp stops, or none
-            *(volatile int *)&sm.abort = 1;
-            return;
-        }
-        const Slot &sl = sm.slot[b];
-        const int tb = tlo + n * CH, rows = min(CH, thi + 1 - tb);
-        // the results of chunk n: row of step tb + s at out0 + s * ostep
-        float *out0 = a.out + tileBase + (size_t)(FWD ? tb : T - 1 - tb) * NP + w0 * TJ + l;
-        const long long ostep = FWD ? NP : -NP;
-        // operands of the next step, loaded while the current one computes
-        float4 Ln[SPW];
-        float rn[SPW], ejn[SPW], ekn = 0.0f;
-        auto load_step = [&](int s) {
-            const int q = FWD ? s : CH - 1 - s;
-#pragma unroll
-            for (int j = 0; j < SPW; j++) {
-                Ln[j] = sl.L[q][(w0 + j) * TJ + l];
-                rn[j] = sl.r[q][(w0 + j) * TJ + l];
-                ejn[j] = sl.eJ[s][w0 + j];
-            }
-            if (slotEdgeIn) ekn = sl.eK[s][l];
-        };
-        auto step = [&](int s, bool more) {
-            const int t = tb + s;
-            float4 Lc[SPW];
-            float rr[SPW], ej[SPW];
-#pragma unroll
-            for (int j = 0; j < SPW; j++) { Lc[j] = Ln[j]; rr[j] = rn[j]; ej[j] = ejn[j]; }
-            const float up = slotEdgeIn ? ekn : upNext;   // the z term of the warp's edge slot
-            if (more) load_step(s + 1);
-            float nb[SPW];   // the lane neighbour's term of each slot
-#pragma unroll
-            for (int j = 0; j < SPW; j++) {
-                nb[j] = FWD ? __shfl_up_sync(0xffffffffu, tl[j], 1) : __shfl_down_sync(0xffffffffu, tx[j], 1);
-                if (l == (FWD ? 0 : TJ - 1)) nb[j] = ej[j];
-            }
-            float nx[SPW], nl[SPW], nw[SPW], res[SPW];
-#pragma unroll
-            for (int j = 0; j < SPW; j++) {
-                if (FWD) {
-                    // terms from the lane and slot neighbours: L of the
-                    // neighbour towards this cell times its y
-                    const float pL = nb[j];
-                    const float pW = j > 0 ? tw[j - 1] : up;
-                    float acc = __fsub_rn(rr[j], SWAP ? pL : pW);   // -z
-                    acc = __fsub_rn(acc, SWAP ? pW : pL);           // -y
-                    acc = __fsub_rn(acc, tx[j]);                    // -x
-                    res[j] = __fmul_rn(acc, Lc[j].x);
-                    nx[j] = __fmul_rn(Lc[j].y, res[j]);
-                    nl[j] = __fmul_rn(SWAP ? Lc[j].w : Lc[j].z, res[j]);   // for the next lane
-                    nw[j] = __fmul_rn(SWAP ? Lc[j].z : Lc[j].w, res[j]);   // for the next slot
-                } else {
-                    const float zL = nb[j];
-                    const float zW = j < SPW - 1 ? tx[j + 1] : up;
-                    float acc = __fsub_rn(rr[j], __fmul_rn(Lc[j].y, tx[j]));          // +x
-                    acc = __fsub_rn(acc, __fmul_rn(Lc[j].z, SWAP ? zW : zL));      // +y
-                    acc = __fsub_rn(acc, __fmul_rn(Lc[j].w, SWAP ? zL : zW));      // +z
-                    res[j] = __fmul_rn(acc, Lc[j].x);
-                    nx[j] = nl[j] = nw[j] = res[j];
-                }
-            }
-            // the edge slot's term for the neighbouring warp, by step parity:
-            // it reads it after this step's barrier, before the next one
-            if (hands) sm.hand[t & 1][bOut][l] = nw[FWD ? SPW - 1 : 0];
-#pragma unroll
-            for (int j = 0; j < SPW; j++) __stcg(out0 + s * ostep + j * TJ, res[j]);
-            // Edge terms of cells outside the grid are published too: a
-            // neighbour only polls the words of cells it needs.
-            st_terms(pubJ, pubJw + (size_t)t * TK, nl, ep);
-            st_term(pubK, pubKw + (size_t)t * TJ, pack(ep, nw[FWD ? SPW - 1 : 0]));
-#pragma unroll
-            for (int j = 0; j < SPW; j++) { tx[j] = nx[j]; tl[j] = nl[j]; tw[j] = nw[j]; }
-            if (NWC > 1) {
-                compute_sync();
-                if (takes) upNext = sm.hand[t & 1][bIn][l];
-            }
-        };
-        load_step(0);
-        if (rows == CH) {
-#pragma unroll
-            for (int s = 0; s < CH; s++) step(s, s + 1 < CH);
-        } else {
-#pragma unroll 1
-            for (int s = 0; s < rows; s++) step(s, s + 1 < rows);
-        }
-        mb_arrive(&sm.done[b]);   // the slot may be refilled
+    // Warp (wa, wb), lane (la, lb): pencil (8 wa + la, 4 wb + lb) of the tile.
+    const int wa = warp % NWA, wb = warp / NWA, la = lane % VA, lb = lane / VA;
+    const bool outEdgeA = la == (FWD ? VA - 1 : 0), outEdgeB = lb == (FWD ? VB - 1 : 0);
+    WarpJob w;
+    w.sm = &sm;
+    w.err = a.err;
+    w.spinLimit = a.spinLimit;
+    w.c0 = c0;
+    w.nChunks = nChunks;
+    w.lane = lane;
+    w.L = &sm.slot[0].L[0][warp * 32 + lane];
+    w.r = &sm.slot[0].r[0][warp * 32 + lane];
+    w.out = a.out + tileBase + warp * 32 + lane;
+    w.lastStep = T - 1;
+    w.inEdgeA = la == (FWD ? 0 : VA - 1);
+    w.inEdgeB = lb == (FWD ? 0 : VB - 1);
+    w.epoch = sm.epoch;
+    const unsigned eb = smem_addr(edge), warpBytes = (unsigned)edgeGroups * GW * 4;
+    w.inA = eb + warp * warpBytes + lb * EC * 4;
+    w.inB = eb + warp * warpBytes + (VB + la) * EC * 4;
+    // To the next warp of the tile, or from the last one to the next tile: the
+    // words of its first warp there (another CTA of the cluster, by its own
+    // steps), or the exchange array.
+    const bool lastA = wa == 1 - W0, lastB = wb == 1 - W0;
+    const unsigned toA = (unsigned)(lastA ? W0 + NWA * wb : 1 - W0 + NWA * wb) * warpBytes + lb * EC * 4;
+    const unsigned toB = (unsigned)(lastB ? wa + NWA * W0 : wa + NWA * (1 - W0)) * warpBytes + (VB + la) * EC * 4;
+    constexpr int GB = GW * 4 / EC;   // edge bytes per step
+    w.unused = smem_addr(&sm.unused[warp][lane]);
+    w.unused = map_rank(w.unused, rank);
+    w.dstA = lastA && dnAcl ? map_rank(eb + toA, (unsigned)((int)rank + dir)) - WA * GB : map_rank(eb + toA, rank);
+    w.dstB = lastB && dnBcl ? map_rank(eb + toB, (unsigned)((int)rank + dir * CA)) - WB * GB : map_rank(eb + toB, rank);
+    const int dA0 = max(lo, rDA.x + WA - 1), dA1 = min(hi, rDA.y + WA - 1);   // steps whose term the next tile takes
+    const int dB0 = max(lo, rDB.x + WB - 1), dB1 = min(hi, rDB.y + WB - 1);
+    // chunks of a window of steps [s0, s1], by `first` step of the chunk (0: its
+    // steps 0-6; 7: step 7)
+    auto chunks = [](bool on, int s0, int s1, int first) {
+        const int k0 = (s0 - first + CH - 1) >> 3, k1 = (s1 - (first | 6)) >> 3;   // floor division
+        return make_int2(k0, on ? max(k1 - k0 + 1, 0) : 0);
+    };
+    const bool smA = outEdgeA && (!lastA || dnAcl), smB = outEdgeB && (!lastB || dnBcl);   // into shared memory
+    const int sA0 = lastA ? dA0 : lo, sA1 = lastA ? dA1 : hi - 1, sB0 = lastB ? dB0 : lo, sB1 = lastB ? dB1 : hi - 1;
+    w.kA = chunks(smA, sA0, sA1, 0);
+    w.kA7 = chunks(smA, sA0, sA1, 7);
+    w.kB = chunks(smB, sB0, sB1, 0);
+    w.kB7 = chunks(smB, sB0, sB1, 7);
+    w.pA = chunks(outEdgeA && !smA, dA0, dA1, 0);
+    w.pA7 = chunks(outEdgeA && !smA, dA0, dA1, 7);
+    w.pB = chunks(outEdgeB && !smB, dB0, dB1, 0);
+    w.pB7 = chunks(outEdgeB && !smB, dB0, dB1, 7);
+    w.xA = a.xchg + (size_t)tile * wordsPerTile + wb * VB + lb;                    // [t][WB]
+    w.xB = a.xchg + (size_t)tile * wordsPerTile + (size_t)T * WB + wa * VA + la;   // [t][WA]
+    const bool pub = __any_sync(0xffffffffu, w.pA.y + w.pA7.y + w.pB.y + w.pB7.y > 0);
+    const bool fine = pub ? run_steps<FWD, SWAP, WHOLE, true>(w) : run_steps<FWD, SWAP, WHOLE, false>(w);
+    if (!fine) {
+        // Peers may still store into this CTA's shared memory: stop the other
+        // warps, let what is in flight land, and stay until the cluster's
+        // other threads have ended or got here.
+        *(volatile int *)&sm.abort = 1;
+        for (int q = 0; q < 32; q++) __nanosleep(1000);
+        __syncwarp();
+        cluster_sync();
     }
 }
 
@@ -558,8 +669,8 @@ __global__ void k_tile_range(const uint8_t *fluid, int I, int J, int K, SweepLay
         int i, j, k;
         unflatten(t, I, J, i, j, k);
         const int aa = (g.swap ? k : j) - 1, bb = (g.swap ? j : k) - 1;
-        tile = aa / TJ + g.ntj * (bb / TK);
-        step = (i - 1) + SL * (aa % TJ) + SW * (bb % TK);
+        tile = aa / WA + g.nta * (bb / WB);
+        step = (i - 1) + aa % WA + bb % WB;
     }
     unsigned int grp = __match_any_sync(0xffffffffu, tile);
     int mn = __reduce_min_sync(grp, f ? step : 0x7fffffff);
@@ -576,20 +687,20 @@ int sweep_tiles_max(int I, int J, int K) {
     int best = 0;
     for (int sw = 0; sw < 2; sw++) {
         const SweepLayout g = sweep_layout(I, J, K, sw);
-        best = std::max(best, g.ntj * g.ntk);
+        best = std::max(best, g.nta * g.ntb);
     }
     return best;
 }
 
-// per tile: TK j-edge words and TJ k-edge words for each of its T steps
+// per tile: WB a-edge words and WA b-edge words for each of its T steps
 long long sweep_exchange_words(int I, int J, int K) {
     const SweepLayout g = sweep_layout(I, J, K);
-    return (long long)sweep_tiles_max(I, J, K) * (TJ + TK) * g.T;
+    return (long long)sweep_tiles_max(I, J, K) * (WA + WB) * g.T;
 }
 
 void launch_sweep_ranges(const StepConsts &c, const SweepLayout &g, const uint8_t *fluid, SweepState &sw,
                          cudaStream_t s) {
-    const int n = g.ntj * g.ntk;
+    const int n = g.nta * g.ntb;
     { FLIP_COUNT(1); k_tile_range_init<<<div_up(n, 256), 256, 0, s>>>(sw.range, n); }
     long long nc = (long long)c.I * c.J * c.K;
     { FLIP_COUNT(1); k_tile_range<<<div_up(nc, 256), 256, 0, s>>>(fluid, c.I, c.J, c.K, g, sw.range); }
@@ -597,33 +708,43 @@ void launch_sweep_ranges(const StepConsts &c, const SweepLayout &g, const uint8_
 
 void launch_sweeps(const StepConsts &c, const SweepLayout &g, const float4 *L, const float *rf, float *z,
                    SweepState &sw, const int *skip, cudaStream_t s, bool prepped) {
-    const int n = g.ntj * g.ntk;
-    static std::atomic<unsigned long long> smemSet{0};   // devices on which the slots' shared memory is opted in
+    static std::atomic<unsigned long long> smemSet{0};   // devices on which the shared memory is opted in
     int dev = 0;
     cudaGetDevice(&dev);
+    // [direction][orientation][whole]
+    using Kernel = void (*)(SweepArgs);
+    static constexpr Kernel kernels[2][2][2] = {
+        {{k_wavefront<true, false, false>, k_wavefront<true, false, true>},
+         {k_wavefront<true, true, false>, k_wavefront<true, true, true>}},
+        {{k_wavefront<false, false, false>, k_wavefront<false, false, true>},
+         {k_wavefront<false, true, false>, k_wavefront<false, true, true>}}};
     if (dev < 64 && !((smemSet.load() >> dev) & 1ull)) {   // idempotent, so a race only repeats it
-        cudaFuncSetAttribute(k_wavefront<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SweepSmem));
-        cudaFuncSetAttribute(k_wavefront<false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SweepSmem));
-        cudaFuncSetAttribute(k_wavefront<true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SweepSmem));
-        cudaFuncSetAttribute(k_wavefront<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SweepSmem));
+        for (auto &byDir : kernels)
+            for (auto &byOrient : byDir)
+                for (Kernel k : byOrient)
+                    cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sweep_smem_bytes(WHOLE_STEPS));
         smemSet.fetch_or(1ull << dev);
     }
     SweepArgs a;
     a.L = L;
-    a.J = g.EA; a.K = g.EB; a.NI = c.I - 2; a.T = g.T;   // extents along the lane and warp axes
-    a.ntj = g.ntj; a.ntk = g.ntk;
+    a.T = g.T;
+    a.nta = g.nta; a.ntb = g.ntb;
+    a.nca = (g.nta + CA - 1) / CA;
+    a.nClusters = a.nca * ((g.ntb + CB - 1) / CB);
     a.range = sw.range; a.xchg = sw.xchg; a.ticket = sw.ticket; a.err = sw.err; a.skip = skip;
     a.spinLimit = sw.spinLimit ? sw.spinLimit : DEFAULT_SPIN_LIMIT;
     a.epochSkew = sw.stall ? 1u : 0u;
-    // forward: y from r
-    a.rin = rf; a.out = z;
+    const bool whole = g.T <= WHOLE_STEPS;
+    const size_t smem = sweep_smem_bytes(whole ? g.T : RC * CH);
+    const unsigned n = (unsigned)a.nClusters * CL;
     if (!prepped) { FLIP_COUNT(1); k_sweep_prep<<<1, 1, 0, s>>>(sw.ticket); }
-    if (g.swap) { FLIP_COUNT(1); k_wavefront<true, true><<<n, NTHREADS, sizeof(SweepSmem), s>>>(a); }
-    else { FLIP_COUNT(1); k_wavefront<true, false><<<n, NTHREADS, sizeof(SweepSmem), s>>>(a); }
-    // backward: z from y, in place
-    a.rin = z; a.out = z;
-    if (g.swap) { FLIP_COUNT(1); k_wavefront<false, true><<<n, NTHREADS, sizeof(SweepSmem), s>>>(a); }
-    else { FLIP_COUNT(1); k_wavefront<false, false><<<n, NTHREADS, sizeof(SweepSmem), s>>>(a); }
+    // forward: y from r; backward: z from y, in place
+    for (int d = 0; d < 2; d++) {
+        a.rin = d == 0 ? rf : z;
+        a.out = z;
+        FLIP_COUNT(1);
+        kernels[d][g.swap ? 1 : 0][whole ? 1 : 0]<<<n, NTHREADS, smem, s>>>(a);
+    }
     sw.epoch += 2;
 }
 
