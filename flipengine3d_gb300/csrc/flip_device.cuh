@@ -151,6 +151,8 @@ inline long long sweep_layout_size(int I, int J, int K) {
     }
     return best;
 }
+// chunks of either orientation: the most items a solve can have
+inline long long sweep_items_max(int I, int J, int K) { return sweep_layout_size(I, J, K) / (SWEEP_CH * SWEEP_NP); }
 // entry of interior cell (i, j, k)
 __host__ __device__ __forceinline__ long long sweep_index(const SweepLayout &g, int i, int j, int k) {
     const int aa = (g.swap ? k : j) - 1, bb = (g.swap ? j : k) - 1;
@@ -177,22 +179,23 @@ constexpr int PCG_BATCH = 8;   // iterations of a captured batch
 
 struct PressureBuffers {
     uint8_t *fluid;        // interior cell with phi < 0 (a row of the system)
-    // the rows as a list, in cell order (built once per solve by a scan):
-    // flat index and sweep-layout index of each row, and their number
-    int *fluidFlag, *fluidPos, *fluidScan, *nFluid;
-    int *fluidIdx, *fluidSk;
+    int *items, *nItems;   // the solve's chunks of the sweep layout, and their number
     double4_32a *Ad;           // rows {diag, to +x, to +y, to +z}, FP64
     double *b;             // right-hand side (negative divergence)
     double *invdiagD;      // MIC(0) inverse pivots, FP64
     float4 *L;             // {invdiag, Lx, Ly, Lz} for the FP32 sweeps, sweep layout
-    float4 *A2;            // per cell {hi, lo}: the rows as exact float pairs (hi + lo = the FP64 value to 48 bits)
-    float2 *x, *r, *q;     // solution, residual, A s: exact float pairs {hi, lo} (hi + lo to ~48 bits)
-    float *z;              // preconditioned residual, sweep layout
-    float *zc;             // the same at the rows in cell order (written by the z.r pass for the SpMV)
+    // The loop's vectors, in the sweep layout (nsl entries each; A, z, s and s2
+    // have a step of zeros after them, planes of A too).  Values kept
+    // to ~48 bits are pairs of floats, leading part h and remainder l.
+    float *A;              // rows as pairs: 8 planes, h of {diag, +x, +y, +z}, then l (also the factor's pivot weights)
+    float *xh, *xl;        // solution
+    float *rh, *rl;        // residual (rh: the forward sweep's right-hand side)
+    float *qh, *ql;        // A s
+    float *z;              // preconditioned residual
     float *s, *s2;         // search direction, double-buffered: an iteration reads one and writes the other
-    float *rf;             // r rounded to FP32, the forward sweep's right-hand side, sweep layout
     SweepLayout sl;        // the orientation of the current solve
     long long nsl;         // entries allocated for the sweep layout
+    bool stale = true;     // z, s, s2 may hold values that are not finite
     double *partials;      // per-block partial sums (deterministic reduction)
     double *scal;          // [0]=s.q [1]=z.r (new rho) [2]=|b|inf [3]=rho [4]=alpha [5]=beta [6]=tol |b|inf
     unsigned long long *rmaxBits;  // [0] |r|inf of the recurrence, [1] of b - A x, as double bits
@@ -264,6 +267,30 @@ int sweep_tiles_max(int I, int J, int K);           // tiles of the larger orien
 long long sweep_exchange_words(int I, int J, int K);   // for the larger orientation
 void launch_sweep_ranges(const StepConsts &c, const SweepLayout &g, const uint8_t *fluid, SweepState &sw,
                          cudaStream_t s);
+// Programmatic dependent launch: a kernel launched with launch_after may start
+// while the kernel before it in the stream still runs; what it reads or
+// overwrites of that kernel's lies after pdl_wait().  Called after pdl_wait,
+// pdl_trigger lets the kernel after it start the same way, which can then
+// rely on everything up to the kernel before this one even ahead of its own
+// wait.
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+template <class... P, class... Q>
+inline void launch_after(bool overlap, void (*k)(P...), unsigned grid, unsigned block, size_t smem, cudaStream_t s,
+                         Q... args) {
+    FLIP_COUNT(1);
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(block);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = overlap ? 1 : 0;
+    cudaLaunchKernelEx(&cfg, k, static_cast<P>(args)...);
+}
 // Before each sweep pair, by one thread of a kernel that runs before it:
 // tile tickets from zero for both sweeps and a fresh epoch for each (the
 // forward sweep publishes under ticket[1], the backward under ticket[1]+1).
@@ -276,9 +303,11 @@ __device__ __forceinline__ void sweep_prep(unsigned int *ticket) {
 }
 // z = M^-1 r with the MIC(0) factor L: forward then backward sweep
 // The launches return at once when *skip is set (a converged solve).
-// `prepped`: a kernel ahead of them on the stream already ran sweep_prep.
+// `prepped`: a kernel ahead of them on the stream already ran sweep_prep;
+// `overlap`: and at least one more lies between, so the forward sweep may set
+// up while that one runs.
 void launch_sweeps(const StepConsts &c, const SweepLayout &g, const float4 *L, const float *rf, float *z,
-                   SweepState &sw, const int *skip, cudaStream_t s, bool prepped = false);
+                   SweepState &sw, const int *skip, cudaStream_t s, bool prepped = false, bool overlap = false);
 void sweep_epoch_guard(const StepConsts &c, SweepState &sw, long long upcoming, cudaStream_t s);
 
 void mic0_factor(const StepConsts &c, const uint8_t *fluid, const double4_32a *Ad, double *invD, double *W0,

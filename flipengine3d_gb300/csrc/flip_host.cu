@@ -289,22 +289,13 @@ int alloc_grids(flip_ctx *x) {
     p.sl = sweep_layout(x->I, x->J, x->K, 0);
     p.nsl = nsl;
     if ((rc = x->alloc(&p.fluid, nc)) || (rc = x->alloc(&p.Ad, nc)) || (rc = x->alloc(&p.L, nsl)) ||
-        (rc = x->alloc(&p.b, nc)) || (rc = x->alloc(&p.invdiagD, nc)) || (rc = x->alloc(&p.x, nc)) ||
-        (rc = x->alloc(&p.r, nc)) || (rc = x->alloc(&p.q, nc)) || (rc = x->alloc(&p.z, nsl)) ||
-        (rc = x->alloc(&p.zc, nc)) ||
-        (rc = x->alloc(&p.A2, 2 * nc)) ||
-        (rc = x->alloc(&p.s, nc)) || (rc = x->alloc(&p.s2, nc)) || (rc = x->alloc(&p.rf, nsl)) ||
-        (rc = x->alloc(&p.pressure, nc)))
+        (rc = x->alloc(&p.b, nc)) || (rc = x->alloc(&p.invdiagD, nc)) ||
+        (rc = x->alloc(&p.A, std::max(8 * (nsl + SWEEP_NP), 6 * nc))) || (rc = x->alloc(&p.xh, nsl)) ||
+        (rc = x->alloc(&p.xl, nsl)) || (rc = x->alloc(&p.rh, nsl)) || (rc = x->alloc(&p.rl, nsl)) ||
+        (rc = x->alloc(&p.qh, nsl)) || (rc = x->alloc(&p.ql, nsl)) || (rc = x->alloc(&p.z, nsl + SWEEP_NP)) ||
+        (rc = x->alloc(&p.s, nsl + SWEEP_NP)) || (rc = x->alloc(&p.s2, nsl + SWEEP_NP)) || (rc = x->alloc(&p.pressure, nc)) ||
+        (rc = x->alloc(&p.items, sweep_items_max(x->I, x->J, x->K))) || (rc = x->alloc(&p.nItems, 4)))
         return rc;
-    if ((rc = x->alloc(&p.fluidFlag, nc + 1)) || (rc = x->alloc(&p.fluidPos, nc + 1)) ||
-        (rc = x->alloc(&p.fluidScan, scan_scratch_ints((int)nc) + 4)) || (rc = x->alloc(&p.nFluid, 4)) ||
-        (rc = x->alloc(&p.fluidIdx, nc)) || (rc = x->alloc(&p.fluidSk, nc)))
-        return rc;
-    // entries of the sweep layout that hold no interior cell stay zero
-    CK(cudaMemsetAsync(p.L, 0, nsl * sizeof(float4), x->stream));
-    CK(cudaMemsetAsync(p.rf, 0, nsl * sizeof(float), x->stream));
-    CK(cudaMemsetAsync(p.z, 0, nsl * sizeof(float), x->stream));
-    CK(cudaMemsetAsync(p.zc, 0, nc * sizeof(float), x->stream));
     p.nPartials = pressure_partials_for(x->I, x->J, x->K, x->pcgCellsPerCta);
     if ((rc = x->alloc(&p.partials, PCG_MAX_PARTIALS + 32)) || (rc = x->alloc(&p.scal, 8)) ||
         (rc = x->alloc(&p.rmaxBits, 2)) || (rc = x->alloc(&p.levelRange, 8)) || (rc = x->alloc(&p.ctl, 1)) ||
@@ -1555,8 +1546,8 @@ int flip_estimate_device_bytes(int isize, int jsize, int ksize, int particles, l
     b += 5 * (nc + 1) * 4 + (scan_scratch_ints((int)nc) + 4) * 4 + 16;   // binning
     b += nc * 4 + (I + 1) * (J + 1) * (K + 1) * 4 + nc;                  // phi, solid phi, solid cells
     b += faces * (4 * 3 + 1 + 1);                                        // weights, velocity, saved, valid, status
-    b += nc * (1 + 32 + 32 + 8 * 5 + 4 * 3 + 4) + nsl * (16 + 4 + 4);     // pressure system (s, s2, zc)
-    b += (nc + 1) * 4 * 2 + nc * 4 * 2 + (scan_scratch_ints((int)nc) + 8) * 4;   // row list
+    b += nc * (1 + 32 + 8 * 2 + 4) + nsl * (16 + 4 * 9) + 12 * SWEEP_NP + 4 * std::max(8 * (nsl + SWEEP_NP), 6 * nc);   // pressure system
+    b += 4 * (sweep_items_max(isize, jsize, ksize) + 8) + 16;              // its items
     b += (PCG_MAX_PARTIALS + 32) * 8 + 64 + 16 + 32;
     b += (mic0_factor_tiles(jsize, ksize) + 1) * 4 + 64;                  // factor tiles, ticket, control
     b += sweep_exchange_words(isize, jsize, ksize) * 8 + 4096;           // sweep exchange, ranges, tables

@@ -41,47 +41,52 @@ __device__ __forceinline__ bool sys_cell(const StepConsts &c, const float *phi, 
     return phi[(long long)i + (long long)c.I * ((long long)j + (long long)c.J * k)] < 0.0f;
 }
 
-__global__ void k_flags(StepConsts c, const float *phi, uint8_t *fluid, int *fluidFlag, int *levelRange) {
-    long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    Dims d{c.I, c.J, c.K};
-    bool f = false;
-    int lv = 0;
-    if (t < d.size()) {
+// The rows' flags, and the extent of their levels i + j + k, their number and
+// their extent in j and k (for the sweep tile orientation).  A CTA reduces
+// over CELLS_PER_CTA cells before its seven atomics: one set per warp of 32
+// cells was bound by them, all on the same addresses (107 us at 128^3).
+constexpr int FLAG_CELLS = 4096;
+__global__ void __launch_bounds__(TPB) k_flags(StepConsts c, const float *phi, uint8_t *fluid, int *levelRange) {
+    __shared__ int sh[7][TPB / 32];
+    const long long base = (long long)blockIdx.x * FLAG_CELLS, n = (long long)c.I * c.J * c.K;
+    int v[7] = {0x7fffffff, -1, 0, 0x7fffffff, -1, 0x7fffffff, -1};
+#pragma unroll 4
+    for (int q = threadIdx.x; q < FLAG_CELLS; q += TPB) {
+        const long long t = base + q;
+        if (t >= n) break;
         int i, j, k;
         unflatten(t, c.I, c.J, i, j, k);
-        f = sys_cell(c, phi, i, j, k);
+        const bool f = sys_cell(c, phi, i, j, k);
         fluid[t] = f ? 1 : 0;
-        fluidFlag[t] = f ? 1 : 0;
-        lv = i + j + k;
+        if (!f) continue;
+        v[0] = min(v[0], i + j + k);
+        v[1] = max(v[1], i + j + k);
+        v[2]++;
+        v[3] = min(v[3], j);
+        v[4] = max(v[4], j);
+        v[5] = min(v[5], k);
+        v[6] = max(v[6], k);
     }
-    // warp-aggregated min/max/count of the system cells' levels, and their
-    // extent in j and k (for the sweep tile orientation)
-    unsigned int m = __ballot_sync(0xffffffffu, f);
-    if (!m) return;
-    int jk[4] = {0x7fffffff, -1, 0x7fffffff, -1};
-    if (f) {
-        int i, j, k;
-        unflatten(t, c.I, c.J, i, j, k);
-        jk[0] = jk[1] = j;
-        jk[2] = jk[3] = k;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    auto reduce = [&](int q, int x) {
+        return q == 2 ? __reduce_add_sync(0xffffffffu, x)
+                      : (q == 0 || q == 3 || q == 5 ? __reduce_min_sync(0xffffffffu, x) : __reduce_max_sync(0xffffffffu, x));
+    };
+#pragma unroll
+    for (int q = 0; q < 7; q++) {
+        const int x = reduce(q, v[q]);
+        if (lane == 0) sh[q][warp] = x;
     }
-    int lo = f ? lv : 0x7fffffff, hi = f ? lv : -1;
-    for (int o = 16; o > 0; o >>= 1) {
-        lo = min(lo, __shfl_xor_sync(0xffffffffu, lo, o));
-        hi = max(hi, __shfl_xor_sync(0xffffffffu, hi, o));
-        jk[0] = min(jk[0], __shfl_xor_sync(0xffffffffu, jk[0], o));
-        jk[1] = max(jk[1], __shfl_xor_sync(0xffffffffu, jk[1], o));
-        jk[2] = min(jk[2], __shfl_xor_sync(0xffffffffu, jk[2], o));
-        jk[3] = max(jk[3], __shfl_xor_sync(0xffffffffu, jk[3], o));
-    }
-    if ((threadIdx.x & 31) == 0) {
-        atomicMin(&levelRange[0], lo);
-        atomicMax(&levelRange[1], hi);
-        atomicAdd(&levelRange[2], __popc(m));
-        atomicMin(&levelRange[3], jk[0]);
-        atomicMax(&levelRange[4], jk[1]);
-        atomicMin(&levelRange[5], jk[2]);
-        atomicMax(&levelRange[6], jk[3]);
+    __syncthreads();
+    if (warp != 0) return;
+#pragma unroll
+    for (int q = 0; q < 7; q++) {
+        const int idle = q == 2 ? 0 : (q == 0 || q == 3 || q == 5 ? 0x7fffffff : -1);
+        const int x = reduce(q, lane < TPB / 32 ? sh[q][lane] : idle);
+        if (lane != 0 || x == idle) continue;
+        if (q == 2) atomicAdd(&levelRange[q], x);
+        else if (q == 0 || q == 3 || q == 5) atomicMin(&levelRange[q], x);
+        else atomicMax(&levelRange[q], x);
     }
 }
 
@@ -144,16 +149,9 @@ __global__ void k_build(StepConsts c, const float *phi, const float *wu, const f
     Dims d{c.I, c.J, c.K};
     double bmag = 0.0;
     if (t < d.size()) {
-        pb.x[t] = make_float2(0.0f, 0.0f);
-        pb.r[t] = make_float2(0.0f, 0.0f);
-        pb.q[t] = make_float2(0.0f, 0.0f);
-        pb.s[t] = 0.0f;
-        pb.s2[t] = 0.0f;
         pb.invdiagD[t] = 0.0;
         if (!pb.fluid[t]) {
-            pb.Ad[t] = make_double4_32a(0.0, 0.0, 0.0, 0.0);
-            pb.A2[2 * t] = pb.A2[2 * t + 1] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-            pb.b[t] = 0.0;
+            pb.b[t] = 0.0;   // the row itself is not read
         } else {
             int i, j, k;
         unflatten(t, c.I, c.J, i, j, k);
@@ -171,12 +169,7 @@ __global__ void k_build(StepConsts c, const float *phi, const float *wu, const f
             div += factor * vK * (double)w[dw.idx(i, j, k)];
             pb.b[t] = div;
             bmag = fabs(div);
-            const double4_32a a = row_coeffs(c, phi, wu, wv, ww, mf, i, j, k);
-            pb.Ad[t] = a;
-            const float4 hi = make_float4((float)a.x, (float)a.y, (float)a.z, (float)a.w);
-            pb.A2[2 * t] = hi;
-            pb.A2[2 * t + 1] = make_float4((float)(a.x - (double)hi.x), (float)(a.y - (double)hi.y),
-                                           (float)(a.z - (double)hi.z), (float)(a.w - (double)hi.w));
+            pb.Ad[t] = row_coeffs(c, phi, wu, wv, ww, mf, i, j, k);
         }
     }
     block_max_to(bmag, (unsigned long long *)pb.scal + 2, false);
@@ -409,47 +402,151 @@ __global__ void __launch_bounds__(FT *FT) k_mic0_tiles(StepConsts c, const uint8
     if (threadIdx.x == 0) st_release(&progress[tile], FACTOR_DONE);
 }
 
-// the FP32 factor rows of the interior cells, into the sweep layout
-__global__ void k_mic0_finalize(StepConsts c, SweepLayout g, const uint8_t *fluid, const double4_32a *Ad,
-                                const double *invD, float4 *L) {
-    long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= (long long)c.I * c.J * c.K) return;
-    int i, j, k;
-    unflatten(t, c.I, c.J, i, j, k);
-    if (i < 1 || j < 1 || k < 1 || i > c.I - 2 || j > c.J - 2 || k > c.K - 2) return;
-    const double inv = invD[t];
-    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (fluid[t] && inv != 0.0) {
-        const double4_32a a = Ad[t];
-        v = make_float4((float)inv, (float)(a.y * inv), (float)(a.z * inv), (float)(a.w * inv));
+// The items of a solve: the chunks (SWEEP_CH steps of a tile, 1024 entries of
+// the sweep layout) that the sweeps pass over, tile by tile.  An item is
+// tile * (T / SWEEP_CH) + chunk.  One CTA.
+__global__ void __launch_bounds__(1024) k_items(SweepLayout g, const int2 *range, int *items, int *nItems) {
+    __shared__ int sh[32], base;
+    const int nt = g.nta * g.ntb, nch = g.T / SWEEP_CH, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (threadIdx.x == 0) base = 0;
+    __syncthreads();
+    for (int t0 = 0; t0 < nt; t0 += 1024) {
+        const int t = t0 + threadIdx.x;
+        const int2 rg = t < nt ? range[t] : make_int2(0, -1);
+        const int c0 = rg.x / SWEEP_CH, n = rg.y < rg.x ? 0 : rg.y / SWEEP_CH - c0 + 1;
+        int x = n;   // inclusive scan over the CTA
+        for (int o = 1; o < 32; o <<= 1) {
+            const int y = __shfl_up_sync(0xffffffffu, x, o);
+            if (lane >= o) x += y;
+        }
+        if (lane == 31) sh[warp] = x;
+        __syncthreads();
+        if (warp == 0) {
+            int w = sh[lane];
+            for (int o = 1; o < 32; o <<= 1) {
+                const int y = __shfl_up_sync(0xffffffffu, w, o);
+                if (lane >= o) w += y;
+            }
+            sh[lane] = w;
+        }
+        __syncthreads();
+        const int at = base + (warp ? sh[warp - 1] : 0) + x - n;
+        for (int q = 0; q < n; q++) items[at + q] = t * nch + c0 + q;
+        __syncthreads();
+        if (threadIdx.x == 0) base += sh[31];
+        __syncthreads();
     }
-    L[sweep_index(g, i, j, k)] = v;
+    if (threadIdx.x == 0) *nItems = base;
 }
 
-template <class T>
-__device__ __forceinline__ T block_sum(T v, T *sh) {
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    if (lane == 0) sh[warp] = v;
+// The grid cell of entry (tile, step tf, pencil p); false outside the interior.
+__device__ __forceinline__ bool entry_cell(const SweepLayout &g, int I, int tile, int tf, int p, int &i, int &j, int &k) {
+    const int A = (p & 7) + ((p >> 5) & 1) * SWEEP_VA, B = ((p >> 3) & 3) + (p >> 6) * SWEEP_VB;
+    const int aa = tile % g.nta * SWEEP_WA + A + 1, bb = tile / g.nta * SWEEP_WB + B + 1;
+    i = tf + 1 - A - B;
+    j = g.swap ? bb : aa;
+    k = g.swap ? aa : bb;
+    return i >= 1 && i <= I - 2 && aa <= g.EA - 2 && bb <= g.EB - 2;
+}
+
+// A system's vectors in the sweep layout, an item per CTA, four consecutive
+// pencils of a step per thread: the FP32 factor rows, the rows as exact float
+// pairs (planes of A: the leading parts of the diagonal and of the couplings
+// to +x, +y, +z, then their remainders), r = b as pairs, x = s = 0.  Reads
+// gather whole 32-byte rows; all writes are coalesced.
+__global__ void __launch_bounds__(TPB) k_layout(StepConsts c, SweepLayout g, const int *items, const int *nItems,
+                                                PressureBuffers pb, unsigned int *sweepTicket) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) sweep_prep(sweepTicket);   // for the first sweep pair
+    const int nch = g.T / SWEEP_CH, p0 = (threadIdx.x & 31) * 4;
+    for (int it = blockIdx.x; it < *nItems; it += gridDim.x) {
+        const int item = items[it], tile = item / nch, tf = item % nch * SWEEP_CH + (threadIdx.x >> 5);
+        const long long e = ((long long)tile * g.T + tf) * SWEEP_NP + p0;
+        float4 hi[4], lo[4], L[4];
+        float rh[4], rl[4];
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+            hi[q] = lo[q] = L[q] = make_float4(0.f, 0.f, 0.f, 0.f);
+            rh[q] = rl[q] = 0.0f;
+            int i, j, k;
+            if (!entry_cell(g, c.I, tile, tf, p0 + q, i, j, k)) continue;
+            const long long t = (long long)i + (long long)c.I * (j + (long long)c.J * k);
+            if (!pb.fluid[t]) continue;
+            const double4_32a a = pb.Ad[t];
+            const double inv = pb.invdiagD[t], b = pb.b[t];
+            hi[q] = make_float4((float)a.x, (float)a.y, (float)a.z, (float)a.w);
+            lo[q] = make_float4((float)(a.x - (double)hi[q].x), (float)(a.y - (double)hi[q].y),
+                                (float)(a.z - (double)hi[q].z), (float)(a.w - (double)hi[q].w));
+            if (inv != 0.0) L[q] = make_float4((float)inv, (float)(a.y * inv), (float)(a.z * inv), (float)(a.w * inv));
+            rh[q] = (float)b;
+            rl[q] = (float)(b - (double)rh[q]);
+        }
+        const long long n = pb.nsl + SWEEP_NP;   // the planes' stride
+        auto put = [&](float *p, float v0, float v1, float v2, float v3) {
+            *reinterpret_cast<float4 *>(p + e) = make_float4(v0, v1, v2, v3);
+        };
+#pragma unroll
+        for (int q = 0; q < 4; q++) pb.L[e + q] = L[q];
+        put(pb.A, hi[0].x, hi[1].x, hi[2].x, hi[3].x);
+        put(pb.A + n, hi[0].y, hi[1].y, hi[2].y, hi[3].y);
+        put(pb.A + 2 * n, hi[0].z, hi[1].z, hi[2].z, hi[3].z);
+        put(pb.A + 3 * n, hi[0].w, hi[1].w, hi[2].w, hi[3].w);
+        put(pb.A + 4 * n, lo[0].x, lo[1].x, lo[2].x, lo[3].x);
+        put(pb.A + 5 * n, lo[0].y, lo[1].y, lo[2].y, lo[3].y);
+        put(pb.A + 6 * n, lo[0].z, lo[1].z, lo[2].z, lo[3].z);
+        put(pb.A + 7 * n, lo[0].w, lo[1].w, lo[2].w, lo[3].w);
+        put(pb.rh, rh[0], rh[1], rh[2], rh[3]);
+        put(pb.rl, rl[0], rl[1], rl[2], rl[3]);
+        put(pb.xh, 0.f, 0.f, 0.f, 0.f);
+        put(pb.xl, 0.f, 0.f, 0.f, 0.f);
+        put(pb.s, 0.f, 0.f, 0.f, 0.f);
+    }
+}
+
+// Sum over a CTA of TPB threads in a fixed order; thread 0 has the result.
+// FP64 runs at 2 lanes a clock on this GPU, so the tree's first steps go
+// through shared memory in one warp (12 FP64 instructions a CTA; shuffles in
+// every warp took 48).
+__device__ __forceinline__ double block_sum(double v, double *sh) {
+    sh[threadIdx.x] = v;
     __syncthreads();
-    T s = 0;
-    if (threadIdx.x == 0)
-        for (int q = 0; q < (int)(blockDim.x >> 5); q++) s += sh[q];
+    double s = 0.0;
+    if (threadIdx.x < 32) {
+        double w[TPB / 32];
+#pragma unroll
+        for (int q = 0; q < TPB / 32; q++) w[q] = sh[threadIdx.x + 32 * q];
+#pragma unroll
+        for (int m = TPB / 64; m > 0; m >>= 1)
+#pragma unroll
+            for (int q = 0; q < m; q++) w[q] += w[q + m];
+        s = w[0];
+        for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    }
     __syncthreads();
     return s;
 }
-
+// Max of non-negative floats over the CTA, a NaN counting as +inf, then one
+// atomic on the bits of the double.
+__device__ __forceinline__ void block_max_float_to(float v, unsigned long long *out) {
+    __shared__ unsigned shm[TPB / 32];
+    unsigned m = __reduce_max_sync(0xffffffffu, v != v ? 0x7f800000u : __float_as_uint(v));
+    if ((threadIdx.x & 31) == 0) shm[threadIdx.x >> 5] = m;
+    __syncthreads();
+    if (threadIdx.x < 32) {
+        m = __reduce_max_sync(0xffffffffu, threadIdx.x < TPB / 32 ? shm[threadIdx.x] : 0u);
+        if (threadIdx.x == 0 && m) atomicMax(out, (unsigned long long)__double_as_longlong((double)__uint_as_float(m)));
+    }
+}
 
 // Each CTA of a reduction takes a ticket once its partial (or atomic) is
 // out; the CTA that takes the last one then sees all of them and finishes the
 // reduction, and resets the ticket for the next launch.  One launch instead
 // of a producer and a one-CTA consumer.
-__device__ __forceinline__ bool last_cta(unsigned int *ticket) {
+__device__ __forceinline__ bool last_cta(unsigned int *ticket, unsigned int ctas) {
     __shared__ int amLast;
     __syncthreads();
     if (threadIdx.x == 0) {
         __threadfence();
-        amLast = atomicAdd(ticket, 1u) == gridDim.x - 1;
+        amLast = atomicAdd(ticket, 1u) == ctas - 1;
         if (amLast) {
             *ticket = 0u;
             __threadfence();
@@ -469,22 +566,15 @@ __device__ __forceinline__ double bits_to_resid(const unsigned long long *p) {
     return __longlong_as_double((long long)__ldcg(p));
 }
 
-// The reductions below run on a fixed grid per context (nPartials CTAs,
-// pressure_partials_for) with grid-stride loops: each thread sums its rows
-// in a fixed order, each CTA writes one partial, and the last CTA adds the
-// partials in a fixed order, so every sum is deterministic and the FP64
-// reduction work is per thread, not per row.
-
-// the rows of the system as a list: flat index and sweep-layout index
-__global__ void k_compact_rows(StepConsts c, SweepLayout g, const uint8_t *fluid, const int *pos, int *idx, int *sk) {
-    long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= (long long)c.I * c.J * c.K || !fluid[t]) return;
-    int i, j, k;
-    unflatten(t, c.I, c.J, i, j, k);
-    const int e = pos[t];
-    idx[e] = (int)t;
-    sk[e] = (int)sweep_index(g, i, j, k);
-}
+// The row kernels below run over the items of the solve on a fixed grid per
+// context (pressure_row_grid CTAs): each thread sums its entries in a fixed
+// order, each CTA writes one partial, and the last CTA adds the partials in a
+// fixed order, so every sum is deterministic.  Entries without a row hold
+// zeros.  The vectors live in the sweep layout: a warp takes one step of a
+// tile, whose entries are contiguous, and a row's six neighbours are entries
+// of the steps before and after it, so loads are 16-byte and coalesced (a row
+// list in cell order gathered every neighbour on its own: 17.7, 15.0 and 13.5
+// us for the three kernels at 518k rows).
 
 // Double-float arithmetic on the FP32 pipe (this GPU's FP64 rate is ~1/64
 // of FP32): a coefficient a = hi + lo (floats, exact to 48 bits) times an
@@ -516,15 +606,67 @@ __device__ __forceinline__ float2 df_scale(float f, float2 v) {
     const float pl = __fmaf_rn(f, v.y, __fmaf_rn(f, v.x, -ph));
     return make_float2(ph, pl);
 }
-__device__ __forceinline__ void df_mul_add(float ah, float al, float sv, float &sh, float &sl) {
-    const float ph = __fmul_rn(ah, sv);
-    float pl = __fmaf_rn(ah, sv, -ph);   // exact error of ah * sv
-    pl = __fmaf_rn(al, sv, pl);
-    const float t = __fadd_rn(sh, ph);
-    const float bb = __fsub_rn(t, sh);
-    const float err = __fadd_rn(__fsub_rn(sh, __fsub_rn(t, bb)), __fsub_rn(ph, bb));   // exact error of sh + ph
-    sl = __fadd_rn(sl, __fadd_rn(err, pl));
+// Pairs of floats in one 64-bit register (two cells): each operation rounds
+// each half as the scalar one does.  Sums and products are written as fused
+// multiply-adds that are exact up to that one rounding (a b + 0, a 1 + b), so
+// the compiler cannot contract two operations into one.
+using F2 = unsigned long long;
+__device__ __forceinline__ F2 f2(float x, float y) {
+    F2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(x), "f"(y));
+    return r;
+}
+__device__ __forceinline__ float f2_x(F2 v) { return __uint_as_float((unsigned)v); }
+__device__ __forceinline__ float f2_y(F2 v) { return __uint_as_float((unsigned)(v >> 32)); }
+__device__ __forceinline__ F2 f2_fma(F2 a, F2 b, F2 c) {
+    F2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+constexpr F2 F2_ONE = 0x3f8000003f800000ull, F2_MINUS = 0xbf800000bf800000ull, F2_ZERO = 0x8000000080000000ull;   // -0
+__device__ __forceinline__ F2 f2_add(F2 a, F2 b) { return f2_fma(a, F2_ONE, b); }
+__device__ __forceinline__ F2 f2_sub(F2 a, F2 b) { return f2_fma(b, F2_MINUS, a); }
+__device__ __forceinline__ F2 f2_mul(F2 a, F2 b) { return f2_fma(a, b, F2_ZERO); }
+// (sh, sl) += (ah, al) s for two cells, ns = -s: the leading product exact as
+// its rounded value plus its FMA-recovered error, the sum's rounding error by
+// Knuth's TwoSum
+__device__ __forceinline__ void df2_mul_add(F2 ah, F2 al, F2 sv, F2 ns, F2 &sh, F2 &sl) {
+    const F2 nph = f2_mul(ah, ns);                        // -(ah s) rounded
+    const F2 pl = f2_fma(al, sv, f2_fma(ah, sv, nph));   // its error, plus al s
+    const F2 t = f2_sub(sh, nph);
+    const F2 bb = f2_sub(t, sh);
+    const F2 err = f2_sub(f2_sub(sh, f2_sub(t, bb)), f2_add(nph, bb));   // exact error of the sum
+    sl = f2_add(sl, f2_add(err, pl));
     sh = t;
+}
+// df_norm, df_add and df_scale for two cells
+__device__ __forceinline__ void df2_norm(F2 h, F2 l, F2 &oh, F2 &ol) {
+    oh = f2_add(h, l);
+    ol = f2_sub(l, f2_sub(oh, h));
+}
+__device__ __forceinline__ void df2_add(F2 ah, F2 al, F2 bh, F2 bl, F2 &oh, F2 &ol) {
+    const F2 t = f2_add(ah, bh);
+    const F2 bb = f2_sub(t, ah);
+    const F2 err = f2_add(f2_sub(ah, f2_sub(t, bb)), f2_sub(bh, bb));
+    df2_norm(t, f2_add(err, f2_add(al, bl)), oh, ol);
+}
+__device__ __forceinline__ void df2_scale(F2 f, F2 nf, F2 vh, F2 vl, F2 &oh, F2 &ol) {   // nf = -f
+    oh = f2_mul(f, vh);
+    ol = f2_fma(f, vl, f2_sub(F2_ZERO, f2_fma(nf, vh, oh)));
+}
+__device__ __forceinline__ void ld2x2(const float *p, F2 (&v)[2]) {
+    const ulonglong2 q = *reinterpret_cast<const ulonglong2 *>(p);
+    v[0] = q.x; v[1] = q.y;
+}
+__device__ __forceinline__ void st2x2(float *p, const F2 (&v)[2]) {
+    *reinterpret_cast<ulonglong2 *>(p) = make_ulonglong2(v[0], v[1]);
+}
+__device__ __forceinline__ void ld4(const float *p, float (&v)[4]) {
+    const float4 q = *reinterpret_cast<const float4 *>(p);
+    v[0] = q.x; v[1] = q.y; v[2] = q.z; v[3] = q.w;
+}
+__device__ __forceinline__ void st4(float *p, const float (&v)[4]) {
+    *reinterpret_cast<float4 *>(p) = make_float4(v[0], v[1], v[2], v[3]);
 }
 
 // s = z + beta s (pcgsolver.h:295-298, beta rounded to float) fused with
@@ -532,55 +674,121 @@ __device__ __forceinline__ void df_mul_add(float ah, float al, float sv, float &
 // double-float per thread and in FP64 across threads.  The new s of a row's
 // stencil is formed from the previous iteration's buffer sIn (so no row
 // reads a value another thread is writing) and the row's own goes to sOut.
-// z is read in cell order (zc, written by the z.r pass before it).  In the
-// first iteration beta = 0 and sIn = 0, so s = z.  A neighbour that
-// is not a row couples with 0 and takes s = 0.  The last CTA sums s.q and
-// sets alpha = rho / s.q, rounded to float as BLAS::addScaled takes it
-// (blaswrapper.h:129-158), and clears the iteration's residual norms.
-__global__ void k_spmv_s(StepConsts c, const int *__restrict__ rows,
-                         const int *nRows, const float4 *__restrict__ A2, const float *__restrict__ z,
-                         const float *__restrict__ sIn, float *__restrict__ sOut, float2 *__restrict__ q,
-                         double *partials, double *scal, unsigned long long *rmaxBits, PcgCtl *ctl) {
-    __shared__ double sh[32];
-    if (ctl->done) return;
-    const int n = *nRows;
-    const float beta = (float)scal[5];   // exact: beta is a float value
-    const long long sy = c.I, sz = (long long)c.I * c.J;
-    float2 dot = make_float2(0.0f, 0.0f);
-    for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < n; e += gridDim.x * blockDim.x) {
-        const long long t = rows[e];
-        const float4 hi = A2[2 * t], lo = A2[2 * t + 1];
-        const float4 hxm = A2[2 * (t - 1)], lxm = A2[2 * (t - 1) + 1];
-        const float4 hym = A2[2 * (t - sy)], lym = A2[2 * (t - sy) + 1];
-        const float4 hzm = A2[2 * (t - sz)], lzm = A2[2 * (t - sz) + 1];
-        // the search direction over the stencil's rows
-        auto snew = [&](bool row, long long tn) {
-            return row ? __fmaf_rn(beta, sIn[tn], z[tn]) : 0.0f;
+// In the first iteration beta = 0 and sIn = 0, so s = z.  A neighbour that
+// is not a row couples with 0 (its entry holds a finite value); one outside
+// the layout is the zero padding after it.  A thread takes four consecutive
+// pencils of a step, two to a packed operation: along a, the neighbours of
+// three of them are in its own vectors of the steps before and after, the
+// fourth's is one word more.  The last CTA sums s.q and sets alpha = rho / s.q,
+// rounded to float as BLAS::addScaled takes it (blaswrapper.h:129-158), and
+// clears the iteration's residual norms.
+template <bool SWAP>
+__global__ void __launch_bounds__(TPB, 3)
+    k_spmv_s(SweepLayout g, long long nsl, const int *__restrict__ items, const int *__restrict__ nItems,
+             const float *__restrict__ A, const float *__restrict__ z, const float *__restrict__ sIn,
+             float *__restrict__ sOut, float *__restrict__ qh, float *__restrict__ ql, double *partials, double *scal,
+             unsigned long long *rmaxBits, PcgCtl *ctl) {
+    __shared__ double sh[TPB];
+    const int n = *nItems, T = g.T, nch = T / SWEEP_CH, ctas = min((int)gridDim.x, n);
+    pdl_wait();
+    pdl_trigger();
+    if (ctl->done || (int)blockIdx.x >= n) return;
+    const float betaf = (float)scal[5];   // exact: beta is a float value
+    const F2 beta = f2(betaf, betaf);
+    constexpr int NP = SWEEP_NP;
+    const long long np = nsl + NP;        // stride of the planes of A
+    const float *Xh = A + np, *Xl = A + 5 * np;
+    const float *Ah = A + (SWAP ? 3 : 2) * np, *Al = A + (SWAP ? 7 : 6) * np;   // couplings along a
+    const float *Bh = A + (SWAP ? 2 : 3) * np, *Bl = A + (SWAP ? 6 : 7) * np;   // and along b
+    const int p0 = (threadIdx.x & 31) * 4, la0 = p0 & 7, lb = (p0 >> 3) & 3, wa = (p0 >> 5) & 1, wb = p0 >> 6;
+    F2 dotH = F2_ZERO, dotL = F2_ZERO;
+    for (int it = blockIdx.x; it < n; it += gridDim.x) {
+        const int item = items[it], tile = item / nch, tf = item % nch * SWEEP_CH + (threadIdx.x >> 5);
+        const int ta = tile % g.nta, tb = tile / g.nta;
+        const long long e = ((long long)tile * T + tf) * NP + p0, none = nsl + p0;
+        // entries of the neighbours: the steps after and before; a+ of the last
+        // pencil and a- of the first; b+ and b- of all four
+        const long long eU = tf + 1 < T ? e + NP : none, eD = tf > 0 ? e - NP : none;
+        long long eaU, eaD, ebU, ebD;
+        if (la0 == 0) eaU = eU + 4;
+        else if (wa == 0) eaU = tf + 1 < T ? eU + 28 : none;
+        else eaU = ta + 1 < g.nta && tf >= SWEEP_WA - 1 ? e + ((long long)T - (SWEEP_WA - 1)) * NP - 36 : none;
+        if (la0 != 0) eaD = eD - 1;
+        else if (wa == 1) eaD = tf > 0 ? eD - 25 : none;
+        else eaD = ta > 0 && tf + SWEEP_WA - 1 < T ? e - ((long long)T - (SWEEP_WA - 1)) * NP + 39 : none;
+        if (lb < 3) ebU = tf + 1 < T ? eU + 8 : none;
+        else if (wb == 0) ebU = tf + 1 < T ? eU + 40 : none;
+        else ebU = tb + 1 < g.ntb && tf >= SWEEP_WB - 1 ? e + ((long long)T * g.nta - (SWEEP_WB - 1)) * NP - 88 : none;
+        if (lb > 0) ebD = tf > 0 ? eD - 8 : none;
+        else if (wb == 1) ebD = tf > 0 ? eD - 40 : none;
+        else ebD = tb > 0 && tf + SWEEP_WB - 1 < T ? e - ((long long)T * g.nta - (SWEEP_WB - 1)) * NP + 88 : none;
+        auto snew = [&](long long at, F2 (&v)[2]) {
+            F2 zz[2], ss[2];
+            ld2x2(z + at, zz);
+            ld2x2(sIn + at, ss);
+            v[0] = f2_fma(beta, ss[0], zz[0]);
+            v[1] = f2_fma(beta, ss[1], zz[1]);
         };
-        const float st = snew(true, t);
-        const float sxp = snew(hi.y != 0.0f || lo.y != 0.0f, t + 1);
-        const float syp = snew(hi.z != 0.0f || lo.z != 0.0f, t + sy);
-        const float szp = snew(hi.w != 0.0f || lo.w != 0.0f, t + sz);
-        const float sxm = snew(hxm.y != 0.0f || lxm.y != 0.0f, t - 1);
-        const float sym = snew(hym.z != 0.0f || lym.z != 0.0f, t - sy);
-        const float szm = snew(hzm.w != 0.0f || lzm.w != 0.0f, t - sz);
-        sOut[t] = st;
-        float accH = 0.0f, accL = 0.0f;
-        df_mul_add(hi.x, lo.x, st, accH, accL);
-        df_mul_add(hi.y, lo.y, sxp, accH, accL);
-        df_mul_add(hi.z, lo.z, syp, accH, accL);
-        df_mul_add(hi.w, lo.w, szp, accH, accL);
-        df_mul_add(hxm.y, lxm.y, sxm, accH, accL);
-        df_mul_add(hym.z, lym.z, sym, accH, accL);
-        df_mul_add(hzm.w, lzm.w, szm, accH, accL);
-        const float2 qt = df_norm(accH, accL);
-        q[t] = qt;
-        dot = df_add(dot, df_scale(st, qt));
+        F2 accH[2] = {F2_ZERO, F2_ZERO}, accL[2] = {F2_ZERO, F2_ZERO};
+        auto couple = [&](const F2 (&h)[2], const F2 (&l)[2], const F2 (&v)[2]) {
+#pragma unroll
+            for (int q = 0; q < 2; q++) df2_mul_add(h[q], l[q], v[q], f2_mul(v[q], F2_MINUS), accH[q], accL[q]);
+        };
+        F2 s0[2], sU[2], sD[2] = {0, 0}, h[2], l[2], v[2];
+        snew(e, s0);
+        snew(eU, sU);
+        const float saU = __fmaf_rn(betaf, sIn[eaU], z[eaU]), saD = __fmaf_rn(betaf, sIn[eaD], z[eaD]);
+        ld2x2(A + e, h); ld2x2(A + 4 * np + e, l);
+        couple(h, l, s0);
+        ld2x2(Xh + e, h); ld2x2(Xl + e, l);
+        couple(h, l, sU);   // +x
+        auto plusA = [&] {
+            ld2x2(Ah + e, h); ld2x2(Al + e, l);
+            v[0] = f2(f2_y(sU[0]), f2_x(sU[1]));
+            v[1] = f2(f2_y(sU[1]), saU);
+            couple(h, l, v);
+        };
+        auto plusB = [&] {
+            ld2x2(Bh + e, h); ld2x2(Bl + e, l);
+            snew(ebU, v);
+            couple(h, l, v);
+        };
+        auto minusA = [&] {
+            F2 ch[2], cl[2];
+            ld2x2(Ah + eD, ch); ld2x2(Al + eD, cl);
+            h[0] = f2(Ah[eaD], f2_x(ch[0])); h[1] = f2(f2_y(ch[0]), f2_x(ch[1]));
+            l[0] = f2(Al[eaD], f2_x(cl[0])); l[1] = f2(f2_y(cl[0]), f2_x(cl[1]));
+            v[0] = f2(saD, f2_x(sD[0]));
+            v[1] = f2(f2_y(sD[0]), f2_x(sD[1]));
+            couple(h, l, v);
+        };
+        auto minusB = [&] {
+            ld2x2(Bh + ebD, h); ld2x2(Bl + ebD, l);
+            snew(ebD, v);
+            couple(h, l, v);
+        };
+        // +y, +z, then -x, -y, -z
+        if (SWAP) { plusB(); plusA(); } else { plusA(); plusB(); }
+        snew(eD, sD);
+        ld2x2(Xh + eD, h); ld2x2(Xl + eD, l);
+        couple(h, l, sD);
+        if (SWAP) { minusB(); minusA(); } else { minusA(); minusB(); }
+        F2 oh[2], ol[2];
+#pragma unroll
+        for (int q = 0; q < 2; q++) {
+            df2_norm(accH[q], accL[q], oh[q], ol[q]);
+            F2 ph, pl;
+            df2_scale(s0[q], f2_mul(s0[q], F2_MINUS), oh[q], ol[q], ph, pl);
+            df2_add(dotH, dotL, ph, pl, dotH, dotL);
+        }
+        st2x2(sOut + e, s0);
+        st2x2(qh + e, oh);
+        st2x2(ql + e, ol);
     }
-    double b = block_sum(df_to(dot), sh);
+    double b = block_sum(df_to(make_float2(f2_x(dotH), f2_x(dotL))) + df_to(make_float2(f2_y(dotH), f2_y(dotL))), sh);
     if (threadIdx.x == 0) partials[blockIdx.x] = b;
-    if (last_cta(&ctl->ticket[0])) {
-        const double sq = sum_partials_fixed(partials, gridDim.x, sh);
+    if (last_cta(&ctl->ticket[0], ctas)) {
+        const double sq = sum_partials_fixed(partials, ctas, sh);
         if (threadIdx.x == 0) {
             scal[0] = sq;
             scal[4] = (double)(float)(scal[3] / sq);
@@ -592,27 +800,39 @@ __global__ void k_spmv_s(StepConsts c, const int *__restrict__ rows,
 
 // rho_new = z.r.  The last CTA sums it; inside the loop (inLoop) it also
 // sets beta = rho_new / rho as float (pcgsolver.h:295-298) and ends the
-// iteration: rho = rho_new, next iteration index.  Each row's z, gathered
-// from the sweep layout, is also stored in cell order, so that the SpMV's
-// stencil reads of z are coalesced.
-__global__ void k_dot_zr(const int *__restrict__ rows, const int *__restrict__ rowsSk, const int *nRows,
-                         const float *__restrict__ z, float *__restrict__ zc, const float2 *__restrict__ r,
-                         double *partials, double *scal,
-                         PcgCtl *ctl, int inLoop) {
-    __shared__ double sh[32];
-    if (ctl->done) return;
-    const int n = *nRows;
+// iteration: rho = rho_new, next iteration index.
+__global__ void __launch_bounds__(TPB) k_dot_zr(const int *__restrict__ items, const int *__restrict__ nItems,
+                                                const float *__restrict__ z, const float *__restrict__ rh,
+                                                const float *__restrict__ rl, double *partials, double *scal,
+                                                PcgCtl *ctl, int inLoop) {
+    __shared__ double sh[TPB];
+    const int n = *nItems;
     float2 dot = make_float2(0.0f, 0.0f);   // double-float per thread, FP64 across threads
-    for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < n; e += gridDim.x * blockDim.x) {
-        const int t = rows[e];
-        const float zt = z[rowsSk[e]];
-        zc[t] = zt;   // z in cell order, where the SpMV reads its stencil
-        dot = df_add(dot, df_scale(zt, r[t]));
+    float h[4], l[4];
+    auto entry = [&](int it) { return (long long)items[it] * (SWEEP_CH * SWEEP_NP) + threadIdx.x * 4; };
+    const int ctas = min((int)gridDim.x, n);
+    if ((int)blockIdx.x < n) {   // r does not depend on the sweeps
+        ld4(rh + entry(blockIdx.x), h);
+        ld4(rl + entry(blockIdx.x), l);
+    }
+    pdl_wait();
+    pdl_trigger();
+    if (ctl->done || (int)blockIdx.x >= n) return;
+    for (int it = blockIdx.x; it < n; it += gridDim.x) {
+        const long long e = entry(it);
+        float zv[4];
+        ld4(z + e, zv);
+        if (it != (int)blockIdx.x) {
+            ld4(rh + e, h);
+            ld4(rl + e, l);
+        }
+#pragma unroll
+        for (int q = 0; q < 4; q++) dot = df_add(dot, df_scale(zv[q], make_float2(h[q], l[q])));
     }
     double s = block_sum(df_to(dot), sh);
     if (threadIdx.x == 0) partials[blockIdx.x] = s;
-    if (last_cta(&ctl->ticket[1])) {
-        const double zr = sum_partials_fixed(partials, gridDim.x, sh);
+    if (last_cta(&ctl->ticket[1], ctas)) {
+        const double zr = sum_partials_fixed(partials, ctas, sh);
         if (threadIdx.x == 0) {
             scal[1] = zr;
             if (inLoop) {
@@ -645,25 +865,50 @@ __device__ __forceinline__ void convergence_test(PcgCtl *ctl, double resid, doub
 // x += alpha s, r -= alpha q with alpha = rho / s.q passed on as float, as
 // BLAS::addScaled(float alpha, ...) does (blaswrapper.h:129-158); |r|inf,
 // tested by the last CTA except on the iterations of the periodic recompute
-__global__ void k_update_xr(const int *__restrict__ rows, const int *__restrict__ rowsSk, const int *nRows,
-                            float2 *__restrict__ x, float2 *__restrict__ r, float *__restrict__ rf,
-                            const float *__restrict__ s, const float2 *__restrict__ q, const double *scal,
-                            unsigned long long *rmaxBits, PcgCtl *ctl) {
-    if (ctl->done) return;
-    const int n = *nRows;
+__global__ void __launch_bounds__(TPB) k_update_xr(const int *__restrict__ items, const int *__restrict__ nItems,
+                                                   float *__restrict__ xh, float *__restrict__ xl,
+                                                   float *__restrict__ rh, float *__restrict__ rl,
+                                                   const float *__restrict__ s, const float *__restrict__ qh,
+                                                   const float *__restrict__ ql, const double *scal,
+                                                   unsigned long long *rmaxBits, PcgCtl *ctl,
+                                                   unsigned int *sweepTicket) {
+    const int n = *nItems;
+    float vxh[4], vxl[4], vrh[4], vrl[4];
+    auto entry = [&](int it) { return (long long)items[it] * (SWEEP_CH * SWEEP_NP) + threadIdx.x * 4; };
+    auto load_xr = [&](long long e) {
+        ld4(xh + e, vxh); ld4(xl + e, vxl);
+        ld4(rh + e, vrh); ld4(rl + e, vrl);
+    };
+    if ((int)blockIdx.x < n) load_xr(entry(blockIdx.x));   // the SpMV before does not touch them
+    pdl_wait();
+    pdl_trigger();
+    if (blockIdx.x == 0 && threadIdx.x == 0) sweep_prep(sweepTicket);   // for the sweep pair that follows
+    if (ctl->done || (int)blockIdx.x >= n) return;
+    const int ctas = min((int)gridDim.x, n);
     const float alpha = (float)scal[4];   // exact: alpha is a float value
     float m = 0.0f;
-    for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < n; e += gridDim.x * blockDim.x) {
-        const int t = rows[e];
-        x[t] = df_add(x[t], df_scale(alpha, make_float2(s[t], 0.0f)));   // alpha s is exact as a pair
-        const float2 rv = df_add(r[t], df_scale(-alpha, q[t]));
-        r[t] = rv;
-        rf[rowsSk[e]] = rv.x;   // normalised: the pair rounded to float
-        const float av = fabsf(rv.x);
-        m = (av != av || av > m) ? av : m;   // a NaN sticks
+    for (int it = blockIdx.x; it < n; it += gridDim.x) {
+        const long long e = entry(it);
+        float vs[4], vqh[4], vql[4];
+        if (it != (int)blockIdx.x) load_xr(e);
+        ld4(s + e, vs); ld4(qh + e, vqh); ld4(ql + e, vql);
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            const float2 xv = df_add(make_float2(vxh[k], vxl[k]),
+                                     df_scale(alpha, make_float2(vs[k], 0.0f)));   // alpha s is exact as a pair
+            const float2 rv = df_add(make_float2(vrh[k], vrl[k]), df_scale(-alpha, make_float2(vqh[k], vql[k])));
+            vxh[k] = xv.x;
+            vxl[k] = xv.y;
+            vrh[k] = rv.x;   // normalised: the pair rounded to float, the sweeps' right-hand side
+            vrl[k] = rv.y;
+            const float av = fabsf(rv.x);
+            m = (av != av || av > m) ? av : m;   // a NaN sticks
+        }
+        st4(xh + e, vxh); st4(xl + e, vxl);
+        st4(rh + e, vrh); st4(rl + e, vrl);
     }
-    block_max_to((double)m, rmaxBits);
-    if (last_cta(&ctl->ticket[2]) && threadIdx.x == 0 && (ctl->it + 1) % 25 != 0)
+    block_max_float_to(m, rmaxBits);
+    if (last_cta(&ctl->ticket[2], ctas) && threadIdx.x == 0 && (ctl->it + 1) % 25 != 0)
         convergence_test(ctl, bits_to_resid(rmaxBits), scal[6], false);
 }
 
@@ -672,61 +917,70 @@ __global__ void k_update_xr(const int *__restrict__ rows, const int *__restrict_
 // (pcgsolver.h's periodic recompute, here before the test) and when the
 // recurrence just claimed convergence (a claim is only made on the other
 // iterations, so one launch serves both); never once converged.
-__global__ void k_true_residual(StepConsts c, const int *__restrict__ rows, const int *__restrict__ rowsSk,
-                                const int *nRows, const double4_32a *__restrict__ Ad, const double *__restrict__ b,
-                                const float2 *__restrict__ x, float2 *__restrict__ r, float *__restrict__ rf,
-                                unsigned long long *rmaxBits, const double *scal, PcgCtl *ctl,
-                                unsigned int *sweepTicket) {
-    if (blockIdx.x == 0 && threadIdx.x == 0) sweep_prep(sweepTicket);   // for the sweep pair that follows
+__global__ void __launch_bounds__(TPB) k_true_residual(StepConsts c, SweepLayout g, const int *__restrict__ items,
+                                                       const int *__restrict__ nItems,
+                                                       const uint8_t *__restrict__ fluid,
+                                                       const double4_32a *__restrict__ Ad, const double *__restrict__ b,
+                                                       const float *__restrict__ xh, const float *__restrict__ xl,
+                                                       float *__restrict__ rh, float *__restrict__ rl,
+                                                       unsigned long long *rmaxBits, const double *scal, PcgCtl *ctl) {
+    pdl_wait();
+    pdl_trigger();
     if (ctl->done) return;
     if ((ctl->it + 1) % 25 != 0 && !ctl->claim) return;
-    const int n = *nRows;
+    const int n = *nItems, nch = g.T / SWEEP_CH;
     const long long sy = c.I, sz = (long long)c.I * c.J;
     double m = 0.0;
-    for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < n; e += gridDim.x * blockDim.x) {
-        const long long t = rows[e];
+    for (long long w = (long long)blockIdx.x * TPB + threadIdx.x; w < (long long)n * (SWEEP_CH * SWEEP_NP);
+         w += (long long)gridDim.x * TPB) {
+        const int item = items[w / (SWEEP_CH * SWEEP_NP)], in = (int)(w % (SWEEP_CH * SWEEP_NP));
+        const int tile = item / nch, tf = item % nch * SWEEP_CH + in / SWEEP_NP, p = in % SWEEP_NP;
+        int i, j, k;
+        if (!entry_cell(g, c.I, tile, tf, p, i, j, k)) continue;
+        const long long t = i + sy * j + sz * k;
+        if (!fluid[t]) continue;
+        const long long e = ((long long)tile * g.T + tf) * SWEEP_NP + p;
+        // x at the row and, where they are rows, at its neighbours
+        auto xat = [&](bool row, int ni, int nj, int nk) {
+            if (!row) return 0.0;
+            const long long en = sweep_index(g, ni, nj, nk);
+            return df_to(make_float2(xh[en], xl[en]));
+        };
         const double4_32a a = Ad[t];
-        double ax = a.x * df_to(x[t]);
-        ax = fma(a.y, df_to(x[t + 1]), ax);
-        ax = fma(a.z, df_to(x[t + sy]), ax);
-        ax = fma(a.w, df_to(x[t + sz]), ax);
-        ax = fma(Ad[t - 1].y, df_to(x[t - 1]), ax);
-        ax = fma(Ad[t - sy].z, df_to(x[t - sy]), ax);
-        ax = fma(Ad[t - sz].w, df_to(x[t - sz]), ax);
+        double ax = a.x * df_to(make_float2(xh[e], xl[e]));
+        ax = fma(a.y, xat(fluid[t + 1], i + 1, j, k), ax);
+        ax = fma(a.z, xat(fluid[t + sy], i, j + 1, k), ax);
+        ax = fma(a.w, xat(fluid[t + sz], i, j, k + 1), ax);
+        if (fluid[t - 1]) ax = fma(Ad[t - 1].y, xat(true, i - 1, j, k), ax);
+        if (fluid[t - sy]) ax = fma(Ad[t - sy].z, xat(true, i, j - 1, k), ax);
+        if (fluid[t - sz]) ax = fma(Ad[t - sz].w, xat(true, i, j, k - 1), ax);
         const double rv = b[t] - ax;
         const float2 rp = df_from(rv);
-        r[t] = rp;
-        rf[rowsSk[e]] = rp.x;
+        rh[e] = rp.x;
+        rl[e] = rp.y;
         const double av = fabs(rv);
         m = (av != av || av > m) ? av : m;
     }
     block_max_to(m, rmaxBits);
-    if (last_cta(&ctl->ticket[3]) && threadIdx.x == 0) convergence_test(ctl, bits_to_resid(rmaxBits), scal[6], true);
+    if (last_cta(&ctl->ticket[3], gridDim.x) && threadIdx.x == 0) convergence_test(ctl, bits_to_resid(rmaxBits), scal[6], true);
 }
 
-// r = b (and its FP32 copy in the sweep layout), x = 0, |b|inf
-__global__ void k_init_r(StepConsts c, SweepLayout g, const double *b, float2 *r, float *rf, float2 *x,
-                         unsigned long long *rmaxBits, unsigned int *sweepTicket) {
-    const long long n = (long long)c.I * c.J * c.K;
-    if (blockIdx.x == 0 && threadIdx.x == 0) sweep_prep(sweepTicket);   // for the first sweep pair
-    double m = 0.0;
-#pragma unroll 4
-    for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < n; t += (long long)gridDim.x * blockDim.x) {
-        r[t] = df_from(b[t]);
-        x[t] = make_float2(0.0f, 0.0f);
-        int i, j, k;
-    unflatten(t, c.I, c.J, i, j, k);
-        if (i >= 1 && j >= 1 && k >= 1 && i <= c.I - 2 && j <= c.J - 2 && k <= c.K - 2)
-            rf[sweep_index(g, i, j, k)] = (float)b[t];
-        double av = fabs(b[t]);
-        m = (av != av || av > m) ? av : m;
+// The solution to a float per cell (zero off the rows: cleared before).
+__global__ void __launch_bounds__(TPB) k_x_to_cells(StepConsts c, SweepLayout g, const int *items, const int *nItems,
+                                                    const uint8_t *fluid, const float *xh, const float *xl, float *P) {
+    const int nch = g.T / SWEEP_CH;
+    for (int it = blockIdx.x; it < *nItems; it += gridDim.x) {
+        const int item = items[it], tile = item / nch;
+        for (int in = threadIdx.x; in < SWEEP_CH * SWEEP_NP; in += TPB) {
+            const int tf = item % nch * SWEEP_CH + in / SWEEP_NP, p = in % SWEEP_NP;
+            int i, j, k;
+            if (!entry_cell(g, c.I, tile, tf, p, i, j, k)) continue;
+            const long long t = (long long)i + (long long)c.I * (j + (long long)c.J * k);
+            if (!fluid[t]) continue;
+            const long long e = ((long long)tile * g.T + tf) * SWEEP_NP + p;
+            P[t] = (float)df_to(make_float2(xh[e], xl[e]));
+        }
     }
-    block_max_to(m, rmaxBits);
-}
-
-__global__ void k_x_to_float(long long n, const float2 *x, float *p) {
-    long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t < n) p[t] = (float)df_to(x[t]);
 }
 
 // _applyPressureToVelocityFieldThread (pressuresolver.cpp:896-1046) without
@@ -791,13 +1045,18 @@ int cuda_fail(cudaError_t e, const char *what, std::string *msg) {
 }  // namespace
 
 int mic0_factor_tiles(int J, int K) { return std::max(1, (J - 2 + FT - 1) / FT) * std::max(1, (K - 2 + FT - 1) / FT); }
-// One reduction CTA per `cellsPerCta` grid cells (4096 by default), at most
-// RBLOCKS.  A liquid fills a fraction of the grid, so a thread takes a few
-// rows; a smaller grid spares the GPU's CTA dispatch, which many scenes
-// running at once share.
+// One CTA of the row kernels per `cellsPerCta` grid cells (4096 by default),
+// at least 128 where there are as many items, at most RBLOCKS.  A liquid fills
+// a fraction of the grid, so a CTA takes one to three items of 1024 entries,
+// and CTAs beyond the items leave at once.  Twice as many CTAs: 128^3 frame
+// 11.66 against 11.53 ms, 16 scenes at once 16.56 against 16.35 ms (CTA
+// dispatch and reductions are shared limits); without the floor of 128, 64^3
+// frames take 3.40 against 3.30 ms.
 int pressure_partials_for(int I, int J, int K, int cellsPerCta) {
     static_assert(RBLOCKS == PCG_MAX_PARTIALS, "the partials buffer holds RBLOCKS sums");
-    return std::min((int)div_up((long long)I * J * K, std::max(cellsPerCta, 256)), RBLOCKS);
+    const long long items = sweep_items_max(I, J, K);
+    const long long ctas = std::max<long long>(div_up((long long)I * J * K, std::max(cellsPerCta, 256)), 128);
+    return (int)std::max(1LL, std::min({ctas, items, (long long)RBLOCKS}));
 }
 
 #define PCK(call)                                               \
@@ -874,7 +1133,7 @@ int pressure_project(const StepConsts &c, const PressureArgs &a, PressureBuffers
     std::memcpy(mail->levelRange, lr, sizeof(lr));
     PCK(cudaMemcpyAsync(pb.levelRange, mail->levelRange, sizeof(lr), cudaMemcpyHostToDevice, s));
     PCK(cudaMemsetAsync(pb.scal, 0, 8 * sizeof(double), s));
-    { FLIP_COUNT(1); k_flags<<<nb, TPB, 0, s>>>(c, a.phi, pb.fluid, pb.fluidFlag, pb.levelRange); }
+    { FLIP_COUNT(1); k_flags<<<div_up(n, FLAG_CELLS), TPB, 0, s>>>(c, a.phi, pb.fluid, pb.levelRange); }
     { FLIP_COUNT(1); k_build<<<nb, TPB, 0, s>>>(c, a.phi, a.wu, a.wv, a.ww, a.u, a.v, a.w, mf, pb); }
     PCK(cudaMemcpyAsync(mail->levelRange, pb.levelRange, 7 * sizeof(int), cudaMemcpyDeviceToHost, s));
     PCK(cudaMemcpyAsync(&mail->bmax, pb.scal + 2, sizeof(double), cudaMemcpyDeviceToHost, s));
@@ -907,25 +1166,26 @@ int pressure_project(const StepConsts &c, const PressureArgs &a, PressureBuffers
         const int cost1 = lag(klo, khi, SWEEP_WA, SWEEP_CA) + lag(jlo, jhi, SWEEP_WB, SWEEP_CB);
         int want = cost1 < cost0 ? 1 : (cost0 < cost1 ? 0 : pb.sl.swap);
         if (a.sweepOrientation == 0 || a.sweepOrientation == 1) want = a.sweepOrientation;
-        if (want != pb.sl.swap) {
-            pb.sl = sweep_layout(c.I, c.J, c.K, want);
-            // entries that hold no interior cell in the new orientation must read zero
-            PCK(cudaMemsetAsync(pb.L, 0, pb.nsl * sizeof(float4), s));
-            PCK(cudaMemsetAsync(pb.rf, 0, pb.nsl * sizeof(float), s));
-            PCK(cudaMemsetAsync(pb.z, 0, pb.nsl * sizeof(float), s));
-        }
+        if (want != pb.sl.swap) pb.sl = sweep_layout(c.I, c.J, c.K, want);
     }
-    // the rows as a list in cell order (a scan keeps it deterministic)
-    launch_scan_cells(pb.fluidFlag, (int)n, pb.fluidPos, pb.fluidScan, pb.nFluid, s);
-    { FLIP_COUNT(1); k_compact_rows<<<nb, TPB, 0, s>>>(c, pb.sl, pb.fluid, pb.fluidPos, pb.fluidIdx, pb.fluidSk); }
+    const SweepLayout sl = pb.sl;
+    const unsigned ib = (unsigned)std::max(1LL, std::min<long long>(sweep_items_max(c.I, c.J, c.K), RBLOCKS));   // item loops
+    launch_sweep_ranges(c, sl, pb.fluid, sw, s);
+    { FLIP_COUNT(1); k_items<<<1, 1024, 0, s>>>(sl, sw.range, pb.items, pb.nItems); }
 
-    // MIC(0) factor; the pivot weights go to q, r and x (as FP64 arrays),
-    // which the loop set-up rewrites
-    mic0_factor(c, pb.fluid, pb.Ad, pb.invdiagD, reinterpret_cast<double *>(pb.q), reinterpret_cast<double *>(pb.r),
-                reinterpret_cast<double *>(pb.x), pb.factorProgress, pb.factorTicket, sw.err,
+    // MIC(0) factor; the pivot weights go to A's buffer, which is filled after
+    // it: zero wherever no item of this solve writes a coupling
+    double *W = reinterpret_cast<double *>(pb.A);
+    mic0_factor(c, pb.fluid, pb.Ad, pb.invdiagD, W, W + n, W + 2 * n, pb.factorProgress, pb.factorTicket, sw.err,
                 sw.spinLimit ? sw.spinLimit : DEFAULT_SPIN_LIMIT, lo, hi, s);
-    { FLIP_COUNT(1); k_mic0_finalize<<<nb, TPB, 0, s>>>(c, pb.sl, pb.fluid, pb.Ad, pb.invdiagD, pb.L); }
-    launch_sweep_ranges(c, pb.sl, pb.fluid, sw, s);
+    PCK(cudaMemsetAsync(pb.A, 0, 8 * (pb.nsl + SWEEP_NP) * sizeof(float), s));
+    if (pb.stale) {   // entries off this solve's items are read (and multiplied by zero): finite values only
+        PCK(cudaMemsetAsync(pb.z, 0, (pb.nsl + SWEEP_NP) * sizeof(float), s));
+        PCK(cudaMemsetAsync(pb.s, 0, (pb.nsl + SWEEP_NP) * sizeof(float), s));
+        PCK(cudaMemsetAsync(pb.s2, 0, (pb.nsl + SWEEP_NP) * sizeof(float), s));
+    }
+    pb.stale = true;   // until this solve has converged
+    { FLIP_COUNT(1); k_layout<<<ib, TPB, 0, s>>>(c, sl, pb.items, pb.nItems, pb, sw.ticket); }
 
     unsigned long long *rmax = pb.rmaxBits;
     SweepTiming *tm = a.sweepTiming;
@@ -948,11 +1208,12 @@ int pressure_project(const StepConsts &c, const PressureArgs &a, PressureBuffers
     };
     // z = M^-1 r, then rho_new = z.r; with `timed` the sweeps sit between
     // event pair q (recorded as graph nodes when captured)
+    // (the kernels of an iteration overlap with the end of the one before each)
     auto precondition = [&](int q, bool timed) {
         if (timed) record(tm->ev[2 * q]);
-        launch_sweeps(c, pb.sl, pb.L, pb.rf, pb.z, sw, &pb.ctl->done, s, true);   // prepared by the kernel before
+        launch_sweeps(c, sl, pb.L, pb.rh, pb.z, sw, &pb.ctl->done, s, true, q > 0);   // prepared by a kernel before
         if (timed) record(tm->ev[2 * q + 1]);
-        { FLIP_COUNT(1); k_dot_zr<<<rb, TPB, 0, s>>>(pb.fluidIdx, pb.fluidSk, pb.nFluid, pb.z, pb.zc, pb.r, pb.partials, pb.scal, pb.ctl, q > 0); }
+        launch_after(true, k_dot_zr, rb, TPB, 0, s, pb.items, pb.nItems, pb.z, pb.rh, pb.rl, pb.partials, pb.scal, pb.ctl, q > 0);
     };
     // one PCG iteration (pcgsolver.h:263-300); every launch is the same for
     // every iteration but the search direction's two buffers, which swap
@@ -961,9 +1222,12 @@ int pressure_project(const StepConsts &c, const PressureArgs &a, PressureBuffers
     int sPar = 0;
     auto iteration = [&](int k, bool timed) {
         float *sIn = sPar ? pb.s2 : pb.s, *sOut = sPar ? pb.s : pb.s2;
-        { FLIP_COUNT(1); k_spmv_s<<<rb, TPB, 0, s>>>(c, pb.fluidIdx, pb.nFluid, pb.A2, pb.zc, sIn, sOut, pb.q, pb.partials, pb.scal, rmax, pb.ctl); }
-        { FLIP_COUNT(1); k_update_xr<<<rb, TPB, 0, s>>>(pb.fluidIdx, pb.fluidSk, pb.nFluid, pb.x, pb.r, pb.rf, sOut, pb.q, pb.scal, rmax, pb.ctl); }
-        { FLIP_COUNT(1); k_true_residual<<<rb, TPB, 0, s>>>(c, pb.fluidIdx, pb.fluidSk, pb.nFluid, pb.Ad, pb.b, pb.x, pb.r, pb.rf, rmax + 1, pb.scal, pb.ctl, sw.ticket); }
+        launch_after(true, sl.swap ? k_spmv_s<true> : k_spmv_s<false>, rb, TPB, 0, s, sl, pb.nsl, pb.items, pb.nItems, pb.A,
+                     pb.z, sIn, sOut, pb.qh, pb.ql, pb.partials, pb.scal, rmax, pb.ctl);
+        launch_after(true, k_update_xr, rb, TPB, 0, s, pb.items, pb.nItems, pb.xh, pb.xl, pb.rh, pb.rl, sOut, pb.qh, pb.ql,
+                     pb.scal, rmax, pb.ctl, sw.ticket);
+        launch_after(true, k_true_residual, rb, TPB, 0, s, c, sl, pb.items, pb.nItems, pb.fluid, pb.Ad, pb.b, pb.xh, pb.xl,
+                     pb.rh, pb.rl, rmax + 1, pb.scal, pb.ctl);
         precondition(1 + k, timed);
         sPar ^= 1;
     };
@@ -974,7 +1238,6 @@ int pressure_project(const StepConsts &c, const PressureArgs &a, PressureBuffers
     PCK(cudaMemsetAsync(rmax, 0, 2 * sizeof(unsigned long long), s));
     PCK(cudaMemcpyAsync(pb.scal + 6, &mail->ptol, sizeof(double), cudaMemcpyHostToDevice, s));
     sweep_epoch_guard(c, sw, 2, s);
-    { FLIP_COUNT(1); k_init_r<<<rb, TPB, 0, s>>>(c, pb.sl, pb.b, pb.r, pb.rf, pb.x, rmax, sw.ticket); }
     precondition(0, tm != nullptr);
     PCK(cudaMemcpyAsync(&mail->rho, pb.scal + 1, sizeof(double), cudaMemcpyDeviceToHost, s));
     PCK(cudaMemcpyAsync(&mail->sweepErr, sw.err, sizeof(int), cudaMemcpyDeviceToHost, s));
@@ -1115,8 +1378,10 @@ int pressure_project(const StepConsts &c, const PressureArgs &a, PressureBuffers
     }
     res->iterations = iterations;
     res->residual = resid;
+    pb.stale = !ok;
     const bool accept = ok || (iterations == a.maxIter && resid < a.accTol);   // pressuresolver.cpp:810-840
-    { FLIP_COUNT(1); k_x_to_float<<<nb, TPB, 0, s>>>(n, pb.x, pb.pressure); }
+    PCK(cudaMemsetAsync(pb.pressure, 0, n * sizeof(float), s));
+    { FLIP_COUNT(1); k_x_to_cells<<<ib, TPB, 0, s>>>(c, sl, pb.items, pb.nItems, pb.fluid, pb.xh, pb.xl, pb.pressure); }
     if (a.dumpPressure) {
         PCK(sync());
         PCK(cudaMemcpy(a.dumpPressure, pb.pressure, n * sizeof(float), cudaMemcpyDeviceToHost));

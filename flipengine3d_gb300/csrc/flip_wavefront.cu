@@ -320,6 +320,7 @@ __device__ __forceinline__ bool run_steps(const WarpJob &w) {
                     na = ld_edge(w.inA + off);
                     nb = ld_edge(w.inB + off);
                     if (!__any_sync(0xffffffffu, any_absent(na, nb))) break;
+                    __nanosleep(20);   // leaves the issue slots to the kernels of other streams; no cost alone
                     if (edge_gives_up(++spin, &w.sm->abort, w.err, w.spinLimit)) { fine = false; return; }
                 }
             }
@@ -407,14 +408,17 @@ template <bool FWD, bool SWAP, bool WHOLE>
 __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(NTHREADS) k_wavefront(SweepArgs a) {
     extern __shared__ __align__(128) unsigned char smemRaw[];
     SweepSmem &sm = *reinterpret_cast<SweepSmem *>(smemRaw);
-    if (*(volatile const int *)a.skip) return;   // converged: nothing to do (all CTAs see the same)
     const int T = a.T;
     const int edgeGroups = (WHOLE ? T : RC * CH) / EC;   // groups of edge words per warp
     float *edge = reinterpret_cast<float *>(smemRaw + sizeof(SweepSmem));   // [warp][group][GW]
     const unsigned rank = cluster_rank();
     if (threadIdx.x == 0) {
+        // Nothing to do once converged or after an earlier sweep gave up.  One
+        // thread decides for the cluster: the flags may change while its CTAs
+        // start, and a CTA must not leave while another reads its shared memory.
         if (rank == 0)
-            sm.cluster = *(volatile int *)a.err ? -1 : (int)atomicAdd(&a.ticket[FWD ? 0 : 2], 1u);
+            sm.cluster = *(volatile const int *)a.skip || *(volatile int *)a.err ? -1
+                                                                                  : (int)atomicAdd(&a.ticket[FWD ? 0 : 2], 1u);
         sm.abort = 0;
         sm.epoch = *(volatile unsigned int *)&a.ticket[1] + (FWD ? 0u : 1u);   // forward e, backward e + 1
         for (int b = 0; b < NBUF; b++) {
@@ -483,7 +487,6 @@ __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(NTHREADS) k_wavefro
         prefetch_l2(a.L + chunk_entry(n), bl);
         prefetch_l2(a.rin + chunk_entry(n), br);
     };
-    if (work && threadIdx.x == LOADER * 32) issue(0);   // comes while the edge words are set up
     if (work) {
         // Words that will come are ABSENT, the others are zero terms.  In the
         // ring everything comes, the other tiles' zero terms too, except a
@@ -505,15 +508,17 @@ __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(NTHREADS) k_wavefro
         }
     }
     cluster_sync();   // also keeps rank 0 until every CTA has read its ticket
-    if (!work) return;
+    // All of the above may run while the kernel before this one ends.
+    pdl_wait();
+    pdl_trigger();
+    if (!work || *(volatile const int *)a.skip) return;   // converged meanwhile: every CTA sees the same now
     const size_t wordsPerTile = (size_t)T * (WA + WB);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
     if (warp == LOADER) {
         // ================================================== loader thread
         if (lane != 0) return;
-        prefetch(NBUF);
-        int issued = 1;
+        int issued = 0;
         for (; issued < nChunks; issued++) {
             const int before = issued - NBUF;
             if (before >= 0 && !mb_wait(smem_addr(&sm.done[before % NBUF]), (before / NBUF) & 1, &sm.abort, a.err, a.spinLimit)) break;
@@ -707,7 +712,7 @@ void launch_sweep_ranges(const StepConsts &c, const SweepLayout &g, const uint8_
 }
 
 void launch_sweeps(const StepConsts &c, const SweepLayout &g, const float4 *L, const float *rf, float *z,
-                   SweepState &sw, const int *skip, cudaStream_t s, bool prepped) {
+                   SweepState &sw, const int *skip, cudaStream_t s, bool prepped, bool overlap) {
     static std::atomic<unsigned long long> smemSet{0};   // devices on which the shared memory is opted in
     int dev = 0;
     cudaGetDevice(&dev);
@@ -742,8 +747,7 @@ void launch_sweeps(const StepConsts &c, const SweepLayout &g, const float4 *L, c
     for (int d = 0; d < 2; d++) {
         a.rin = d == 0 ? rf : z;
         a.out = z;
-        FLIP_COUNT(1);
-        kernels[d][g.swap ? 1 : 0][whole ? 1 : 0]<<<n, NTHREADS, smem, s>>>(a);
+        launch_after(overlap || d == 1, kernels[d][g.swap ? 1 : 0][whole ? 1 : 0], n, NTHREADS, smem, s, a);
     }
     sw.epoch += 2;
 }
