@@ -168,9 +168,8 @@ __host__ __device__ __forceinline__ long long sweep_index(const SweepLayout &g, 
 struct PcgCtl {
     int done;      // converged
     int iters;     // iterations to convergence
-    int claim;     // the recurrence residual passed the test; b - A x must confirm
     int it;        // index of the iteration being run
-    unsigned int ticket[4];   // per reduction kernel (spmv, dot_zr, update_xr, true residual): CTAs done
+    unsigned int ticket[4];   // CTAs done, of [1] the first z.r and [3] the true residual
     double resid;  // last residual norm tested
     int batches;     // batches run by the device-side loop
     int maxBatches;  // its limit (maximum iterations / PCG_BATCH)
@@ -196,8 +195,8 @@ struct PressureBuffers {
     SweepLayout sl;        // the orientation of the current solve
     long long nsl;         // entries allocated for the sweep layout
     bool stale = true;     // z, s, s2 may hold values that are not finite
-    double *partials;      // per-block partial sums (deterministic reduction)
-    double *scal;          // [0]=s.q [1]=z.r (new rho) [2]=|b|inf [3]=rho [4]=alpha [5]=beta [6]=tol |b|inf
+    double *partials;      // per-block partial sums of s.q, then of z.r (PCG_MAX_PARTIALS each; deterministic)
+    double *scal;          // [1]=the first z.r [2]=|b|inf [3], [7]=rho of even and odd iterations [6]=tol |b|inf
     unsigned long long *rmaxBits;  // [0] |r|inf of the recurrence, [1] of b - A x, as double bits
     PcgCtl *ctl;
     // PCG_BATCH iterations captured as a CUDA graph, replayed per batch;

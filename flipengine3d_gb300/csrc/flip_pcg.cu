@@ -537,10 +537,12 @@ __device__ __forceinline__ void block_max_float_to(float v, unsigned long long *
     }
 }
 
-// Each CTA of a reduction takes a ticket once its partial (or atomic) is
-// out; the CTA that takes the last one then sees all of them and finishes the
-// reduction, and resets the ticket for the next launch.  One launch instead
-// of a producer and a one-CTA consumer.
+// The sums of the loop are finished by the kernel that needs them: every one
+// of its CTAs adds the block partials of the kernel before it, in the same
+// fixed order.  A fence, a ticket and a last CTA that adds them at the end of
+// the producer took about 2 us longer per sum.  Where the host needs a
+// result, the CTA that takes the last ticket sees all partials (or atomics),
+// finishes and resets the ticket for the next launch.
 __device__ __forceinline__ bool last_cta(unsigned int *ticket, unsigned int ctas) {
     __shared__ int amLast;
     __syncthreads();
@@ -562,6 +564,15 @@ __device__ __forceinline__ double sum_partials_fixed(const double *partials, int
     for (int q = threadIdx.x; q < n; q += blockDim.x) v += __ldcg(partials + q);
     return block_sum(v, sh);
 }
+// The same sum for every thread of the CTA.
+__device__ __forceinline__ double sum_partials_all(const double *partials, int n, double *sh) {
+    const double v = sum_partials_fixed(partials, n, sh);
+    if (threadIdx.x == 0) sh[0] = v;
+    __syncthreads();
+    const double r = sh[0];
+    __syncthreads();
+    return r;
+}
 __device__ __forceinline__ double bits_to_resid(const unsigned long long *p) {
     return __longlong_as_double((long long)__ldcg(p));
 }
@@ -573,8 +584,9 @@ __device__ __forceinline__ double bits_to_resid(const unsigned long long *p) {
 // zeros.  The vectors live in the sweep layout: a warp takes one step of a
 // tile, whose entries are contiguous, and a row's six neighbours are entries
 // of the steps before and after it, so loads are 16-byte and coalesced (a row
-// list in cell order gathered every neighbour on its own: 17.7, 15.0 and 13.5
-// us for the three kernels at 518k rows).
+// list in cell order gathered every neighbour on its own).  Warm times of the
+// SpMV, the update and z.r: 17.3, 8.9 and 5.0 us at 518k rows (16.4, 12.4 and
+// 12.5 us with the row list), 8.2, 4.9 and 3.8 us at 59k rows (11.1, 9.2, 8.8).
 
 // Double-float arithmetic on the FP32 pipe (this GPU's FP64 rate is ~1/64
 // of FP32): a coefficient a = hi + lo (floats, exact to 48 bits) times an
@@ -676,101 +688,199 @@ __device__ __forceinline__ void st4(float *p, const float (&v)[4]) {
 // reads a value another thread is writing) and the row's own goes to sOut.
 // In the first iteration beta = 0 and sIn = 0, so s = z.  A neighbour that
 // is not a row couples with 0 (its entry holds a finite value); one outside
-// the layout is the zero padding after it.  A thread takes four consecutive
-// pencils of a step, two to a packed operation: along a, the neighbours of
-// three of them are in its own vectors of the steps before and after, the
-// fourth's is one word more.  The last CTA sums s.q and sets alpha = rho / s.q,
-// rounded to float as BLAS::addScaled takes it (blaswrapper.h:129-158), and
-// clears the iteration's residual norms.
+// the layout is the zero padding after it.
+//
+// An item's operands are whole steps of the layout, contiguous in every
+// plane, so one thread brings them to shared memory with ten bulk copies (the
+// rows' planes and sIn already while the kernel before this one ends): a
+// single latency per item, where loads into registers exposed one per
+// coupling.  A
+// thread takes four consecutive pencils of a step, two to a packed operation;
+// only the neighbours in other tiles are read from global memory.
+struct SpmvSmem {
+    float S[SWEEP_CH + 2][SWEEP_NP], Z[SWEEP_CH + 2][SWEEP_NP];   // steps -1 .. 8 of the item
+    float C[6][SWEEP_CH + 1][SWEEP_NP];   // couplings +x, +y, +z: leading parts, remainders; steps -1 .. 7
+    float D[2][SWEEP_CH][SWEEP_NP];       // diagonal
+    unsigned long long bar;
+    int failed, issued;
+};
+static_assert(sizeof(SpmvSmem) + sizeof(double) * TPB <= 48 * 1024, "static shared memory");
+__device__ __forceinline__ unsigned smem_addr(const void *p) { return (unsigned)__cvta_generic_to_shared(p); }
+__device__ __forceinline__ void bulk_steps(float *dst, const float *src, int steps, unsigned bar) {
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+                 ::"r"(smem_addr(dst)), "l"(src), "r"(steps * SWEEP_NP * 4), "r"(bar) : "memory");
+}
 template <bool SWAP>
 __global__ void __launch_bounds__(TPB, 3)
     k_spmv_s(SweepLayout g, long long nsl, const int *__restrict__ items, const int *__restrict__ nItems,
              const float *__restrict__ A, const float *__restrict__ z, const float *__restrict__ sIn,
-             float *__restrict__ sOut, float *__restrict__ qh, float *__restrict__ ql, double *partials, double *scal,
-             unsigned long long *rmaxBits, PcgCtl *ctl) {
+             float *__restrict__ sOut, float *__restrict__ qh, float *__restrict__ ql, const double *zrPartials,
+             double *partials, double *scal, PcgCtl *ctl, int *err) {
+    __shared__ __align__(128) SpmvSmem sm;
     __shared__ double sh[TPB];
     const int n = *nItems, T = g.T, nch = T / SWEEP_CH, ctas = min((int)gridDim.x, n);
-    pdl_wait();
-    pdl_trigger();
-    if (ctl->done || (int)blockIdx.x >= n) return;
-    const float betaf = (float)scal[5];   // exact: beta is a float value
-    const F2 beta = f2(betaf, betaf);
     constexpr int NP = SWEEP_NP;
     const long long np = nsl + NP;        // stride of the planes of A
-    const float *Xh = A + np, *Xl = A + 5 * np;
-    const float *Ah = A + (SWAP ? 3 : 2) * np, *Al = A + (SWAP ? 7 : 6) * np;   // couplings along a
-    const float *Bh = A + (SWAP ? 2 : 3) * np, *Bl = A + (SWAP ? 6 : 7) * np;   // and along b
-    const int p0 = (threadIdx.x & 31) * 4, la0 = p0 & 7, lb = (p0 >> 3) & 3, wa = (p0 >> 5) & 1, wb = p0 >> 6;
+    const unsigned bar = smem_addr(&sm.bar);
+    // The couplings along a and b are planes 1 + CA and 1 + CB (C[CA], C[CB]).
+    constexpr int CA = SWAP ? 2 : 1, CB = SWAP ? 1 : 2;
+    auto issue = [&](int it, bool rows, bool zed) {   // one thread
+        const int item = items[it], tile = item / nch, t0 = item % nch * SWEEP_CH;
+        const int lo = t0 > 0, hi = t0 + SWEEP_CH < T;
+        const long long e0 = ((long long)tile * T + t0) * NP;
+        if (rows) {
+            const unsigned steps = 2 * (SWEEP_CH + lo + hi) + 6 * (SWEEP_CH + lo) + 2 * SWEEP_CH;
+            asm volatile("{\n .reg .b64 st;\n mbarrier.arrive.expect_tx.shared::cta.b64 st, [%0], %1;\n}" ::"r"(bar),
+                         "r"(steps * (NP * 4)) : "memory");
+            for (int q = 0; q < 6; q++)
+                bulk_steps(sm.C[q][1 - lo], A + (q < 3 ? 1 + q : 2 + q) * np + e0 - lo * NP, SWEEP_CH + lo, bar);
+            bulk_steps(sm.D[0][0], A + e0, SWEEP_CH, bar);
+            bulk_steps(sm.D[1][0], A + 4 * np + e0, SWEEP_CH, bar);
+            bulk_steps(sm.S[1 - lo], sIn + e0 - lo * NP, SWEEP_CH + lo + hi, bar);
+        }
+        if (zed) bulk_steps(sm.Z[1 - lo], z + e0 - lo * NP, SWEEP_CH + lo + hi, bar);
+    };
+    if (threadIdx.x == 0) {
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar) : "memory");
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        sm.failed = 0;
+        // The rows and sIn were written before the kernel ahead of this one;
+        // the flag may still be set, and what is started is waited for.
+        sm.issued = (int)blockIdx.x < n && !*(volatile int *)&ctl->done;
+        if (sm.issued) issue(blockIdx.x, true, false);
+    }
+    pdl_wait();
+    pdl_trigger();
+    __syncthreads();
+    const bool done = ctl->done != 0;
+    if ((int)blockIdx.x >= n || (done && !sm.issued)) return;
+    if (threadIdx.x == 0) issue(blockIdx.x, false, true);
+    // rho of this iteration, and beta = rho / rho of the one before as float
+    // (pcgsolver.h:295-298); the two alternate between two places
+    const int odd = ctl->it & 1;
+    const double rho = sum_partials_all(zrPartials, ctas, sh), before = scal[odd ? 3 : 7];
+    if (blockIdx.x == 0 && threadIdx.x == 0) scal[odd ? 7 : 3] = rho;
+    const float betaf = ctl->it > 0 && before != 0.0 ? (float)(rho / before) : 0.0f;
+    const F2 beta = f2(betaf, betaf);
+    const int u = threadIdx.x >> 5, p0 = (threadIdx.x & 31) * 4, la0 = p0 & 7, lb = (p0 >> 3) & 3, wa = (p0 >> 5) & 1,
+              wb = p0 >> 6;
     F2 dotH = F2_ZERO, dotL = F2_ZERO;
+    unsigned phase = 0;
     for (int it = blockIdx.x; it < n; it += gridDim.x) {
-        const int item = items[it], tile = item / nch, tf = item % nch * SWEEP_CH + (threadIdx.x >> 5);
+        if (threadIdx.x == 0 && it != (int)blockIdx.x) issue(it, true, true);
+        const int item = items[it], tile = item / nch, tf = item % nch * SWEEP_CH + u;
         const int ta = tile % g.nta, tb = tile / g.nta;
         const long long e = ((long long)tile * T + tf) * NP + p0, none = nsl + p0;
-        // entries of the neighbours: the steps after and before; a+ of the last
-        // pencil and a- of the first; b+ and b- of all four
-        const long long eU = tf + 1 < T ? e + NP : none, eD = tf > 0 ? e - NP : none;
-        long long eaU, eaD, ebU, ebD;
-        if (la0 == 0) eaU = eU + 4;
-        else if (wa == 0) eaU = tf + 1 < T ? eU + 28 : none;
-        else eaU = ta + 1 < g.nta && tf >= SWEEP_WA - 1 ? e + ((long long)T - (SWEEP_WA - 1)) * NP - 36 : none;
-        if (la0 != 0) eaD = eD - 1;
-        else if (wa == 1) eaD = tf > 0 ? eD - 25 : none;
-        else eaD = ta > 0 && tf + SWEEP_WA - 1 < T ? e - ((long long)T - (SWEEP_WA - 1)) * NP + 39 : none;
-        if (lb < 3) ebU = tf + 1 < T ? eU + 8 : none;
-        else if (wb == 0) ebU = tf + 1 < T ? eU + 40 : none;
-        else ebU = tb + 1 < g.ntb && tf >= SWEEP_WB - 1 ? e + ((long long)T * g.nta - (SWEEP_WB - 1)) * NP - 88 : none;
-        if (lb > 0) ebD = tf > 0 ? eD - 8 : none;
-        else if (wb == 1) ebD = tf > 0 ? eD - 40 : none;
-        else ebD = tb > 0 && tf + SWEEP_WB - 1 < T ? e - ((long long)T * g.nta - (SWEEP_WB - 1)) * NP + 88 : none;
-        auto snew = [&](long long at, F2 (&v)[2]) {
+        const bool up = tf + 1 < T, down = tf > 0;
+        // Neighbours in other tiles, read while the copies run: a+ of the last
+        // pencil, a- of the first; b+ or b- of all four.
+        const bool farU = la0 != 0 && wa == 1, farD = la0 == 0 && wa == 0;
+        const bool farBU = lb == 3 && wb == 1, farBD = lb == 0 && wb == 0;
+        float saU = 0.f, saD = 0.f, caH = 0.f, caL = 0.f;
+        F2 fz[2] = {0, 0}, fs[2] = {0, 0}, fh[2] = {0, 0}, fl[2] = {0, 0};
+        auto snew_at = [&](long long at) { return __fmaf_rn(betaf, sIn[at], z[at]); };
+        if (farU)
+            saU = snew_at(ta + 1 < g.nta && tf >= SWEEP_WA - 1 ? e + ((long long)T - (SWEEP_WA - 1)) * NP - 36 : none);
+        if (farD) {
+            const long long at =
+                ta > 0 && tf + SWEEP_WA - 1 < T ? e - ((long long)T - (SWEEP_WA - 1)) * NP + 39 : none;
+            saD = snew_at(at);
+            caH = A[(1 + CA) * np + at];
+            caL = A[(5 + CA) * np + at];
+        }
+        if (farBU || farBD) {
+            const long long step = ((long long)T * g.nta - (SWEEP_WB - 1)) * NP - 88;
+            long long at = none;
+            if (farBU && tb + 1 < g.ntb && tf >= SWEEP_WB - 1) at = e + step;
+            if (farBD && tb > 0 && tf + SWEEP_WB - 1 < T) at = e - step;
+            ld2x2(z + at, fz);
+            ld2x2(sIn + at, fs);
+            if (farBD) {
+                ld2x2(A + (1 + CB) * np + at, fh);
+                ld2x2(A + (5 + CB) * np + at, fl);
+            }
+        }
+        bool in = false;
+        for (unsigned spin = 0; spin < DEFAULT_SPIN_LIMIT && !in; spin++) {
+            unsigned ok;
+            asm volatile("{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, 256;\n selp.u32 %0, 1, 0, p;\n}"
+                         : "=r"(ok) : "r"(bar), "r"(phase) : "memory");
+            in = ok != 0;
+        }
+        if (!in) sm.failed = 1;
+        phase ^= 1;
+        if (done) return;   // what was started is in
+        auto from = [&](const float *row, int p, F2 (&v)[2]) { ld2x2(row + p, v); };
+        auto snew = [&](int r, int p, F2 (&v)[2]) {   // of step r - 1 of the item
             F2 zz[2], ss[2];
-            ld2x2(z + at, zz);
-            ld2x2(sIn + at, ss);
+            from(sm.Z[r], p, zz);
+            from(sm.S[r], p, ss);
             v[0] = f2_fma(beta, ss[0], zz[0]);
             v[1] = f2_fma(beta, ss[1], zz[1]);
         };
+        auto snew1 = [&](int r, int p) { return __fmaf_rn(betaf, sm.S[r][p], sm.Z[r][p]); };
         F2 accH[2] = {F2_ZERO, F2_ZERO}, accL[2] = {F2_ZERO, F2_ZERO};
         auto couple = [&](const F2 (&h)[2], const F2 (&l)[2], const F2 (&v)[2]) {
 #pragma unroll
             for (int q = 0; q < 2; q++) df2_mul_add(h[q], l[q], v[q], f2_mul(v[q], F2_MINUS), accH[q], accL[q]);
         };
-        F2 s0[2], sU[2], sD[2] = {0, 0}, h[2], l[2], v[2];
-        snew(e, s0);
-        snew(eU, sU);
-        const float saU = __fmaf_rn(betaf, sIn[eaU], z[eaU]), saD = __fmaf_rn(betaf, sIn[eaD], z[eaD]);
-        ld2x2(A + e, h); ld2x2(A + 4 * np + e, l);
+        // sU, sD: the steps after and before; nothing beyond the tile's ends
+        F2 s0[2], sU[2] = {0, 0}, sD[2] = {0, 0}, h[2], l[2], v[2];
+        snew(u + 1, p0, s0);
+        if (up) {
+            snew(u + 2, p0, sU);
+            if (!farU) saU = snew1(u + 2, la0 == 0 ? p0 + 4 : p0 + 28);
+        }
+        if (down) {
+            snew(u, p0, sD);
+            if (!farD) {
+                const int p = la0 != 0 ? p0 - 1 : p0 - 25;
+                saD = snew1(u, p);
+                caH = sm.C[CA][u][p];
+                caL = sm.C[3 + CA][u][p];
+            }
+        }
+        from(sm.D[0][u], p0, h); from(sm.D[1][u], p0, l);
         couple(h, l, s0);
-        ld2x2(Xh + e, h); ld2x2(Xl + e, l);
+        from(sm.C[0][u + 1], p0, h); from(sm.C[3][u + 1], p0, l);
         couple(h, l, sU);   // +x
         auto plusA = [&] {
-            ld2x2(Ah + e, h); ld2x2(Al + e, l);
+            from(sm.C[CA][u + 1], p0, h); from(sm.C[3 + CA][u + 1], p0, l);
             v[0] = f2(f2_y(sU[0]), f2_x(sU[1]));
             v[1] = f2(f2_y(sU[1]), saU);
             couple(h, l, v);
         };
         auto plusB = [&] {
-            ld2x2(Bh + e, h); ld2x2(Bl + e, l);
-            snew(ebU, v);
+            from(sm.C[CB][u + 1], p0, h); from(sm.C[3 + CB][u + 1], p0, l);
+            v[0] = v[1] = 0;
+            if (farBU) { v[0] = f2_fma(beta, fs[0], fz[0]); v[1] = f2_fma(beta, fs[1], fz[1]); }
+            else if (up) snew(u + 2, lb < 3 ? p0 + 8 : p0 + 40, v);
             couple(h, l, v);
         };
         auto minusA = [&] {
-            F2 ch[2], cl[2];
-            ld2x2(Ah + eD, ch); ld2x2(Al + eD, cl);
-            h[0] = f2(Ah[eaD], f2_x(ch[0])); h[1] = f2(f2_y(ch[0]), f2_x(ch[1]));
-            l[0] = f2(Al[eaD], f2_x(cl[0])); l[1] = f2(f2_y(cl[0]), f2_x(cl[1]));
+            F2 ch[2] = {0, 0}, cl[2] = {0, 0};
+            if (down) { from(sm.C[CA][u], p0, ch); from(sm.C[3 + CA][u], p0, cl); }
+            h[0] = f2(caH, f2_x(ch[0])); h[1] = f2(f2_y(ch[0]), f2_x(ch[1]));
+            l[0] = f2(caL, f2_x(cl[0])); l[1] = f2(f2_y(cl[0]), f2_x(cl[1]));
             v[0] = f2(saD, f2_x(sD[0]));
             v[1] = f2(f2_y(sD[0]), f2_x(sD[1]));
             couple(h, l, v);
         };
         auto minusB = [&] {
-            ld2x2(Bh + ebD, h); ld2x2(Bl + ebD, l);
-            snew(ebD, v);
+            h[0] = fh[0]; h[1] = fh[1]; l[0] = fl[0]; l[1] = fl[1];
+            v[0] = v[1] = 0;
+            if (farBD) { v[0] = f2_fma(beta, fs[0], fz[0]); v[1] = f2_fma(beta, fs[1], fz[1]); }
+            else if (down) {
+                const int p = lb > 0 ? p0 - 8 : p0 - 40;
+                from(sm.C[CB][u], p, h); from(sm.C[3 + CB][u], p, l);
+                snew(u, p, v);
+            }
             couple(h, l, v);
         };
         // +y, +z, then -x, -y, -z
         if (SWAP) { plusB(); plusA(); } else { plusA(); plusB(); }
-        snew(eD, sD);
-        ld2x2(Xh + eD, h); ld2x2(Xl + eD, l);
+        h[0] = h[1] = l[0] = l[1] = 0;
+        if (down) { from(sm.C[0][u], p0, h); from(sm.C[3][u], p0, l); }
         couple(h, l, sD);
         if (SWAP) { minusB(); minusA(); } else { minusA(); minusB(); }
         F2 oh[2], ol[2];
@@ -784,27 +894,20 @@ __global__ void __launch_bounds__(TPB, 3)
         st2x2(sOut + e, s0);
         st2x2(qh + e, oh);
         st2x2(ql + e, ol);
+        __syncthreads();   // the operands are free again
     }
+    if (threadIdx.x == 0 && sm.failed) atomicExch(err, 1);
     double b = block_sum(df_to(make_float2(f2_x(dotH), f2_x(dotL))) + df_to(make_float2(f2_y(dotH), f2_y(dotL))), sh);
     if (threadIdx.x == 0) partials[blockIdx.x] = b;
-    if (last_cta(&ctl->ticket[0], ctas)) {
-        const double sq = sum_partials_fixed(partials, ctas, sh);
-        if (threadIdx.x == 0) {
-            scal[0] = sq;
-            scal[4] = (double)(float)(scal[3] / sq);
-            rmaxBits[0] = 0ull;
-            rmaxBits[1] = 0ull;
-        }
-    }
 }
 
-// rho_new = z.r.  The last CTA sums it; inside the loop (inLoop) it also
-// sets beta = rho_new / rho as float (pcgsolver.h:295-298) and ends the
-// iteration: rho = rho_new, next iteration index.
+// The partial sums of rho_new = z.r; inside the loop (inLoop) it also begins
+// the next iteration: its index, its residual norms cleared.  Before the loop
+// the last CTA sums rho for the host.
 __global__ void __launch_bounds__(TPB) k_dot_zr(const int *__restrict__ items, const int *__restrict__ nItems,
                                                 const float *__restrict__ z, const float *__restrict__ rh,
                                                 const float *__restrict__ rl, double *partials, double *scal,
-                                                PcgCtl *ctl, int inLoop) {
+                                                unsigned long long *rmaxBits, PcgCtl *ctl, int inLoop) {
     __shared__ double sh[TPB];
     const int n = *nItems;
     float2 dot = make_float2(0.0f, 0.0f);   // double-float per thread, FP64 across threads
@@ -831,47 +934,39 @@ __global__ void __launch_bounds__(TPB) k_dot_zr(const int *__restrict__ items, c
     }
     double s = block_sum(df_to(dot), sh);
     if (threadIdx.x == 0) partials[blockIdx.x] = s;
-    if (last_cta(&ctl->ticket[1], ctas)) {
-        const double zr = sum_partials_fixed(partials, ctas, sh);
-        if (threadIdx.x == 0) {
-            scal[1] = zr;
-            if (inLoop) {
-                scal[5] = scal[3] != 0.0 ? (double)(float)(zr / scal[3]) : 0.0;
-                ctl->it += 1;
-            }
-            scal[3] = zr;
+    if (inLoop) {
+        if (blockIdx.x == 0 && threadIdx.x == 0) {
+            ctl->it += 1;
+            rmaxBits[0] = rmaxBits[1] = 0ull;
         }
+    } else if (last_cta(&ctl->ticket[1], ctas)) {
+        const double zr = sum_partials_fixed(partials, ctas, sh);
+        if (threadIdx.x == 0) scal[1] = zr;
     }
 }
 
 // The reference's convergence test |r|inf <= tol |b|inf (pcgsolver.h:
-// 263-288) on the device, by the last CTA of the kernel that produced the
-// norm.  On the iterations where r is recomputed as b - A x (every 25th)
-// that norm decides; otherwise a pass of the recurrence's norm is only a
-// claim, which the recompute of b - A x then settles (final).
-__device__ __forceinline__ void convergence_test(PcgCtl *ctl, double resid, double ptol, bool final) {
+// 263-288) on the device.  On the iterations where r is recomputed as b - A x
+// (every 25th) that norm decides; otherwise a pass of the recurrence's norm is
+// only a claim, which the recompute of b - A x then settles.
+__device__ __forceinline__ void convergence_test(PcgCtl *ctl, double resid, double ptol) {
     ctl->resid = resid;
-    ctl->claim = 0;
     if (resid <= ptol) {
-        if (final) {
-            ctl->done = 1;
-            ctl->iters = ctl->it + 1;
-        } else {
-            ctl->claim = 1;
-        }
+        ctl->done = 1;
+        ctl->iters = ctl->it + 1;
     }
 }
 
 // x += alpha s, r -= alpha q with alpha = rho / s.q passed on as float, as
-// BLAS::addScaled(float alpha, ...) does (blaswrapper.h:129-158); |r|inf,
-// tested by the last CTA except on the iterations of the periodic recompute
+// BLAS::addScaled(float alpha, ...) does (blaswrapper.h:129-158); |r|inf
 __global__ void __launch_bounds__(TPB) k_update_xr(const int *__restrict__ items, const int *__restrict__ nItems,
                                                    float *__restrict__ xh, float *__restrict__ xl,
                                                    float *__restrict__ rh, float *__restrict__ rl,
                                                    const float *__restrict__ s, const float *__restrict__ qh,
-                                                   const float *__restrict__ ql, const double *scal,
-                                                   unsigned long long *rmaxBits, PcgCtl *ctl,
+                                                   const float *__restrict__ ql, const double *sqPartials,
+                                                   const double *scal, unsigned long long *rmaxBits, PcgCtl *ctl,
                                                    unsigned int *sweepTicket) {
+    __shared__ double sh[TPB];
     const int n = *nItems;
     float vxh[4], vxl[4], vrh[4], vrl[4];
     auto entry = [&](int it) { return (long long)items[it] * (SWEEP_CH * SWEEP_NP) + threadIdx.x * 4; };
@@ -885,7 +980,7 @@ __global__ void __launch_bounds__(TPB) k_update_xr(const int *__restrict__ items
     if (blockIdx.x == 0 && threadIdx.x == 0) sweep_prep(sweepTicket);   // for the sweep pair that follows
     if (ctl->done || (int)blockIdx.x >= n) return;
     const int ctas = min((int)gridDim.x, n);
-    const float alpha = (float)scal[4];   // exact: alpha is a float value
+    const float alpha = (float)(scal[ctl->it & 1 ? 7 : 3] / sum_partials_all(sqPartials, ctas, sh));
     float m = 0.0f;
     for (int it = blockIdx.x; it < n; it += gridDim.x) {
         const long long e = entry(it);
@@ -908,8 +1003,6 @@ __global__ void __launch_bounds__(TPB) k_update_xr(const int *__restrict__ items
         st4(rh + e, vrh); st4(rl + e, vrl);
     }
     block_max_float_to(m, rmaxBits);
-    if (last_cta(&ctl->ticket[2], ctas) && threadIdx.x == 0 && (ctl->it + 1) % 25 != 0)
-        convergence_test(ctl, bits_to_resid(rmaxBits), scal[6], false);
 }
 
 // r = b - A x (residual replacement); |r|inf, which the last CTA tests as
@@ -927,7 +1020,11 @@ __global__ void __launch_bounds__(TPB) k_true_residual(StepConsts c, SweepLayout
     pdl_wait();
     pdl_trigger();
     if (ctl->done) return;
-    if ((ctl->it + 1) % 25 != 0 && !ctl->claim) return;
+    const double claimed = bits_to_resid(rmaxBits);   // of the recurrence
+    if ((ctl->it + 1) % 25 != 0 && !(claimed <= scal[6])) {
+        if (blockIdx.x == 0 && threadIdx.x == 0) ctl->resid = claimed;
+        return;
+    }
     const int n = *nItems, nch = g.T / SWEEP_CH;
     const long long sy = c.I, sz = (long long)c.I * c.J;
     double m = 0.0;
@@ -961,8 +1058,8 @@ __global__ void __launch_bounds__(TPB) k_true_residual(StepConsts c, SweepLayout
         const double av = fabs(rv);
         m = (av != av || av > m) ? av : m;
     }
-    block_max_to(m, rmaxBits);
-    if (last_cta(&ctl->ticket[3], gridDim.x) && threadIdx.x == 0) convergence_test(ctl, bits_to_resid(rmaxBits), scal[6], true);
+    block_max_to(m, rmaxBits + 1);
+    if (last_cta(&ctl->ticket[3], gridDim.x) && threadIdx.x == 0) convergence_test(ctl, bits_to_resid(rmaxBits + 1), scal[6]);
 }
 
 // The solution to a float per cell (zero off the rows: cleared before).
@@ -1046,17 +1143,18 @@ int cuda_fail(cudaError_t e, const char *what, std::string *msg) {
 
 int mic0_factor_tiles(int J, int K) { return std::max(1, (J - 2 + FT - 1) / FT) * std::max(1, (K - 2 + FT - 1) / FT); }
 // One CTA of the row kernels per `cellsPerCta` grid cells (4096 by default),
-// at least 128 where there are as many items, at most RBLOCKS.  A liquid fills
-// a fraction of the grid, so a CTA takes one to three items of 1024 entries,
-// and CTAs beyond the items leave at once.  Twice as many CTAs: 128^3 frame
-// 11.66 against 11.53 ms, 16 scenes at once 16.56 against 16.35 ms (CTA
-// dispatch and reductions are shared limits); without the floor of 128, 64^3
-// frames take 3.40 against 3.30 ms.
+// at least 128 where there are as many items, at most the three per SM that
+// the SpMV's shared memory leaves resident.  A liquid fills a fraction of the
+// grid, so a CTA takes a few items of 1024 entries, and CTAs beyond the items
+// leave at once.  The floor of 128: 64^3 frames 3.40 -> 3.30 ms; the cap:
+// 128^3 frames 11.63 -> 11.40 ms, 256x128x128 27.2 -> 26.3 ms (a partial last
+// wave, and more partials for every CTA to add).
+constexpr long long ROW_CTAS = 152 * 3;
 int pressure_partials_for(int I, int J, int K, int cellsPerCta) {
     static_assert(RBLOCKS == PCG_MAX_PARTIALS, "the partials buffer holds RBLOCKS sums");
     const long long items = sweep_items_max(I, J, K);
     const long long ctas = std::max<long long>(div_up((long long)I * J * K, std::max(cellsPerCta, 256)), 128);
-    return (int)std::max(1LL, std::min({ctas, items, (long long)RBLOCKS}));
+    return (int)std::max(1LL, std::min({ctas, items, ROW_CTAS}));
 }
 
 #define PCK(call)                                               \
@@ -1188,6 +1286,7 @@ int pressure_project(const StepConsts &c, const PressureArgs &a, PressureBuffers
     { FLIP_COUNT(1); k_layout<<<ib, TPB, 0, s>>>(c, sl, pb.items, pb.nItems, pb, sw.ticket); }
 
     unsigned long long *rmax = pb.rmaxBits;
+    double *zrPartials = pb.partials + PCG_MAX_PARTIALS;
     SweepTiming *tm = a.sweepTiming;
     // sweep pairs timed but not yet added: event pair index q
     auto tally_pair = [&](int q) {
@@ -1213,7 +1312,8 @@ int pressure_project(const StepConsts &c, const PressureArgs &a, PressureBuffers
         if (timed) record(tm->ev[2 * q]);
         launch_sweeps(c, sl, pb.L, pb.rh, pb.z, sw, &pb.ctl->done, s, true, q > 0);   // prepared by a kernel before
         if (timed) record(tm->ev[2 * q + 1]);
-        launch_after(true, k_dot_zr, rb, TPB, 0, s, pb.items, pb.nItems, pb.z, pb.rh, pb.rl, pb.partials, pb.scal, pb.ctl, q > 0);
+        launch_after(true, k_dot_zr, rb, TPB, 0, s, pb.items, pb.nItems, pb.z, pb.rh, pb.rl, zrPartials, pb.scal, rmax,
+                     pb.ctl, q > 0);
     };
     // one PCG iteration (pcgsolver.h:263-300); every launch is the same for
     // every iteration but the search direction's two buffers, which swap
@@ -1223,11 +1323,11 @@ int pressure_project(const StepConsts &c, const PressureArgs &a, PressureBuffers
     auto iteration = [&](int k, bool timed) {
         float *sIn = sPar ? pb.s2 : pb.s, *sOut = sPar ? pb.s : pb.s2;
         launch_after(true, sl.swap ? k_spmv_s<true> : k_spmv_s<false>, rb, TPB, 0, s, sl, pb.nsl, pb.items, pb.nItems, pb.A,
-                     pb.z, sIn, sOut, pb.qh, pb.ql, pb.partials, pb.scal, rmax, pb.ctl);
+                     pb.z, sIn, sOut, pb.qh, pb.ql, zrPartials, pb.partials, pb.scal, pb.ctl, sw.err);
         launch_after(true, k_update_xr, rb, TPB, 0, s, pb.items, pb.nItems, pb.xh, pb.xl, pb.rh, pb.rl, sOut, pb.qh, pb.ql,
-                     pb.scal, rmax, pb.ctl, sw.ticket);
+                     pb.partials, pb.scal, rmax, pb.ctl, sw.ticket);
         launch_after(true, k_true_residual, rb, TPB, 0, s, c, sl, pb.items, pb.nItems, pb.fluid, pb.Ad, pb.b, pb.xh, pb.xl,
-                     pb.rh, pb.rl, rmax + 1, pb.scal, pb.ctl);
+                     pb.rh, pb.rl, rmax, pb.scal, pb.ctl);
         precondition(1 + k, timed);
         sPar ^= 1;
     };
