@@ -26,6 +26,9 @@ struct StepConsts {
     double radius;               // liquid SDF / P2G particle radius, 0.5*sqrt(3)*dx
     double cfl;
     int maxPerCell;
+    // the reference's blocks of 10 cells, for its particle lists: float edge, 1 / edge
+    float blockdxf, invBlockf;
+    double invBlock;
     // near-solid coarse grid
     int nsi, nsj, nsk;
     double nearCell, invNearCell;

@@ -1099,6 +1099,9 @@ int flip_create(int isize, int jsize, int ksize, double dx, flip_ctx **out) {
     c.I = isize; c.J = jsize; c.K = ksize;
     c.dx = dx; c.invdx = 1.0 / dx; c.invdxf = (float)(1.0 / dx); c.dxf = (float)dx;
     c.radius = 0.5 * 1.0 * dx * std::sqrt(3.0);
+    c.blockdxf = (float)(10 * dx);
+    c.invBlock = 1.0 / (double)c.blockdxf;
+    c.invBlockf = (float)c.invBlock;
     auto below = [](double bound) {   // largest float v with (double)v < bound
         float v = (float)bound;
         while ((double)v >= bound) v = std::nextafter(v, 0.0f);
