@@ -335,14 +335,25 @@ __global__ void __launch_bounds__(1024) k_liquid_sdf(ParticleSoA ps, const int *
 
 // ---------------------------------------------------------------------- P2G
 // Gather form of VelocityAdvector (velocityadvector.cpp:38-459): one thread
-// per face; candidate particles come from the 18 cells that can hold a
-// particle within r of the face; each particle's weight is evaluated in the
-// reference's 10^3-block frame.  Sums run in a fixed (cell, id) order, so
-// the result is deterministic (no float atomics).
-__global__ void __launch_bounds__(TPB) k_p2g(ParticleSoA p, const int *cellStart, StepConsts c, int dir,
-                                             float *G, uint8_t *valid) {
-    const int ni = c.I + (dir == 0), nj = c.J + (dir == 1), nk = c.K + (dir == 2);
-    long long f = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+// per grid index (i, j, k) for its u, v and w face together; candidate
+// particles come from the 27 cells that can hold a particle within r of one of
+// them (18 per face); each particle's weight is evaluated in the reference's
+// 10^3-block frame, which the three faces share.  Sums run in a fixed (cell,
+// id) order, so the result is deterministic (no float atomics).
+// Bound by L1: the lanes of a warp visit different cells, so a load touches 32
+// lines.  Three scalar loads a particle for three faces, against three a face
+// in a kernel per direction: P2G and extrapolation 2195 -> 1260 us at
+// 256x128x128, 857 -> 756 us at 128^3 (of which the extrapolation is 100).
+// 16-byte vectors instead of scalars touch four times the lines: slower.
+// The reference also requires the face to lie in the particle's local box and
+// the particle to be in the block's list, both taken with the support radius
+// sr = r + 1e-6.  A particle within r of the face meets both: every coordinate
+// of the face is within r of the particle, and the 1e-6 margin is far above
+// the rounding of these float expressions (ulp(1) ~ 1.2e-7).
+__global__ void __launch_bounds__(TPB) k_p2g(ParticleSoA p, const int *cellStart, StepConsts c,
+                                             float *U, float *V, float *W, uint8_t *vu, uint8_t *vv, uint8_t *vw) {
+    const int ni = c.I + 1, nj = c.J + 1, nk = c.K + 1;
+    const long long f = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (f >= (long long)ni * nj * nk) return;
     int fi, fj, fk;
     unflatten(f, ni, nj, fi, fj, fk);
@@ -353,50 +364,54 @@ __global__ void __launch_bounds__(TPB) k_p2g(ParticleSoA p, const int *cellStart
     const float coef1 = __fmul_rn(4.0f / 9.0f, __fdiv_rn(1.0f, __fmul_rn(__fmul_rn(__fmul_rn(__fmul_rn(__fmul_rn(r, r), r), r), r), r)));
     const float coef2 = __fmul_rn(17.0f / 9.0f, __fdiv_rn(1.0f, __fmul_rn(__fmul_rn(__fmul_rn(r, r), r), r)));
     const float coef3 = __fmul_rn(22.0f / 9.0f, __fdiv_rn(1.0f, __fmul_rn(r, r)));
-    const float halfdx = (float)(0.5 * dx);
-    const float ox = dir == 0 ? 0.0f : halfdx, oy = dir == 1 ? 0.0f : halfdx, oz = dir == 2 ? 0.0f : halfdx;
+    const float h = (float)(0.5 * dx);
     const int bx = fi / BW, by = fj / BW, bz = fk / BW;
-    const float offx = c.blockPos[bx + 1], offy = c.blockPos[by + 1],
-                offz = c.blockPos[bz + 1];
-    const int la = fi - bx * BW, lb = fj - by * BW, lc = fk - bz * BW;
-    const float gx = c.nodePos[la], gy = c.nodePos[lb], gz = c.nodePos[lc];
-    // candidate cells of the cell grid
-    int cx0 = dir == 0 ? fi - 1 : fi - 1, cx1 = dir == 0 ? fi : fi + 1;
-    int cy0 = fj - 1, cy1 = dir == 1 ? fj : fj + 1;
-    int cz0 = fk - 1, cz1 = dir == 2 ? fk : fk + 1;
-    cx0 = max(cx0, 0); cy0 = max(cy0, 0); cz0 = max(cz0, 0);
-    cx1 = min(cx1, c.I - 1); cy1 = min(cy1, c.J - 1); cz1 = min(cz1, c.K - 1);
+    const float offx = c.blockPos[bx + 1], offy = c.blockPos[by + 1], offz = c.blockPos[bz + 1];
+    const float gx = c.nodePos[fi - bx * BW], gy = c.nodePos[fj - by * BW], gz = c.nodePos[fk - bz * BW];
+    const bool isU = fj < c.J && fk < c.K, isV = fi < c.I && fk < c.K, isW = fi < c.I && fj < c.J;
+    const int cx0 = max(fi - 1, 0), cx1 = min(fi + 1, c.I - 1), cy0 = max(fj - 1, 0), cy1 = min(fj + 1, c.J - 1),
+              cz0 = max(fk - 1, 0), cz1 = min(fk + 1, c.K - 1);
     Dims cells{c.I, c.J, c.K};
-    float sc = 0.0f, wt = 0.0f;
+    float sc[3] = {0.0f, 0.0f, 0.0f}, wt[3] = {0.0f, 0.0f, 0.0f};
+    auto take = [&](int d, float d2, float v) {
+        const float w3 = __fmul_rn(__fmul_rn(__fmul_rn(coef1, d2), d2), d2);
+        const float w2 = __fmul_rn(__fmul_rn(coef2, d2), d2);
+        const float w1 = __fmul_rn(coef3, d2);
+        const float wgt = __fsub_rn(__fadd_rn(__fsub_rn(1.0f, w3), w2), w1);
+        sc[d] = __fadd_rn(sc[d], __fmul_rn(wgt, v));
+        wt[d] = __fadd_rn(wt[d], wgt);
+    };
     for (int cz = cz0; cz <= cz1; cz++)
         for (int cy = cy0; cy <= cy1; cy++) {
-            int pb = cellStart[cells.idx(cx0, cy, cz)], pe = cellStart[cells.idx(cx1, cy, cz) + 1];
+            // the row's particles; those of cells up to fi can reach the u face
+            const long long base = cells.idx(0, cy, cz);
+            const int pb = cellStart[base + cx0], pe = cellStart[base + cx1 + 1];
+            if (pb == pe) continue;
+            const int pu = isU ? cellStart[base + min(fi, c.I - 1) + 1] : pb;
+            const bool rowV = isV && cy <= fj, rowW = isW && cz <= fk;
             for (int t = pb; t < pe; t++) {
-                float px = __fsub_rn(p.px[t], ox), py = __fsub_rn(p.py[t], oy), pz = __fsub_rn(p.pz[t], oz);
-                float lx = __fsub_rn(px, offx), ly = __fsub_rn(py, offy), lz = __fsub_rn(pz, offz);
-                float ddx = __fsub_rn(gx, lx), ddy = __fsub_rn(gy, ly), ddz = __fsub_rn(gz, lz);
-                float d2 = __fadd_rn(__fadd_rn(__fmul_rn(ddx, ddx), __fmul_rn(ddy, ddy)), __fmul_rn(ddz, ddz));
-                if (!(d2 < rsq)) continue;
-                // The reference also requires the face to lie in the particle's
-                // local box and the particle to be in the block's list, both
-                // taken with the support radius sr = r + 1e-6.  A particle
-                // within r of the face meets both: every coordinate of the face
-                // is within r of the particle, and the 1e-6 margin is far above
-                // the rounding of these float expressions (ulp(1) ~ 1.2e-7).
-                float vel = dir == 0 ? p.vx[t] : dir == 1 ? p.vy[t] : p.vz[t];
-                float w3 = __fmul_rn(__fmul_rn(__fmul_rn(coef1, d2), d2), d2);
-                float w2 = __fmul_rn(__fmul_rn(coef2, d2), d2);
-                float w1 = __fmul_rn(coef3, d2);
-                float wgt = __fsub_rn(__fadd_rn(__fsub_rn(1.0f, w3), w2), w1);
-                sc = __fadd_rn(sc, __fmul_rn(wgt, vel));
-                wt = __fadd_rn(wt, wgt);
+                const float px = p.px[t], py = p.py[t], pz = p.pz[t];
+                const float x0 = __fsub_rn(gx, __fsub_rn(px, offx)), x1 = __fsub_rn(gx, __fsub_rn(__fsub_rn(px, h), offx));
+                const float y0 = __fsub_rn(gy, __fsub_rn(py, offy)), y1 = __fsub_rn(gy, __fsub_rn(__fsub_rn(py, h), offy));
+                const float z0 = __fsub_rn(gz, __fsub_rn(pz, offz)), z1 = __fsub_rn(gz, __fsub_rn(__fsub_rn(pz, h), offz));
+                const float xx0 = __fmul_rn(x0, x0), xx1 = __fmul_rn(x1, x1), yy0 = __fmul_rn(y0, y0), yy1 = __fmul_rn(y1, y1),
+                            zz0 = __fmul_rn(z0, z0), zz1 = __fmul_rn(z1, z1);
+                const float du = __fadd_rn(__fadd_rn(xx0, yy1), zz1), dv = __fadd_rn(__fadd_rn(xx1, yy0), zz1),
+                            dw = __fadd_rn(__fadd_rn(xx1, yy1), zz0);
+                if (t < pu && du < rsq) take(0, du, p.vx[t]);
+                if (rowV && dv < rsq) take(1, dv, p.vy[t]);
+                if (rowW && dw < rsq) take(2, dw, p.vz[t]);
             }
         }
     const float eps = 1e-6f;
-    bool ok = wt > eps;
-    if (ok) sc = __fdiv_rn(sc, wt);
-    G[f] = sc;
-    valid[f] = ok ? 1 : 0;
+    auto put = [&](int d, float *G, uint8_t *valid, long long l) {
+        const bool ok = wt[d] > eps;
+        G[l] = ok ? __fdiv_rn(sc[d], wt[d]) : sc[d];
+        valid[l] = ok ? 1 : 0;
+    };
+    if (isU) put(0, U, vu, (long long)fi + (long long)(c.I + 1) * (fj + (long long)c.J * fk));
+    if (isV) put(1, V, vv, (long long)fi + (long long)c.I * (fj + (long long)(c.J + 1) * fk));
+    if (isW) put(2, W, vw, (long long)fi + (long long)c.I * (fj + (long long)c.J * fk));
 }
 
 // ------------------------------------------------------------ extrapolation
@@ -794,13 +809,10 @@ void launch_liquid_sdf(const ParticleSoA &p, const int *cellStart, const StepCon
     FLIP_COUNT(1);
     k_liquid_sdf<<<div_up((long long)c.I * c.J * c.K, threads), threads, 0, s>>>(p, cellStart, c, solidCC, phi);
 }
-void launch_p2g(const ParticleSoA &p, const int *cellStart, const StepConsts &c, float *u, float *v, float *w,
-                uint8_t *vu, uint8_t *vv, uint8_t *vw, cudaStream_t s) {
-    long long nu = (long long)(c.I + 1) * c.J * c.K, nv = (long long)c.I * (c.J + 1) * c.K,
-              nw = (long long)c.I * c.J * (c.K + 1);
-    { FLIP_COUNT(1); k_p2g<<<div_up(nu, TPB), TPB, 0, s>>>(p, cellStart, c, 0, u, vu); }
-    { FLIP_COUNT(1); k_p2g<<<div_up(nv, TPB), TPB, 0, s>>>(p, cellStart, c, 1, v, vv); }
-    { FLIP_COUNT(1); k_p2g<<<div_up(nw, TPB), TPB, 0, s>>>(p, cellStart, c, 2, w, vw); }
+void launch_p2g(const ParticleSoA &p, const int *cellStart, const StepConsts &c, float *u, float *v,
+                float *w, uint8_t *vu, uint8_t *vv, uint8_t *vw, cudaStream_t s) {
+    FLIP_COUNT(1);
+    k_p2g<<<div_up((long long)(c.I + 1) * (c.J + 1) * (c.K + 1), TPB), TPB, 0, s>>>(p, cellStart, c, u, v, w, vu, vv, vw);
 }
 void launch_extrapolate(const StepConsts &c, float *u, float *v, float *w, const uint8_t *vu, const uint8_t *vv,
                         const uint8_t *vw, uint8_t *status, int layers, cudaStream_t s) {
