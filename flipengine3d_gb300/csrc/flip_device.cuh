@@ -44,6 +44,31 @@ struct StepConsts {
     const float *blockPosF;
 };
 
+// Programmatic dependent launch: a kernel launched with launch_after may start
+// while the kernel before it in the stream still runs; what it reads or
+// overwrites of that kernel's lies after pdl_wait().  Called after pdl_wait,
+// pdl_trigger lets the kernel after it start the same way, which can then
+// rely on everything up to the kernel before this one even ahead of its own
+// wait.
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+template <class... P, class... Q>
+inline void launch_after(bool overlap, void (*k)(P...), unsigned grid, unsigned block, size_t smem, cudaStream_t s,
+                         Q... args) {
+    FLIP_COUNT(1);
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(block);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = overlap ? 1 : 0;
+    cudaLaunchKernelEx(&cfg, k, static_cast<P>(args)...);
+}
+
 // -- seeding from fluid meshes (flip_seed.cu); mask: one 8-bit sub-cell
 // mask per cell, four cells to a word; owner: 8 I J K words, all ones
 void launch_mask_particles(const ParticleSoA &p, int n, const StepConsts &c, unsigned int *mask, cudaStream_t s);
@@ -71,10 +96,18 @@ void launch_gather_particles(const ParticleSoA &src, ParticleSoA dst, int n,
 // threads: the CTA size, 256, 512 (default) or 1024
 void launch_liquid_sdf(const ParticleSoA &p, const int *cellStart, const StepConsts &c, const uint8_t *solidCC,
                        float *phi, int threads, cudaStream_t s);
-void launch_p2g(const ParticleSoA &p, const int *cellStart, const StepConsts &c, float *u, float *v, float *w,
-                uint8_t *vu, uint8_t *vv, uint8_t *vw, cudaStream_t s);
+void launch_p2g(const ParticleSoA &p, const int *cellStart, const StepConsts &c, float *u, float *v,
+                float *w, uint8_t *vu, uint8_t *vv, uint8_t *vw, cudaStream_t s);
+// The faces as bits: per direction the extents, words per row of 32 faces
+// along x, and the first word.
+struct FaceBits {
+    int ni[3], nj[3], nk[3], wpr[3];
+    long long base[3], words;
+};
+FaceBits face_bits(int I, int J, int K);
+// known: scratch of 2 * face_bits().words words
 void launch_extrapolate(const StepConsts &c, float *u, float *v, float *w, const uint8_t *vu, const uint8_t *vv,
-                        const uint8_t *vw, uint8_t *status, int layers, cudaStream_t s);
+                        const uint8_t *vw, unsigned *known, int layers, cudaStream_t s);
 // The force-field grid on the device (flip_forces.cu): faces of an
 // ni x nj x nk grid of cell size dx, and the body force it reads outside them
 struct ForceFieldView {
@@ -270,30 +303,6 @@ int sweep_tiles_max(int I, int J, int K);           // tiles of the larger orien
 long long sweep_exchange_words(int I, int J, int K);   // for the larger orientation
 void launch_sweep_ranges(const StepConsts &c, const SweepLayout &g, const uint8_t *fluid, SweepState &sw,
                          cudaStream_t s);
-// Programmatic dependent launch: a kernel launched with launch_after may start
-// while the kernel before it in the stream still runs; what it reads or
-// overwrites of that kernel's lies after pdl_wait().  Called after pdl_wait,
-// pdl_trigger lets the kernel after it start the same way, which can then
-// rely on everything up to the kernel before this one even ahead of its own
-// wait.
-__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-template <class... P, class... Q>
-inline void launch_after(bool overlap, void (*k)(P...), unsigned grid, unsigned block, size_t smem, cudaStream_t s,
-                         Q... args) {
-    FLIP_COUNT(1);
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(grid);
-    cfg.blockDim = dim3(block);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = s;
-    cudaLaunchAttribute at{};
-    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at.val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = &at;
-    cfg.numAttrs = overlap ? 1 : 0;
-    cudaLaunchKernelEx(&cfg, k, static_cast<P>(args)...);
-}
 // Before each sweep pair, by one thread of a kernel that runs before it:
 // tile tickets from zero for both sweeps and a fresh epoch for each (the
 // forward sweep publishes under ticket[1], the backward under ticket[1]+1).

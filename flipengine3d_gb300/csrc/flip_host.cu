@@ -163,7 +163,8 @@ struct flip_ctx {
     float *phi = nullptr, *solidPhi = nullptr, *wu = nullptr, *wv = nullptr, *ww = nullptr;
     uint8_t *solidCC = nullptr, *nearSolid = nullptr;
     float *u = nullptr, *v = nullptr, *w = nullptr, *su = nullptr, *sv = nullptr, *sw = nullptr;
-    uint8_t *vu = nullptr, *vv = nullptr, *vw = nullptr, *status = nullptr;
+    uint8_t *vu = nullptr, *vv = nullptr, *vw = nullptr;
+    unsigned *known = nullptr;   // extrapolation: known faces as bits, two sets
     PressureBuffers pr{};
     SweepState sweep{};
     unsigned int *speedHist = nullptr, *maxVelSqBits = nullptr;
@@ -283,7 +284,7 @@ int alloc_grids(flip_ctx *x) {
         return rc;
     if ((rc = x->alloc(&x->vu, x->nu())) || (rc = x->alloc(&x->vv, x->nv())) || (rc = x->alloc(&x->vw, x->nw())))
         return rc;
-    if ((rc = x->alloc(&x->status, x->nu() + x->nv() + x->nw()))) return rc;
+    if ((rc = x->alloc(&x->known, 2 * face_bits(x->I, x->J, x->K).words))) return rc;
     PressureBuffers &p = x->pr;
     const long long nsl = sweep_layout_size(x->I, x->J, x->K);
     p.sl = sweep_layout(x->I, x->J, x->K, 0);
@@ -831,7 +832,7 @@ int step_fluid(flip_ctx *x, double dt, flip_stage_dump *d) {
             CK(cudaMemcpy(d->vv_p2g, x->vv, x->nv(), cudaMemcpyDeviceToHost));
             CK(cudaMemcpy(d->vw_p2g, x->vw, x->nw(), cudaMemcpyDeviceToHost));
         }
-        launch_extrapolate(c, x->u, x->v, x->w, x->vu, x->vv, x->vw, x->status, layers, s);
+        launch_extrapolate(c, x->u, x->v, x->w, x->vu, x->vv, x->vw, x->known, layers, s);
     } else {
         CK(cudaMemsetAsync(x->u, 0, x->nu() * 4, s));
         CK(cudaMemsetAsync(x->v, 0, x->nv() * 4, s));
@@ -876,7 +877,7 @@ int step_fluid(flip_ctx *x, double dt, flip_stage_dump *d) {
     if (d && d->pcg_iters) *d->pcg_iters = x->stats.pressure_iterations;
     if (d && d->pcg_error) *d->pcg_error = x->stats.pressure_error;
     x->mark(FLIP_STAGE_CONSTRAIN);
-    launch_extrapolate(c, x->u, x->v, x->w, x->vu, x->vv, x->vw, x->status, layers, s);
+    launch_extrapolate(c, x->u, x->v, x->w, x->vu, x->vv, x->vw, x->known, layers, s);
     if (d && (rc = dump_mac(x, d->u_press, d->v_press, d->w_press, x->u, x->v, x->w))) return rc;
     // constrain saved and current fields (fluidsimulation.cpp:3937-3950)
     const bool fr = x->box.anyFriction;
@@ -1548,7 +1549,7 @@ int flip_estimate_device_bytes(int isize, int jsize, int ksize, int particles, l
     long long b = 0;
     b += 5 * (nc + 1) * 4 + (scan_scratch_ints((int)nc) + 4) * 4 + 16;   // binning
     b += nc * 4 + (I + 1) * (J + 1) * (K + 1) * 4 + nc;                  // phi, solid phi, solid cells
-    b += faces * (4 * 3 + 1 + 1);                                        // weights, velocity, saved, valid, status
+    b += faces * (4 * 3 + 1) + 8 * face_bits(isize, jsize, ksize).words;                                        // weights, velocity, saved, valid, status
     b += nc * (1 + 32 + 8 * 2 + 4) + nsl * (16 + 4 * 9) + 12 * SWEEP_NP + 4 * std::max(8 * (nsl + SWEEP_NP), 6 * nc);   // pressure system
     b += 4 * (sweep_items_max(isize, jsize, ksize) + 8) + 16;              // its items
     b += 2 * PCG_MAX_PARTIALS * 8 + 64 + 16 + 32;
