@@ -360,10 +360,14 @@ int viscosity_apply(const StepConsts &c, const ViscosityBuffers &vb, const float
 // -- surface reconstruction (flip_mesh.cu)
 // The frame of the mesher's one compute chunk: the subdivided grid, its
 // blocks of 10^3 nodes, the chunk's nodes and offset, and the particle radii.
+struct MeshRow {           // a row of cells around a node's: its offset, and the least squared distance to it
+    float least;
+    short y, z;
+};
 struct MeshFrame {
     int I, J, K;
     double dx, invdx, subdx, invsub;
-    float invsubf;
+    float dxf, invdxf, subdxf, invsubf;
     double blockdx, invBlock;      // 10 subdx, occupancy pass
     float invBlockf;
     float blockdxF;                // (float)(10 subdx), the count pass's block size
@@ -374,8 +378,17 @@ struct MeshFrame {
     int cbI, cbJ, cbK;             // chunk blocks
     float offx, offy, offz;        // chunk offset
     float r, sr, maxd;             // radius, search radius, initial distance
-    float bbx, bby, bbz;           // the chunk's expanded box
-    double bbw, bbh, bbd;
+    // how far along an axis a particle can reach a node, how far it can make one inside, and the squared
+    // distance below which its search box surely holds the node
+    float reach, signReach, near2, slack;
+    // where node a of the chunk lies along an axis with chunk offset off, in cells
+    __device__ float cellAt(float off, int a) const { return (off + (float)a * subdxf) * invdxf; }
+    const MeshRow *rows;           // rows to search, nearest first
+    int nrows;
+    int wpr, wpc;                  // words of 32 nodes a row of the chunk, of 32 cells a row of the grid
+    float nodePos[10];             // a node's place in its block's frame
+    const float *blockPos[3];      // origins of the blocks' frames along each axis
+    float bbx, bby, bbz, bhx, bhy, bhz;   // the chunk's expanded box: from bb (inside) to bh (outside)
     int solidMode;                 // 0 interpolated, 1 subdivision 2 at offset 0, 2 same grid
     float scalef, invscalef;
 };
@@ -395,12 +408,12 @@ struct MeshJob {
 struct MeshBuffers {
     long long bytes = 0;
     uint8_t *occ = nullptr, *active = nullptr, *cube = nullptr;
-    float *field = nullptr;
-    int *vstart = nullptr, *tstart = nullptr, *totals = nullptr;
+    unsigned *inside = nullptr, *occupied = nullptr;   // nodes inside; cells with particles, cells near those: bits
+    int *vstart = nullptr, *totals = nullptr;
     int2 *tiles = nullptr, *adj = nullptr, *adjStart = nullptr;
     int *adjCursor = nullptr, *adjList = nullptr, *tris = nullptr;
     float *verts[2] = {nullptr, nullptr};
-    long long occCap = 0, activeCap = 0, cubeCap = 0, fieldCap = 0, vstartCap = 0, tstartCap = 0, totalsCap = 0,
+    long long occCap = 0, activeCap = 0, cubeCap = 0, insideCap = 0, occupiedCap = 0, vstartCap = 0, totalsCap = 0,
               tilesCap = 0, adjCap = 0, adjStartCap = 0, adjCursorCap = 0, adjListCap = 0, trisCap = 0;
     long long vertsCap[2] = {0, 0};
     int nverts = 0, ntris = 0, cur = 0;

@@ -18,10 +18,11 @@
 //   meshParticles; TriangleMesh::smooth (trianglemesh.cpp:481-585).
 //
 // The GPU work is organised for parallelism, not as the reference's loops:
-//   * field: one CTA per 10^3-node block, particles found through the cell
-//     bins, each particle's node box scattered into the block's shared
-//     memory with an atomic minimum of squared distances (sqrt and the
-//     subtraction of r are monotone, so min(|d|) - r comes out exactly);
+//   * field: of most nodes only the side is needed (is a particle within r,
+//     is the node in the solid), as a bit; the value only at the ends of the
+//     cut edges.  Both come from a search for the node's nearest particle
+//     through the cell bins (sqrt and the subtraction of r are monotone, so
+//     min(|d|) - r comes out exactly);
 //   * numbering: a vertex belongs to the first cell in flat order that holds
 //     its edge (for an edge, the cell below it in every perpendicular axis
 //     where there is one).  So a cell's new vertices and its triangles are
@@ -37,6 +38,7 @@
 // triangles come out identical to the reference's for the same particles.
 #include <algorithm>
 #include <cmath>
+#include <cstring>
 #include <string>
 #include <vector>
 
@@ -48,6 +50,7 @@ namespace {
 
 constexpr int MB = 10;          // ParticleMesher::_blockwidth (particlemesher.h:190)
 constexpr int MESH_TPB = 256;
+constexpr int SEARCH_TPB = 128;   // searches differ in length: small CTAs
 constexpr int CELLS_PER_THREAD = 8;
 constexpr int TILE = MESH_TPB * CELLS_PER_THREAD;   // cells per scan tile
 
@@ -57,7 +60,7 @@ constexpr int TILE = MESH_TPB * CELLS_PER_THREAD;   // cells per scan tile
 // in the 4-bit fields of kTri[q], lowest first, three per triangle, ended by
 // 0xF.  The edge table is not stored: edge e is cut when its two corners
 // differ in the cube index.
-__constant__ unsigned long long kTri[256] = {
+__device__ const unsigned long long kTri[256] = {
     0xffffffffffffffffull, 0xfffffffffffff380ull, 0xfffffffffffff910ull, 0xffffffffff189381ull,
     0xfffffffffffffa21ull, 0xffffffffffa21380ull, 0xffffffffff920a29ull, 0xfffffff89a8a2382ull,
     0xfffffffffffff2b3ull, 0xffffffffff0b82b0ull, 0xffffffffffb32091ull, 0xfffffffb89b912b1ull,
@@ -126,42 +129,44 @@ __constant__ unsigned long long kTri[256] = {
 
 // Cube corners (Grid3d::getGridIndexVertices, grid3d.h:304-313): corner q at
 // (i + kCx[q], j + kCy[q], k + kCz[q]).
-__constant__ int kCx[8] = {0, 1, 1, 0, 0, 1, 1, 0};
-__constant__ int kCy[8] = {0, 0, 0, 0, 1, 1, 1, 1};
-__constant__ int kCz[8] = {0, 0, 1, 1, 0, 0, 1, 1};
+#define FLIP_CORNERS_X {0, 1, 1, 0, 0, 1, 1, 0}
+#define FLIP_CORNERS_Y {0, 0, 0, 0, 1, 1, 1, 1}
+#define FLIP_CORNERS_Z {0, 0, 1, 1, 0, 0, 1, 1}
+__constant__ int kCx[8] = FLIP_CORNERS_X;
+__constant__ int kCy[8] = FLIP_CORNERS_Y;
+__constant__ int kCz[8] = FLIP_CORNERS_Z;
 // Edges in the reference's order (polygonizer3d.cpp:495-630): the corners
 // interpolated from and to, the axis of the edge and the corner it starts
 // from along that axis (which names the edge in the grid of edges).
+#define FLIP_EDGE_DIR {0, 2, 0, 2, 0, 2, 0, 2, 1, 1, 1, 1}
+#define FLIP_EDGE_ORG {0, 1, 3, 0, 4, 5, 7, 4, 0, 1, 2, 3}
 __constant__ int kEa[12] = {0, 1, 2, 3, 4, 5, 6, 7, 0, 1, 2, 3};
 __constant__ int kEb[12] = {1, 2, 3, 0, 5, 6, 7, 4, 4, 5, 6, 7};
-__constant__ int kEdir[12] = {0, 2, 0, 2, 0, 2, 0, 2, 1, 1, 1, 1};
-__constant__ int kEorg[12] = {0, 1, 3, 0, 4, 5, 7, 4, 0, 1, 2, 3};
+__constant__ int kEdir[12] = FLIP_EDGE_DIR;
+__constant__ int kEorg[12] = FLIP_EDGE_ORG;
 
+// Edges whose two corners differ in the cube index: edges 0-3 join corner e of
+// the lower four with the next one round, 4-7 of the upper four, 8-11 a lower
+// corner with the one above.
 __device__ __forceinline__ unsigned cut_mask(int q) {
-    unsigned m = 0;
-#pragma unroll
-    for (int e = 0; e < 12; e++)
-        if (((q >> kEa[e]) ^ (q >> kEb[e])) & 1) m |= 1u << e;
-    return m;
+    const unsigned lo = q & 15, hi = (unsigned)q >> 4;
+    return (lo ^ (lo >> 1 | (lo & 1) << 3)) | (hi ^ (hi >> 1 | (hi & 1) << 3)) << 4 | (lo ^ hi) << 8;
 }
-__device__ __forceinline__ int tri_count(int q) {
-    const unsigned long long w = kTri[q];
-    int n = 0;
-    while (n < 16 && ((w >> (4 * n)) & 0xF) != 0xF) n++;
-    return n / 3;
+// A case's fields past its last triangle are all 0xF, and an edge id is below 12.
+__device__ __forceinline__ int tri_count(int q) { return (16 - __clzll(~(long long)kTri[q]) / 4) / 3; }
+// Edges that lie along an axis or start from its upper corner.
+__host__ __device__ constexpr unsigned edges_off(int axis) {
+    constexpr int c[3][8] = {FLIP_CORNERS_X, FLIP_CORNERS_Y, FLIP_CORNERS_Z}, dir[12] = FLIP_EDGE_DIR, org[12] = FLIP_EDGE_ORG;
+    unsigned m = 0;
+    for (int e = 0; e < 12; e++)
+        if (dir[e] == axis || c[axis][org[e]] == 1) m |= 1u << e;
+    return m;
 }
 // Edges that cell (i, j, k) creates: the first cell in flat order holding an
 // edge is the one below it in each perpendicular axis, where that cell exists.
 __device__ __forceinline__ unsigned created_mask(int i, int j, int k) {
-    unsigned m = 0;
-#pragma unroll
-    for (int e = 0; e < 12; e++) {
-        const int o = kEorg[e], d = kEdir[e];
-        const bool ok = (d == 0 || kCx[o] == 1 || i == 0) && (d == 1 || kCy[o] == 1 || j == 0) &&
-                        (d == 2 || kCz[o] == 1 || k == 0);
-        if (ok) m |= 1u << e;
-    }
-    return m;
+    constexpr unsigned x = edges_off(0), y = edges_off(1), z = edges_off(2);
+    return (i == 0 ? 0xfffu : x) & (j == 0 ? 0xfffu : y) & (k == 0 ? 0xfffu : z);
 }
 
 // Nodal solid level set at a point, in FP64 as Interpolation::
@@ -189,15 +194,55 @@ __device__ double solid_sample(const MeshFrame &m, const float *S, float px, flo
            p7 * x * y * z;
 }
 
+// The sign of solid_sample where it is plain, else 0: all nodes around the point
+// of one sign and within a factor of 20, far beyond what the rounding of the
+// weights (which add up to 1, none below -1e-3) can turn, or a value
+// interpolated in 32 bits of more than 1% of the largest of them.  The cell is
+// found in 32 bits, and where the point is within 0.01 of a cell's face, the
+// nodes of both cells count.  Spares nearly all of the FP64 interpolation: an
+// SM does two FP64 operations a cycle.
+__device__ __forceinline__ int solid_sign(const MeshFrame &m, const float *S, float px, float py, float pz) {
+    const float gx = px * m.invdxf, gy = py * m.invdxf, gz = pz * m.invdxf;
+    const int i0 = (int)floorf(gx - 0.01f), i1 = (int)floorf(gx + 0.01f) + 1, j0 = (int)floorf(gy - 0.01f),
+              j1 = (int)floorf(gy + 0.01f) + 1, k0 = (int)floorf(gz - 0.01f), k1 = (int)floorf(gz + 0.01f) + 1;
+    if (i0 < 0 || j0 < 0 || k0 < 0 || i1 > m.I || j1 > m.J || k1 > m.K) return 0;
+    const int ni = m.I + 1, nj = m.J + 1;
+    float lo = __uint_as_float(0x7f800000u), hi = -lo;
+    for (int k = k0; k <= k1; k++)
+        for (int j = j0; j <= j1; j++) {
+            const float *s = S + i0 + (long long)ni * (j + (long long)nj * k);
+            const float a = s[0], b = s[1], c = s[i1 - i0];
+            lo = fminf(fminf(lo, a), fminf(b, c));
+            hi = fmaxf(fmaxf(hi, a), fmaxf(b, c));
+        }
+    if (lo > fmaxf(0.05f * hi, 1e-20f)) return 1;
+    if (hi < fminf(0.05f * lo, -1e-20f)) return -1;
+    // mixed: by interpolation in 32 bits, where it is far from 0
+    const int i = min(max((int)floorf(gx), 0), m.I - 1), j = min(max((int)floorf(gy), 0), m.J - 1),
+              k = min(max((int)floorf(gz), 0), m.K - 1);
+    const float x = gx - (float)i, y = gy - (float)j, z = gz - (float)k;
+    const float *s = S + i + (long long)ni * (j + (long long)nj * k);
+    auto along = [&](const float *r) { return r[0] + x * (r[1] - r[0]); };
+    const float c0 = along(s), c1 = along(s + ni), c2 = along(s + (long long)ni * nj), c3 = along(s + (long long)ni * (nj + 1));
+    const float b0 = c0 + y * (c1 - c0), b1 = c2 + y * (c3 - c2), d = b0 + z * (b1 - b0);
+    const float sure = fmaxf(0.01f * fmaxf(hi, -lo), 1e-20f);
+    return d > sure ? 1 : (d < -sure ? -1 : 0);
+}
+
 // Is chunk node (a, b, c) a solid vertex (ScalarField::setSolidSDF,
 // scalarfield.cpp:372-395, MeshLevelSet::_trilinearInterpolateSolidGridPointsThread,
 // meshlevelset.cpp:309-340)?
-__device__ bool solid_vertex(const MeshFrame &m, const float *S, int a, int b, int c) {
+// -1: solid, 1: not, 0: the level set has to be interpolated there.
+__device__ __forceinline__ int solid_vertex_sign(const MeshFrame &m, const float *S, int a, int b, int c) {
     if (m.solidMode == 2)   // the scalar field's grid is the level set's
-        return S[(long long)a + (long long)(m.I + 1) * ((long long)b + (long long)(m.J + 1) * c)] < 0.0f;
+        return S[(long long)a + (long long)(m.I + 1) * ((long long)b + (long long)(m.J + 1) * c)] < 0.0f ? -1 : 1;
     if (m.solidMode == 1 && !(a & 1) && !(b & 1) && !(c & 1))   // subdivision 2 at offset 0: even nodes
-        return S[(long long)(a >> 1) + (long long)(m.I + 1) * ((long long)(b >> 1) + (long long)(m.J + 1) * (c >> 1))] <
-               0.0f;
+        return S[(long long)(a >> 1) + (long long)(m.I + 1) * ((long long)(b >> 1) + (long long)(m.J + 1) * (c >> 1))] < 0.0f
+                   ? -1
+                   : 1;
+    return solid_sign(m, S, (float)a * m.subdxf + m.offx, (float)b * m.subdxf + m.offy, (float)c * m.subdxf + m.offz);
+}
+__device__ bool solid_vertex_value(const MeshFrame &m, const float *S, int a, int b, int c) {
     const float px = __fadd_rn((float)((double)(float)a * m.subdx), m.offx);
     const float py = __fadd_rn((float)((double)(float)b * m.subdx), m.offy);
     const float pz = __fadd_rn((float)((double)(float)c * m.subdx), m.offz);
@@ -210,167 +255,337 @@ __device__ bool solid_vertex(const MeshFrame &m, const float *S, int a, int b, i
 // _initializeComputeChunkDataActiveBlocks, particlemesher.cpp:116-137).
 __global__ void k_mesh_occupancy(ParticleSoA p, int n, MeshFrame m, uint8_t *occ) {
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= n) return;
-    const int bi = exact_floor(p.px[t], m.invBlock, m.invBlockf), bj = exact_floor(p.py[t], m.invBlock, m.invBlockf),
-              bk = exact_floor(p.pz[t], m.invBlock, m.invBlockf);
-    if (bi >= 0 && bj >= 0 && bk >= 0 && bi < m.nbI && bj < m.nbJ && bk < m.nbK)
-        occ[bi + m.nbI * (bj + m.nbJ * bk)] = 1;
+    int at = -1;
+    if (t < n) {
+        const int bi = exact_floor(p.px[t], m.invBlock, m.invBlockf), bj = exact_floor(p.py[t], m.invBlock, m.invBlockf),
+                  bk = exact_floor(p.pz[t], m.invBlock, m.invBlockf);
+        if (bi >= 0 && bj >= 0 && bk >= 0 && bi < m.nbI && bj < m.nbJ && bk < m.nbK) at = bi + m.nbI * (bj + m.nbJ * bk);
+    }
+    // the lane before mostly has the same block to mark
+    const int before = __shfl_up_sync(0xffffffffu, at, 1);
+    if (at >= 0 && ((threadIdx.x & 31) == 0 || at != before)) occ[at] = 1;
 }
 
 // -------------------------------------------------------------- scalar field
-// One CTA per block of the chunk (chunk-frame block index = blockIdx).
-__global__ void __launch_bounds__(MESH_TPB) k_mesh_field(ParticleSoA p, const int *cellStart, MeshFrame m,
-                                                         const uint8_t *active, const float *solidPhi,
-                                                         float *field) {
-    __shared__ unsigned int smin[MB * MB * MB];
-    __shared__ float npos[MB];
-    __shared__ float4 recs[MESH_TPB / 32][32];   // per warp: a pass's particles {lx, ly, lz, box}
-    const int bx = blockIdx.x, by = blockIdx.y, bz = blockIdx.z;
-    for (int q = threadIdx.x; q < MB * MB * MB; q += blockDim.x) smin[q] = 0x7f800000u;   // +inf
-    if (threadIdx.x < MB) npos[threadIdx.x] = (float)((double)(float)threadIdx.x * m.subdx);
-    __syncthreads();
-    if (active[bx + m.cbI * (by + m.cbJ * bz)]) {
-        // block frame (_scalarFieldProducerThread, particlemesher.cpp:498-549)
-        const float bofx = (float)((double)(float)bx * m.blockdx), bofy = (float)((double)(float)by * m.blockdx),
-                    bofz = (float)((double)(float)bz * m.blockdx);
-        // candidate cells: every particle whose search box can overlap the
-        // block (its list holds no other), with slack for rounding
-        const double reach = (double)m.sr + 0.01 * m.dx;
-        const double lox = (double)m.offx + bx * m.blockdx - reach, hix = (double)m.offx + (bx + 1) * m.blockdx + reach;
-        const double loy = (double)m.offy + by * m.blockdx - reach, hiy = (double)m.offy + (by + 1) * m.blockdx + reach;
-        const double loz = (double)m.offz + bz * m.blockdx - reach, hiz = (double)m.offz + (bz + 1) * m.blockdx + reach;
-        const int x0 = max((int)floor(lox * m.invdx), 0), x1 = min((int)floor(hix * m.invdx), m.I - 1);
-        const int y0 = max((int)floor(loy * m.invdx), 0), y1 = min((int)floor(hiy * m.invdx), m.J - 1);
-        const int z0 = max((int)floor(loz * m.invdx), 0), z1 = min((int)floor(hiz * m.invdx), m.K - 1);
-        const int ny = y1 - y0 + 1, nrows = x1 >= x0 ? ny * (z1 - z0 + 1) : 0;
-        const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
-        const float sr = m.sr;
-        float4 *wrec = recs[warp];
-        // col / n = (col * ceil(2^11 / n)) >> 11, exact for n <= MB and
-        // col < n * MB; lane n holds the multiplier
-        const int divLane = lane > 0 ? (2048 + lane - 1) / lane : 0;
-        for (int row = warp; row < nrows; row += nwarps) {
-            const int cy = y0 + row % ny, cz = z0 + row / ny;
-            const long long rbase = (long long)m.I * (cy + (long long)m.J * cz);
-            const int pb = cellStart[rbase + x0], pe = cellStart[rbase + x1 + 1];
-            for (int base = pb; base < pe; base += 32) {
-                // phase 1, a lane per particle: is it in this block's list,
-                // and which of the block's nodes does its box cover
-                const int t = base + lane;
-                int ncol = 0, na = 0;
-                float4 rec = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-                unsigned packed = 0;
-                if (t < pe) {
-                    const float px = p.px[t], py = p.py[t], pz = p.pz[t];
-                    // the chunk's box, expanded (particlemesher.cpp:287-301, aabb.cpp:122-133)
-                    const bool in = px >= m.bbx && py >= m.bby && pz >= m.bbz && (double)px < (double)m.bbx + m.bbw &&
-                                    (double)py < (double)m.bby + m.bbh && (double)pz < (double)m.bbz + m.bbd;
-                    const float cx = __fsub_rn(px, m.offx), cy2 = __fsub_rn(py, m.offy), cz2 = __fsub_rn(pz, m.offz);
-                    // the count pass's block lists (particlemesher.cpp:400-446)
-                    const int oi = exact_floor(cx, m.invBlockF, m.invBlockFf),
-                              oj = exact_floor(cy2, m.invBlockF, m.invBlockFf),
-                              ok = exact_floor(cz2, m.invBlockF, m.invBlockFf);
-                    const float bpx = (float)((double)(float)oi * (double)m.blockdxF),
-                                bpy = (float)((double)(float)oj * (double)m.blockdxF),
-                                bpz = (float)((double)(float)ok * (double)m.blockdxF);
-                    bool mine;
-                    if (__fsub_rn(cx, sr) > bpx && __fsub_rn(cy2, sr) > bpy && __fsub_rn(cz2, sr) > bpz &&
-                        __fadd_rn(cx, sr) < __fadd_rn(bpx, m.blockdxF) &&
-                        __fadd_rn(cy2, sr) < __fadd_rn(bpy, m.blockdxF) &&
-                        __fadd_rn(cz2, sr) < __fadd_rn(bpz, m.blockdxF)) {
-                        mine = oi == bx && oj == by && ok == bz;
-                    } else {
-                        const int i0 = exact_floor(__fsub_rn(cx, sr), m.invBlockF, m.invBlockFf),
-                                  i1 = exact_floor(__fadd_rn(cx, sr), m.invBlockF, m.invBlockFf);
-                        const int j0 = exact_floor(__fsub_rn(cy2, sr), m.invBlockF, m.invBlockFf),
-                                  j1 = exact_floor(__fadd_rn(cy2, sr), m.invBlockF, m.invBlockFf);
-                        const int k0 = exact_floor(__fsub_rn(cz2, sr), m.invBlockF, m.invBlockFf),
-                                  k1 = exact_floor(__fadd_rn(cz2, sr), m.invBlockF, m.invBlockFf);
-                        mine = bx >= i0 && bx <= i1 && by >= j0 && by <= j1 && bz >= k0 && bz <= k1;
-                    }
-                    if (in && mine) {
-                        const float lx = __fsub_rn(cx, bofx), ly = __fsub_rn(cy2, bofy), lz = __fsub_rn(cz2, bofz);
-                        const int a0 = max(exact_floor(__fsub_rn(lx, sr), m.invsub, m.invsubf), 0);
-                        const int b0 = max(exact_floor(__fsub_rn(ly, sr), m.invsub, m.invsubf), 0);
-                        const int c0 = max(exact_floor(__fsub_rn(lz, sr), m.invsub, m.invsubf), 0);
-                        const int a1 = min(exact_floor(__fadd_rn(lx, sr), m.invsub, m.invsubf) + 1, MB - 1);
-                        const int b1 = min(exact_floor(__fadd_rn(ly, sr), m.invsub, m.invsubf) + 1, MB - 1);
-                        const int c1 = min(exact_floor(__fadd_rn(lz, sr), m.invsub, m.invsubf) + 1, MB - 1);
-                        if (a1 >= a0 && b1 >= b0 && c1 >= c0) {
-                            na = a1 - a0 + 1;
-                            ncol = na * (b1 - b0 + 1);
-                            packed = (unsigned)a0 | (unsigned)na << 4 | (unsigned)b0 << 8 | (unsigned)c0 << 12 |
-                                     (unsigned)c1 << 16;
-                            rec = make_float4(lx, ly, lz, 0.0f);
-                        }
-                    }
-                }
-                const unsigned div = (unsigned)__shfl_sync(0xffffffffu, divLane, na);
-                if (ncol > 0) {
-                    rec.w = __uint_as_float(packed | div << 20);
-                    wrec[lane] = rec;
-                }
-                int incl = ncol;   // inclusive prefix sum of the column counts over the lanes
+// Does the reference's scatter take particle p to node (a, b, c) of block
+// (bx, by, bz)?  The count pass's block lists (particlemesher.cpp:400-446) and
+// the particle's node box in the block's frame; cx..cz: p in the chunk's frame,
+// lx..lz: in the block's.
+__device__ __noinline__ bool field_reaches(const MeshFrame &m, float cx, float cy, float cz, float lx, float ly, float lz,
+                                           int bx, int by, int bz, int a, int b, int c) {
+    const float sr = m.sr;
+    const int oi = exact_floor(cx, m.invBlockF, m.invBlockFf), oj = exact_floor(cy, m.invBlockF, m.invBlockFf),
+              ok = exact_floor(cz, m.invBlockF, m.invBlockFf);
+    const float bpx = (float)((double)(float)oi * (double)m.blockdxF), bpy = (float)((double)(float)oj * (double)m.blockdxF),
+                bpz = (float)((double)(float)ok * (double)m.blockdxF);
+    bool mine;
+    if (__fsub_rn(cx, sr) > bpx && __fsub_rn(cy, sr) > bpy && __fsub_rn(cz, sr) > bpz &&
+        __fadd_rn(cx, sr) < __fadd_rn(bpx, m.blockdxF) && __fadd_rn(cy, sr) < __fadd_rn(bpy, m.blockdxF) &&
+        __fadd_rn(cz, sr) < __fadd_rn(bpz, m.blockdxF)) {
+        mine = oi == bx && oj == by && ok == bz;
+    } else {
+        mine = bx >= exact_floor(__fsub_rn(cx, sr), m.invBlockF, m.invBlockFf) &&
+               bx <= exact_floor(__fadd_rn(cx, sr), m.invBlockF, m.invBlockFf) &&
+               by >= exact_floor(__fsub_rn(cy, sr), m.invBlockF, m.invBlockFf) &&
+               by <= exact_floor(__fadd_rn(cy, sr), m.invBlockF, m.invBlockFf) &&
+               bz >= exact_floor(__fsub_rn(cz, sr), m.invBlockF, m.invBlockFf) &&
+               bz <= exact_floor(__fadd_rn(cz, sr), m.invBlockF, m.invBlockFf);
+    }
+    return mine && a >= exact_floor(__fsub_rn(lx, sr), m.invsub, m.invsubf) &&
+           a <= exact_floor(__fadd_rn(lx, sr), m.invsub, m.invsubf) + 1 &&
+           b >= exact_floor(__fsub_rn(ly, sr), m.invsub, m.invsubf) &&
+           b <= exact_floor(__fadd_rn(ly, sr), m.invsub, m.invsubf) + 1 &&
+           c >= exact_floor(__fsub_rn(lz, sr), m.invsub, m.invsubf) &&
+           c <= exact_floor(__fadd_rn(lz, sr), m.invsub, m.invsubf) + 1;
+}
+
+// The reference scatters every particle over the nodes of its search box
+// (hundreds of them); a node's value is that of its nearest particle, since the
+// rounded square root and the subtraction of r are monotone.  So a node looks
+// for it.  A Seeker holds what a search needs of its node and tests particles.
+template <bool SIGN>
+struct Seeker {
+    const ParticleSoA &p;
+    const MeshFrame &m;
+    int A, B, C;
+    float bofx, bofy, bofz, nx, ny, nz;   // the frame of the node's block, the node there
+    float px, py, pz;                     // the node in the simulation's frame
+    float best;                           // SIGN: best < 0 once one nearer than r is found
+    __device__ Seeker(const ParticleSoA &p_, const MeshFrame &m_, int A_, int B_, int C_)
+        : p(p_), m(m_), A(A_), B(B_), C(C_) {
+        const int bx = A / MB, by = B / MB, bz = C / MB;
+        bofx = m.blockPos[0][bx];
+        bofy = m.blockPos[1][by];
+        bofz = m.blockPos[2][bz];
+        nx = m.nodePos[A - bx * MB];
+        ny = m.nodePos[B - by * MB];
+        nz = m.nodePos[C - bz * MB];
+        px = m.offx + (float)A * m.subdxf;
+        py = m.offy + (float)B * m.subdxf;
+        pz = m.offz + (float)C * m.subdxf;
+        best = SIGN ? m.signReach * m.signReach : __uint_as_float(0x7f800000u);
+    }
+    // squared distance in the frame of the node's block, as the reference finds
+    // it (_scalarFieldProducerThread, particlemesher.cpp:498-549)
+    __device__ float dist2(float qx, float qy, float qz) const {
+        const float dx = __fsub_rn(nx, __fsub_rn(__fsub_rn(qx, m.offx), bofx)),
+                    dy = __fsub_rn(ny, __fsub_rn(__fsub_rn(qy, m.offy), bofy)),
+                    dz = __fsub_rn(nz, __fsub_rn(__fsub_rn(qz, m.offz), bofz));
+        return __fadd_rn(__fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy)), __fmul_rn(dz, dz));
+    }
+    // the chunk's box, expanded (particlemesher.cpp:287-301, aabb.cpp:122-133)
+    __device__ bool in_box(float qx, float qy, float qz) const {
+        return qx >= m.bbx && qy >= m.bby && qz >= m.bbz && qx < m.bhx && qy < m.bhy && qz < m.bhz;
+    }
+    __device__ void test(float qx, float qy, float qz) {
+        const float d2 = dist2(qx, qy, qz);
+        if (!(d2 < best) || (SIGN && !(__fsqrt_rn(d2) < m.r)) || !in_box(qx, qy, qz)) return;
+        if (!(d2 < m.near2)) {
+            const float cx = __fsub_rn(qx, m.offx), cy = __fsub_rn(qy, m.offy), cz = __fsub_rn(qz, m.offz);
+            const int bx = A / MB, by = B / MB, bz = C / MB;
+            if (!field_reaches(m, cx, cy, cz, __fsub_rn(cx, bofx), __fsub_rn(cy, bofy), __fsub_rn(cz, bofz), bx, by, bz,
+                               A - bx * MB, B - by * MB, C - bz * MB))
+                return;
+        }
+        best = SIGN ? -1.0f : d2;
+    }
+    __device__ void look(int from, int to, int step) {   // particles from, from + step, ...
+        for (int t = from; t < to; t += 4 * step) {
+            float qx[4], qy[4], qz[4];
 #pragma unroll
-                for (int o = 1; o < 32; o <<= 1) {
-                    const int v = __shfl_up_sync(0xffffffffu, incl, o);
-                    if (lane >= o) incl += v;
-                }
-                const int total = __shfl_sync(0xffffffffu, incl, 31);
-                __syncwarp();
-                // phase 2, a lane per (particle, column of its box along k):
-                // the lanes of one step walk distinct columns
-                for (int first = 0; first < total; first += 32) {
-                    const int item = first + lane;
-                    int L = 0;   // the smallest lane whose inclusive sum exceeds item
-#pragma unroll
-                    for (int step = 16; step > 0; step >>= 1)
-                        if (__shfl_sync(0xffffffffu, incl, L + step - 1) <= item) L += step;
-                    const int startL = __shfl_sync(0xffffffffu, incl, L) - __shfl_sync(0xffffffffu, ncol, L);
-                    if (item < total) {
-                        const float4 pr = wrec[L];
-                        const unsigned w = __float_as_uint(pr.w);
-                        const int a0 = w & 15, nA = (w >> 4) & 15, b0 = (w >> 8) & 15;
-                        const int c0 = (w >> 12) & 15, c1 = (w >> 16) & 15;
-                        const int col = item - startL;
-                        const int bq = (col * (int)(w >> 20)) >> 11;   // col / nA
-                        const int aa = a0 + col - bq * nA, bb = b0 + bq;
-                        const float ddx = __fsub_rn(npos[aa], pr.x);
-                        const float dy = __fsub_rn(npos[bb], pr.y);
-                        const float dxy = __fadd_rn(__fmul_rn(ddx, ddx), __fmul_rn(dy, dy));
-                        unsigned int *dst = &smin[aa + MB * (bb + MB * c0)];
-                        for (int cc = c0; cc <= c1; cc++, dst += MB * MB) {
-                            const float dz = __fsub_rn(npos[cc], pr.z);
-                            atomicMin(dst, __float_as_uint(__fadd_rn(dxy, __fmul_rn(dz, dz))));
-                        }
-                    }
-                }
-                __syncwarp();
+            for (int q = 0; q < 4; q++) {   // four at a time, so that their loads overlap
+                const int tq = t + q * step < to ? t + q * step : t;
+                qx[q] = p.px[tq];
+                qy[q] = p.py[tq];
+                qz[q] = p.pz[tq];
             }
+            // a first look in plain coordinates; `slack` is far above what
+            // their rounding and the block frame's make of a squared distance
+            bool hit = false;
+            const float bar = best + m.slack;
+#pragma unroll
+            for (int q = 0; q < 4; q++) {
+                const float ex = qx[q] - px, ey = qy[q] - py, ez = qz[q] - pz;
+                hit |= __fmaf_rn(ez, ez, __fmaf_rn(ey, ey, ex * ex)) < bar;
+            }
+            if (!hit) continue;
+            // the nearest of the four; below near2 its list and box surely hold
+            // the node, which leaves nothing to look up
+            float d2 = dist2(qx[0], qy[0], qz[0]), x = qx[0], y = qy[0], z = qz[0];
+#pragma unroll
+            for (int q = 1; q < 4; q++) {
+                const float e2 = dist2(qx[q], qy[q], qz[q]);
+                const bool nearer = e2 < d2;
+                d2 = nearer ? e2 : d2;
+                x = nearer ? qx[q] : x;
+                y = nearer ? qy[q] : y;
+                z = nearer ? qz[q] : z;
+            }
+            if (!(d2 < best)) continue;
+            if (d2 < m.near2 && in_box(x, y, z)) {
+                if (!SIGN) best = d2;
+                else if (__fsqrt_rn(d2) < m.r) best = -1.0f;
+            } else {
+                for (int q = 0; q < 4; q++)
+                    if (t + q * step < to) test(p.px[t + q * step], p.py[t + q * step], p.pz[t + q * step]);
+            }
+            if (SIGN && best < 0.0f) return;
         }
     }
-    __syncthreads();
-    for (int q = threadIdx.x; q < MB * MB * MB; q += blockDim.x) {
-        const int a = MB * bx + q % MB, b = MB * by + (q / MB) % MB, c = MB * bz + q / (MB * MB);
-        if (a >= m.ni || b >= m.nj || c >= m.nk) continue;
-        const unsigned int s = smin[q];
-        const float d = s == 0x7f800000u ? m.maxd : fminf(m.maxd, __fsub_rn(__fsqrt_rn(__uint_as_float(s)), m.r));
-        float f = -d;
-        if (f > 0.0f && solid_vertex(m, solidPhi, a, b, c)) f = 0.0f;
-        field[(long long)a + (long long)m.ni * ((long long)b + (long long)m.nj * c)] = f;
+};
+
+// A search by GROUP lanes (all of a group call it with the same node): its own
+// cell together, then the rows of cells around it, nearest first, a row a lane,
+// as long as one can hold a nearer particle.  Returns the squared distance to
+// the nearest particle, +inf without one; with SIGN 0 if one is nearer than r,
+// else +inf.  Particles beyond near2 have to be looked up in the lists, with
+// FP64: a first pass leaves them out, and mostly finds a nearer one.
+template <bool SIGN, int GROUP>
+__device__ float nearest(const ParticleSoA &p, const int *cellStart, const MeshFrame &m, int A, int B, int C) {
+    const float kInf = __uint_as_float(0x7f800000u);
+    const int lane = threadIdx.x & 31, g = lane & (GROUP - 1);
+    const unsigned group = ((1u << GROUP) - 1) << (lane - g);
+    Seeker<SIGN> sk(p, m, A, B, C);
+    // the cell the node lies in and its place there, in cells
+    const float gx = m.cellAt(m.offx, A), gy = m.cellAt(m.offy, B), gz = m.cellAt(m.offz, C);
+    const int i = (int)floorf(gx), j = (int)floorf(gy), k = (int)floorf(gz);
+    const float fy = gy - (float)j, fz = gz - (float)k;
+    auto least = [&]() {
+#pragma unroll
+        for (int o = GROUP / 2; o > 0; o >>= 1) sk.best = fminf(sk.best, __shfl_xor_sync(group, sk.best, o));
+    };
+    // squared distance along an axis to the cells o away, less a margin far
+    // above the rounding of the positions
+    auto away = [&](int o, float f) {
+        const float d = fmaxf((o > 0 ? (float)o - f : (o < 0 ? f - (float)(o + 1) : 0.0f)) - 0.01f, 0.0f) * m.dxf;
+        return d * d;
+    };
+    const int sy = fy < 0.5f ? -1 : 1, sz = fz < 0.5f ? -1 : 1;   // towards the nearer side
+    const float all = sk.best;
+#pragma unroll 1
+    for (int pass = 0; pass < 2; pass++) {
+        const float bound = pass == 0 ? fminf(all, m.near2) : all;
+        sk.best = bound;
+        if (i < m.I && j < m.J && k < m.K) {
+            const long long own = i + (long long)m.I * (j + (long long)m.J * k);
+            sk.look(cellStart[own] + g, cellStart[own + 1], GROUP);
+        }
+        __syncwarp(group);
+        least();
+#pragma unroll 1
+        for (int n0 = 0; n0 < m.nrows && m.rows[n0].least < sk.best; n0 += GROUP) {
+            if (n0 + g < m.nrows) {
+                const MeshRow row = m.rows[n0 + g];
+                const int oy = sy * row.y, oz = sz * row.z, y = j + oy, z = k + oz;
+                const float d = away(oy, fy) + away(oz, fz);
+                if (d < sk.best && y >= 0 && z >= 0 && y < m.J && z < m.K) {
+                    // how far along the row a nearer particle can be
+                    const float w = fminf(sqrtf(sk.best - d), m.reach) * m.invdxf + 0.02f;
+                    const int x0 = max((int)floorf(gx - w), 0), x1 = min((int)floorf(gx + w), m.I - 1);
+                    const long long base = (long long)m.I * (y + (long long)m.J * z);
+                    if (x0 <= x1) sk.look(cellStart[base + x0], cellStart[base + x1 + 1], 1);
+                }
+            }
+            __syncwarp(group);
+            least();
+        }
+        if (sk.best < bound) return SIGN ? 0.0f : sk.best;
+        if (bound == all) break;
+    }
+    return kInf;
+}
+__device__ __forceinline__ bool block_active(const MeshFrame &m, const uint8_t *active, int A, int B, int C) {
+    return active[A / MB + m.cbI * (B / MB + m.cbJ * (C / MB))];
+}
+
+// Cells with a particle as bits, 32 along x to a word (a warp a word), and the
+// cells with one within R cells of them along each axis: nodes elsewhere are
+// outside without a search, most of the air.
+__global__ void __launch_bounds__(MESH_TPB) k_mesh_occupied(const int *cellStart, MeshFrame m, unsigned *occupied) {
+    const long long word = (long long)blockIdx.x * (MESH_TPB / 32) + (threadIdx.x >> 5);
+    if (word >= (long long)m.wpc * m.J * m.K) return;
+    int wx, j, k;
+    unflatten(word, m.wpc, m.J, wx, j, k);
+    const int i = wx * 32 + (threadIdx.x & 31);
+    const int *s = cellStart + i + (long long)m.I * (j + (long long)m.J * k);
+    const unsigned w = __ballot_sync(0xffffffffu, i < m.I && s[0] != s[1]);
+    if ((threadIdx.x & 31) == 0) occupied[word] = w;
+}
+__global__ void __launch_bounds__(MESH_TPB) k_mesh_around(MeshFrame m, const unsigned *occupied, int R, unsigned *around) {
+    const long long word = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (word >= (long long)m.wpc * m.J * m.K) return;
+    int wx, j, k;
+    unflatten(word, m.wpc, m.J, wx, j, k);
+    unsigned w = 0, below = 0, above = 0;   // the rows' words together
+    for (int z = max(k - R, 0); z <= min(k + R, m.K - 1); z++)
+        for (int y = max(j - R, 0); y <= min(j + R, m.J - 1); y++) {
+            const unsigned *row = occupied + (long long)m.wpc * (y + (long long)m.J * z);
+            w |= row[wx];
+            if (wx > 0) below |= row[wx - 1];
+            if (wx + 1 < m.wpc) above |= row[wx + 1];
+        }
+    unsigned out = w;
+    for (int q = 1; q <= R; q++) out |= __funnelshift_l(below, w, q) | __funnelshift_r(w, above, q);
+    around[word] = out;
+}
+
+__device__ __forceinline__ bool near_particles(const MeshFrame &m, const unsigned *around, int A, int B, int C) {
+    if (!around) return true;
+    const int i = min((int)m.cellAt(m.offx, A), m.I - 1), j = min((int)m.cellAt(m.offy, B), m.J - 1),
+              k = min((int)m.cellAt(m.offz, C), m.K - 1);
+    return around[(i >> 5) + (long long)m.wpc * (j + (long long)m.J * k)] >> (i & 31) & 1u;
+}
+
+// Which nodes are inside (field above the threshold, not solid), as bits, 32
+// along x to a word: all that the polygoniser asks of a node, but for those at
+// the ends of a cut edge.  A warp a word.  A lane looks at its node's own cell,
+// which decides nearly all nodes of the liquid; the air is decided without
+// particles; the nodes left, near the surface, are searched by groups of lanes.
+// Nodes where the solid level set has to be interpolated in FP64, a few at the
+// walls' ends of many rows, go to a list (as long as it has room) for
+// k_mesh_walls, which works on full warps.
+// Bound by the searches near the surface and their latency: 345 us at 128^3,
+// subdivision 2 (17M nodes), where scattering every particle over its box took
+// 2250 us for all values; 21 us at 71x59x83, subdivision 1.
+__global__ void __launch_bounds__(SEARCH_TPB, 1024 / SEARCH_TPB) k_mesh_inside(ParticleSoA p, const int *cellStart, MeshFrame m,
+                                                                               const uint8_t *active, const unsigned *around,
+                                                                               const float *solidPhi, unsigned *inside,
+                                                                               int *walls, int room, int *nwalls) {
+    __shared__ int lists[SEARCH_TPB];
+    __shared__ unsigned founds[SEARCH_TPB / 32];
+    const int lane = threadIdx.x & 31;
+    int *list = lists + (threadIdx.x - lane);
+    unsigned *found = founds + (threadIdx.x >> 5);
+    const long long word = (long long)blockIdx.x * (SEARCH_TPB / 32) + (threadIdx.x >> 5);
+    if (word >= (long long)m.wpr * m.nj * m.nk) return;
+    int wx, B, C;
+    unflatten(word, m.wpr, m.nj, wx, B, C);
+    const int A = wx * 32 + lane;
+    bool in = false, open = false;
+    if (A < m.ni && block_active(m, active, A, B, C) && near_particles(m, around, A, B, C)) {
+        Seeker<true> sk(p, m, A, B, C);
+        const int i = (int)floorf(m.cellAt(m.offx, A)), j = (int)floorf(m.cellAt(m.offy, B)), k = (int)floorf(m.cellAt(m.offz, C));
+        if (i < m.I && j < m.J && k < m.K) {
+            const long long own = i + (long long)m.I * (j + (long long)m.J * k);
+            sk.look(cellStart[own], cellStart[own + 1], 1);
+        }
+        in = sk.best < 0.0f;
+        open = !in;
+    }
+    const unsigned opens = __ballot_sync(0xffffffffu, open);
+    if (opens) {
+        if (open) list[__popc(opens & ((1u << lane) - 1u))] = lane;
+        if (lane == 0) *found = 0;
+        __syncwarp();
+        for (int n = lane / 4; n < __popc(opens); n += 8) {
+            const int t = list[n];
+            if (nearest<true, 4>(p, cellStart, m, wx * 32 + t, B, C) == 0.0f && lane % 4 == 0) atomicOr(found, 1u << t);
+        }
+        __syncwarp();
+        in |= *found >> lane & 1u;
+    }
+    int sign = in ? solid_vertex_sign(m, solidPhi, A, B, C) : -1;
+    if (sign == 0) {
+        const int at = atomicAdd(nwalls, 1);
+        if (at < room) walls[at] = (int)(word * 32 + lane);
+        else sign = solid_vertex_value(m, solidPhi, A, B, C) ? -1 : 1;
+    }
+    const unsigned w = __ballot_sync(0xffffffffu, sign > 0);
+    if (lane == 0) inside[word] = w;
+}
+__global__ void __launch_bounds__(MESH_TPB) k_mesh_walls(MeshFrame m, const float *solidPhi, const int *walls, int room,
+                                                         const int *nwalls, unsigned *inside) {
+    const int n = min(*nwalls, room);
+    for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < n; q += gridDim.x * blockDim.x) {
+        const unsigned t = (unsigned)walls[q];
+        int wx, b, c;
+        unflatten(t >> 5, m.wpr, m.nj, wx, b, c);
+        if (!solid_vertex_value(m, solidPhi, wx * 32 + (int)(t & 31), b, c)) atomicOr(&inside[t >> 5], 1u << (t & 31));
     }
 }
 
 // ------------------------------------------------------------------- cells
-__device__ __forceinline__ float fld(const MeshFrame &m, const float *F, int a, int b, int c) {
-    return F[(long long)a + (long long)m.ni * ((long long)b + (long long)m.nj * c)];
+__device__ __forceinline__ unsigned inside_bit(const MeshFrame &m, const unsigned *inside, int a, int b, int c) {
+    return inside[(a >> 5) + (long long)m.wpr * ((long long)b + (long long)m.nj * c)] >> (a & 31) & 1u;
 }
-__device__ __forceinline__ int cube_index(const MeshFrame &m, const float *F, int i, int j, int k) {
-    int q = 0;
-#pragma unroll
-    for (int v = 0; v < 8; v++)
-        if (fld(m, F, i + kCx[v], j + kCy[v], k + kCz[v]) > 0.0f) q |= 1 << v;
-    return q;
+// A node's field value: of its nearest particle, 0 in the solid.
+template <int GROUP>
+__device__ float node_value(const ParticleSoA &p, const int *cellStart, const MeshFrame &m, const uint8_t *active,
+                            const unsigned *inside, int a, int b, int c) {
+    const float kInf = __uint_as_float(0x7f800000u);
+    const float best = block_active(m, active, a, b, c) ? nearest<false, GROUP>(p, cellStart, m, a, b, c) : kInf;
+    const float f = -(best == kInf ? m.maxd : fminf(m.maxd, __fsub_rn(__fsqrt_rn(best), m.r)));
+    return f > 0.0f && !inside_bit(m, inside, a, b, c) ? 0.0f : f;
+}
+__device__ __forceinline__ int cube_index(const MeshFrame &m, const unsigned *inside, int i, int j, int k) {
+    const unsigned *row = inside + (i >> 5) + (long long)m.wpr * ((long long)j + (long long)m.nj * k);
+    const bool across = (i & 31) == 31;
+    auto pair = [&](long long o) {   // nodes i and i + 1 of a row
+        return across ? row[o] >> 31 | (row[o + 1] & 1u) << 1 : row[o] >> (i & 31) & 3u;
+    };
+    // corners 0 1 / 3 2 below, 4 5 / 7 6 above (kCx, kCy, kCz)
+    const unsigned a = pair(0), b = pair((long long)m.wpr * m.nj), c = pair(m.wpr), d = pair((long long)m.wpr * (m.nj + 1));
+    return (int)(a | (b >> 1) << 2 | (b & 1) << 3 | c << 4 | (d >> 1) << 6 | (d & 1) << 7);
 }
 
 // inclusive warp scan of int2, then the block's exclusive prefix and total
@@ -396,18 +611,20 @@ __device__ int2 block_scan_int2(int2 v, int2 *total) {
     return make_int2(before.x + x.x - v.x, before.y + x.y - v.y);
 }
 
-// Per cell: cube index; per tile: vertices created and triangles.
-__global__ void __launch_bounds__(MESH_TPB) k_mesh_count(MeshFrame m, const float *F, long long ncells,
+// Per cell: cube index; per tile: vertices created and triangles (their order
+// within a tile does not matter here, so neighbouring threads take
+// neighbouring cells).
+__global__ void __launch_bounds__(MESH_TPB) k_mesh_count(MeshFrame m, const unsigned *inside, long long ncells,
                                                          uint8_t *cube, int2 *tileSums) {
-    const long long base = (long long)blockIdx.x * TILE + (long long)threadIdx.x * CELLS_PER_THREAD;
+    const long long base = (long long)blockIdx.x * TILE + threadIdx.x;
     int2 own = make_int2(0, 0);
     const int ci = m.ni - 1, cj = m.nj - 1;
     for (int q = 0; q < CELLS_PER_THREAD; q++) {
-        const long long c = base + q;
+        const long long c = base + q * MESH_TPB;
         if (c >= ncells) break;
         int i, j, k;
         unflatten(c, ci, cj, i, j, k);
-        const int cq = cube_index(m, F, i, j, k);
+        const int cq = cube_index(m, inside, i, j, k);
         cube[c] = (uint8_t)cq;
         if (cq != 0 && cq != 255) {
             own.x += __popc(cut_mask(cq) & created_mask(i, j, k));
@@ -421,20 +638,30 @@ __global__ void __launch_bounds__(MESH_TPB) k_mesh_count(MeshFrame m, const floa
 
 // Exclusive scan of the tile sums in place (one CTA, any number of tiles);
 // the totals to totals[0..1].
-__global__ void k_mesh_scan_tiles(int2 *tileSums, int ntiles, int *totals) {
-    __shared__ int2 carry;
-    if (threadIdx.x == 0) carry = make_int2(0, 0);
-    __syncthreads();
-    for (int b0 = 0; b0 < ntiles; b0 += MESH_TPB) {
-        const int t = b0 + threadIdx.x;
-        const int2 v = t < ntiles ? tileSums[t] : make_int2(0, 0);
+__global__ void __launch_bounds__(MESH_TPB) k_mesh_scan_tiles(int2 *tileSums, int ntiles, int *totals) {
+    constexpr int PER = 8;
+    int2 carry = make_int2(0, 0);
+    for (int b0 = 0; b0 < ntiles; b0 += MESH_TPB * PER) {
+        const int t0 = b0 + threadIdx.x * PER;
+        int2 v[PER], own = make_int2(0, 0);
+#pragma unroll
+        for (int q = 0; q < PER; q++) {
+            v[q] = t0 + q < ntiles ? tileSums[t0 + q] : make_int2(0, 0);
+            own.x += v[q].x;
+            own.y += v[q].y;
+        }
         int2 tot;
-        const int2 ex = block_scan_int2(v, &tot);
-        const int2 cr = carry;
-        if (t < ntiles) tileSums[t] = make_int2(cr.x + ex.x, cr.y + ex.y);
-        __syncthreads();
-        if (threadIdx.x == 0) carry = make_int2(cr.x + tot.x, cr.y + tot.y);
-        __syncthreads();
+        int2 run = block_scan_int2(own, &tot);
+        run.x += carry.x;
+        run.y += carry.y;
+#pragma unroll
+        for (int q = 0; q < PER; q++) {
+            if (t0 + q < ntiles) tileSums[t0 + q] = run;
+            run.x += v[q].x;
+            run.y += v[q].y;
+        }
+        carry.x += tot.x;
+        carry.y += tot.y;
     }
     if (threadIdx.x == 0) {
         totals[0] = carry.x;
@@ -445,14 +672,10 @@ __global__ void k_mesh_scan_tiles(int2 *tileSums, int ntiles, int *totals) {
 // Polygonizer3d::_vertexInterp (polygonizer3d.cpp:455-491): the point where
 // the field crosses the threshold on the edge from corner 1 to corner 2,
 // kept on the liquid side of a solid crossing.
-__device__ void vertex_interp(const MeshFrame &m, const float *S, float p1x, float p1y, float p1z, float p2x,
-                              float p2y, float p2z, double v1, double v2, float *out) {
+__device__ void vertex_interp(float p1x, float p1y, float p1z, float p2x, float p2y, float p2z, double v1, double v2,
+                              double s1, double s2, float *out) {
     double minmu = 0.0, maxmu = 1.0;
     const double eps = 1e-10;
-    const double s1 = (double)(float)solid_sample(m, S, __fadd_rn(p1x, m.offx), __fadd_rn(p1y, m.offy),
-                                                  __fadd_rn(p1z, m.offz));
-    const double s2 = (double)(float)solid_sample(m, S, __fadd_rn(p2x, m.offx), __fadd_rn(p2y, m.offy),
-                                                  __fadd_rn(p2z, m.offz));
     if ((s1 < 0.0 && s2 >= 0.0) || (s2 < 0.0 && s1 >= 0.0)) {
         const double diff = s2 - s1;
         if (fabs(diff) > eps) {
@@ -474,61 +697,118 @@ __device__ void vertex_interp(const MeshFrame &m, const float *S, float p1x, flo
     out[2] = __fadd_rn(p1z, __fmul_rn(fm, __fsub_rn(p2z, p1z)));
 }
 
-// Every cell's first vertex and triangle; the vertices it creates, moved to
-// the simulation's frame (translate by the chunk offset, scale, unscale:
-// particlemesher.cpp:35-55, 271-280).
-__global__ void __launch_bounds__(MESH_TPB) k_mesh_vertices(MeshFrame m, const float *F, const float *S,
-                                                            long long ncells, const uint8_t *cube,
-                                                            const int2 *tileBase, int *vstart, int *tstart,
-                                                            float *verts) {
+// Numbers the vertices and triangles: the first vertex of every cell that the
+// surface cuts, and for each vertex and triangle where it comes from (cell *
+// 16 + edge, cell * 16 + number in the cell), as the first two words of the
+// place its kernel will fill.  Vertices and triangles are thin on the ground
+// (one cell in twenty), so a thread each afterwards keeps the warps full,
+// where a kernel over the cells had a few lanes at work.
+// With one kernel over the cells for all of it, the numbering and the vertices
+// took 1240 us and the triangles 283 us at 128^3, subdivision 2 (209k
+// vertices); now 45 us for the numbers, 84 for the vertices, 13 for the
+// triangles.
+__device__ __forceinline__ void put_origin(int *o, long long code) {
+    o[0] = (int)(unsigned)code;
+    o[1] = (int)(code >> 32);
+}
+__device__ __forceinline__ long long get_origin(const int *o) {
+    return (long long)((unsigned long long)(unsigned)o[0] | (unsigned long long)(unsigned)o[1] << 32);
+}
+__global__ void __launch_bounds__(MESH_TPB) k_mesh_number(MeshFrame m, long long ncells, const uint8_t *cube,
+                                                          const int2 *tileBase, int *vstart, int *verts, int *tris) {
     const long long base = (long long)blockIdx.x * TILE + (long long)threadIdx.x * CELLS_PER_THREAD;
     const int ci = m.ni - 1, cj = m.nj - 1;
+    static_assert(CELLS_PER_THREAD == 8, "a thread's cube indices are one 8-byte word");
+    unsigned long long cubes = 0;   // of the thread's cells, those past the end outside
+    if (base + CELLS_PER_THREAD <= ncells) {
+        cubes = *reinterpret_cast<const unsigned long long *>(cube + base);
+    } else {
+        for (int q = 0; q < CELLS_PER_THREAD; q++)
+            if (base + q < ncells) cubes |= (unsigned long long)cube[base + q] << (8 * q);
+    }
+    const bool plain = cubes == 0ull || cubes == ~0ull;
     int2 own = make_int2(0, 0);
-    for (int q = 0; q < CELLS_PER_THREAD; q++) {
-        const long long c = base + q;
-        if (c >= ncells) break;
-        const int cq = cube[c];
-        if (cq != 0 && cq != 255) {
+    if (!plain)
+        for (int q = 0; q < CELLS_PER_THREAD; q++) {
+            const int cq = (int)(cubes >> (8 * q) & 255);
+            if (cq == 0 || cq == 255) continue;
             int i, j, k;
-            unflatten(c, ci, cj, i, j, k);
+            unflatten(base + q, ci, cj, i, j, k);
             own.x += __popc(cut_mask(cq) & created_mask(i, j, k));
             own.y += tri_count(cq);
         }
-    }
     int2 tot;
     int2 run = block_scan_int2(own, &tot);
+    if (plain) return;
     const int2 tb = tileBase[blockIdx.x];
     run.x += tb.x;
     run.y += tb.y;
-    const float sdx = (float)m.subdx;
     for (int q = 0; q < CELLS_PER_THREAD; q++) {
-        const long long c = base + q;
-        if (c >= ncells) break;
-        vstart[c] = run.x;
-        tstart[c] = run.y;
-        const int cq = cube[c];
+        const int cq = (int)(cubes >> (8 * q) & 255);
         if (cq == 0 || cq == 255) continue;
+        const long long c = base + q;
         int i, j, k;
         unflatten(c, ci, cj, i, j, k);
-        const unsigned mk = cut_mask(cq) & created_mask(i, j, k);
-        for (int e = 0; e < 12; e++) {
-            if (!(mk >> e & 1u)) continue;
-            const int A = kEa[e], B = kEb[e];
-            const int ai = i + kCx[A], aj = j + kCy[A], ak = k + kCz[A];
-            const int bi = i + kCx[B], bj = j + kCy[B], bk = k + kCz[B];
-            float v[3];
-            // Polygonizer3d::_getVertexPosition (polygonizer3d.cpp:356-359)
-            vertex_interp(m, S, __fmul_rn(sdx, (float)ai), __fmul_rn(sdx, (float)aj), __fmul_rn(sdx, (float)ak),
-                          __fmul_rn(sdx, (float)bi), __fmul_rn(sdx, (float)bj), __fmul_rn(sdx, (float)bk),
-                          (double)fld(m, F, ai, aj, ak), (double)fld(m, F, bi, bj, bk), v);
-            float *o = verts + 3LL * run.x;
-            o[0] = __fmul_rn(__fmul_rn(__fadd_rn(v[0], m.offx), m.scalef), m.invscalef);
-            o[1] = __fmul_rn(__fmul_rn(__fadd_rn(v[1], m.offy), m.scalef), m.invscalef);
-            o[2] = __fmul_rn(__fmul_rn(__fadd_rn(v[2], m.offz), m.scalef), m.invscalef);
-            run.x++;
-        }
-        run.y += tri_count(cq);
+        vstart[c] = run.x;
+        for (unsigned mk = cut_mask(cq) & created_mask(i, j, k); mk; mk &= mk - 1)
+            put_origin(verts + 3LL * run.x++, c * 16 + (__ffs(mk) - 1));
+        const int nt = tri_count(cq);
+        for (int t = 0; t < nt; t++) put_origin(tris + 3LL * run.y++, c * 16 + t);
     }
+}
+
+// The ends of the vertices' edges: their nodes.
+__device__ __forceinline__ void edge_end(const MeshFrame &m, long long code, int side, int &a, int &b, int &c) {
+    int i, j, k;
+    unflatten(code >> 4, m.ni - 1, m.nj - 1, i, j, k);
+    const int e = (int)(code & 15), q = side ? kEb[e] : kEa[e];
+    a = i + kCx[q];
+    b = j + kCy[q];
+    c = k + kCz[q];
+}
+// The ends' field values, a group of lanes each.
+template <int GROUP>
+__global__ void __launch_bounds__(SEARCH_TPB, 1024 / SEARCH_TPB) k_mesh_ends(ParticleSoA p, const int *cellStart, MeshFrame m,
+                                                                             const uint8_t *active, const unsigned *inside,
+                                                                             int nverts, const int *origins, float *values) {
+    const long long t = ((long long)blockIdx.x * blockDim.x + threadIdx.x) / GROUP;
+    if (t >= 2LL * nverts) return;
+    int a, b, c;
+    edge_end(m, get_origin(origins + 3 * (t >> 1)), (int)(t & 1), a, b, c);
+    const float f = node_value<GROUP>(p, cellStart, m, active, inside, a, b, c);
+    if (threadIdx.x % GROUP == 0) values[t] = f;
+}
+// A vertex, moved to the simulation's frame (translate by the chunk offset,
+// scale, unscale: particlemesher.cpp:35-55, 271-280).  Apart from the search,
+// so that its FP64 work has full warps.
+__global__ void __launch_bounds__(MESH_TPB) k_mesh_vertices(MeshFrame m, const float *S, int nverts, const float *values,
+                                                            float *verts) {
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= nverts) return;
+    float *o = verts + 3LL * t;
+    const long long code = get_origin(reinterpret_cast<const int *>(o));
+    float x[2], y[2], z[2];
+    double sd[2];
+    int sign[2];
+#pragma unroll
+    for (int q = 0; q < 2; q++) {
+        int a, b, c;
+        edge_end(m, code, q, a, b, c);
+        // Polygonizer3d::_getVertexPosition (polygonizer3d.cpp:356-359)
+        x[q] = __fmul_rn(m.subdxf, (float)a);
+        y[q] = __fmul_rn(m.subdxf, (float)b);
+        z[q] = __fmul_rn(m.subdxf, (float)c);
+        sign[q] = solid_sign(m, S, __fadd_rn(x[q], m.offx), __fadd_rn(y[q], m.offy), __fadd_rn(z[q], m.offz));
+        sd[q] = (double)sign[q];
+    }
+    if (sign[0] * sign[1] <= 0)   // the solid's values matter only where the ends' signs differ
+        for (int q = 0; q < 2; q++)
+            sd[q] = (double)(float)solid_sample(m, S, __fadd_rn(x[q], m.offx), __fadd_rn(y[q], m.offy), __fadd_rn(z[q], m.offz));
+    float v[3];
+    vertex_interp(x[0], y[0], z[0], x[1], y[1], z[1], (double)values[2LL * t], (double)values[2LL * t + 1], sd[0], sd[1], v);
+    o[0] = __fmul_rn(__fmul_rn(__fadd_rn(v[0], m.offx), m.scalef), m.invscalef);
+    o[1] = __fmul_rn(__fmul_rn(__fadd_rn(v[1], m.offy), m.scalef), m.invscalef);
+    o[2] = __fmul_rn(__fmul_rn(__fadd_rn(v[2], m.offz), m.scalef), m.invscalef);
 }
 
 // The vertex on edge e of cell (i, j, k): the cell that creates it, the
@@ -549,22 +829,17 @@ __device__ int edge_vertex(const MeshFrame &m, const uint8_t *cube, const int *v
     return vstart[c2] + __popc(mk & ((1u << e2) - 1u));
 }
 
-// Polygonizer3d::_polygonizeCell (polygonizer3d.cpp:635-656)
-__global__ void k_mesh_triangles(MeshFrame m, long long ncells, const uint8_t *cube, const int *vstart,
-                                 const int *tstart, int *tris) {
-    const long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= ncells) return;
-    const int cq = cube[c];
-    if (cq == 0 || cq == 255) return;
+// A triangle (Polygonizer3d::_polygonizeCell, polygonizer3d.cpp:635-656)
+__global__ void k_mesh_triangles(MeshFrame m, int ntris, const uint8_t *cube, const int *vstart, int *tris) {
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= ntris) return;
+    int *o = tris + 3LL * t;
+    const long long code = get_origin(o), c = code >> 4;
     int i, j, k;
     unflatten(c, m.ni - 1, m.nj - 1, i, j, k);
-    const unsigned long long w = kTri[cq];
-    int *o = tris + 3LL * tstart[c];
-    for (int t = 0; t < 15; t++) {
-        const int e = (int)((w >> (4 * t)) & 0xF);
-        if (e == 0xF) break;
-        o[t] = edge_vertex(m, cube, vstart, i, j, k, e);
-    }
+    const unsigned w = (unsigned)(kTri[cube[c]] >> (12 * (int)(code & 15)));
+#pragma unroll
+    for (int q = 0; q < 3; q++) o[q] = edge_vertex(m, cube, vstart, i, j, k, (int)(w >> (4 * q) & 15));
 }
 
 // -------------------------------------------------------------- smoothing
@@ -698,7 +973,7 @@ int grow(MeshBuffers &mb, T **p, long long *cap, long long need) {
 }  // namespace
 
 void mesh_release(MeshBuffers &mb) {
-    void *ptrs[] = {mb.occ, mb.active, mb.field, mb.cube, mb.vstart, mb.tstart, mb.tiles, mb.totals,
+    void *ptrs[] = {mb.occ, mb.active, mb.inside, mb.occupied, mb.cube, mb.vstart, mb.tiles, mb.totals,
                     mb.verts[0], mb.verts[1], mb.tris, mb.adj, mb.adjStart, mb.adjCursor, mb.adjList};
     for (void *q : ptrs)
         if (q) cudaFree(q);
@@ -720,6 +995,10 @@ int mesh_surface(const MeshJob &job, MeshBuffers &mb, cudaStream_t s) {
     m.subdx = c.dx / (double)sd;
     m.invsub = 1.0 / m.subdx;
     m.invsubf = (float)m.invsub;
+    m.dxf = (float)m.dx;
+    m.invdxf = (float)m.invdx;
+    m.subdxf = (float)m.subdx;
+    for (int a = 0; a < MB; a++) m.nodePos[a] = (float)((double)(float)a * m.subdx);
     m.blockdx = MB * m.subdx;
     m.invBlock = 1.0 / m.blockdx;
     m.invBlockf = (float)m.invBlock;
@@ -799,9 +1078,15 @@ int mesh_surface(const MeshJob &job, MeshBuffers &mb, cudaStream_t s) {
         m.bbx = m.offx - (float)h;
         m.bby = m.offy - (float)h;
         m.bbz = m.offz - (float)h;
-        m.bbw = ((double)pmx - (double)m.offx) + v;
-        m.bbh = ((double)pmy - (double)m.offy) + v;
-        m.bbd = ((double)pmz - (double)m.offz) + v;
+        // a coordinate p is inside where (double)p < bb + extent: where p is
+        // below the smallest float that is no less
+        auto upper = [](double x) {
+            const float f = (float)x;
+            return (double)f < x ? std::nextafter(f, INFINITY) : f;
+        };
+        m.bhx = upper((double)m.bbx + (((double)pmx - (double)m.offx) + v));
+        m.bhy = upper((double)m.bby + (((double)pmy - (double)m.offy) + v));
+        m.bhz = upper((double)m.bbz + (((double)pmz - (double)m.offz) + v));
     }
     // how ScalarField::setSolidSDF finds solid nodes (scalarfield.cpp:372-395)
     const float offLen = std::sqrt(m.offx * m.offx + m.offy * m.offy + m.offz * m.offz);
@@ -816,29 +1101,79 @@ int mesh_surface(const MeshJob &job, MeshBuffers &mb, cudaStream_t s) {
     m.invscalef = (float)(1.0 / scale);
 
     const long long ncb = (long long)m.cbI * m.cbJ * m.cbK;
-    std::vector<uint8_t> cact(ncb);
+    // the chunk's blocks: their frames' origins along each axis, then which are active
+    const int nb1[3] = {m.cbI, m.cbJ, m.cbK};
+    // the rows of cells that a search visits, nearest first, for a node nearer
+    // to the lower side of its cell in y and z
+    m.reach = m.sr + 1.02f * m.subdxf;
+    m.signReach = std::min(m.r * 1.001f, m.reach);
+    m.slack = 0.01f * m.dxf * (m.dxf + m.reach);
+    m.near2 = std::max(m.sr - 0.02f * m.subdxf, 0.0f) * std::max(m.sr - 0.02f * m.subdxf, 0.0f);
+    std::vector<MeshRow> rows;
+    const int R2 = (int)std::ceil(m.reach * m.invdxf + 0.02f);
+    auto side = [](int o) { return o == 0 ? 0.0f : (o > 0 ? o - 1.0f : -o - 0.5f); };   // at least so far, in cells
+    for (int z = -std::min(R2, c.K); z <= std::min(R2, c.K); z++)
+        for (int y = -std::min(R2, c.J); y <= std::min(R2, c.J); y++) {
+            const float dy = std::max(side(y) - 0.01f, 0.0f) * m.dxf, dz = std::max(side(z) - 0.01f, 0.0f) * m.dxf;
+            rows.push_back({dy * dy + dz * dz, (short)y, (short)z});
+        }
+    std::stable_sort(rows.begin(), rows.end(), [&](const MeshRow &a, const MeshRow &b) {
+        return a.least != b.least ? a.least < b.least
+                                  : std::abs(a.y) + std::abs(a.z) < std::abs(b.y) + std::abs(b.z);
+    });
+    m.nrows = (int)rows.size();
+    const size_t rowBytes = rows.size() * sizeof(MeshRow);
+    const size_t tables = rowBytes + sizeof(float) * ((size_t)m.cbI + m.cbJ + m.cbK);
+    std::vector<uint8_t> blocks(tables + ncb);
+    uint8_t *cact = blocks.data() + tables;
+    for (int d = 0, at = 0; d < 3; at += nb1[d++])
+        for (int b = 0; b < nb1[d]; b++) {
+            const float o = (float)((double)(float)b * m.blockdx);
+            std::memcpy(blocks.data() + rowBytes + sizeof(float) * (at + b), &o, sizeof(o));
+        }
+    std::memcpy(blocks.data(), rows.data(), rowBytes);
     for (int e = 0; e < m.cbK; e++)
         for (int b = 0; b < m.cbJ; b++)
             for (int a = 0; a < m.cbI; a++)
                 cact[a + (long long)m.cbI * (b + (long long)m.cbJ * e)] = act[bidx(a + lo[0], b + lo[1], e + lo[2])];
-    const long long nnodes = (long long)m.ni * m.nj * m.nk;
+    m.wpr = (m.ni + 31) / 32;
+    const long long nwords = (long long)m.wpr * m.nj * m.nk;
     const long long ncells = (long long)(m.ni - 1) * (m.nj - 1) * (m.nk - 1);
     const long long ntiles = std::max<long long>((ncells + TILE - 1) / TILE, 1);
-    MRC(grow(mb, &mb.active, &mb.activeCap, ncb));
-    MRC(grow(mb, &mb.field, &mb.fieldCap, nnodes));
+    MRC(grow(mb, &mb.active, &mb.activeCap, (long long)blocks.size()));
+    MRC(grow(mb, &mb.inside, &mb.insideCap, nwords));
     MRC(grow(mb, &mb.cube, &mb.cubeCap, std::max<long long>(ncells, 1)));
     MRC(grow(mb, &mb.vstart, &mb.vstartCap, std::max<long long>(ncells, 1)));
-    MRC(grow(mb, &mb.tstart, &mb.tstartCap, std::max<long long>(ncells, 1)));
     MRC(grow(mb, &mb.tiles, &mb.tilesCap, ntiles));
     MRC(grow(mb, &mb.totals, &mb.totalsCap, 2));
-    MCK(cudaMemcpyAsync(mb.active, cact.data(), ncb, cudaMemcpyHostToDevice, s));
-    {
-        dim3 grid(m.cbI, m.cbJ, m.cbK);
-        FLIP_COUNT(1);
-        k_mesh_field<<<grid, MESH_TPB, 0, s>>>(job.p, job.cellStart, m, mb.active, job.solidPhi, mb.field);
+    MCK(cudaMemcpyAsync(mb.active, blocks.data(), blocks.size(), cudaMemcpyHostToDevice, s));
+    m.rows = reinterpret_cast<const MeshRow *>(mb.active);
+    m.blockPos[0] = reinterpret_cast<const float *>(mb.active + rowBytes);
+    m.blockPos[1] = m.blockPos[0] + m.cbI;
+    m.blockPos[2] = m.blockPos[1] + m.cbJ;
+    const uint8_t *active = mb.active + tables;
+    // no farther than the word of cells beside a cell's own
+    const int R = (int)std::ceil(m.signReach * m.invdxf + 0.02f);
+    unsigned *around = nullptr;
+    if (R < 32) {
+        m.wpc = (c.I + 31) / 32;
+        const long long cw = (long long)m.wpc * c.J * c.K;
+        MRC(grow(mb, &mb.occupied, &mb.occupiedCap, 2 * cw));
+        around = mb.occupied + cw;
+        { FLIP_COUNT(1); k_mesh_occupied<<<div_up(cw, MESH_TPB / 32), MESH_TPB, 0, s>>>(job.cellStart, m, mb.occupied); }
+        { FLIP_COUNT(1); k_mesh_around<<<div_up(cw, MESH_TPB), MESH_TPB, 0, s>>>(m, mb.occupied, R, around); }
     }
+    // the list of wall nodes lies where vstart will
+    const int room = (int)std::min<long long>(mb.vstartCap, 0x7fffffff);
+    MCK(cudaMemsetAsync(mb.totals, 0, sizeof(int), s));
+    {
+        FLIP_COUNT(1);
+        k_mesh_inside<<<div_up(nwords, SEARCH_TPB / 32), SEARCH_TPB, 0, s>>>(job.p, job.cellStart, m, active, around, job.solidPhi,
+                                                                              mb.inside, mb.vstart, room, mb.totals);
+    }
+    { FLIP_COUNT(1); k_mesh_walls<<<152, MESH_TPB, 0, s>>>(m, job.solidPhi, mb.vstart, room, mb.totals, mb.inside); }
     if (ncells <= 0) return FLIP_OK;
-    { FLIP_COUNT(1); k_mesh_count<<<(unsigned)ntiles, MESH_TPB, 0, s>>>(m, mb.field, ncells, mb.cube, mb.tiles); }
+    { FLIP_COUNT(1); k_mesh_count<<<(unsigned)ntiles, MESH_TPB, 0, s>>>(m, mb.inside, ncells, mb.cube, mb.tiles); }
     { FLIP_COUNT(1); k_mesh_scan_tiles<<<1, MESH_TPB, 0, s>>>(mb.tiles, (int)ntiles, mb.totals); }
     int totals[2];
     MCK(cudaMemcpyAsync(totals, mb.totals, sizeof(totals), cudaMemcpyDeviceToHost, s));
@@ -851,10 +1186,23 @@ int mesh_surface(const MeshJob &job, MeshBuffers &mb, cudaStream_t s) {
     MRC(grow(mb, &mb.tris, &mb.trisCap, 3LL * ntris));
     {
         FLIP_COUNT(1);
-        k_mesh_vertices<<<(unsigned)ntiles, MESH_TPB, 0, s>>>(m, mb.field, job.solidPhi, ncells, mb.cube, mb.tiles,
-                                                               mb.vstart, mb.tstart, mb.verts[0]);
+        k_mesh_number<<<(unsigned)ntiles, MESH_TPB, 0, s>>>(m, ncells, mb.cube, mb.tiles, mb.vstart,
+                                                             reinterpret_cast<int *>(mb.verts[0]), mb.tris);
     }
-    { FLIP_COUNT(1); k_mesh_triangles<<<div_up(ncells, MESH_TPB), MESH_TPB, 0, s>>>(m, ncells, mb.cube, mb.vstart, mb.tstart, mb.tris); }
+    {
+        // few vertices: more lanes to a search, which then ends sooner (12650
+        // vertices: 112 us with eight, 163 with four); many: fewer, which look
+        // at less (208844: 245 us with eight, 174 with four)
+        auto ends = [&](auto kernel, int group) {
+            FLIP_COUNT(1);
+            kernel<<<div_up(2LL * group * nverts, SEARCH_TPB), SEARCH_TPB, 0, s>>>(
+                job.p, job.cellStart, m, active, mb.inside, nverts, reinterpret_cast<const int *>(mb.verts[0]), mb.verts[1]);
+        };
+        if (nverts < 65536) ends(k_mesh_ends<8>, 8);
+        else ends(k_mesh_ends<4>, 4);
+    }
+    { FLIP_COUNT(1); k_mesh_vertices<<<div_up(nverts, MESH_TPB), MESH_TPB, 0, s>>>(m, job.solidPhi, nverts, mb.verts[1], mb.verts[0]); }
+    { FLIP_COUNT(1); k_mesh_triangles<<<div_up(ntris, MESH_TPB), MESH_TPB, 0, s>>>(m, ntris, mb.cube, mb.vstart, mb.tris); }
     mb.nverts = nverts;
     mb.ntris = ntris;
     if (job.smoothIterations > 0) {

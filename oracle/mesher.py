@@ -227,9 +227,10 @@ def mesh_particles(pos, isize, jsize, ksize, dx, solid_phi, subdivisions=1, part
     best = np.full(nn[::-1], np.inf, f32)   # smallest squared distance per chunk node (k, j, i)
     npos = _idx_pos(np.arange(MB), subdx)
     invs = 1.0 / subdx
-    for dk in (0, 1):
-        for dj in (0, 1):
-            for di in (0, 1):
+    most = range(int((b1 - b0).max(initial=0)) + 1)   # blocks a search box spans along an axis
+    for dk in most:
+        for dj in most:
+            for di in most:
                 B = b0 + np.array([di, dj, dk])
                 ok = np.all(B <= b1, axis=1) & np.all(B >= 0, axis=1) & np.all(B < cb, axis=1)
                 ok[ok] &= cact[B[ok, 2], B[ok, 1], B[ok, 0]]
