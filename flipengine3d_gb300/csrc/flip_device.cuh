@@ -342,10 +342,12 @@ namespace flip {
 // -- viscosity (flip_viscosity.cu)
 struct ViscosityBuffers {
     uint8_t *fluidFace, *valid, *valid2, *inSys;   // per face; per node (two); per face
-    float *node;                                   // corner values of one control-volume grid
-    float *vol[7];                                 // control-volume fractions
-    float4 *fac, *dr;                              // per face: six factors (two float4); {diag, rhs}
-    double *x, *r, *z, *p, *q, *part, *scal;       // CG vectors, partials (3 x blocks), scalars (8)
+    float *node[7], *vol[7];                       // per control-volume grid: corner values, fractions
+    double *coefs;                                 // per row: six factors, diagonal, 1 / diagonal
+    double *x, *r, *p, *q, *scal;                  // per row: CG vectors; scalars (8)
+    double2 *zp;                                   // per face {z, the last p}
+    int *list, *blockRows;                         // the system's faces; counts per block of faces and their scan
+    unsigned long long *slots;                     // the CTAs' shares of the CG's sums
 };
 struct ViscosityResult {
     long long rows;
@@ -353,7 +355,7 @@ struct ViscosityResult {
     double residual;   // |r|inf / |b|inf
 };
 void viscosity_buffer_sizes(int I, int J, int K, long long *nf, long long *nn, long long *ncorner,
-                            long long vol[7], int *reductionBlocks);
+                            long long vol[7], long long *rowBlocks, long long *slotWords);
 int viscosity_apply(const StepConsts &c, const ViscosityBuffers &vb, const float *liquidPhi, const float *solidPhi,
                     float *u, float *v, float *w, double visc, double dt, ViscosityResult *res, cudaStream_t s);
 

@@ -729,19 +729,19 @@ int dump_mac(flip_ctx *x, float *a, float *b, float *e, const float *u, const fl
 // The viscosity solve's device buffers, made with the first viscous step.
 int alloc_viscosity(flip_ctx *x) {
     if (x->vbReady) return FLIP_OK;
-    long long nf, nn, ncorner, vol[7];
-    int rb;
-    viscosity_buffer_sizes(x->I, x->J, x->K, &nf, &nn, &ncorner, vol, &rb);
+    long long nf, nn, ncorner, vol[7], rowBlocks, slotWords;
+    viscosity_buffer_sizes(x->I, x->J, x->K, &nf, &nn, &ncorner, vol, &rowBlocks, &slotWords);
     ViscosityBuffers &b = x->vb;
     int rc;
     if ((rc = x->alloc(&b.fluidFace, nf)) || (rc = x->alloc(&b.valid, nn)) || (rc = x->alloc(&b.valid2, nn)) ||
-        (rc = x->alloc(&b.inSys, nf)) || (rc = x->alloc(&b.node, ncorner)) || (rc = x->alloc(&b.fac, 2 * nf)) ||
-        (rc = x->alloc(&b.dr, nf)) || (rc = x->alloc(&b.x, nf)) || (rc = x->alloc(&b.r, nf)) ||
-        (rc = x->alloc(&b.z, nf)) || (rc = x->alloc(&b.p, nf)) || (rc = x->alloc(&b.q, nf)) ||
-        (rc = x->alloc(&b.part, 3 * (long long)rb)) || (rc = x->alloc(&b.scal, 8)))
+        (rc = x->alloc(&b.inSys, nf)) || (rc = x->alloc(&b.coefs, 8 * nf)) ||
+        (rc = x->alloc(&b.x, nf)) || (rc = x->alloc(&b.r, nf)) ||
+        (rc = x->alloc(&b.zp, nf)) || (rc = x->alloc(&b.p, nf)) || (rc = x->alloc(&b.q, nf)) ||
+        (rc = x->alloc(&b.list, nf)) || (rc = x->alloc(&b.blockRows, rowBlocks)) ||
+        (rc = x->alloc(&b.slots, slotWords)) || (rc = x->alloc(&b.scal, 8)))
         return rc;
     for (int g = 0; g < 7; g++)
-        if ((rc = x->alloc(&b.vol[g], vol[g]))) return rc;
+        if ((rc = x->alloc(&b.vol[g], vol[g])) || (rc = x->alloc(&b.node[g], ncorner))) return rc;
     x->vbReady = true;
     return FLIP_OK;
 }

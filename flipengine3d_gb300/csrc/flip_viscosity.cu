@@ -16,12 +16,13 @@
 //
 // The solve differs on purpose.  The reference runs its FP32 MIC(0)-PCG to
 // a relative residual of 1e-4 (at most 700 iterations).  Here the system is
-// solved matrix-free by Jacobi-preconditioned CG in FP64 to 1e-9, so the
+// solved by Jacobi-preconditioned CG in FP64 to 1e-9, so the
 // result is the system's solution to well inside the reference's own
 // tolerance; a reference-exact MIC(0) over this 15-point, three-component
 // system would be a sequential triangular solve.  The faces of the system
 // then take the solution and every other face is zeroed, as the reference's
 // _applySolutionToVelocityField (:856-891) does.
+#include <algorithm>
 #include <cmath>
 #include <string>
 
@@ -160,11 +161,23 @@ __global__ void k_visc_dilate(StepConsts c, const uint8_t *in, uint8_t *out) {
               v(i, j, k + 1)) ? 1 : 0;
 }
 
-// Corner values of one control-volume grid (viscositysolver.cpp:278-368):
-// node (a, b, d) of the grid's (ni+1)(nj+1)(nk+1) corners takes its value
-// from the first valid volume in flat order among the eight that share it,
-// sampled at that volume's centre plus the corner's offset.
-__global__ void k_visc_corners(StepConsts c, VGrid g, const uint8_t *valid, const float *phi, float *node) {
+// The control-volume grids, in the order of ViscosityVolumeGrid
+// (viscositysolver.h:57-78): centre, U, V, W, edgeU, edgeV, edgeW.  All seven
+// go through one launch (blockIdx.y: the grid).
+enum { VC = 0, VU, VV, VW, EU, EV, EW, NVOL };
+struct VGrids {
+    VGrid g[NVOL];
+    float *node[NVOL], *vol[NVOL];
+};
+
+// Corner values (viscositysolver.cpp:278-368): node (a, b, d) of a grid's
+// (ni+1)(nj+1)(nk+1) corners takes its value from the first valid volume in
+// flat order among the eight that share it, sampled at that volume's centre
+// plus the corner's offset.  The volume is found first and the sample, FP64,
+// taken once for all lanes: in the search's loop it ran up to eight times a
+// warp (16.5 us a grid at 40^3; all seven now 60 us).
+__global__ void __launch_bounds__(TPB) k_visc_corners(StepConsts c, VGrids grids, const uint8_t *valid, const float *phi) {
+    const VGrid g = grids.g[blockIdx.y];
     const int ni = g.ni + 1, nj = g.nj + 1, nk = g.nk + 1;
     const long long n = (long long)ni * nj * nk;
     const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -172,13 +185,18 @@ __global__ void k_visc_corners(StepConsts c, VGrid g, const uint8_t *valid, cons
     int a, b, d;
     unflatten(t, ni, nj, a, b, d);
     const int vi = c.I + 1, vj = c.J + 1;
-    float val = 0.0f;
     // cells in ascending flat order: lower k first, then lower j, then lower i
-    for (int q = 0; q < 8; q++) {
-        const int dz = (q >> 2) & 1, dy = (q >> 1) & 1, dxx = q & 1;
-        const int ci = a - 1 + dxx, cj = b - 1 + dy, ck = d - 1 + dz;
+    int first = -1;
+#pragma unroll
+    for (int q = 7; q >= 0; q--) {
+        const int ci = a - 1 + (q & 1), cj = b - 1 + (q >> 1 & 1), ck = d - 1 + (q >> 2);
         if (ci < 0 || cj < 0 || ck < 0 || ci >= g.ni || cj >= g.nj || ck >= g.nk) continue;
-        if (!valid[(long long)ci + (long long)vi * ((long long)cj + (long long)vj * ck)]) continue;
+        if (valid[(long long)ci + (long long)vi * ((long long)cj + (long long)vj * ck)]) first = q;
+    }
+    float val = 0.0f;
+    if (first >= 0) {
+        const int dxx = first & 1, dy = first >> 1 & 1, dz = first >> 2;
+        const int ci = a - 1 + dxx, cj = b - 1 + dy, ck = d - 1 + dz;
         // centre = centerStart + GridIndexToCellCenter(ci, cj, ck, dx), then +-dx/2
         const float hdx = __fmul_rn(0.5f, (float)c.dx);
         const float cx = __fadd_rn(g.ox, (float)((double)(float)ci * c.dx + 0.5 * c.dx));
@@ -189,11 +207,13 @@ __global__ void k_visc_corners(StepConsts c, VGrid g, const uint8_t *valid, cons
         const float py = __fadd_rn(cy, dy ? -hdx : hdx);
         const float pz = __fadd_rn(cz, dz ? -hdx : hdx);
         val = liquid_at(c, phi, px, py, pz);
-        break;
     }
-    node[t] = val;
+    grids.node[blockIdx.y][t] = val;
 }
-__global__ void k_visc_volumes(StepConsts c, VGrid g, const uint8_t *valid, const float *node, float *vol) {
+__global__ void __launch_bounds__(TPB) k_visc_volumes(StepConsts c, VGrids grids, const uint8_t *valid) {
+    const VGrid g = grids.g[blockIdx.y];
+    const float *node = grids.node[blockIdx.y];
+    float *vol = grids.vol[blockIdx.y];
     const long long n = (long long)g.ni * g.nj * g.nk;
     const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= n) return;
@@ -218,9 +238,6 @@ __global__ void k_visc_volumes(StepConsts c, VGrid g, const uint8_t *valid, cons
 }
 
 // ------------------------------------------------------------------ system
-// The control-volume grids, in the order of ViscosityVolumeGrid
-// (viscositysolver.h:57-78): centre, U, V, W, edgeU, edgeV, edgeW.
-enum { VC = 0, VU, VV, VW, EU, EV, EW, NVOL };
 struct VolPtrs {
     const float *v[NVOL];
     int ni[NVOL], nj[NVOL];
@@ -240,7 +257,8 @@ struct FaceIdx {   // flat index of a face over the U, V, W grids, one after the
 // (direction, offset), which of the six factors, and its sign.
 struct Term { signed char d, di, dj, dk, f, s; };
 enum { FR = 0, FL, FT, FB, FF, FK };
-__constant__ Term kTerms[3][14] = {
+struct TermTable {
+    Term t[3][14] = {
     {{0, 1, 0, 0, FR, -1}, {0, -1, 0, 0, FL, -1}, {0, 0, 1, 0, FT, -1}, {0, 0, -1, 0, FB, -1}, {0, 0, 0, 1, FF, -1},
      {0, 0, 0, -1, FK, -1}, {1, 0, 1, 0, FT, -1}, {1, -1, 1, 0, FT, 1}, {1, 0, 0, 0, FB, 1}, {1, -1, 0, 0, FB, -1},
      {2, 0, 0, 1, FF, -1}, {2, -1, 0, 1, FF, 1}, {2, 0, 0, 0, FK, 1}, {2, -1, 0, 0, FK, -1}},
@@ -250,11 +268,21 @@ __constant__ Term kTerms[3][14] = {
     {{2, 1, 0, 0, FR, -1}, {2, -1, 0, 0, FL, -1}, {2, 0, 1, 0, FT, -1}, {2, 0, -1, 0, FB, -1}, {2, 0, 0, 1, FF, -1},
      {2, 0, 0, -1, FK, -1}, {0, 1, 0, 0, FR, -1}, {0, 1, 0, -1, FR, 1}, {0, 0, 0, 0, FL, 1}, {0, 0, 0, -1, FL, -1},
      {1, 0, 1, 0, FT, -1}, {1, 0, 1, -1, FT, 1}, {1, 0, 0, 0, FB, 1}, {1, 0, 0, -1, FB, -1}}};
+};
+__constant__ TermTable kTerms;
 // The control volume behind each factor of a row of direction d: (grid, di, dj, dk)
 __constant__ signed char kVol[3][7][4] = {
     {{VU, 0, 0, 0}, {VC, 0, 0, 0}, {VC, -1, 0, 0}, {EW, 0, 1, 0}, {EW, 0, 0, 0}, {EV, 0, 0, 1}, {EV, 0, 0, 0}},
     {{VV, 0, 0, 0}, {EW, 1, 0, 0}, {EW, 0, 0, 0}, {VC, 0, 0, 0}, {VC, 0, -1, 0}, {EU, 0, 0, 1}, {EU, 0, 0, 0}},
     {{VW, 0, 0, 0}, {EV, 1, 0, 0}, {EV, 0, 0, 0}, {EU, 0, 1, 0}, {EU, 0, 0, 0}, {VC, 0, 0, 0}, {VC, 0, 0, -1}}};
+
+// The rows' coefficients by place in the list: six factors, diagonal, 1 /
+// diagonal, each an array; the right-hand side (which becomes the residual).
+struct RowCoefs {
+    double *base, *rhs;
+    long long room;
+    __device__ double *at(int q) const { return base + q * room; }
+};
 
 struct SysArgs {
     FaceIdx fx;
@@ -265,219 +293,314 @@ struct SysArgs {
     float factor;   // dt / dx^2 as the reference rounds it
 };
 
-// Per face: in the system or not (viscositysolver.cpp:374-464), its six
-// factors, diagonal and right-hand side (:550-821), all in float.
-__global__ void k_visc_rows(SysArgs a, uint8_t *inSys, float4 *fac, float4 *dr) {
-    const long long nf = a.fx.nu + a.fx.nv + (long long)a.fx.I * a.fx.J * (a.fx.K + 1);
-    const long long f = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (f >= nf) return;
-    int d, i, j, k;
-    if (f < a.fx.nu) { d = 0; unflatten(f, a.fx.I + 1, a.fx.J, i, j, k); }
-    else if (f < a.fx.nu + a.fx.nv) { d = 1; unflatten(f - a.fx.nu, a.fx.I, a.fx.J + 1, i, j, k); }
-    else { d = 2; unflatten(f - a.fx.nu - a.fx.nv, a.fx.I, a.fx.J, i, j, k); }
-    uint8_t in = 0;
-    if (i >= 1 && j >= 1 && k >= 1 && i < a.fx.I && j < a.fx.J && k < a.fx.K && a.fluidFace[f]) {
-        float vv[7];
+__device__ __forceinline__ int face_of(const FaceIdx &fx, long long f, int &i, int &j, int &k) {
+    if (f < fx.nu) { unflatten(f, fx.I + 1, fx.J, i, j, k); return 0; }
+    if (f < fx.nu + fx.nv) { unflatten(f - fx.nu, fx.I, fx.J + 1, i, j, k); return 1; }
+    unflatten(f - fx.nu - fx.nv, fx.I, fx.J, i, j, k);
+    return 2;
+}
+__device__ __forceinline__ void row_volumes(const SysArgs &a, int d, int i, int j, int k, float *vv) {
 #pragma unroll
-        for (int q = 0; q < 7; q++)
-            vv[q] = vol(a.vp, kVol[d][q][0], i + kVol[d][q][1], j + kVol[d][q][2], k + kVol[d][q][3]);
-        in = (vv[0] > 0.0f || vv[1] > 0.0f || vv[2] > 0.0f || vv[3] > 0.0f || vv[4] > 0.0f || vv[5] > 0.0f ||
-              vv[6] > 0.0f) ? 1 : 0;
-        if (in) {
-            const float v = a.visc;
-            const float vq = __fmul_rn(0.25f, __fadd_rn(__fadd_rn(__fadd_rn(v, v), v), v));
-            const float two = __fmul_rn(2.0f, a.factor);
-            float F[6];
-#pragma unroll
-            for (int q = 0; q < 6; q++) {
-                // the two factors across the row's own direction use the
-                // viscosity at the cell centres, doubled; the others the
-                // mean of four
-                const bool own = (d == 0 && q < 2) || (d == 1 && (q == 2 || q == 3)) || (d == 2 && q >= 4);
-                F[q] = own ? __fmul_rn(__fmul_rn(two, v), vv[q + 1]) : __fmul_rn(__fmul_rn(a.factor, vq), vv[q + 1]);
-            }
-            float diag = vv[0];
-#pragma unroll
-            for (int q = 0; q < 6; q++) diag = __fadd_rn(diag, F[q]);
-            const float *G[3] = {a.u, a.v, a.w};
-            const long long self = f - (d == 0 ? 0 : d == 1 ? a.fx.nu : a.fx.nu + a.fx.nv);
-            float rval = __fmul_rn(vv[0], G[d][self]);
-            for (int q = 0; q < 14; q++) {
-                const Term t = kTerms[d][q];
-                const long long g = a.fx.of(t.d, i + t.di, j + t.dj, k + t.dk);
-                if (a.fluidFace[g]) continue;   // SOLID: the known velocity moves to the right-hand side
-                const long long gl = g - (t.d == 0 ? 0 : t.d == 1 ? a.fx.nu : a.fx.nu + a.fx.nv);
-                const float entry = t.s < 0 ? -F[t.f] : F[t.f];
-                rval = __fsub_rn(rval, __fmul_rn(entry, G[t.d][gl]));
-            }
-            fac[2 * f] = make_float4(F[0], F[1], F[2], F[3]);
-            fac[2 * f + 1] = make_float4(F[4], F[5], 0.0f, 0.0f);
-            dr[f] = make_float4(diag, rval, 0.0f, 0.0f);
+    for (int q = 0; q < 7; q++)
+        vv[q] = vol(a.vp, kVol[d][q][0], i + kVol[d][q][1], j + kVol[d][q][2], k + kVol[d][q][3]);
+}
+
+// Per face: in the system or not (viscositysolver.cpp:374-464); per block of
+// faces, how many are.
+__global__ void __launch_bounds__(TPB) k_visc_system(SysArgs a, long long nf, uint8_t *inSys, int *blockRows) {
+    const long long f = (long long)blockIdx.x * TPB + threadIdx.x;
+    bool in = false;
+    if (f < nf) {
+        int i, j, k;
+        const int d = face_of(a.fx, f, i, j, k);
+        if (i >= 1 && j >= 1 && k >= 1 && i < a.fx.I && j < a.fx.J && k < a.fx.K && a.fluidFace[f]) {
+            float vv[7];
+            row_volumes(a, d, i, j, k, vv);
+            in = vv[0] > 0.0f || vv[1] > 0.0f || vv[2] > 0.0f || vv[3] > 0.0f || vv[4] > 0.0f || vv[5] > 0.0f || vv[6] > 0.0f;
         }
+        inSys[f] = in;
     }
-    inSys[f] = in;
+    const int rows = __syncthreads_count(in);
+    if (threadIdx.x == 0) blockRows[blockIdx.x] = rows;
+}
+
+// The system's faces, in order.
+__global__ void __launch_bounds__(TPB) k_visc_list(const uint8_t *inSys, long long nf, const int *start, int *list) {
+    __shared__ int warps[TPB / 32];
+    const long long f = (long long)blockIdx.x * TPB + threadIdx.x;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const bool in = f < nf && inSys[f];
+    const unsigned m = __ballot_sync(0xffffffffu, in);
+    if (lane == 0) warps[warp] = __popc(m);
+    __syncthreads();
+    int at = start[blockIdx.x] + __popc(m & ((1u << lane) - 1u));
+    for (int w = 0; w < warp; w++) at += warps[w];
+    if (in) list[at] = (int)f;
+}
+
+// Per row: its six factors, diagonal and right-hand side (:550-821), all in
+// float, kept as doubles, which they are multiplied with.
+__global__ void __launch_bounds__(TPB) k_visc_rows(SysArgs a, const int *list, const int *listed, RowCoefs c) {
+    const int rows = *listed;
+    for (int n = blockIdx.x * TPB + threadIdx.x; n < rows; n += gridDim.x * TPB) {
+        const long long f = list[n];
+        int i, j, k;
+        const int d = face_of(a.fx, f, i, j, k);
+        float vv[7];
+        row_volumes(a, d, i, j, k, vv);
+        const float v = a.visc;
+        const float vq = __fmul_rn(0.25f, __fadd_rn(__fadd_rn(__fadd_rn(v, v), v), v));
+        const float two = __fmul_rn(2.0f, a.factor);
+        float F[6];
+#pragma unroll
+        for (int q = 0; q < 6; q++) {
+            // the two factors across the row's own direction use the
+            // viscosity at the cell centres, doubled; the others the
+            // mean of four
+            const bool own = (d == 0 && q < 2) || (d == 1 && (q == 2 || q == 3)) || (d == 2 && q >= 4);
+            F[q] = own ? __fmul_rn(__fmul_rn(two, v), vv[q + 1]) : __fmul_rn(__fmul_rn(a.factor, vq), vv[q + 1]);
+        }
+        float diag = vv[0];
+#pragma unroll
+        for (int q = 0; q < 6; q++) diag = __fadd_rn(diag, F[q]);
+        const float *G[3] = {a.u, a.v, a.w};
+        const long long self = f - (d == 0 ? 0 : d == 1 ? a.fx.nu : a.fx.nu + a.fx.nv);
+        float rval = __fmul_rn(vv[0], G[d][self]);
+        for (int q = 0; q < 14; q++) {
+            const Term t = kTerms.t[d][q];
+            const long long g = a.fx.of(t.d, i + t.di, j + t.dj, k + t.dk);
+            if (a.fluidFace[g]) continue;   // SOLID: the known velocity moves to the right-hand side
+            const long long gl = g - (t.d == 0 ? 0 : t.d == 1 ? a.fx.nu : a.fx.nu + a.fx.nv);
+            const float entry = t.s < 0 ? -F[t.f] : F[t.f];
+            rval = __fsub_rn(rval, __fmul_rn(entry, G[t.d][gl]));
+        }
+#pragma unroll
+        for (int q = 0; q < 6; q++) c.at(q)[n] = (double)F[q];
+        c.at(6)[n] = (double)diag;
+        c.at(7)[n] = 1.0 / (double)diag;
+        c.rhs[n] = (double)rval;
+    }
+}
+// _applySolutionToVelocityField (viscositysolver.cpp:856-891): the field is
+// cleared before the system's faces take the solution; without a system it is
+// left as it is (:55-58).
+__global__ void __launch_bounds__(TPB) k_visc_clear(SysArgs a, long long nf, const int *listed, float *u, float *v, float *w) {
+    const long long f = (long long)blockIdx.x * TPB + threadIdx.x;
+    if (f >= nf || *listed == 0) return;
+    if (f < a.fx.nu) u[f] = 0.0f;
+    else if (f < a.fx.nu + a.fx.nv) v[f - a.fx.nu] = 0.0f;
+    else w[f - a.fx.nu - a.fx.nv] = 0.0f;
 }
 
 // ------------------------------------------------------------------- solve
-// Jacobi-preconditioned CG in FP64 over the faces in the system.  Reductions
-// go through fixed per-block partials summed by one block, so they are
-// deterministic.  scal: [0] r.z  [1] p.q  [2] new r.z  [3] |r|inf  [4] |b|inf
-// [5] rows  [6] alpha  [7] beta
-constexpr int RB = 1024;   // reduction blocks
-
-__device__ __forceinline__ double block_sum(double v, double *sh) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    if (lane == 0) sh[warp] = v;
-    __syncthreads();
-    double s = 0.0;
-    if (threadIdx.x == 0)
-        for (int q = 0; q < (int)(blockDim.x >> 5); q++) s += sh[q];
-    __syncthreads();
-    return s;
-}
-__device__ __forceinline__ double block_max(double v, double *sh) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_down_sync(0xffffffffu, v, o));
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    if (lane == 0) sh[warp] = v;
-    __syncthreads();
-    double s = 0.0;
-    if (threadIdx.x == 0)
-        for (int q = 0; q < (int)(blockDim.x >> 5); q++) s = fmax(s, sh[q]);
-    __syncthreads();
-    return s;
-}
+// Jacobi-preconditioned CG in FP64 over the faces in the system, all
+// iterations in one cooperative launch.  The systems are small (41k rows at
+// 40^3, a few MB), so what counts are the steps' latencies and FP64, of which an
+// SM does two operations a cycle.  As five launches an iteration, two of them a
+// sum in one CTA, it took 70 us at 40^3 (apply 24, sums 2 x 13, update 14,
+// direction 4); here 15 us.
+//   * chunks of 32 rows go to the SMs in turn, so that all have equally many;
+//   * p stays implicit off its own row: p = z + beta p_old from the pair
+//     {z, p_old} of a neighbour's row, zero off the system, so that a direction
+//     needs no step of its own;
+//   * products are added with one rounding (fma), and z = r (1 / diagonal);
+//   * a sum over the rows is also the barrier: a CTA writes its share into a
+//     slot, tagged with the number of the sum, and every CTA reads all slots,
+//     in the same order.
+// scal: [3] |r|inf  [4] |b|inf  [5] rows  [6] iterations  [7] 1: a wait ran out
+constexpr int CG_CTAS = 320, CG_TPB = 512;
+constexpr int CG_BATCH = 8;            // |r|inf is compared with the tolerance every so many iterations
+constexpr int CG_MAX_ITER = 2000;
+constexpr unsigned CG_SPINS = 1u << 24;   // of a wait, about 10 s
 
 struct CgArgs {
-    SysArgs s;
-    const uint8_t *inSys;
-    const float4 *fac, *dr;
-    long long nf;
-    double *x, *r, *z, *p, *q;
-    double *part;    // 3 x RB partials
+    FaceIdx fx;
+    RowCoefs c;
+    const int *list, *listed;   // the rows' faces; how many
+    double *x, *p, *q;          // a row's own, by place in the list (and c.rhs: r)
+    double2 *zp;                // {z, p_old} by face
+    unsigned long long *slots;  // [2][CG_CTAS][4]
     double *scal;
+    float *u, *v, *w;           // take the solution
 };
 
-// A p for row f (zero off the system): diagonal plus the row's couplings to
-// faces in the system, as the reference's matrix holds them.
-__device__ double apply_row(const CgArgs &a, long long f) {
-    int d, i, j, k;
-    if (f < a.s.fx.nu) { d = 0; unflatten(f, a.s.fx.I + 1, a.s.fx.J, i, j, k); }
-    else if (f < a.s.fx.nu + a.s.fx.nv) { d = 1; unflatten(f - a.s.fx.nu, a.s.fx.I, a.s.fx.J + 1, i, j, k); }
-    else { d = 2; unflatten(f - a.s.fx.nu - a.s.fx.nv, a.s.fx.I, a.s.fx.J, i, j, k); }
-    const float4 f0 = a.fac[2 * f], f1 = a.fac[2 * f + 1];
-    const float F[6] = {f0.x, f0.y, f0.z, f0.w, f1.x, f1.y};
-    double y = (double)a.dr[f].x * a.p[f];
+// Sums a0 and takes the maximum of a1 >= 0 over the grid, in a fixed order, and
+// is a barrier: what a CTA wrote to global memory before is seen after.  False
+// once a wait ran out.
+__device__ bool cg_all(const CgArgs &a, unsigned epoch, double &a0, double &a1) {
+    constexpr int WARPS = CG_TPB / 32;
+    __shared__ double s0[WARPS], t0;
+    __shared__ long long s1[WARPS], t1;
+    __shared__ int good;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    long long m = __double_as_longlong(a1);   // as integers in the same order
+    auto lanes = [&]() {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            a0 += __shfl_xor_sync(0xffffffffu, a0, o);
+            m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
+        }
+    };
+    if (__any_sync(0xffffffffu, a0 != 0.0 || m != 0)) lanes();
+    if (lane == 0) {
+        s0[warp] = a0;
+        s1[warp] = m;
+    }
+    __threadfence();
+    __syncthreads();
+    if (warp == 0) {
+        a0 = lane < WARPS ? s0[lane] : 0.0;
+        m = lane < WARPS ? s1[lane] : 0;
+        lanes();
+        // a slot's words: the halves of the two numbers, each with the sum's
+        // number, so that a word is new or not as a whole.  Two sets in turn: a
+        // CTA writes one again only after every CTA has read it.
+        unsigned long long *set = a.slots + (size_t)(epoch & 1) * CG_CTAS * 4;
+        if (lane < 4) {
+            const unsigned long long v = (unsigned long long)(lane < 2 ? __double_as_longlong(a0) : m);
+            asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(set + 4 * blockIdx.x + lane),
+                         "l"((unsigned long long)epoch << 32 | (v >> (lane & 1 ? 32 : 0) & 0xffffffffull))
+                         : "memory");
+        }
+        a0 = 0.0;
+        m = 0;
+        bool ok = true;
+        for (int first = lane; ok && first < (int)gridDim.x; first += 128) {   // four slots a lane at a time
+            unsigned long long w[4][4];
+            for (unsigned spin = 0;; spin++) {
+                bool all = true;
+#pragma unroll
+                for (int h = 0; h < 4; h++) {
+                    const int t = min(first + 32 * h, (int)gridDim.x - 1);
+#pragma unroll
+                    for (int q = 0; q < 4; q += 2)
+                        asm volatile("ld.relaxed.gpu.global.v2.u64 {%0, %1}, [%2];"
+                                     : "=l"(w[h][q]), "=l"(w[h][q + 1])
+                                     : "l"(set + 4 * t + q)
+                                     : "memory");
+                }
+#pragma unroll
+                for (int h = 0; h < 4; h++)
+#pragma unroll
+                    for (int q = 0; q < 4; q++) all &= (unsigned)(w[h][q] >> 32) == epoch;
+                if (all) break;
+                if (spin > CG_SPINS || ((spin & 1023u) == 1023u && *(volatile double *)&a.scal[7] != 0.0)) {
+                    ok = false;
+                    break;
+                }
+            }
+#pragma unroll
+            for (int h = 0; h < 4; h++)
+                if (first + 32 * h < (int)gridDim.x) {
+                    a0 += __longlong_as_double((long long)((w[h][0] & 0xffffffffull) | w[h][1] << 32));
+                    m = max(m, (long long)((w[h][2] & 0xffffffffull) | w[h][3] << 32));
+                }
+        }
+        __threadfence();
+        if (!ok) *(volatile double *)&a.scal[7] = 1.0;
+        ok = __all_sync(0xffffffffu, ok);
+        lanes();
+        if (lane == 0) {
+            t0 = a0;
+            t1 = m;
+            good = ok;
+        }
+    }
+    __syncthreads();
+    a0 = t0;
+    a1 = __longlong_as_double(t1);
+    return good != 0;   // written again only after the next sum's first barrier
+}
+
+// The couplings of row (i, j, k) of direction D, added to y in the reference's
+// order: entries times the neighbours' p, which is 0 off the system.
+template <int D>
+__device__ __forceinline__ double couple(const CgArgs &a, int i, int j, int k, const double *F, double beta, double y) {
+    double2 v[14];
+#pragma unroll
     for (int q = 0; q < 14; q++) {
-        const Term t = kTerms[d][q];
-        const long long g = a.s.fx.of(t.d, i + t.di, j + t.dj, k + t.dk);
-        if (!a.s.fluidFace[g] || !a.inSys[g]) continue;
-        const double entry = t.s < 0 ? -(double)F[t.f] : (double)F[t.f];
-        y += entry * a.p[g];
+        constexpr TermTable T;
+        const Term t = T.t[D][q];
+        v[q] = __ldcg(&a.zp[a.fx.of(t.d, i + t.di, j + t.dj, k + t.dk)]);
+    }
+#pragma unroll
+    for (int q = 0; q < 14; q++) {
+        constexpr TermTable T;
+        const Term t = T.t[D][q];
+        y = __fma_rn(t.s < 0 ? -F[t.f] : F[t.f], __fma_rn(beta, v[q].y, v[q].x), y);
     }
     return y;
 }
 
-__global__ void k_cg_init(CgArgs a) {
-    __shared__ double sh[32];
-    double rz = 0.0, bmax = 0.0, rows = 0.0;
-    for (long long f = (long long)blockIdx.x * blockDim.x + threadIdx.x; f < a.nf; f += (long long)gridDim.x * blockDim.x) {
-        double b = 0.0, z = 0.0;
-        if (a.inSys[f]) {
-            b = (double)a.dr[f].y;
-            z = b / (double)a.dr[f].x;
-            rz += b * z;
-            bmax = fmax(bmax, fabs(b));
-            rows += 1.0;
+__global__ void __launch_bounds__(CG_TPB, 1) k_cg(CgArgs a) {
+    const int rows = *a.listed, step = gridDim.x * CG_TPB;
+    const int first = ((threadIdx.x >> 5) * gridDim.x + blockIdx.x) * 32 + (threadIdx.x & 31);
+    unsigned epoch = 0;
+    double rz = 0.0, bmax = 0.0;
+    for (int n = first; n < rows; n += step) {
+        const double b = a.c.rhs[n], z = b * a.c.at(7)[n];
+        rz = __fma_rn(b, z, rz);
+        bmax = fmax(bmax, fabs(b));
+        a.x[n] = 0.0;
+        __stcg(&a.zp[a.list[n]], make_double2(z, 0.0));
+    }
+    bool ok = cg_all(a, ++epoch, rz, bmax);
+    const double tol = 1e-9 * bmax;
+    double beta = 0.0, rmax = bmax;
+    int it = 0;
+    while (ok && it < CG_MAX_ITER && rmax > tol) {
+        double pq = 0.0, none = 0.0;
+        for (int n = first; n < rows; n += step) {
+            const int f = a.list[n];
+            int i, j, k;
+            const int d = face_of(a.fx, f, i, j, k);
+            double F[6];
+#pragma unroll
+            for (int q = 0; q < 6; q++) F[q] = a.c.at(q)[n];
+            const double2 own = __ldcg(&a.zp[f]);
+            const double p = __fma_rn(beta, own.y, own.x);
+            double y = a.c.at(6)[n] * p;
+            y = d == 0 ? couple<0>(a, i, j, k, F, beta, y) : d == 1 ? couple<1>(a, i, j, k, F, beta, y) : couple<2>(a, i, j, k, F, beta, y);
+            a.p[n] = p;
+            a.q[n] = y;
+            pq = __fma_rn(p, y, pq);
         }
-        a.x[f] = 0.0;
-        a.r[f] = b;
-        a.z[f] = z;
-        a.p[f] = z;
-    }
-    const double s0 = block_sum(rz, sh), s1 = block_max(bmax, sh), s2 = block_sum(rows, sh);
-    if (threadIdx.x == 0) {
-        a.part[blockIdx.x] = s0;
-        a.part[RB + blockIdx.x] = s1;
-        a.part[2 * RB + blockIdx.x] = s2;
-    }
-}
-// mode 0: init sums -> rz, |b|, rows; 1: p.q; 2: new rz, |r| and beta
-__global__ void k_cg_sum(CgArgs a, int mode) {
-    __shared__ double sh[32];
-    double s0 = 0.0, s1 = 0.0, s2 = 0.0;
-    for (int q = threadIdx.x; q < RB; q += blockDim.x) {
-        s0 += a.part[q];
-        s1 = fmax(s1, a.part[RB + q]);
-        s2 += a.part[2 * RB + q];
-    }
-    const double t0 = block_sum(s0, sh), t1 = block_max(s1, sh), t2 = block_sum(s2, sh);
-    if (threadIdx.x != 0) return;
-    if (mode == 0) { a.scal[0] = t0; a.scal[4] = t1; a.scal[3] = t1; a.scal[5] = t2; }
-    else if (mode == 1) { a.scal[1] = t0; a.scal[6] = t0 != 0.0 ? a.scal[0] / t0 : 0.0; }
-    else { a.scal[7] = a.scal[0] != 0.0 ? t0 / a.scal[0] : 0.0; a.scal[0] = t0; a.scal[3] = t1; }
-}
-__global__ void k_cg_apply(CgArgs a) {
-    __shared__ double sh[32];
-    double pq = 0.0;
-    for (long long f = (long long)blockIdx.x * blockDim.x + threadIdx.x; f < a.nf; f += (long long)gridDim.x * blockDim.x) {
-        double y = 0.0;
-        if (a.inSys[f]) {
-            y = apply_row(a, f);
-            pq += a.p[f] * y;
+        if (!(ok = cg_all(a, ++epoch, pq, none))) break;
+        const double alpha = pq != 0.0 ? rz / pq : 0.0;
+        double nrz = 0.0, nmax = 0.0;
+        for (int n = first; n < rows; n += step) {
+            const double p = a.p[n], r = __fma_rn(-alpha, a.q[n], a.c.rhs[n]), z = r * a.c.at(7)[n];
+            a.x[n] = __fma_rn(alpha, p, a.x[n]);
+            a.c.rhs[n] = r;
+            __stcg(&a.zp[a.list[n]], make_double2(z, p));
+            nrz = __fma_rn(r, z, nrz);
+            nmax = fmax(nmax, fabs(r));
         }
-        a.q[f] = y;
+        if (!(ok = cg_all(a, ++epoch, nrz, nmax))) break;
+        beta = rz != 0.0 ? nrz / rz : 0.0;
+        rz = nrz;
+        if (++it % CG_BATCH == 0) rmax = nmax;
     }
-    const double s0 = block_sum(pq, sh);
-    if (threadIdx.x == 0) {
-        a.part[blockIdx.x] = s0;
-        a.part[RB + blockIdx.x] = 0.0;
-        a.part[2 * RB + blockIdx.x] = 0.0;
+    if (ok)
+        for (int n = first; n < rows; n += step) {
+            const long long f = a.list[n];
+            const float x = (float)a.x[n];
+            if (f < a.fx.nu) a.u[f] = x;
+            else if (f < a.fx.nu + a.fx.nv) a.v[f - a.fx.nu] = x;
+            else a.w[f - a.fx.nu - a.fx.nv] = x;
+        }
+    if (first == 0) {
+        a.scal[3] = rmax;
+        a.scal[4] = bmax;
+        a.scal[5] = (double)rows;
+        a.scal[6] = (double)it;
     }
-}
-__global__ void k_cg_update(CgArgs a) {
-    __shared__ double sh[32];
-    const double alpha = a.scal[6];
-    double rz = 0.0, rmax = 0.0;
-    for (long long f = (long long)blockIdx.x * blockDim.x + threadIdx.x; f < a.nf; f += (long long)gridDim.x * blockDim.x) {
-        if (!a.inSys[f]) continue;
-        a.x[f] += alpha * a.p[f];
-        const double r = a.r[f] - alpha * a.q[f];
-        a.r[f] = r;
-        const double z = r / (double)a.dr[f].x;
-        a.z[f] = z;
-        rz += r * z;
-        rmax = fmax(rmax, fabs(r));
-    }
-    const double s0 = block_sum(rz, sh), s1 = block_max(rmax, sh);
-    if (threadIdx.x == 0) {
-        a.part[blockIdx.x] = s0;
-        a.part[RB + blockIdx.x] = s1;
-        a.part[2 * RB + blockIdx.x] = 0.0;
-    }
-}
-__global__ void k_cg_direction(CgArgs a) {
-    const double beta = a.scal[7];
-    for (long long f = (long long)blockIdx.x * blockDim.x + threadIdx.x; f < a.nf; f += (long long)gridDim.x * blockDim.x)
-        if (a.inSys[f]) a.p[f] = a.z[f] + beta * a.p[f];
-}
-// _applySolutionToVelocityField (viscositysolver.cpp:856-891): the field is
-// cleared, then the system's faces take the solution.
-__global__ void k_visc_write(CgArgs a, float *u, float *v, float *w) {
-    const long long f = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (f >= a.nf) return;
-    const float val = a.inSys[f] ? (float)a.x[f] : 0.0f;
-    if (f < a.s.fx.nu) u[f] = val;
-    else if (f < a.s.fx.nu + a.s.fx.nv) v[f - a.s.fx.nu] = val;
-    else w[f - a.s.fx.nu - a.s.fx.nv] = val;
 }
 
 }  // namespace
 
 void viscosity_buffer_sizes(int I, int J, int K, long long *nf, long long *nn, long long *ncorner,
-                            long long vol[7], int *reductionBlocks) {
+                            long long vol[7], long long *rowBlocks, long long *slotWords) {
     const long long nu = (long long)(I + 1) * J * K, nv = (long long)I * (J + 1) * K, nw = (long long)I * J * (K + 1);
     *nf = nu + nv + nw;
     *nn = (long long)(I + 1) * (J + 1) * (K + 1);
@@ -485,7 +608,9 @@ void viscosity_buffer_sizes(int I, int J, int K, long long *nf, long long *nn, l
     const long long g[7][3] = {{I, J, K}, {I + 1, J, K}, {I, J + 1, K}, {I, J, K + 1}, {I, J + 1, K + 1},
                                {I + 1, J, K + 1}, {I + 1, J + 1, K}};
     for (int q = 0; q < 7; q++) vol[q] = g[q][0] * g[q][1] * g[q][2];
-    *reductionBlocks = RB;
+    const long long blocks = div_up(*nf, TPB);   // their counts, the counts' scan, its total and scratch
+    *rowBlocks = 2 * blocks + 2 + scan_scratch_ints((int)blocks);
+    *slotWords = 8LL * CG_CTAS;
 }
 
 // The viscosity step on the device (buffers from the caller, sized by
@@ -501,20 +626,23 @@ int viscosity_apply(const StepConsts &c, const ViscosityBuffers &vb, const float
     { FLIP_COUNT(1); k_visc_dilate<<<div_up(nn, TPB), TPB, 0, s>>>(c, vb.valid2, vb.valid); }
     // the seven control-volume grids and their corner offsets (viscositysolver.cpp:240-248)
     const float h = (float)(0.5 * c.dx);
-    const VGrid grids[NVOL] = {{c.I, c.J, c.K, h, h, h},         {c.I + 1, c.J, c.K, 0, h, h},
-                               {c.I, c.J + 1, c.K, h, 0, h},     {c.I, c.J, c.K + 1, h, h, 0},
-                               {c.I, c.J + 1, c.K + 1, h, 0, 0}, {c.I + 1, c.J, c.K + 1, 0, h, 0},
-                               {c.I + 1, c.J + 1, c.K, 0, 0, h}};
+    VGrids grids = {{{c.I, c.J, c.K, h, h, h},         {c.I + 1, c.J, c.K, 0, h, h},
+                     {c.I, c.J + 1, c.K, h, 0, h},     {c.I, c.J, c.K + 1, h, h, 0},
+                     {c.I, c.J + 1, c.K + 1, h, 0, 0}, {c.I + 1, c.J, c.K + 1, 0, h, 0},
+                     {c.I + 1, c.J + 1, c.K, 0, 0, h}}, {}, {}};
     VolPtrs vp;
+    long long ncorner = 0;   // of the largest grid, which bounds its volumes too
     for (int g = 0; g < NVOL; g++) {
-        const VGrid &G = grids[g];
-        const long long ncorner = (long long)(G.ni + 1) * (G.nj + 1) * (G.nk + 1), ncell = (long long)G.ni * G.nj * G.nk;
-        { FLIP_COUNT(1); k_visc_corners<<<div_up(ncorner, TPB), TPB, 0, s>>>(c, G, vb.valid, liquidPhi, vb.node); }
-        { FLIP_COUNT(1); k_visc_volumes<<<div_up(ncell, TPB), TPB, 0, s>>>(c, G, vb.valid, vb.node, vb.vol[g]); }
+        const VGrid &G = grids.g[g];
+        ncorner = std::max(ncorner, (long long)(G.ni + 1) * (G.nj + 1) * (G.nk + 1));
+        grids.node[g] = vb.node[g];
+        grids.vol[g] = vb.vol[g];
         vp.v[g] = vb.vol[g];
         vp.ni[g] = G.ni;
         vp.nj[g] = G.nj;
     }
+    { FLIP_COUNT(1); k_visc_corners<<<dim3(div_up(ncorner, TPB), NVOL), TPB, 0, s>>>(c, grids, vb.valid, liquidPhi); }
+    { FLIP_COUNT(1); k_visc_volumes<<<dim3(div_up(ncorner, TPB), NVOL), TPB, 0, s>>>(c, grids, vb.valid); }
     SysArgs sa;
     sa.fx = FaceIdx{c.I, c.J, c.K, nu, nv};
     sa.vp = vp;
@@ -525,47 +653,38 @@ int viscosity_apply(const StepConsts &c, const ViscosityBuffers &vb, const float
     sa.visc = (float)visc;
     const float invdx = (float)(1.0 / c.dx);
     sa.factor = (float)(dt * (double)invdx * (double)invdx);
-    { FLIP_COUNT(1); k_visc_rows<<<div_up(nf, TPB), TPB, 0, s>>>(sa, vb.inSys, vb.fac, vb.dr); }
-    CgArgs a;
-    a.s = sa;
-    a.inSys = vb.inSys;
-    a.fac = vb.fac;
-    a.dr = vb.dr;
-    a.nf = nf;
-    a.x = vb.x; a.r = vb.r; a.z = vb.z; a.p = vb.p; a.q = vb.q;
-    a.part = vb.part;
-    a.scal = vb.scal;
-    { FLIP_COUNT(1); k_cg_init<<<RB, TPB, 0, s>>>(a); }
-    { FLIP_COUNT(1); k_cg_sum<<<1, 1024, 0, s>>>(a, 0); }
+    const int blocks = (int)div_up(nf, TPB);
+    int *start = vb.blockRows + blocks, *total = start + blocks + 1;
+    const RowCoefs coefs{vb.coefs, vb.r, nf};
+    { FLIP_COUNT(1); k_visc_system<<<blocks, TPB, 0, s>>>(sa, nf, vb.inSys, vb.blockRows); }
+    launch_scan_cells(vb.blockRows, blocks, start, total + 1, total, s);
+    { FLIP_COUNT(1); k_visc_list<<<blocks, TPB, 0, s>>>(vb.inSys, nf, start, vb.list); }
+    { FLIP_COUNT(1); k_visc_rows<<<std::min(blocks, 152 * 8), TPB, 0, s>>>(sa, vb.list, total, coefs); }
+    { FLIP_COUNT(1); k_visc_clear<<<blocks, TPB, 0, s>>>(sa, nf, total, u, v, w); }
+    const CgArgs a{sa.fx, coefs, vb.list, total, vb.x, vb.p, vb.q, vb.zp, vb.slots, vb.scal, u, v, w};
+    cudaError_t e = cudaMemsetAsync(vb.zp, 0, (size_t)nf * sizeof(double2), s);   // off the system
+    if (e == cudaSuccess) e = cudaMemsetAsync(vb.slots, 0, sizeof(unsigned long long) * 8 * CG_CTAS, s);
+    if (e == cudaSuccess) e = cudaMemsetAsync(vb.scal, 0, 8 * sizeof(double), s);
+    // a CTA per SM, fewer where they would have less than a chunk of rows each
+    // (one face in five is in a system as a rule)
+    int dev = 0, sms = 0;
+    if (e == cudaSuccess) e = cudaGetDevice(&dev);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    if (e == cudaSuccess) {
+        const int ctas = std::max(std::min({(int)div_up(nf, 5 * 32), sms, CG_CTAS}), 1);
+        void *args[] = {const_cast<CgArgs *>(&a)};
+        FLIP_COUNT(1);
+        e = cudaLaunchCooperativeKernel((const void *)k_cg, dim3(ctas), dim3(CG_TPB), args, 0, s);
+    }
+    if (e != cudaSuccess) return record_error(FLIP_E_CUDA, std::string("viscosity: ") + cudaGetErrorString(e));
     double hs[8];
-    cudaError_t e = cudaMemcpyAsync(hs, vb.scal, sizeof(hs), cudaMemcpyDeviceToHost, s);
+    e = cudaMemcpyAsync(hs, vb.scal, sizeof(hs), cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess) { FLIP_SYNC_COUNT(); e = cudaStreamSynchronize(s); }
     if (e != cudaSuccess) return record_error(FLIP_E_CUDA, std::string("viscosity: ") + cudaGetErrorString(e));
+    if (hs[7] != 0.0) return record_error(FLIP_E_CUDA, "viscosity: a wait of the solver ran out");
     res->rows = (long long)hs[5];
-    res->iterations = 0;
-    res->residual = 0.0;
-    if (res->rows == 0) return FLIP_OK;   // nothing to solve: the field is left as it is (:55-58)
-    const double bmax = hs[4], tol = 1e-9 * bmax;
-    const int maxIter = 2000, batch = 8;
-    double rmax = hs[3];
-    int it = 0;
-    while (it < maxIter && rmax > tol) {
-        for (int q = 0; q < batch; q++) {
-            { FLIP_COUNT(1); k_cg_apply<<<RB, TPB, 0, s>>>(a); }
-            { FLIP_COUNT(1); k_cg_sum<<<1, 1024, 0, s>>>(a, 1); }
-            { FLIP_COUNT(1); k_cg_update<<<RB, TPB, 0, s>>>(a); }
-            { FLIP_COUNT(1); k_cg_sum<<<1, 1024, 0, s>>>(a, 2); }
-            { FLIP_COUNT(1); k_cg_direction<<<RB, TPB, 0, s>>>(a); }
-        }
-        it += batch;
-        e = cudaMemcpyAsync(hs, vb.scal, sizeof(hs), cudaMemcpyDeviceToHost, s);
-        if (e == cudaSuccess) { FLIP_SYNC_COUNT(); e = cudaStreamSynchronize(s); }
-        if (e != cudaSuccess) return record_error(FLIP_E_CUDA, std::string("viscosity: ") + cudaGetErrorString(e));
-        rmax = hs[3];
-    }
-    res->iterations = it;
-    res->residual = bmax > 0 ? rmax / bmax : 0.0;
-    { FLIP_COUNT(1); k_visc_write<<<div_up(nf, TPB), TPB, 0, s>>>(a, u, v, w); }
+    res->iterations = (int)hs[6];
+    res->residual = hs[4] > 0 && res->rows > 0 ? hs[3] / hs[4] : 0.0;
     e = cudaGetLastError();
     if (e != cudaSuccess) return record_error(FLIP_E_CUDA, std::string("viscosity: ") + cudaGetErrorString(e));
     return FLIP_OK;
