@@ -428,8 +428,7 @@ int record_error(int code, const std::string &msg);   // sets flip_last_error()
 // Packed xyz positions/velocities (either may be null) of the n particles in
 // the reference's order; flags/rank hold idSpace+1 ints, scratch
 // scan_scratch_ints(idSpace) ints.
-void launch_readback_order(const ParticleSoA &p, int n, int idSpace, int *flags, int *rank, int *scratch,
-                           int *total, float *pos, float *vel, cudaStream_t s);
+void launch_readback_order(const ParticleSoA &p, int n, float *pos, float *vel, cudaStream_t s);
 void launch_compact_ids(const ParticleSoA &p, int n, int idSpace, int *flags, int *rank, int *scratch, int *total,
                         cudaStream_t s);
 }  // namespace flip

@@ -456,6 +456,12 @@ int inflow_constraint(flip_ctx *x, InflowConstraint *ic) {
     return FLIP_OK;
 }
 
+// Ids become ranks 0..n-1 in the load order.
+void compact_ids(flip_ctx *x) {
+    launch_compact_ids(x->pa, x->n, (int)x->idNext, x->idFlags, x->idRank, x->idScratch, x->idTotal, x->stream);
+    x->idNext = (unsigned int)x->n;
+}
+
 // _updateFluidObjects (fluidsimulation.cpp:4794-4806) after a substep: the
 // queued fluid meshes (_updateAddedFluidMeshObjectQueue, :4724-4759), then
 // the inflow sources' emission (_updateInflowMeshFluidSources, :4676-4698,
@@ -504,8 +510,7 @@ int update_fluid_objects(flip_ctx *x) {
         // ids are ranks below the id space, which is the storage's capacity:
         // once emission and removal have spread them out, renumber them
         if ((long long)x->idNext + ncand > x->capacity && x->idNext > (unsigned int)x->n) {
-            launch_compact_ids(x->pa, x->n, x->idSpace, x->idFlags, x->idRank, x->idScratch, x->idTotal, s);
-            x->idNext = (unsigned int)x->n;
+            compact_ids(x);
         }
         if ((rc = grow_particles(x, std::max(x->capacity, (int)(x->idNext + ncand))))) return rc;
     }
@@ -678,8 +683,8 @@ int particles_to_host(flip_ctx *x, float *pos, float *vel, int start, int end) {
     int n = x->n;
     if (n == 0 || end <= start) return FLIP_OK;
     float *dpos = x->pb.px, *dvel = x->pb.px + 3 * (size_t)x->capacity;
-    launch_readback_order(x->pa, n, x->idSpace, x->idFlags, x->idRank, x->idScratch, x->idTotal,
-                          pos ? dpos : nullptr, vel ? dvel : nullptr, x->stream);
+    if (x->idNext != (unsigned int)n) compact_ids(x);
+    launch_readback_order(x->pa, n, pos ? dpos : nullptr, vel ? dvel : nullptr, x->stream);
     size_t off = 3 * (size_t)start, bytes = 3 * (size_t)(end - start) * sizeof(float);
     if (pos) CK(cudaMemcpyAsync(pos, dpos + off, bytes, cudaMemcpyDeviceToHost, x->stream));
     if (vel) CK(cudaMemcpyAsync(vel, dvel + off, bytes, cudaMemcpyDeviceToHost, x->stream));
