@@ -218,7 +218,7 @@ struct PressureBuffers {
     int *items, *nItems;   // the solve's chunks of the sweep layout, and their number
     double4_32a *Ad;           // rows {diag, to +x, to +y, to +z}, FP64
     double *b;             // right-hand side (negative divergence)
-    double *invdiagD;      // MIC(0) inverse pivots, FP64
+    double *pivotInv;      // reciprocals of the MIC(0) pivots, FP64
     float4 *L;             // {invdiag, Lx, Ly, Lz} for the FP32 sweeps, sweep layout
     // The loop's vectors, in the sweep layout (nsl entries each; A, z, s and s2
     // have a step of zeros after them, planes of A too).  Values kept
@@ -247,7 +247,6 @@ struct PressureBuffers {
     long long loopKernels[2] = {};       // kernels per pass of the loop body
     bool noLoopGraph = false;            // the loop could not be built: batches from the host
     int *levelRange;       // [0]=min(i+j+k) [1]=max(i+j+k) [2]=system size [3..6]=min/max j, min/max k
-    int *factorProgress;   // per factor tile: the last level it finished
     unsigned int *factorTicket;
     float *pressure;       // float copy of x for the velocity update
     int nPartials;
@@ -322,14 +321,13 @@ void launch_sweeps(const StepConsts &c, const SweepLayout &g, const float4 *L, c
                    SweepState &sw, const int *skip, cudaStream_t s, bool prepped = false, bool overlap = false);
 void sweep_epoch_guard(const StepConsts &c, SweepState &sw, long long upcoming, cudaStream_t s);
 
-void mic0_factor(const StepConsts &c, const uint8_t *fluid, const double4_32a *Ad, double *invD, double *W0,
-                 double *W1, double *W2, int *progress, unsigned int *ticket, int *err, unsigned int spinLimit,
-                 int lo, int hi, cudaStream_t s);
+void mic0_factor(const StepConsts &c, const uint8_t *fluid, const double4_32a *Ad, double *E, double *W0, double *W1,
+                 double *W2, unsigned int *ticket, int *err, unsigned int spinLimit, cudaStream_t s);
+void mic0_inverse_pivots(const uint8_t *fluid, long long n, double *E, cudaStream_t s);
 // The reduction grid of the PCG row kernels: one CTA per `cellsPerCta` grid
 // cells (a tuning knob, default 4096), at most PCG_MAX_PARTIALS.
 constexpr int PCG_MAX_PARTIALS = 152 * 8;
 int pressure_partials_for(int I, int J, int K, int cellsPerCta = 4096);
-int mic0_factor_tiles(int J, int K);   // tiles of the wavefront factorisation
 // PressureSolver::solve (pressuresolver.cpp:44-76) on the device.  Returns
 // FLIP_OK (velocities updated, or nothing to solve), FLIP_E_SOLVER_NOCONV
 // (left unchanged), FLIP_E_DEVICE_TIMEOUT or FLIP_E_CUDA.

@@ -290,7 +290,7 @@ int alloc_grids(flip_ctx *x) {
     p.sl = sweep_layout(x->I, x->J, x->K, 0);
     p.nsl = nsl;
     if ((rc = x->alloc(&p.fluid, nc)) || (rc = x->alloc(&p.Ad, nc)) || (rc = x->alloc(&p.L, nsl)) ||
-        (rc = x->alloc(&p.b, nc)) || (rc = x->alloc(&p.invdiagD, nc)) ||
+        (rc = x->alloc(&p.b, nc)) || (rc = x->alloc(&p.pivotInv, nc)) ||
         (rc = x->alloc(&p.A, std::max(8 * (nsl + SWEEP_NP), 6 * nc))) || (rc = x->alloc(&p.xh, nsl)) ||
         (rc = x->alloc(&p.xl, nsl)) || (rc = x->alloc(&p.rh, nsl)) || (rc = x->alloc(&p.rl, nsl)) ||
         (rc = x->alloc(&p.qh, nsl)) || (rc = x->alloc(&p.ql, nsl)) || (rc = x->alloc(&p.z, nsl + SWEEP_NP)) ||
@@ -300,7 +300,7 @@ int alloc_grids(flip_ctx *x) {
     p.nPartials = pressure_partials_for(x->I, x->J, x->K, x->pcgCellsPerCta);
     if ((rc = x->alloc(&p.partials, 2 * PCG_MAX_PARTIALS)) || (rc = x->alloc(&p.scal, 8)) ||
         (rc = x->alloc(&p.rmaxBits, 2)) || (rc = x->alloc(&p.levelRange, 8)) || (rc = x->alloc(&p.ctl, 1)) ||
-        (rc = x->alloc(&p.factorProgress, mic0_factor_tiles(x->J, x->K))) || (rc = x->alloc(&p.factorTicket, 1)))
+        (rc = x->alloc(&p.factorTicket, 1)))
         return rc;
     {
         int nt = sweep_tiles_max(x->I, x->J, x->K);
@@ -1558,7 +1558,7 @@ int flip_estimate_device_bytes(int isize, int jsize, int ksize, int particles, l
     b += nc * (1 + 32 + 8 * 2 + 4) + nsl * (16 + 4 * 9) + 12 * SWEEP_NP + 4 * std::max(8 * (nsl + SWEEP_NP), 6 * nc);   // pressure system
     b += 4 * (sweep_items_max(isize, jsize, ksize) + 8) + 16;              // its items
     b += 2 * PCG_MAX_PARTIALS * 8 + 64 + 16 + 32;
-    b += (mic0_factor_tiles(jsize, ksize) + 1) * 4 + 64;                  // factor tiles, ticket, control
+    b += 4 + 64;                                                          // factor ticket, control
     b += sweep_exchange_words(isize, jsize, ksize) * 8 + 4096;           // sweep exchange, ranges, tables
     b += cap * (7 * 4 * 2 + 4 * 4) + (scan_scratch_ints((int)cap) + 4) * 4 + 64;   // particles
     *bytes = b;

@@ -142,6 +142,8 @@ __device__ __forceinline__ void block_max_to(double v, unsigned long long *out, 
     }
 }
 
+constexpr long long NOT_YET = -1LL;   // the bits of a pivot's reciprocal before it is found: a NaN that no operation returns
+
 // RHS (pressuresolver.cpp:580-669; the domain walls do not move) and the rows.
 __global__ void k_build(StepConsts c, const float *phi, const float *wu, const float *wv, const float *ww,
                         const float *u, const float *v, const float *w, double mf, PressureBuffers pb) {
@@ -149,7 +151,7 @@ __global__ void k_build(StepConsts c, const float *phi, const float *wu, const f
     Dims d{c.I, c.J, c.K};
     double bmag = 0.0;
     if (t < d.size()) {
-        pb.invdiagD[t] = 0.0;
+        pb.pivotInv[t] = __longlong_as_double(NOT_YET);
         if (!pb.fluid[t]) {
             pb.b[t] = 0.0;   // the row itself is not read
         } else {
@@ -175,72 +177,18 @@ __global__ void k_build(StepConsts c, const float *phi, const float *wu, const f
     block_max_to(bmag, (unsigned long long *)pb.scal + 2, false);
 }
 
-// MIC(0) pivots of one wavefront i+j+k = level, FP64.  For 7-point rows the
-// column-oriented elimination of factorModifiedIncompleteColesky0 reduces to:
-//   d_c = A_cc - sum over earlier neighbours k (ascending index) of
-//         L_ck^2 + 0.97 L_ck (sum of k's other later-neighbour entries L_mk),
-//   L_mk = A_mk / sqrt(pivot_k); a pivot below 0.25 A_kk falls back to A_kk.
-__device__ __forceinline__ void mic0_cell(const StepConsts &c, const uint8_t *fluid, const double4_32a *Ad, double *invD,
-                                          int level, int jj) {
-    int nj = c.J - 2;
-    int j = 1 + jj % nj, k = 1 + jj / nj;
-    int i = level - j - k;
-    if (i < 1 || i > c.I - 2) return;
-    const long long sy = c.I, sz = (long long)c.I * c.J;
-    long long t = i + sy * j + sz * k;
-    if (!fluid[t]) return;
-    double ad = Ad[t].x;
-    double d = ad;
-    const long long back[3] = {t - sz, t - sy, t - 1};   // ascending: -z, -y, -x
-#pragma unroll
-    for (int q = 0; q < 3; q++) {
-        long long kk = back[q];
-        if (!fluid[kk]) continue;
-        double4_32a ak = Ad[kk];
-        if (ak.x == 0.0) continue;
-        double inv = invD[kk];
-        double Lck = (q == 0 ? ak.w : (q == 1 ? ak.z : ak.y)) * inv;
-        // k's later neighbours, ascending +x, +y, +z, without c itself
-        double miss = 0.0;
-        if (q != 2 && fluid[kk + 1]) miss += ak.y * inv;
-        if (q != 1 && fluid[kk + sy]) miss += ak.z * inv;
-        if (q != 0 && fluid[kk + sz]) miss += ak.w * inv;
-        d -= Lck * Lck;
-        d -= 0.97 * Lck * miss;
-    }
-    double inv;
-    if (ad == 0.0) inv = 0.0;
-    else if (d < 0.25 * ad) inv = 1 / sqrt(ad);
-    else inv = 1 / sqrt(d);
-    invD[t] = inv;
-}
-
-__global__ void k_mic0_level(StepConsts c, const uint8_t *fluid, const double4_32a *Ad, double *invD, int level) {
-    int jj = blockIdx.x * blockDim.x + threadIdx.x;
-    if (jj < (c.J - 2) * (c.K - 2)) mic0_cell(c, fluid, Ad, invD, level, jj);
-}
-
-// All wavefronts lo..hi in one cooperative launch: the cells of a level in
-// parallel, a grid-wide barrier between levels (every block is resident, so
-// the barrier completes).
-__global__ void k_mic0_levels(StepConsts c, const uint8_t *fluid, const double4_32a *Ad, double *invD, int lo, int hi) {
-    cg::grid_group grid = cg::this_grid();
-    const int np = (c.J - 2) * (c.K - 2);
-    for (int lv = lo; lv <= hi; lv++) {
-        for (int jj = blockIdx.x * blockDim.x + threadIdx.x; jj < np; jj += gridDim.x * blockDim.x)
-            mic0_cell(c, fluid, Ad, invD, lv, jj);
-        grid.sync();
-    }
-}
-
-// The pivot of cell c (mic0_cell) regrouped per earlier neighbour q:
-//   L_cq^2 + 0.97 L_cq miss_q = inv_q^2 (a_q^2 + 0.97 a_q (m1_q + m2_q)),
+// MIC(0) pivots in FP64.  For 7-point rows the column-oriented elimination of
+// factorModifiedIncompleteColesky0 reduces to:
+//   d_c = A_cc - sum over earlier neighbours q of
+//         L_cq^2 + 0.97 L_cq (sum of q's other later-neighbour entries L_mq),
+//   L_mq = A_mq / sqrt(pivot_q); a pivot below 0.25 A_cc falls back to A_cc.
+// Regrouped per earlier neighbour q:
+//   L_cq^2 + 0.97 L_cq miss_q = (a_q^2 + 0.97 a_q (m1_q + m2_q)) / pivot_q,
 // with a_q the coupling of q to c and m1_q, m2_q q's other later-neighbour
-// couplings (0 where mic0_cell skips them).  The bracket depends on the rows
-// only; this pass computes it for every cell and earlier neighbour, so a
-// level needs three multiply-subtracts and a reciprocal square root.  The
-// FP64 results differ from mic0_cell's order in the last bits; the factor
-// is used rounded to FP32.
+// couplings (0 off the system).  The bracket depends on the rows only; this
+// pass computes it for every cell and earlier neighbour, so a level needs
+// three multiply-subtracts and a reciprocal.  The FP64 results differ from the
+// elimination's order in the last bits; the factor is used rounded to FP32.
 __global__ void k_mic0_weights(StepConsts c, const uint8_t *fluid, const double4_32a *Ad, double *W0, double *W1,
                                double *W2) {
     const long long n = (long long)c.I * c.J * c.K;
@@ -268,44 +216,92 @@ __global__ void k_mic0_weights(StepConsts c, const uint8_t *fluid, const double4
     W2[t] = w[2];
 }
 
-// The factor as a tiled wavefront, with no grid-wide barrier: a CTA per
-// tile of FT x FT (j, k) pencils, tiles taken by ticket in diagonal order
-// (a tile only waits on tiles with smaller tickets, which are running or
-// done).  Within a tile a level costs one __syncthreads: the -y and -z
-// neighbours' pivots of the level before sit in shared memory, the -x one
-// in a register.  Across tiles a tile publishes the last level it finished
-// every FCH levels (release), and a tile's edge threads read FCH levels of
-// the neighbouring pencil's pivots at once, after acquiring its progress.
-// Every wait is bounded: past the limit the tile sets *err and all tiles
-// that depend on it give up too (the solve reports a device timeout).
-// A level is bound by the latency of its FP64 chain (a dependent FP64
-// operation takes ~64 cycles on this GPU, rsqrt ~430), not by throughput:
-// tiles of 8, 12 and 16 pencils a side time the same.
+// FP64 to FP32 and back with integer operations, which are far cheaper than the
+// FP64 unit's conversions: for magnitudes well inside the range of FP32 (in_fp32),
+// rounded towards zero.
+__device__ __forceinline__ bool in_fp32(double d) {
+    return (unsigned)((__double2hiint(d) >> 20 & 0x7ff) - (1023 - 120)) <= 240u;
+}
+__device__ __forceinline__ float narrow(double d) {
+    const int hi = __double2hiint(d);
+    return __int_as_float((hi & 0x80000000) | ((hi & 0x7fffffff) - (896 << 20)) << 3 | (int)((unsigned)__double2loint(d) >> 29));
+}
+__device__ __forceinline__ double widen(float f) {
+    const int b = __float_as_int(f);
+    return __hiloint2double((b & 0x80000000) | (((b & 0x7fffffff) >> 3) + (896 << 20)), b << 29);
+}
+__device__ __forceinline__ float narrow_or_0(double d) { return in_fp32(d) ? narrow(d) : 0.0f; }
+// 1 / d from a guess g: one third-order step, e (1 + r + r^2) with r = 1 - d e,
+// which leaves r^3 < 2^-57; the division for a guess with fewer than 19 bits.
+__device__ __forceinline__ double reciprocal(double d, float g) {
+    const double e = widen(g), r = __fma_rn(-d, e, 1.0);
+    if ((__double2hiint(r) >> 20 & 0x7ff) >= 1023 - 19) return 1.0 / d;
+    return __fma_rn(e, __fma_rn(r, r, r), e);
+}
+__device__ __forceinline__ float guess_reciprocal(float f) {
+    float g;
+    asm("rcp.approx.f32 %0, %1;" : "=f"(g) : "f"(f));
+    return g;
+}
+// sqrt(e), e the reciprocal of a pivot: the inverse pivot.  The same way: a
+// guess from the FP32 unit, then two Newton steps.
+__device__ __forceinline__ double inverse_pivot(double e) {
+    if (!(e > 0.0) || !in_fp32(e)) return sqrt(e);
+    const float f = narrow(e);
+    float g;
+    asm("rsqrt.approx.f32 %0, %1;" : "=f"(g) : "f"(f));
+    const double y = widen(0.5f * g);
+    double x = widen(f * g);
+    x = __fma_rn(__fma_rn(-x, x, e), y, x);
+    return __fma_rn(__fma_rn(-x, x, e), y, x);
+}
+
+// The factor as a tiled wavefront, with no grid-wide barrier: a CTA per tile of
+// FT x FT (j, k) pencils, tiles taken by ticket in diagonal order (a tile only
+// waits on tiles with smaller tickets, which are running or done).  E, the
+// pivots' reciprocals, is all that the cells exchange.  Within a tile a level
+// costs one __syncthreads: the -y and -z neighbours' values of the level before
+// sit in shared memory, the -x one in a register.  Between tiles the values
+// themselves are the message: every cell starts as NOT_YET, and a tile's edge
+// threads read the neighbouring pencil's cells until they are there.  Rows,
+// weights and edges are loaded a chunk of FCH levels ahead.  A tile starts at
+// its first level with a cell in the system and ends with the last; one
+// without cells ends at once.  Every wait is bounded: past the limit the tile
+// sets *err and stops, and all tiles that wait on it give up too (the solve
+// reports a device timeout).
+// Bound by latencies: a level's FP64 chain of two multiply-adds and a reciprocal
+// of three more (about 64 cycles each; 820 cycles a level in all) and the hops
+// between tiles (L2, about 3 us each).  290 us at 128^3, 127 at 64^3, 42 at 32^3
+// with tiles of 8 x 8 and chunks of 2 (16 x 16, 4: 394, 174, 51).  Exchanging
+// rsqrt(pivot), with a progress counter per tile released every eight levels,
+// took 600 us at 128^3.
 #ifndef MIC0_FT
-#define MIC0_FT 16
+#define MIC0_FT 8
 #endif
 #ifndef MIC0_FCH
-#define MIC0_FCH 8
+#define MIC0_FCH 2
 #endif
-constexpr int FT = MIC0_FT, FCH = MIC0_FCH;
+constexpr int FT = MIC0_FT, FCH = MIC0_FCH, FTHREADS = (FT * FT + 31) / 32 * 32;
 static_assert(FT * FT >= 32 && FT * FT <= 1024, "a tile is one CTA");
-constexpr int FACTOR_DONE = 0x7fffffff;   // progress of a tile with all its levels done
 
-__device__ __forceinline__ int ld_acquire(const int *p) {
-    int v;
-    asm volatile("ld.acquire.gpu.b32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+__device__ __forceinline__ double ld_value(const double *p) {
+    double v;
+    asm volatile("ld.relaxed.gpu.f64 %0, [%1];" : "=d"(v) : "l"(p) : "memory");
     return v;
 }
-__device__ __forceinline__ void st_release(int *p, int v) {
-    asm volatile("st.release.gpu.b32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+__device__ __forceinline__ void st_value(double *p, double v) {
+    asm volatile("st.relaxed.gpu.f64 [%0], %1;" ::"l"(p), "d"(v) : "memory");
 }
+struct FactorChunk {
+    double ad[FCH], w0[FCH], w1[FCH], w2[FCH], ey[FCH], ez[FCH];
+    unsigned cells;   // which of its levels have a cell of this pencil
+};
 
-__global__ void __launch_bounds__(FT *FT) k_mic0_tiles(StepConsts c, const uint8_t *fluid, const double4_32a *Ad,
-                                                       const double *W0, const double *W1, const double *W2,
-                                                       double *invD, int lo, int hi, unsigned int *ticket,
-                                                       int *progress, int *err, unsigned int spinLimit) {
-    __shared__ double prev[2][FT][FT];
-    __shared__ int tileSh, abortSh;
+__global__ void __launch_bounds__(FTHREADS) k_mic0_tiles(StepConsts c, const uint8_t *fluid, const double4_32a *Ad,
+                                                         const double *W0, const double *W1, const double *W2, double *E,
+                                                         unsigned int *ticket, int *err, unsigned int spinLimit) {
+    __shared__ double prev[2][FT + 1][FT + 1];   // of the level before; row and column 0 stand for the edges
+    __shared__ int tileSh, lvLo, lvHi;
     const int ntj = (c.J - 2 + FT - 1) / FT, ntk = (c.K - 2 + FT - 1) / FT;
     if (threadIdx.x == 0) {
         // ticket -> tile in diagonal order (tj + tk, then tj)
@@ -315,91 +311,132 @@ __global__ void __launch_bounds__(FT *FT) k_mic0_tiles(StepConsts c, const uint8
             if (q < n) break;
             q -= n;
         }
-        abortSh = d >= ntj + ntk - 1;   // more CTAs than tiles: the launch is wrong
-        if (abortSh) atomicExch(err, 1);
+        const bool wrong = d >= ntj + ntk - 1;   // more CTAs than tiles: the launch is wrong
+        if (wrong) atomicExch(err, 1);
         const int tj = max(0, d - ntk + 1) + q;
-        tileSh = tj + ntj * (d - tj);
+        tileSh = wrong ? -1 : tj + ntj * (d - tj);
+        lvLo = 0x7fffffff;
+        lvHi = -1;
     }
     __syncthreads();
-    if (abortSh) return;
-    const int tile = tileSh, tj = tile % ntj, tk = tile / ntj;
+    const int tile = tileSh;
+    if (tile < 0) return;
+    const int tj = tile % ntj, tk = tile / ntj;
+    const int sy = c.I, sz = c.I * c.J;
+    // the levels with cells of this tile, 32 cells of a pencil at a time
+    {
+        const int lane = threadIdx.x & 31;
+        int lo = 0x7fffffff, hi = -1;
+        for (int p = threadIdx.x >> 5; p < FT * FT; p += FTHREADS / 32) {
+            const int j = 1 + tj * FT + p % FT, k = 1 + tk * FT + p / FT;
+            if (j > c.J - 2 || k > c.K - 2) continue;
+            for (int i = 1 + lane; i <= c.I - 2; i += 32)
+                if (fluid[i + sy * j + sz * k]) {
+                    lo = min(lo, i + j + k);
+                    hi = max(hi, i + j + k);
+                }
+        }
+        lo = __reduce_min_sync(0xffffffffu, lo);
+        hi = __reduce_max_sync(0xffffffffu, hi);
+        if (lane == 0 && hi >= 0) {
+            atomicMin(&lvLo, lo);
+            atomicMax(&lvHi, hi);
+        }
+    }
+    for (int q = threadIdx.x; q < 2 * (FT + 1) * (FT + 1); q += FTHREADS) (&prev[0][0][0])[q] = 0.0;
+    __syncthreads();
+    const int lvStart = lvLo, lvEnd = lvHi;
     const int a = threadIdx.x % FT, b = threadIdx.x / FT;   // j and k within the tile
     const int j = 1 + tj * FT + a, k = 1 + tk * FT + b;
-    const bool mine = j <= c.J - 2 && k <= c.K - 2;
-    const int sy = c.I, sz = c.I * c.J;
-    // the levels holding cells of this tile, within lo..hi
-    const int jhi = min(c.J - 2, 1 + tj * FT + FT - 1), khi = min(c.K - 2, 1 + tk * FT + FT - 1);
-    const int lvStart = max(lo, 1 + (1 + tj * FT) + (1 + tk * FT));
-    const int lvEnd = min(hi, (c.I - 2) + jhi + khi);
-    const int left = tj > 0 ? tile - 1 : -1, down = tk > 0 ? tile - ntj : -1;
-    prev[0][b][a] = prev[1][b][a] = 0.0;
-    if (threadIdx.x == 0) st_release(&progress[tile], lvStart - 1);   // the levels below hold no cell of the tile
+    const bool mine = b < FT && j <= c.J - 2 && k <= c.K - 2;
+    const int pencil = sy * j + sz * k - j - k;   // cell of level lv: pencil + lv
+    const bool edgeY = mine && a == 0 && tj > 0, edgeZ = mine && b == 0 && tk > 0;
+    auto load = [&](int lvc, FactorChunk &n) {
+        n.cells = 0;
+#pragma unroll
+        for (int m = 0; m < FCH; m++) {
+            const int i = lvc + m - j - k, t = pencil + lvc + m;
+            const bool in = mine && i >= 1 && i <= c.I - 2 && lvc + m <= lvEnd && fluid[t];
+            n.cells |= (unsigned)in << m;
+            n.ad[m] = in ? Ad[t].x : 0.0;
+            n.w0[m] = in ? W0[t] : 0.0;
+            n.w1[m] = in ? W1[t] : 0.0;
+            n.w2[m] = in ? W2[t] : 0.0;
+            n.ey[m] = in && edgeY ? ld_value(E + t - sy) : 0.0;
+            n.ez[m] = in && edgeZ ? ld_value(E + t - sz) : 0.0;
+        }
+    };
+    // Edge values that a weight asks for and that were not there when the chunk
+    // was loaded, all at once; a cell without weight may be off the system.
+    auto await = [&](int lvc, FactorChunk &n) {
+        unsigned miss = 0;
+#pragma unroll
+        for (int m = 0; m < FCH; m++) {
+            if (edgeY && n.w1[m] == 0.0) n.ey[m] = 0.0;
+            if (edgeZ && n.w0[m] == 0.0) n.ez[m] = 0.0;
+            miss |= (unsigned)(__double_as_longlong(n.ey[m]) == NOT_YET) << m;
+            miss |= (unsigned)(__double_as_longlong(n.ez[m]) == NOT_YET) << (FCH + m);
+        }
+        for (unsigned spin = 1; miss; spin++) {
+            if (spin >= spinLimit || ((spin & 255u) == 0u && *(volatile const int *)err)) {
+                atomicExch(err, 1);
+                return false;
+            }
+#pragma unroll
+            for (int m = 0; m < FCH; m++) {
+                if (miss >> m & 1u) n.ey[m] = ld_value(E + pencil + lvc + m - sy);
+                if (miss >> (FCH + m) & 1u) n.ez[m] = ld_value(E + pencil + lvc + m - sz);
+            }
+#pragma unroll
+            for (int m = 0; m < FCH; m++) {
+                if (__double_as_longlong(n.ey[m]) != NOT_YET) miss &= ~(1u << m);
+                if (__double_as_longlong(n.ez[m]) != NOT_YET) miss &= ~(1u << (FCH + m));
+            }
+        }
+        return true;
+    };
+    FactorChunk now, next;
+    double own = 0.0;   // this pencil's value of the level before (the -x neighbour's)
     int cur = 0;
-    double own = 0.0;   // this pencil's pivot at the level before (the -x neighbour's)
+    if (lvStart <= lvEnd) load(lvStart, now);
     for (int lvc = lvStart; lvc <= lvEnd; lvc += FCH) {
-        // the chunk's boundary values are the neighbours' levels lvc-1 .. lvc+FCH-2
-        if (threadIdx.x == 0) {
-            const int need = lvc + FCH - 2;
-            const int nbr[2] = {left, down};
-            for (int q = 0; q < 2 && !abortSh; q++) {
-                if (nbr[q] < 0) continue;
-                unsigned int spin = 0;
-                while (ld_acquire(&progress[nbr[q]]) < need) {
-                    if (++spin >= spinLimit || ld_acquire(err)) {
-                        atomicExch(err, 1);
-                        abortSh = 1;
-                        break;
-                    }
-                    if (spin > 256) __nanosleep(128);
-                }
-            }
-        }
-        __syncthreads();
-        if (abortSh) return;
-        // the chunk's cells of this pencil are consecutive along i: their
-        // rows, flags and weights, and the edge pencils' pivots, load at once
-        double bY[FCH], bZ[FCH], pad[FCH], pw0[FCH], pw1[FCH], pw2[FCH];
-        bool pcell[FCH];
+        load(lvc + FCH, next);
+        const bool failed = (edgeY || edgeZ) && !await(lvc, now);
+        if (__syncthreads_or(failed)) return;
 #pragma unroll
         for (int m = 0; m < FCH; m++) {
-            const int i = lvc + m - j - k;
-            const bool in = mine && i >= 1 && i <= c.I - 2 && lvc + m <= lvEnd;
-            const int t = i + sy * j + sz * k;
-            pcell[m] = in && fluid[t];
-            pad[m] = pcell[m] ? Ad[t].x : 0.0;
-            pw0[m] = pcell[m] ? W0[t] : 0.0;
-            pw1[m] = pcell[m] ? W1[t] : 0.0;
-            pw2[m] = pcell[m] ? W2[t] : 0.0;
-            bY[m] = (pcell[m] && a == 0 && left >= 0) ? __ldcg(invD + t - sy) : 0.0;
-            bZ[m] = (pcell[m] && b == 0 && down >= 0) ? __ldcg(invD + t - sz) : 0.0;
-        }
-#pragma unroll
-        for (int m = 0; m < FCH; m++) {
-            const int lv = lvc + m;
-            if (lv > lvEnd) break;
-            double inv = 0.0;
-            if (pcell[m]) {
-                const int t = (lv - j - k) + sy * j + sz * k;
-                const double ad = pad[m];
-                const double nz = b > 0 ? prev[cur ^ 1][b - 1][a] : bZ[m];
-                const double ny = a > 0 ? prev[cur ^ 1][b][a - 1] : bY[m];
-                double d = ad;
-                d -= pw0[m] * (nz * nz);
-                d -= pw1[m] * (ny * ny);
-                d -= pw2[m] * (own * own);
-                if (ad == 0.0) inv = 0.0;
-                else if (d < 0.25 * ad) inv = rsqrt(ad);
-                else inv = rsqrt(d);
-                invD[t] = inv;
+            double e = 0.0;
+            const float f0 = narrow_or_0(now.w0[m]), f1 = narrow_or_0(now.w1[m]);
+            if (now.cells >> m & 1u) {
+                const double ad = now.ad[m];
+                const double ez = edgeZ ? now.ez[m] : prev[cur ^ 1][b][a + 1];
+                const double ey = edgeY ? now.ey[m] : prev[cur ^ 1][b + 1][a];
+                double d = __fma_rn(-now.w2[m], own, ad);
+                // the guess comes from the same steps in FP32, while FP64 takes them
+                const float g = guess_reciprocal(
+                    __fmaf_rn(-f1, narrow_or_0(ey), __fmaf_rn(-f0, narrow_or_0(ez), narrow_or_0(d))));
+                d = __fma_rn(-now.w0[m], ez, d);
+                d = __fma_rn(-now.w1[m], ey, d);
+                const double least = 0.25 * ad;
+                // positive doubles compare as integers
+                const bool low = ad > 0.0 ? __double_as_longlong(d) < __double_as_longlong(least) : d < least;
+                if (low) e = 1.0 / ad;
+                else if (ad != 0.0) e = reciprocal(d, g);
+                if (__double_as_longlong(e) == NOT_YET) e = __longlong_as_double(NOT_YET - 1);
+                st_value(E + pencil + lvc + m, e);
             }
-            prev[cur][b][a] = inv;
-            own = inv;
+            if (b < FT) prev[cur][b + 1][a + 1] = e;
+            own = e;
             cur ^= 1;
             __syncthreads();
         }
-        if (threadIdx.x == 0) st_release(&progress[tile], min(lvc + FCH - 1, lvEnd));
+        now = next;
     }
-    if (threadIdx.x == 0) st_release(&progress[tile], FACTOR_DONE);
+}
+// Pivots' reciprocals to inverse pivots, 0 off the system.
+__global__ void k_mic0_inverse(const uint8_t *fluid, long long n, double *E) {
+    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (t < n) E[t] = fluid[t] ? inverse_pivot(E[t]) : 0.0;
 }
 
 // The items of a solve: the chunks (SWEEP_CH steps of a tile, 1024 entries of
@@ -472,7 +509,7 @@ __global__ void __launch_bounds__(TPB) k_layout(StepConsts c, SweepLayout g, con
             const long long t = (long long)i + (long long)c.I * (j + (long long)c.J * k);
             if (!pb.fluid[t]) continue;
             const double4_32a a = pb.Ad[t];
-            const double inv = pb.invdiagD[t], b = pb.b[t];
+            const double inv = inverse_pivot(pb.pivotInv[t]), b = pb.b[t];
             hi[q] = make_float4((float)a.x, (float)a.y, (float)a.z, (float)a.w);
             lo[q] = make_float4((float)(a.x - (double)hi[q].x), (float)(a.y - (double)hi[q].y),
                                 (float)(a.z - (double)hi[q].z), (float)(a.w - (double)hi[q].w));
@@ -1141,7 +1178,6 @@ int cuda_fail(cudaError_t e, const char *what, std::string *msg) {
 
 }  // namespace
 
-int mic0_factor_tiles(int J, int K) { return std::max(1, (J - 2 + FT - 1) / FT) * std::max(1, (K - 2 + FT - 1) / FT); }
 // One CTA of the row kernels per `cellsPerCta` grid cells (4096 by default),
 // at least 128 where there are as many items, at most the three per SM that
 // the SpMV's shared memory leaves resident.  A liquid fills a fraction of the
@@ -1163,42 +1199,22 @@ int pressure_partials_for(int I, int J, int K, int cellsPerCta) {
         if (e_ != cudaSuccess) return cuda_fail(e_, #call, errMsg); \
     } while (0)
 
-// MIC(0) factor of the rows Ad over the cells flagged in `fluid`, whose
-// levels i+j+k lie in lo..hi: the inverse pivots invD (FP64).  The tiled
-// wavefront runs where it launches; otherwise one cooperative launch over all
-// levels, else one launch per level.  W0..W2: n doubles each of scratch;
-// progress: mic0_factor_tiles ints; err: set when a bounded wait gave up.
-void mic0_factor(const StepConsts &c, const uint8_t *fluid, const double4_32a *Ad, double *invD, double *W0,
-                 double *W1, double *W2, int *progress, unsigned int *ticket, int *err, unsigned int spinLimit,
-                 int lo, int hi, cudaStream_t s) {
+// MIC(0) factor of the rows Ad over the cells flagged in `fluid`: E, the
+// pivots' reciprocals (FP64), which starts with all bits set.  W0..W2: n
+// doubles each of scratch; err: set when a bounded wait gave up.
+void mic0_factor(const StepConsts &c, const uint8_t *fluid, const double4_32a *Ad, double *E, double *W0, double *W1,
+                 double *W2, unsigned int *ticket, int *err, unsigned int spinLimit, cudaStream_t s) {
     const long long n = (long long)c.I * c.J * c.K;
-    const unsigned nb = div_up(n, TPB);
-    const int np = (c.J - 2) * (c.K - 2);
-    const int ntiles = mic0_factor_tiles(c.J, c.K);
-    cudaMemsetAsync(progress, 0xff, ntiles * sizeof(int), s);
+    const int ntiles = div_up(c.J - 2, FT) * div_up(c.K - 2, FT);
     cudaMemsetAsync(ticket, 0, sizeof(unsigned int), s);
-    { FLIP_COUNT(1); k_mic0_weights<<<nb, TPB, 0, s>>>(c, fluid, Ad, W0, W1, W2); }
+    { FLIP_COUNT(1); k_mic0_weights<<<div_up(n, TPB), TPB, 0, s>>>(c, fluid, Ad, W0, W1, W2); }
     FLIP_COUNT(1);
-    k_mic0_tiles<<<ntiles, FT * FT, 0, s>>>(c, fluid, Ad, W0, W1, W2, invD, lo, hi, ticket, progress, err, spinLimit);
-    if (cudaGetLastError() == cudaSuccess) return;
-    int dev = 0, coop = 0, perSM = 0, sms = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSM, k_mic0_levels, TPB, 0);
-    if (coop && perSM > 0) {
-        StepConsts c_ = c;
-        int lo_ = lo, hi_ = hi;
-        void *args[] = {&c_, &fluid, &Ad, &invD, &lo_, &hi_};
-        const int grid = std::max(1, std::min((int)div_up(np, TPB), perSM * sms));
-        FLIP_COUNT(1);
-        if (cudaLaunchCooperativeKernel((const void *)k_mic0_levels, grid, TPB, args, 0, s) == cudaSuccess) return;
-        cudaGetLastError();
-    }
-    for (int lv = lo; lv <= hi; lv++) {
-        FLIP_COUNT(1);
-        k_mic0_level<<<div_up(np, TPB), TPB, 0, s>>>(c, fluid, Ad, invD, lv);
-    }
+    k_mic0_tiles<<<ntiles, FTHREADS, 0, s>>>(c, fluid, Ad, W0, W1, W2, E, ticket, err, spinLimit);
+}
+// E to inverse pivots, 0 off the system.
+void mic0_inverse_pivots(const uint8_t *fluid, long long n, double *E, cudaStream_t s) {
+    FLIP_COUNT(1);
+    k_mic0_inverse<<<div_up(n, TPB), TPB, 0, s>>>(fluid, n, E);
 }
 
 // The condition of the device-side loop over batches of PCG iterations: one
@@ -1274,8 +1290,8 @@ int pressure_project(const StepConsts &c, const PressureArgs &a, PressureBuffers
     // MIC(0) factor; the pivot weights go to A's buffer, which is filled after
     // it: zero wherever no item of this solve writes a coupling
     double *W = reinterpret_cast<double *>(pb.A);
-    mic0_factor(c, pb.fluid, pb.Ad, pb.invdiagD, W, W + n, W + 2 * n, pb.factorProgress, pb.factorTicket, sw.err,
-                sw.spinLimit ? sw.spinLimit : DEFAULT_SPIN_LIMIT, lo, hi, s);
+    mic0_factor(c, pb.fluid, pb.Ad, pb.pivotInv, W, W + n, W + 2 * n, pb.factorTicket, sw.err,
+                sw.spinLimit ? sw.spinLimit : DEFAULT_SPIN_LIMIT, s);
     PCK(cudaMemsetAsync(pb.A, 0, 8 * (pb.nsl + SWEEP_NP) * sizeof(float), s));
     if (pb.stale) {   // entries off this solve's items are read (and multiplied by zero): finite values only
         PCK(cudaMemsetAsync(pb.z, 0, (pb.nsl + SWEEP_NP) * sizeof(float), s));

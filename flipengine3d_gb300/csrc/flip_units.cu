@@ -68,34 +68,26 @@ extern "C" int flip_mic0_factor(int I, int J, int K, const uint8_t *fluid, const
     int rc = check_system(I, J, K, fluid);
     if (rc) return rc;
     const size_t n = (size_t)I * J * K;
-    int lo = 0x7fffffff, hi = -1;
-    for (int k = 0; k < K; k++)
-        for (int j = 0; j < J; j++)
-            for (int i = 0; i < I; i++)
-                if (fluid[i + (size_t)I * (j + (size_t)J * k)]) {
-                    lo = std::min(lo, i + j + k);
-                    hi = std::max(hi, i + j + k);
-                }
+    const bool any = std::find_if(fluid, fluid + n, [](uint8_t f) { return f != 0; }) != fluid + n;
     std::memset(invdiag, 0, n * sizeof(double));
-    if (hi < lo) return FLIP_OK;
+    if (!any) return FLIP_OK;
     Scratch sc;
     uint8_t *dFluid;
     double4_32a *dAd;
     double *dInv, *dW;
-    int *dProgress, *dErr;
+    int *dErr;
     unsigned int *dTicket;
-    const int ntiles = mic0_factor_tiles(J, K);
     if (!sc.get(&dFluid, n) || !sc.get(&dAd, n) || !sc.get(&dInv, n) || !sc.get(&dW, 3 * n) ||
-        !sc.get(&dProgress, ntiles) || !sc.get(&dErr, 1) || !sc.get(&dTicket, 1))
+        !sc.get(&dErr, 1) || !sc.get(&dTicket, 1))
         return record_error(FLIP_E_NOMEM, "cudaMalloc failed");
     cudaStream_t s = nullptr;
     if ((rc = cuda_status(cudaMemcpy(dFluid, fluid, n, cudaMemcpyHostToDevice), "copy flags")) ||
         (rc = cuda_status(cudaMemcpy(dAd, rows, n * sizeof(double4_32a), cudaMemcpyHostToDevice), "copy rows")) ||
-        (rc = cuda_status(cudaMemset(dInv, 0, n * sizeof(double)), "clear")) ||
+        (rc = cuda_status(cudaMemset(dInv, 0xff, n * sizeof(double)), "clear")) ||
         (rc = cuda_status(cudaMemset(dErr, 0, sizeof(int)), "clear")))
         return rc;
-    mic0_factor(grid_consts(I, J, K), dFluid, dAd, dInv, dW, dW + n, dW + 2 * n, dProgress, dTicket, dErr,
-                DEFAULT_SPIN_LIMIT, lo, hi, s);
+    mic0_factor(grid_consts(I, J, K), dFluid, dAd, dInv, dW, dW + n, dW + 2 * n, dTicket, dErr, DEFAULT_SPIN_LIMIT, s);
+    mic0_inverse_pivots(dFluid, n, dInv, s);
     if ((rc = cuda_status(cudaDeviceSynchronize(), "factor"))) return rc;
     int err = 0;
     if ((rc = cuda_status(cudaMemcpy(&err, dErr, sizeof(int), cudaMemcpyDeviceToHost), "read flag"))) return rc;
