@@ -1,5 +1,5 @@
-"""Liquid level set, particle-to-grid and extrapolation at the sizes where
-their kernels change over: rows of faces that end at, before and after a
+"""Liquid level set, particle-to-grid, extrapolation and the particle update at
+the sizes where their kernels change over: rows of faces that end at, before and after a
 32-bit word, grids smaller than one block of ten cells, and grids on both
 sides of the line between the two extrapolation variants.  Against the CPU
 oracle: level set and known faces bit for bit, velocities to the bound of the
@@ -31,3 +31,5 @@ def test_level_set_and_face_velocities(gpu, dims, fill):
         assert np.array_equal(st[f"v{f}_p2g"], ref[f"v{f}_p2g"])
         assert rel_err(st[f"{f}_p2g"], ref[f"{f}_p2g"]) <= 1e-5
         assert rel_err(st[f"{f}_final"], ref[f"{f}_final"]) <= 1e-5
+    assert rel_err(st["vel_g2p"], ref["vel_g2p"]) <= 1e-5
+    assert rel_err(st["pos_adv"], ref["pos_adv"]) <= 1e-5
