@@ -344,6 +344,7 @@ int alloc_grids(flip_ctx *x) {
 
 int alloc_particles(flip_ctx *x, int cap) {
     int rc;
+    cap += cap & 1;   // planes of pairs of floats
     x->capacity = cap;
     x->idSpace = cap;
     ParticleSoA *bufs[2] = {&x->pa, &x->pb};
@@ -370,6 +371,7 @@ int grow_particles(flip_ctx *x, int cap) {
     // a quarter more than asked for, so that steady emission grows the
     // storage rarely
     cap = (int)std::min<long long>(std::max<long long>(cap, (long long)x->capacity * 5 / 4), 0x7ffffff0LL);
+    cap += cap & 1;   // as alloc_particles does
     ParticleSoA keep = x->pa;
     const int oldCap = x->capacity;
     void *old[] = {x->pa.px, x->pb.px, x->keys, x->slots, x->idFlags, x->idRank, x->idScratch, x->idTotal};

@@ -3,6 +3,7 @@
 // collision particle update.  Every kernel is an HBM-bound gather/stencil;
 // nothing here is a dense contraction, so no tensor cores are involved.
 #include <cstdio>
+#include <type_traits>
 
 #include "flip_device.cuh"
 
@@ -340,17 +341,20 @@ __global__ void __launch_bounds__(1024) k_liquid_sdf(ParticleSoA ps, const int *
 // them (18 per face); each particle's weight is evaluated in the reference's
 // 10^3-block frame, which the three faces share.  Sums run in a fixed (cell,
 // id) order, so the result is deterministic (no float atomics).
-// Bound by L1: the lanes of a warp visit different cells, so a load touches 32
-// lines.  Three scalar loads a particle for three faces, against three a face
-// in a kernel per direction: P2G and extrapolation 2195 -> 1260 us at
-// 256x128x128, 857 -> 756 us at 128^3 (of which the extrapolation is 100).
-// 16-byte vectors instead of scalars touch four times the lines: slower.
+// Bound by instructions: 144 candidates a face, 22 within r.  So two particles
+// at a time, in packed arithmetic (each half rounds as the scalar operation),
+// and of each row of cells only the faces it can reach.  The lanes of a warp
+// visit different cells, so a load touches 32 lines; positions and velocities
+// load in pairs.  P2G at 128^3 (4.1M particles), at 256x128x128 (14.0M): a kernel
+// per direction 740, 2000 us; one for the three 640, 1160; now 433, 730.  16-byte
+// vectors of a particle's coordinates touch four times the lines: slower.
 // The reference also requires the face to lie in the particle's local box and
 // the particle to be in the block's list, both taken with the support radius
 // sr = r + 1e-6.  A particle within r of the face meets both: every coordinate
 // of the face is within r of the particle, and the 1e-6 margin is far above
 // the rounding of these float expressions (ulp(1) ~ 1.2e-7).
-__global__ void __launch_bounds__(TPB) k_p2g(ParticleSoA p, const int *cellStart, StepConsts c,
+constexpr int P2G_TPB = 128;
+__global__ void __launch_bounds__(P2G_TPB, 1024 / P2G_TPB) k_p2g(ParticleSoA p, const int *cellStart, StepConsts c,
                                              float *U, float *V, float *W, uint8_t *vu, uint8_t *vv, uint8_t *vw) {
     const int ni = c.I + 1, nj = c.J + 1, nk = c.K + 1;
     const long long f = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -372,35 +376,67 @@ __global__ void __launch_bounds__(TPB) k_p2g(ParticleSoA p, const int *cellStart
     const int cx0 = max(fi - 1, 0), cx1 = min(fi + 1, c.I - 1), cy0 = max(fj - 1, 0), cy1 = min(fj + 1, c.J - 1),
               cz0 = max(fk - 1, 0), cz1 = min(fk + 1, c.K - 1);
     Dims cells{c.I, c.J, c.K};
+    const F2 nox = f2(-offx, -offx), noy = f2(-offy, -offy), noz = f2(-offz, -offz), nh = f2(-h, -h);
+    const F2 pgx = f2(gx, gx), pgy = f2(gy, gy), pgz = f2(gz, gz);
+    const F2 c1 = f2(coef1, coef1), c2 = f2(coef2, coef2), c3 = f2(coef3, coef3), one = F2_ONE;
     float sc[3] = {0.0f, 0.0f, 0.0f}, wt[3] = {0.0f, 0.0f, 0.0f};
-    auto take = [&](int d, float d2, float v) {
-        const float w3 = __fmul_rn(__fmul_rn(__fmul_rn(coef1, d2), d2), d2);
-        const float w2 = __fmul_rn(__fmul_rn(coef2, d2), d2);
-        const float w1 = __fmul_rn(coef3, d2);
-        const float wgt = __fsub_rn(__fadd_rn(__fsub_rn(1.0f, w3), w2), w1);
-        sc[d] = __fadd_rn(sc[d], __fmul_rn(wgt, v));
-        wt[d] = __fadd_rn(wt[d], wgt);
+    // Two particles' shares of a face: weights of the two together, then the
+    // sums in the particles' order.
+    auto take = [&](int d, F2 d2, const F2 *vel, bool first, bool second) {
+        const bool h0 = first && f2_x(d2) < rsq, h1 = second && f2_y(d2) < rsq;
+        if (!(h0 | h1)) return;
+        const F2 v = *vel;
+        const F2 w3 = f2_mul(f2_mul(f2_mul(c1, d2), d2), d2), w2 = f2_mul(f2_mul(c2, d2), d2), w1 = f2_mul(c3, d2);
+        const F2 wgt = f2_sub(f2_add(f2_sub(one, w3), w2), w1), wv = f2_mul(wgt, v);
+        if (h0) {
+            sc[d] = __fadd_rn(sc[d], f2_x(wv));
+            wt[d] = __fadd_rn(wt[d], f2_x(wgt));
+        }
+        if (h1) {
+            sc[d] = __fadd_rn(sc[d], f2_y(wv));
+            wt[d] = __fadd_rn(wt[d], f2_y(wgt));
+        }
     };
+    // Particles [from, to) for those of the three faces that they can reach,
+    // in pairs as they lie in memory (the planes hold an even number).
+    auto row = [&](auto useU, auto useV, auto useW, int from, int to) {
+        for (int t = from & ~1; t < to; t += 2) {
+            const bool first = t >= from, second = t + 1 < to;
+            auto pair = [&](const float *plane) { return reinterpret_cast<const F2 *>(plane + t); };
+            const F2 px = *pair(p.px), py = *pair(p.py), pz = *pair(p.pz);
+            auto square = [](F2 g, F2 q, F2 no) {   // (g - (q - off))^2
+                const F2 d = f2_sub(g, f2_add(q, no));
+                return f2_mul(d, d);
+            };
+            const F2 xx1 = square(pgx, f2_add(px, nh), nox), yy1 = square(pgy, f2_add(py, nh), noy),
+                     zz1 = square(pgz, f2_add(pz, nh), noz);
+            if (useU.value) take(0, f2_add(f2_add(square(pgx, px, nox), yy1), zz1), pair(p.vx), first, second);
+            if (useV.value) take(1, f2_add(f2_add(xx1, square(pgy, py, noy)), zz1), pair(p.vy), first, second);
+            if (useW.value) take(2, f2_add(f2_add(xx1, yy1), square(pgz, pz, noz)), pair(p.vz), first, second);
+        }
+    };
+    using Yes = std::true_type;
+    using No = std::false_type;
     for (int cz = cz0; cz <= cz1; cz++)
         for (int cy = cy0; cy <= cy1; cy++) {
-            // the row's particles; those of cells up to fi can reach the u face
+            // the row's particles: cells up to fi can reach the u face (those in
+            // pb..pu), rows up to fj the v face, up to fk the w face
             const long long base = cells.idx(0, cy, cz);
             const int pb = cellStart[base + cx0], pe = cellStart[base + cx1 + 1];
             if (pb == pe) continue;
             const int pu = isU ? cellStart[base + min(fi, c.I - 1) + 1] : pb;
             const bool rowV = isV && cy <= fj, rowW = isW && cz <= fk;
-            for (int t = pb; t < pe; t++) {
-                const float px = p.px[t], py = p.py[t], pz = p.pz[t];
-                const float x0 = __fsub_rn(gx, __fsub_rn(px, offx)), x1 = __fsub_rn(gx, __fsub_rn(__fsub_rn(px, h), offx));
-                const float y0 = __fsub_rn(gy, __fsub_rn(py, offy)), y1 = __fsub_rn(gy, __fsub_rn(__fsub_rn(py, h), offy));
-                const float z0 = __fsub_rn(gz, __fsub_rn(pz, offz)), z1 = __fsub_rn(gz, __fsub_rn(__fsub_rn(pz, h), offz));
-                const float xx0 = __fmul_rn(x0, x0), xx1 = __fmul_rn(x1, x1), yy0 = __fmul_rn(y0, y0), yy1 = __fmul_rn(y1, y1),
-                            zz0 = __fmul_rn(z0, z0), zz1 = __fmul_rn(z1, z1);
-                const float du = __fadd_rn(__fadd_rn(xx0, yy1), zz1), dv = __fadd_rn(__fadd_rn(xx1, yy0), zz1),
-                            dw = __fadd_rn(__fadd_rn(xx1, yy1), zz0);
-                if (t < pu && du < rsq) take(0, du, p.vx[t]);
-                if (rowV && dv < rsq) take(1, dv, p.vy[t]);
-                if (rowW && dw < rsq) take(2, dw, p.vz[t]);
+            if (rowV && rowW) {
+                row(Yes{}, Yes{}, Yes{}, pb, pu);
+                row(No{}, Yes{}, Yes{}, pu, pe);
+            } else if (rowV) {
+                row(Yes{}, Yes{}, No{}, pb, pu);
+                row(No{}, Yes{}, No{}, pu, pe);
+            } else if (rowW) {
+                row(Yes{}, No{}, Yes{}, pb, pu);
+                row(No{}, No{}, Yes{}, pu, pe);
+            } else {
+                row(Yes{}, No{}, No{}, pb, pu);
             }
         }
     const float eps = 1e-6f;
@@ -890,7 +926,7 @@ void launch_liquid_sdf(const ParticleSoA &p, const int *cellStart, const StepCon
 void launch_p2g(const ParticleSoA &p, const int *cellStart, const StepConsts &c, float *u, float *v,
                 float *w, uint8_t *vu, uint8_t *vv, uint8_t *vw, cudaStream_t s) {
     FLIP_COUNT(1);
-    k_p2g<<<div_up((long long)(c.I + 1) * (c.J + 1) * (c.K + 1), TPB), TPB, 0, s>>>(p, cellStart, c, u, v, w, vu, vv, vw);
+    k_p2g<<<div_up((long long)(c.I + 1) * (c.J + 1) * (c.K + 1), P2G_TPB), P2G_TPB, 0, s>>>(p, cellStart, c, u, v, w, vu, vv, vw);
 }
 FaceBits face_bits(int I, int J, int K) {
     FaceBits b;

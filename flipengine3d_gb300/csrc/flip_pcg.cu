@@ -655,27 +655,6 @@ __device__ __forceinline__ float2 df_scale(float f, float2 v) {
     const float pl = __fmaf_rn(f, v.y, __fmaf_rn(f, v.x, -ph));
     return make_float2(ph, pl);
 }
-// Pairs of floats in one 64-bit register (two cells): each operation rounds
-// each half as the scalar one does.  Sums and products are written as fused
-// multiply-adds that are exact up to that one rounding (a b + 0, a 1 + b), so
-// the compiler cannot contract two operations into one.
-using F2 = unsigned long long;
-__device__ __forceinline__ F2 f2(float x, float y) {
-    F2 r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(x), "f"(y));
-    return r;
-}
-__device__ __forceinline__ float f2_x(F2 v) { return __uint_as_float((unsigned)v); }
-__device__ __forceinline__ float f2_y(F2 v) { return __uint_as_float((unsigned)(v >> 32)); }
-__device__ __forceinline__ F2 f2_fma(F2 a, F2 b, F2 c) {
-    F2 r;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-    return r;
-}
-constexpr F2 F2_ONE = 0x3f8000003f800000ull, F2_MINUS = 0xbf800000bf800000ull, F2_ZERO = 0x8000000080000000ull;   // -0
-__device__ __forceinline__ F2 f2_add(F2 a, F2 b) { return f2_fma(a, F2_ONE, b); }
-__device__ __forceinline__ F2 f2_sub(F2 a, F2 b) { return f2_fma(b, F2_MINUS, a); }
-__device__ __forceinline__ F2 f2_mul(F2 a, F2 b) { return f2_fma(a, b, F2_ZERO); }
 // (sh, sl) += (ah, al) s for two cells, ns = -s: the leading product exact as
 // its rounded value plus its FMA-recovered error, the sum's rounding error by
 // Knuth's TwoSum
