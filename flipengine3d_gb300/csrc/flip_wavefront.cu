@@ -282,10 +282,11 @@ __device__ __forceinline__ bool run_steps(const WarpJob &w) {
     constexpr unsigned CHB = (CH / EC) * GW * 4;   // edge bytes of a chunk
     // forward: the products of the last cell, for the next one along i, a and
     // b; backward: its z, which all three take
-    float tx = 0.0f, sA = 0.0f, sB = 0.0f;
+    float tx = 0.0f, sA = 0.0f, sB = 0.0f, nA = 0.0f, nB = 0.0f;
     // the edge words of the next group, read ahead
     uint4 na = ld_edge(w.inA + (WHOLE ? w.c0 * CHB : 0)), nb = ld_edge(w.inB + (WHOLE ? w.c0 * CHB : 0));
     unsigned ready = 0;   // the next chunk's operands were seen to be in
+    bool miss = __any_sync(0xffffffffu, any_absent(na, nb));   // words of the next group had not come
     float *out = w.out + (ptrdiff_t)(FWD ? w.c0 * CH : w.lastStep - w.c0 * CH) * NP;
     unsigned long long *xA = w.xA + (size_t)w.c0 * CH * WB, *xB = w.xB + (size_t)w.c0 * CH * WA;
     unsigned cw = WHOLE ? w.c0 * CHB : 0;   // the chunk's edge words
@@ -314,15 +315,14 @@ __device__ __forceinline__ bool run_steps(const WarpJob &w) {
         float xa[EC], xb[EC];
         bool fine = true;
         // the group's edge words, read ahead or awaited
-        auto take_edges = [&](unsigned off) {
-            while (__any_sync(0xffffffffu, any_absent(na, nb))) {
-                for (unsigned spin = 0;;) {
-                    na = ld_edge(w.inA + off);
-                    nb = ld_edge(w.inB + off);
-                    if (!__any_sync(0xffffffffu, any_absent(na, nb))) break;
-                    __nanosleep(20);   // leaves the issue slots to the kernels of other streams; no cost alone
-                    if (edge_gives_up(++spin, &w.sm->abort, w.err, w.spinLimit)) { fine = false; return; }
-                }
+        auto take_edges = [&](unsigned off, bool miss) {
+            for (unsigned spin = 0; miss;) {
+                na = ld_edge(w.inA + off);
+                nb = ld_edge(w.inB + off);
+                miss = __any_sync(0xffffffffu, any_absent(na, nb));
+                if (!miss) break;
+                __nanosleep(20);   // leaves the issue slots to the kernels of other streams; no cost alone
+                if (edge_gives_up(++spin, &w.sm->abort, w.err, w.spinLimit)) { fine = false; return; }
             }
             if (!WHOLE) {   // the ring's words are free again once all warps are done with the chunk
                 __syncwarp();
@@ -341,8 +341,7 @@ __device__ __forceinline__ bool run_steps(const WarpJob &w) {
                 Ln = L[q * NP];
                 rn = r[q * NP];
             }
-            float vA = FWD ? __shfl_up_sync(0xffffffffu, sA, 1) : __shfl_down_sync(0xffffffffu, sA, 1);
-            float vB = FWD ? __shfl_up_sync(0xffffffffu, sB, VA) : __shfl_down_sync(0xffffffffu, sB, VA);
+            float vA = nA, vB = nB;
             if (w.inEdgeA) vA = xa[s];
             if (w.inEdgeB) vB = xb[s];
             float acc, res;
@@ -361,6 +360,8 @@ __device__ __forceinline__ bool run_steps(const WarpJob &w) {
                 res = __fmul_rn(acc, Lc.x);
                 tx = sA = sB = res;
             }
+            nA = FWD ? __shfl_up_sync(0xffffffffu, sA, 1) : __shfl_down_sync(0xffffffffu, sA, 1);
+            nB = FWD ? __shfl_up_sync(0xffffffffu, sB, VA) : __shfl_down_sync(0xffffffffu, sB, VA);
             __stcg(out + (FWD ? u : -u) * NP, res);
             constexpr int off = ((u + 1) / EC % (CH / EC)) * GW * 4 + (u + 1) % EC * 4;
             hand_on<off>(u < 7 ? dA : dA7, sA);
@@ -371,22 +372,24 @@ __device__ __forceinline__ bool run_steps(const WarpJob &w) {
             }
         };
         using std::integral_constant;
-        take_edges(cw);
+        take_edges(cw, miss);
         if (!fine) return false;
         step(integral_constant<int, 0>{});
         step(integral_constant<int, 1>{});
-        step(integral_constant<int, 2>{});
         na = ld_edge(w.inA + cw + GW * 4);
         nb = ld_edge(w.inB + cw + GW * 4);
+        step(integral_constant<int, 2>{});
+        miss = __any_sync(0xffffffffu, any_absent(na, nb));
         step(integral_constant<int, 3>{});
-        take_edges(cw + GW * 4);
+        take_edges(cw + GW * 4, miss);
         if (!fine) return false;
         step(integral_constant<int, 4>{});
         step(integral_constant<int, 5>{});
-        step(integral_constant<int, 6>{});
         na = ld_edge(w.inA + cw1);   // past the last chunk: a place that is not used
         nb = ld_edge(w.inB + cw1);
         ready = mb_peek(smem_addr(&w.sm->loaded[(n + 1) % NBUF]), ((n + 1) / NBUF) & 1);
+        step(integral_constant<int, 6>{});
+        miss = __any_sync(0xffffffffu, any_absent(na, nb));
         step(integral_constant<int, 7>{});
         out += (FWD ? CH : -CH) * NP;
         cw = cw1;
