@@ -353,9 +353,19 @@ __global__ void __launch_bounds__(1024) k_liquid_sdf(ParticleSoA ps, const int *
 // sr = r + 1e-6.  A particle within r of the face meets both: every coordinate
 // of the face is within r of the particle, and the 1e-6 margin is far above
 // the rounding of these float expressions (ulp(1) ~ 1.2e-7).
+// Packed sums and products as fused multiply-adds that are exact up to the one
+// rounding, with constants that the compiler does not see: it folds a visible 1
+// or 0 away and then contracts a product with the sum after it.
+struct PairConsts {
+    F2 one, minus, zero;   // (1, 1), (-1, -1), (-0, -0)
+    __device__ F2 mul(F2 a, F2 b) const { return f2_fma(a, b, zero); }
+    __device__ F2 add(F2 a, F2 b) const { return f2_fma(a, one, b); }
+    __device__ F2 sub(F2 a, F2 b) const { return f2_fma(b, minus, a); }
+};
 constexpr int P2G_TPB = 128;
 __global__ void __launch_bounds__(P2G_TPB, 1024 / P2G_TPB) k_p2g(ParticleSoA p, const int *cellStart, StepConsts c,
-                                             float *U, float *V, float *W, uint8_t *vu, uint8_t *vv, uint8_t *vw) {
+                                             float *U, float *V, float *W, uint8_t *vu, uint8_t *vv, uint8_t *vw,
+                                             PairConsts k2) {
     const int ni = c.I + 1, nj = c.J + 1, nk = c.K + 1;
     const long long f = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (f >= (long long)ni * nj * nk) return;
@@ -378,7 +388,7 @@ __global__ void __launch_bounds__(P2G_TPB, 1024 / P2G_TPB) k_p2g(ParticleSoA p, 
     Dims cells{c.I, c.J, c.K};
     const F2 nox = f2(-offx, -offx), noy = f2(-offy, -offy), noz = f2(-offz, -offz), nh = f2(-h, -h);
     const F2 pgx = f2(gx, gx), pgy = f2(gy, gy), pgz = f2(gz, gz);
-    const F2 c1 = f2(coef1, coef1), c2 = f2(coef2, coef2), c3 = f2(coef3, coef3), one = F2_ONE;
+    const F2 c1 = f2(coef1, coef1), c2 = f2(coef2, coef2), c3 = f2(coef3, coef3), one = k2.one;
     float sc[3] = {0.0f, 0.0f, 0.0f}, wt[3] = {0.0f, 0.0f, 0.0f};
     // Two particles' shares of a face: weights of the two together, then the
     // sums in the particles' order.
@@ -386,8 +396,8 @@ __global__ void __launch_bounds__(P2G_TPB, 1024 / P2G_TPB) k_p2g(ParticleSoA p, 
         const bool h0 = first && f2_x(d2) < rsq, h1 = second && f2_y(d2) < rsq;
         if (!(h0 | h1)) return;
         const F2 v = *vel;
-        const F2 w3 = f2_mul(f2_mul(f2_mul(c1, d2), d2), d2), w2 = f2_mul(f2_mul(c2, d2), d2), w1 = f2_mul(c3, d2);
-        const F2 wgt = f2_sub(f2_add(f2_sub(one, w3), w2), w1), wv = f2_mul(wgt, v);
+        const F2 w3 = k2.mul(k2.mul(k2.mul(c1, d2), d2), d2), w2 = k2.mul(k2.mul(c2, d2), d2), w1 = k2.mul(c3, d2);
+        const F2 wgt = k2.sub(k2.add(k2.sub(one, w3), w2), w1), wv = k2.mul(wgt, v);
         if (h0) {
             sc[d] = __fadd_rn(sc[d], f2_x(wv));
             wt[d] = __fadd_rn(wt[d], f2_x(wgt));
@@ -404,15 +414,15 @@ __global__ void __launch_bounds__(P2G_TPB, 1024 / P2G_TPB) k_p2g(ParticleSoA p, 
             const bool first = t >= from, second = t + 1 < to;
             auto pair = [&](const float *plane) { return reinterpret_cast<const F2 *>(plane + t); };
             const F2 px = *pair(p.px), py = *pair(p.py), pz = *pair(p.pz);
-            auto square = [](F2 g, F2 q, F2 no) {   // (g - (q - off))^2
-                const F2 d = f2_sub(g, f2_add(q, no));
-                return f2_mul(d, d);
+            auto square = [&](F2 g, F2 q, F2 no) {   // (g - (q - off))^2
+                const F2 d = k2.sub(g, k2.add(q, no));
+                return k2.mul(d, d);
             };
-            const F2 xx1 = square(pgx, f2_add(px, nh), nox), yy1 = square(pgy, f2_add(py, nh), noy),
-                     zz1 = square(pgz, f2_add(pz, nh), noz);
-            if (useU.value) take(0, f2_add(f2_add(square(pgx, px, nox), yy1), zz1), pair(p.vx), first, second);
-            if (useV.value) take(1, f2_add(f2_add(xx1, square(pgy, py, noy)), zz1), pair(p.vy), first, second);
-            if (useW.value) take(2, f2_add(f2_add(xx1, yy1), square(pgz, pz, noz)), pair(p.vz), first, second);
+            const F2 xx1 = square(pgx, k2.add(px, nh), nox), yy1 = square(pgy, k2.add(py, nh), noy),
+                     zz1 = square(pgz, k2.add(pz, nh), noz);
+            if (useU.value) take(0, k2.add(k2.add(square(pgx, px, nox), yy1), zz1), pair(p.vx), first, second);
+            if (useV.value) take(1, k2.add(k2.add(xx1, square(pgy, py, noy)), zz1), pair(p.vy), first, second);
+            if (useW.value) take(2, k2.add(k2.add(xx1, yy1), square(pgz, pz, noz)), pair(p.vz), first, second);
         }
     };
     using Yes = std::true_type;
@@ -926,7 +936,8 @@ void launch_liquid_sdf(const ParticleSoA &p, const int *cellStart, const StepCon
 void launch_p2g(const ParticleSoA &p, const int *cellStart, const StepConsts &c, float *u, float *v,
                 float *w, uint8_t *vu, uint8_t *vv, uint8_t *vw, cudaStream_t s) {
     FLIP_COUNT(1);
-    k_p2g<<<div_up((long long)(c.I + 1) * (c.J + 1) * (c.K + 1), P2G_TPB), P2G_TPB, 0, s>>>(p, cellStart, c, u, v, w, vu, vv, vw);
+    k_p2g<<<div_up((long long)(c.I + 1) * (c.J + 1) * (c.K + 1), P2G_TPB), P2G_TPB, 0, s>>>(p, cellStart, c, u, v, w, vu, vv, vw,
+                                                                                                  PairConsts{F2_ONE, F2_MINUS, F2_ZERO});
 }
 FaceBits face_bits(int I, int J, int K) {
     FaceBits b;
