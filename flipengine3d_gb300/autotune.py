@@ -2,8 +2,8 @@
 
 The knobs change how work is laid on the GPU, not what is computed:
 
-* ``sdf_threads``: the CTA size of the liquid-SDF kernel (one CTA per block
-  of 10^3 cells): 256, 512 or 1024 threads;
+* ``sdf_threads``: the threads of two CTAs of the liquid-SDF kernel (a thread
+  per cell): 256, 512 or 1024;
 * ``pcg_cells_per_cta``: grid cells per CTA of the PCG row kernels'
   reduction grid;
 * ``sweep_orientation``: the preconditioner sweep tiles' lane axis, j (0) or

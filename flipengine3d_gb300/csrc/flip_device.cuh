@@ -28,6 +28,7 @@ struct StepConsts {
     int maxPerCell;
     // the reference's blocks of 10 cells, for its particle lists: float edge, 1 / edge
     float blockdxf, invBlockf;
+    float centre[10];   // a cell's centre in its block's frame, by its place there
     double invBlock;
     // near-solid coarse grid
     int nsi, nsj, nsk;

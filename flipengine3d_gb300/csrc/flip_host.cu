@@ -1108,6 +1108,7 @@ int flip_create(int isize, int jsize, int ksize, double dx, flip_ctx **out) {
     c.dx = dx; c.invdx = 1.0 / dx; c.invdxf = (float)(1.0 / dx); c.dxf = (float)dx;
     c.radius = 0.5 * 1.0 * dx * std::sqrt(3.0);
     c.blockdxf = (float)(10 * dx);
+    for (int a = 0; a < 10; a++) c.centre[a] = (float)((double)(float)a * dx + 0.5 * dx);
     c.invBlock = 1.0 / (double)c.blockdxf;
     c.invBlockf = (float)c.invBlock;
     auto below = [](double bound) {   // largest float v with (double)v < bound

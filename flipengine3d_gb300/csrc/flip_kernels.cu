@@ -209,9 +209,14 @@ __global__ void k_gather(ParticleSoA src, ParticleSoA dst, const int *start, con
 // square root give the reference's bits.  Here each cell looks for its nearest
 // particle: its own cell first, then the rows of cells around it, nearest
 // first, as long as a row can still hold a nearer one.  A cell inside the
-// liquid has a particle within half a cell and stops at its own; scattering
-// every particle into the ~100 cells of its box through shared-memory atomics
-// took 830 us at 128^3 (4.1M particles), 380 us at 64^3.
+// liquid has a particle within half a cell and stops at its own, and the air
+// far from it knows from a look of the warp at the 25 rows around.  Bound by the
+// latency and the instructions of the cells near the surface: 223 us at 128^3
+// (4.1M particles), 68 at 64^3; scattering every particle
+// into the ~100 cells of its box through shared-memory atomics took 820, 370.
+// 64 registers a thread: with 128 the occupancy is too low, with 42 small grids
+// lose what large ones gain (in CTAs of 512: 313, 456 and 274 us at 128^3, 68, 94
+// and 74 at 64^3).
 // Then the solid post-process (particlelevelset.cpp:172-196).
 constexpr int BW = 10;
 
@@ -251,21 +256,38 @@ __constant__ signed char kRing[25][2] = {
     {0, 0},  {-1, 0}, {1, 0},  {0, -1},  {0, 1},  {-1, -1}, {1, -1}, {-1, 1}, {1, 1},  {-2, 0}, {2, 0},  {0, -2}, {0, 2},
     {-2, -1}, {2, -1}, {-2, 1}, {2, 1}, {-1, -2}, {1, -2}, {-1, 2}, {1, 2}, {-2, -2}, {2, -2}, {-2, 2}, {2, 2}};
 
-// The CTA size is a tuning knob (256, 512 or 1024 threads; default 512).
-__global__ void __launch_bounds__(1024) k_liquid_sdf(ParticleSoA ps, const int *cellStart, StepConsts c,
+// A tuning knob sets the threads of two CTAs (256, 512 or 1024; default 512).
+template <int SDF_TPB>
+__global__ void __launch_bounds__(SDF_TPB, 1024 / SDF_TPB) k_liquid_sdf(ParticleSoA ps, const int *cellStart, StepConsts c,
                                                      const uint8_t *solidCC, float *phi) {
     const long long ci = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     Dims cells{c.I, c.J, c.K};
-    if (ci >= cells.size()) return;
+    const bool valid = ci < cells.size();
     int gi, gj, gk;
-    unflatten(ci, c.I, c.J, gi, gj, gk);
+    unflatten(valid ? ci : 0, c.I, c.J, gi, gj, gk);
+    // Which of the rows around hold particles that the warp's cells could reach:
+    // where the cells are of one row, a lane looks at a row; no row, no search.
+    const int lane = threadIdx.x & 31, gi0 = __shfl_sync(0xffffffffu, gi, 0), gi1 = __shfl_sync(0xffffffffu, gi, 31);
+    unsigned rows = 0x1ffffffu;
+    if (__all_sync(0xffffffffu, valid && gi == gi0 + lane)) {
+        bool any = false;
+        if (lane < 25) {
+            const int y = gj + kRing[lane][0], z = gk + kRing[lane][1];
+            if (y >= 0 && z >= 0 && y < c.J && z < c.K) {
+                const long long base = cells.idx(0, y, z);
+                any = cellStart[base + max(gi0 - 2, 0)] != cellStart[base + min(gi1 + 2, c.I - 1) + 1];
+            }
+        }
+        rows = __ballot_sync(0xffffffffu, any);
+    }
+    if (!valid) return;
     const double dx = c.dx;
     const float maxd = (float)(3.0 * dx);
     const float r = (float)c.radius;
     const float sr = __fmul_rn(2.0f, r);
     const int bx = gi / BW, by = gj / BW, bz = gk / BW, a = gi - bx * BW, b = gj - by * BW, cc = gk - bz * BW;
     const float offx = c.blockPos[bx + 1], offy = c.blockPos[by + 1], offz = c.blockPos[bz + 1];
-    const float cx = cell_centre(a, dx), cy = cell_centre(b, dx), cz = cell_centre(cc, dx);
+    const float cx = c.centre[a], cy = c.centre[b], cz = c.centre[cc];
     // A particle nearer than this is within the search radius and so in the
     // list and the box, whatever the rounding; farther ones are looked up.
     // The box reaches sr + dx / 2 = 2.2321 dx along an axis.
@@ -274,22 +296,34 @@ __global__ void __launch_bounds__(1024) k_liquid_sdf(ParticleSoA ps, const int *
     // axis, less a margin far above the rounding of the distances below.
     const float h1 = 0.499f * c.dxf, h2 = 1.499f * c.dxf, q1 = h1 * h1, q2 = h2 * h2;
     float best = __uint_as_float(0x7f800000u);   // +inf
+    // The cell's centre in the simulation's frame, for a first look: `slack` is far
+    // above what the rounding of such coordinates makes of a squared distance.
+    const float mx = offx + cx, my = offy + cy, mz = offz + cz, slack = 0.03f * c.dxf * c.dxf;
     // four particles at a time, so that their loads overlap (the last one
     // repeated at the end does not change the minimum)
     auto look = [&](int from, int to) {
         for (int t = from; t < to; t += 4) {
-            float4 p[4];
-            float d2[4];
+            float x[4], y[4], z[4], d2[4];
 #pragma unroll
             for (int q = 0; q < 4; q++) {
                 const int tq = min(t + q, to - 1);
-                p[q] = make_float4(ps.px[tq], ps.py[tq], ps.pz[tq], 0.0f);
+                x[q] = ps.px[tq];
+                y[q] = ps.py[tq];
+                z[q] = ps.pz[tq];
             }
             bool hit = false;
+            const float bar = best + slack;
 #pragma unroll
             for (int q = 0; q < 4; q++) {
-                const float ddx = __fsub_rn(cx, __fsub_rn(p[q].x, offx)), dy = __fsub_rn(cy, __fsub_rn(p[q].y, offy)),
-                            dz = __fsub_rn(cz, __fsub_rn(p[q].z, offz));
+                const float ex = x[q] - mx, ey = y[q] - my, ez = z[q] - mz;
+                hit |= __fmaf_rn(ez, ez, __fmaf_rn(ey, ey, ex * ex)) < bar;
+            }
+            if (!hit) continue;
+            hit = false;
+#pragma unroll
+            for (int q = 0; q < 4; q++) {
+                const float ddx = __fsub_rn(cx, __fsub_rn(x[q], offx)), dy = __fsub_rn(cy, __fsub_rn(y[q], offy)),
+                            dz = __fsub_rn(cz, __fsub_rn(z[q], offz));
                 d2[q] = __fadd_rn(__fadd_rn(__fmul_rn(ddx, ddx), __fmul_rn(dy, dy)), __fmul_rn(dz, dz));
                 // beyond the box along an axis: out, whatever the rounding
                 if (fmaxf(fabsf(ddx), fmaxf(fabsf(dy), fabsf(dz))) > reach) d2[q] = __uint_as_float(0x7f800000u);
@@ -298,17 +332,16 @@ __global__ void __launch_bounds__(1024) k_liquid_sdf(ParticleSoA ps, const int *
             if (!hit) continue;
 #pragma unroll
             for (int q = 0; q < 4; q++)
-                if (d2[q] < best && (d2[q] < near2 || sdf_reaches(c, p[q].x, p[q].y, p[q].z, __fsub_rn(p[q].x, offx),
-                                                                 __fsub_rn(p[q].y, offy), __fsub_rn(p[q].z, offz), sr, bx, by,
+                if (d2[q] < best && (d2[q] < near2 || sdf_reaches(c, x[q], y[q], z[q], __fsub_rn(x[q], offx),
+                                                                 __fsub_rn(y[q], offy), __fsub_rn(z[q], offz), sr, bx, by,
                                                                  bz, a, b, cc)))
                     best = d2[q];
         }
     };
-    look(cellStart[ci], cellStart[ci + 1]);
+    if (rows & 1) look(cellStart[ci], cellStart[ci + 1]);
     if (best > q1) {
-#pragma unroll 1
-        for (int n = 0; n < 25; n++) {
-            const int oy = kRing[n][0], oz = kRing[n][1];
+        for (unsigned left = rows; left; left &= left - 1) {
+            const int n = __ffs(left) - 1, oy = kRing[n][0], oz = kRing[n][1];
             const float ly = oy == 0 ? 0.0f : (oy == 1 || oy == -1 ? q1 : q2), lz = oz == 0 ? 0.0f : (oz == 1 || oz == -1 ? q1 : q2);
             const float row = ly + lz;   // as near as the row can be
             if (!(best > row)) continue;
@@ -931,7 +964,11 @@ void launch_gather_particles(const ParticleSoA &src, ParticleSoA dst, int n,
 void launch_liquid_sdf(const ParticleSoA &p, const int *cellStart, const StepConsts &c, const uint8_t *solidCC,
                        float *phi, int threads, cudaStream_t s) {
     FLIP_COUNT(1);
-    k_liquid_sdf<<<div_up((long long)c.I * c.J * c.K, threads), threads, 0, s>>>(p, cellStart, c, solidCC, phi);
+    // CTAs of half the knob's threads: a CTA lasts as long as its slowest warp
+    // (128^3: 223 us with CTAs of 256 threads, 299 with 512, 370 with 1024)
+    const int cta = threads / 2;
+    auto *kernel = cta == 128 ? k_liquid_sdf<128> : cta == 512 ? k_liquid_sdf<512> : k_liquid_sdf<256>;
+    kernel<<<div_up((long long)c.I * c.J * c.K, cta), cta, 0, s>>>(p, cellStart, c, solidCC, phi);
 }
 void launch_p2g(const ParticleSoA &p, const int *cellStart, const StepConsts &c, float *u, float *v,
                 float *w, uint8_t *vu, uint8_t *vv, uint8_t *vw, cudaStream_t s) {
