@@ -355,7 +355,7 @@ int flip_point_force_grid(int ni, int nj, int nk, double dx, int nfields, const 
                           float *w);
 
 /* Tuning knobs of the device kernels, no counterpart in the reference: the
- * liquid-SDF CTA size (256, 512 or 1024 threads), the grid cells per CTA of
+ * threads of two liquid-SDF CTAs (256, 512 or 1024), the grid cells per CTA of
  * the PCG row kernels' reduction grid (256 .. 2^20), and the preconditioner
  * sweep orientation (as flip_set_sweep_orientation).  A different reduction
  * grid sums the PCG's dot products in another order, so results move in the
