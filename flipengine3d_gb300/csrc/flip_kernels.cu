@@ -30,6 +30,8 @@ __device__ __forceinline__ F3 normalize3(F3 v) {
 
 // ------------------------------------------------------------------ binning
 __global__ void k_keys(ParticleSoA p, int n, StepConsts c, unsigned int *keys) {
+    pdl_wait();
+    pdl_trigger();
     int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= n) return;
     int i = exact_floor(p.px[t], c.invdx, c.invdxf);
@@ -40,6 +42,8 @@ __global__ void k_keys(ParticleSoA p, int n, StepConsts c, unsigned int *keys) {
 }
 
 __global__ void k_bin_count(const unsigned int *keys, int n, int *count) {
+    pdl_wait();
+    pdl_trigger();
     int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= n) return;
     unsigned int k = keys[t];
@@ -78,6 +82,8 @@ __device__ int block_scan_excl(int v, int *sh, int *total) {
 }
 
 __global__ void k_scan_tiles(const int *in, int n, int *out, int *tileSums) {
+    pdl_wait();
+    pdl_trigger();
     __shared__ int sh[32];
     long long base = (long long)blockIdx.x * SCAN_TILE + threadIdx.x * SCAN_PER;
     int v[SCAN_PER];
@@ -100,6 +106,8 @@ __global__ void k_scan_tiles(const int *in, int n, int *out, int *tileSums) {
 }
 
 __global__ void k_scan_sums(int *tileSums, int ntiles, int *grandTotal) {
+    pdl_wait();
+    pdl_trigger();
     __shared__ int sh[32];
     int v[SCAN_PER];
     int sum = 0;
@@ -121,12 +129,16 @@ __global__ void k_scan_sums(int *tileSums, int ntiles, int *grandTotal) {
 }
 
 __global__ void k_scan_add(int *out, int n, const int *tileSums, const int *grandTotal) {
+    pdl_wait();
+    pdl_trigger();
     long long g = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (g < n) out[g] += tileSums[g / SCAN_TILE];
     if (g == n) out[n] = *grandTotal;
 }
 
 __global__ void k_bin_scatter(const unsigned int *keys, int n, const int *start, int *cursor, int *slots) {
+    pdl_wait();
+    pdl_trigger();
     int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= n) return;
     unsigned int k = keys[t];
@@ -142,6 +154,8 @@ __global__ void k_bin_scatter(const unsigned int *keys, int n, const int *start,
 // Kept slots are compacted to the front of the cell's segment.
 __global__ void k_cell_sort_select(const int *start, int ncells, int *slots, const unsigned int *ids,
                                    const unsigned int *keys, int maxPerCell, int *survivors) {
+    pdl_wait();
+    pdl_trigger();
     int c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= ncells) return;
     int b = start[c], e = start[c + 1];
@@ -185,6 +199,8 @@ __device__ __forceinline__ float gather_one(const ParticleSoA &src, const Partic
 }
 __global__ void k_gather(ParticleSoA src, ParticleSoA dst, const int *start, const int *slots,
                          const int *newStart, int ncells, unsigned int *maxSpeedSqBits) {
+    pdl_wait();
+    pdl_trigger();
     const int t = blockIdx.x * blockDim.x + threadIdx.x, total = newStart[ncells];
     float best = 0.0f;
     if (total == start[ncells]) {
@@ -260,6 +276,8 @@ __constant__ signed char kRing[25][2] = {
 template <int SDF_TPB>
 __global__ void __launch_bounds__(SDF_TPB, 1024 / SDF_TPB) k_liquid_sdf(ParticleSoA ps, const int *cellStart, StepConsts c,
                                                      const uint8_t *solidCC, float *phi) {
+    pdl_wait();
+    pdl_trigger();
     const long long ci = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     Dims cells{c.I, c.J, c.K};
     const bool valid = ci < cells.size();
@@ -399,6 +417,8 @@ constexpr int P2G_TPB = 128;
 __global__ void __launch_bounds__(P2G_TPB, 1024 / P2G_TPB) k_p2g(ParticleSoA p, const int *cellStart, StepConsts c,
                                              float *U, float *V, float *W, uint8_t *vu, uint8_t *vv, uint8_t *vw,
                                              PairConsts k2) {
+    pdl_wait();
+    pdl_trigger();
     const int ni = c.I + 1, nj = c.J + 1, nk = c.K + 1;
     const long long f = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (f >= (long long)ni * nj * nk) return;
@@ -510,6 +530,8 @@ __device__ __forceinline__ void face_word(const FaceBits &b, long long t, int &d
 }
 __global__ void __launch_bounds__(TPB) k_extrap_init(FaceBits b, const uint8_t *vu, const uint8_t *vv, const uint8_t *vw,
                                                      unsigned *known) {
+    pdl_wait();
+    pdl_trigger();
     const int lane = threadIdx.x & 31;
     const long long first = ((long long)blockIdx.x * (TPB / 32) + (threadIdx.x >> 5)) * 8;   // eight words a warp
 #pragma unroll
@@ -604,6 +626,8 @@ __global__ void __launch_bounds__(TPB) k_extrap_layer(FaceBits b, const unsigned
 __global__ void k_save_force(long long nu, long long nv, long long nw, float *u, float *v, float *w, float *su,
                              float *sv, float *sw, float fx, float fy, float fz, int ax, int ay, int az,
                              const uint8_t *ex) {
+    pdl_wait();
+    pdl_trigger();
     long long f = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     const bool skip = ex && f < nu + nv + nw && ex[f];
     if (f < nu) {
@@ -623,6 +647,8 @@ __global__ void k_save_force(long long nu, long long nv, long long nw, float *u,
 __global__ void k_constrain(long long nu, long long nv, long long nw, float *u, float *v, float *w, float *su,
                             float *sv, float *sw, const float *wu, const float *wv, const float *ww, const float *fu,
                             const float *fv, const float *fw) {
+    pdl_wait();
+    pdl_trigger();
     long long f = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     float *G, *S;
     const float *W, *F;
@@ -850,6 +876,8 @@ __global__ void __launch_bounds__(TPB) k_advect(ParticleSoA p, int n, StepConsts
                                                 const float *S, const uint8_t *ns, float picRatio, float flipRatio,
                                                 double dt, unsigned int *keys, unsigned int *hist, double speedStep,
                                                 const InflowConstraint ic) {
+    pdl_wait();
+    pdl_trigger();
     __shared__ unsigned int shist[8];
     if (threadIdx.x < 8) shist[threadIdx.x] = 0;
     __syncthreads();
@@ -909,6 +937,8 @@ __global__ void __launch_bounds__(TPB) k_advect(ParticleSoA p, int n, StepConsts
 // _getMarkerParticleSpeedLimit (fluidsimulation.cpp:4298-4322), one thread
 __global__ void k_speed_limit(const unsigned int *hist, int n, int bins, double step, double maxPct, int maxAbs,
                               float *maxSpeedSq) {
+    pdl_wait();
+    pdl_trigger();
     int maxRemoval = (int)fmin((double)(int)((double)n * maxPct), (double)maxAbs);
     double maxspeed = bins * step;
     int cur = 0;
@@ -922,6 +952,8 @@ __global__ void k_speed_limit(const unsigned int *hist, int n, int bins, double 
 }
 
 __global__ void k_mark_fast(ParticleSoA p, int n, const float *maxSpeedSq, unsigned int *keys) {
+    pdl_wait();
+    pdl_trigger();
     int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= n) return;
     unsigned int k = keys[t];
@@ -934,31 +966,30 @@ __global__ void k_mark_fast(ParticleSoA p, int n, const float *maxSpeedSq, unsig
 
 // ------------------------------------------------------------------ launchers
 void launch_keys_from_positions(const ParticleSoA &p, int n, const StepConsts &c, unsigned int *keys, cudaStream_t s) {
-    if (n > 0) { FLIP_COUNT(1); k_keys<<<div_up(n, TPB), TPB, 0, s>>>(p, n, c, keys); }
+    if (n > 0) launch_next(k_keys, div_up(n, TPB), TPB, s, p, n, c, keys);
 }
 void launch_bin_count(const unsigned int *keys, int n, int *cellCount, cudaStream_t s) {
-    if (n > 0) { FLIP_COUNT(1); k_bin_count<<<div_up(n, TPB), TPB, 0, s>>>(keys, n, cellCount); }
+    if (n > 0) launch_next(k_bin_count, div_up(n, TPB), TPB, s, keys, n, cellCount);
 }
 int scan_scratch_ints(int ncells) { return (int)div_up(ncells + 1, SCAN_TILE) + 2; }
 void launch_scan_cells(const int *count, int ncells, int *start, int *scratch, int *total, cudaStream_t s) {
     int ntiles = (int)div_up(ncells, SCAN_TILE);
-    { FLIP_COUNT(1); k_scan_tiles<<<ntiles, SCAN_T, 0, s>>>(count, ncells, start, scratch); }
-    { FLIP_COUNT(1); k_scan_sums<<<1, SCAN_T, 0, s>>>(scratch, ntiles, total); }
-    { FLIP_COUNT(1); k_scan_add<<<div_up(ncells + 1, TPB), TPB, 0, s>>>(start, ncells, scratch, total); }
+    launch_next(k_scan_tiles, ntiles, SCAN_T, s, count, ncells, start, scratch);
+    launch_next(k_scan_sums, 1, SCAN_T, s, scratch, ntiles, total);
+    launch_next(k_scan_add, div_up(ncells + 1, TPB), TPB, s, start, ncells, scratch, total);
 }
 void launch_bin_scatter(const unsigned int *keys, int n, const int *cellStart, int *cursor, int *slots, cudaStream_t s) {
-    if (n > 0) { FLIP_COUNT(1); k_bin_scatter<<<div_up(n, TPB), TPB, 0, s>>>(keys, n, cellStart, cursor, slots); }
+    if (n > 0) launch_next(k_bin_scatter, div_up(n, TPB), TPB, s, keys, n, cellStart, cursor, slots);
 }
 void launch_cell_sort_select(const int *cellStart, int ncells, int *slots, const unsigned int *ids,
                              const unsigned int *keys, int maxPerCell, int *survivorCount, cudaStream_t s) {
-    { FLIP_COUNT(1); k_cell_sort_select<<<div_up(ncells, TPB), TPB, 0, s>>>(cellStart, ncells, slots, ids, keys, maxPerCell, survivorCount); }
+    launch_next(k_cell_sort_select, div_up(ncells, TPB), TPB, s, cellStart, ncells, slots, ids, keys, maxPerCell, survivorCount);
 }
 void launch_gather_particles(const ParticleSoA &src, ParticleSoA dst, int n,
                              const int *cellStart, const int *slots, const int *newStart, int ncells,
                              unsigned int *maxSpeedSqBits, cudaStream_t s) {
     if (n <= 0) return;
-    FLIP_COUNT(1);
-    k_gather<<<std::min(div_up(n, TPB), 152u * 16u), TPB, 0, s>>>(src, dst, cellStart, slots, newStart, ncells,
+    launch_next(k_gather, std::min(div_up(n, TPB), 152u * 16u), TPB, s, src, dst, cellStart, slots, newStart, ncells,
                                                                maxSpeedSqBits);
 }
 void launch_liquid_sdf(const ParticleSoA &p, const int *cellStart, const StepConsts &c, const uint8_t *solidCC,
@@ -972,8 +1003,7 @@ void launch_liquid_sdf(const ParticleSoA &p, const int *cellStart, const StepCon
 }
 void launch_p2g(const ParticleSoA &p, const int *cellStart, const StepConsts &c, float *u, float *v,
                 float *w, uint8_t *vu, uint8_t *vv, uint8_t *vw, cudaStream_t s) {
-    FLIP_COUNT(1);
-    k_p2g<<<div_up((long long)(c.I + 1) * (c.J + 1) * (c.K + 1), P2G_TPB), P2G_TPB, 0, s>>>(p, cellStart, c, u, v, w, vu, vv, vw,
+    launch_next(k_p2g, div_up((long long)(c.I + 1) * (c.J + 1) * (c.K + 1), P2G_TPB), P2G_TPB, s, p, cellStart, c, u, v, w, vu, vv, vw,
                                                                                                   PairConsts{F2_ONE, F2_MINUS, F2_ZERO});
 }
 FaceBits face_bits(int I, int J, int K) {
@@ -993,7 +1023,7 @@ FaceBits face_bits(int I, int J, int K) {
 void launch_extrapolate(const StepConsts &c, float *u, float *v, float *w, const uint8_t *vu, const uint8_t *vv,
                         const uint8_t *vw, unsigned *known, int layers, cudaStream_t s) {
     const FaceBits b = face_bits(c.I, c.J, c.K);
-    { FLIP_COUNT(1); k_extrap_init<<<div_up(b.words, TPB / 4), TPB, 0, s>>>(b, vu, vv, vw, known); }
+    launch_next(k_extrap_init, div_up(b.words, TPB / 4), TPB, s, b, vu, vv, vw, known);
     // Few words: more CTAs, so that their warps share the faces to fill (32^3,
     // 7 layers: 34 us against 48); many: fewer (128^3: 129 us against 187;
     // 64^3, 29000 words: 49 against 53).
@@ -1007,30 +1037,29 @@ void launch_save_and_force(const StepConsts &c, float *u, float *v, float *w, fl
                            cudaStream_t s) {
     long long nu = (long long)(c.I + 1) * c.J * c.K, nv = (long long)c.I * (c.J + 1) * c.K,
               nw = (long long)c.I * c.J * (c.K + 1);
-    { FLIP_COUNT(1); k_save_force<<<div_up(nu + nv + nw, TPB), TPB, 0, s>>>(nu, nv, nw, u, v, w, su, sv, sw, fx, fy, fz, ax, ay, az, ex); }
+    launch_next(k_save_force, div_up(nu + nv + nw, TPB), TPB, s, nu, nv, nw, u, v, w, su, sv, sw, fx, fy, fz, ax, ay, az, ex);
 }
 void launch_constrain(const StepConsts &c, float *u, float *v, float *w, float *su, float *sv, float *sw,
                       const float *wu, const float *wv, const float *ww, const float *fu, const float *fv,
                       const float *fw, cudaStream_t s) {
     long long nu = (long long)(c.I + 1) * c.J * c.K, nv = (long long)c.I * (c.J + 1) * c.K,
               nw = (long long)c.I * c.J * (c.K + 1);
-    { FLIP_COUNT(1); k_constrain<<<div_up(nu + nv + nw, TPB), TPB, 0, s>>>(nu, nv, nw, u, v, w, su, sv, sw, wu, wv, ww, fu, fv, fw); }
+    launch_next(k_constrain, div_up(nu + nv + nw, TPB), TPB, s, nu, nv, nw, u, v, w, su, sv, sw, wu, wv, ww, fu, fv, fw);
 }
 void launch_advect(ParticleSoA p, int n, const StepConsts &c, const float *u, const float *v, const float *w,
                    const float *su, const float *sv, const float *sw, const float *solidPhi,
                    const uint8_t *nearSolid, float picRatio, float flipRatio, double dt, unsigned int *keys,
                    unsigned int *speedHist, double speedStep, const InflowConstraint &ic, cudaStream_t s) {
     if (n <= 0) return;
-    FLIP_COUNT(1);
-    k_advect<<<div_up(n, TPB), TPB, 0, s>>>(p, n, c, u, v, w, su, sv, sw, solidPhi, nearSolid, picRatio,
+    launch_next(k_advect, div_up(n, TPB), TPB, s, p, n, c, u, v, w, su, sv, sw, solidPhi, nearSolid, picRatio,
                                             flipRatio, dt, keys, speedHist, speedStep, ic);
 }
 void launch_speed_limit(const unsigned int *hist, int n, int bins, double speedStep, double maxPct, int maxAbs,
                         float *maxSpeedSq, cudaStream_t s) {
-    { FLIP_COUNT(1); k_speed_limit<<<1, 1, 0, s>>>(hist, n, bins, speedStep, maxPct, maxAbs, maxSpeedSq); }
+    launch_next(k_speed_limit, 1, 1, s, hist, n, bins, speedStep, maxPct, maxAbs, maxSpeedSq);
 }
 void launch_mark_fast(const ParticleSoA &p, int n, const float *maxSpeedSq, unsigned int *keys, cudaStream_t s) {
-    if (n > 0) { FLIP_COUNT(1); k_mark_fast<<<div_up(n, TPB), TPB, 0, s>>>(p, n, maxSpeedSq, keys); }
+    if (n > 0) launch_next(k_mark_fast, div_up(n, TPB), TPB, s, p, n, maxSpeedSq, keys);
 }
 
 }  // namespace flip

@@ -47,6 +47,8 @@ __device__ __forceinline__ bool sys_cell(const StepConsts &c, const float *phi, 
 // cells was bound by them, all on the same addresses (107 us at 128^3).
 constexpr int FLAG_CELLS = 4096;
 __global__ void __launch_bounds__(TPB) k_flags(StepConsts c, const float *phi, uint8_t *fluid, int *levelRange) {
+    pdl_wait();
+    pdl_trigger();
     __shared__ int sh[7][TPB / 32];
     const long long base = (long long)blockIdx.x * FLAG_CELLS, n = (long long)c.I * c.J * c.K;
     int v[7] = {0x7fffffff, -1, 0, 0x7fffffff, -1, 0x7fffffff, -1};
@@ -147,6 +149,8 @@ constexpr long long NOT_YET = -1LL;   // the bits of a pivot's reciprocal before
 // RHS (pressuresolver.cpp:580-669; the domain walls do not move) and the rows.
 __global__ void k_build(StepConsts c, const float *phi, const float *wu, const float *wv, const float *ww,
                         const float *u, const float *v, const float *w, double mf, PressureBuffers pb) {
+    pdl_wait();
+    pdl_trigger();
     long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     Dims d{c.I, c.J, c.K};
     double bmag = 0.0;
@@ -191,6 +195,8 @@ __global__ void k_build(StepConsts c, const float *phi, const float *wu, const f
 // elimination's order in the last bits; the factor is used rounded to FP32.
 __global__ void k_mic0_weights(StepConsts c, const uint8_t *fluid, const double4_32a *Ad, double *W0, double *W1,
                                double *W2) {
+    pdl_wait();
+    pdl_trigger();
     const long long n = (long long)c.I * c.J * c.K;
     const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= n) return;
@@ -300,6 +306,8 @@ struct FactorChunk {
 __global__ void __launch_bounds__(FTHREADS) k_mic0_tiles(StepConsts c, const uint8_t *fluid, const double4_32a *Ad,
                                                          const double *W0, const double *W1, const double *W2, double *E,
                                                          unsigned int *ticket, int *err, unsigned int spinLimit) {
+    pdl_wait();
+    pdl_trigger();
     __shared__ double prev[2][FT + 1][FT + 1];   // of the level before; row and column 0 stand for the edges
     __shared__ int tileSh, lvLo, lvHi;
     const int ntj = (c.J - 2 + FT - 1) / FT, ntk = (c.K - 2 + FT - 1) / FT;
@@ -443,6 +451,8 @@ __global__ void k_mic0_inverse(const uint8_t *fluid, long long n, double *E) {
 // the sweep layout) that the sweeps pass over, tile by tile.  An item is
 // tile * (T / SWEEP_CH) + chunk.  One CTA.
 __global__ void __launch_bounds__(1024) k_items(SweepLayout g, const int2 *range, int *items, int *nItems) {
+    pdl_wait();
+    pdl_trigger();
     __shared__ int sh[32], base;
     const int nt = g.nta * g.ntb, nch = g.T / SWEEP_CH, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     if (threadIdx.x == 0) base = 0;
@@ -1103,6 +1113,8 @@ __global__ void __launch_bounds__(TPB) k_x_to_cells(StepConsts c, SweepLayout g,
 __global__ void k_apply_pressure(StepConsts c, const float *phi, const float *wu, const float *wv, const float *ww,
                                  const float *P, float factor, float *u, float *v, float *w, uint8_t *vu,
                                  uint8_t *vv, uint8_t *vw) {
+    pdl_wait();
+    pdl_trigger();
     long long nu = (long long)(c.I + 1) * c.J * c.K, nv = (long long)c.I * (c.J + 1) * c.K;
     long long nw = (long long)c.I * c.J * (c.K + 1);
     long long f = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -1186,9 +1198,9 @@ void mic0_factor(const StepConsts &c, const uint8_t *fluid, const double4_32a *A
     const long long n = (long long)c.I * c.J * c.K;
     const int ntiles = div_up(c.J - 2, FT) * div_up(c.K - 2, FT);
     cudaMemsetAsync(ticket, 0, sizeof(unsigned int), s);
-    { FLIP_COUNT(1); k_mic0_weights<<<div_up(n, TPB), TPB, 0, s>>>(c, fluid, Ad, W0, W1, W2); }
-    FLIP_COUNT(1);
-    k_mic0_tiles<<<ntiles, FTHREADS, 0, s>>>(c, fluid, Ad, W0, W1, W2, E, ticket, err, spinLimit);
+    launch_next(k_mic0_weights, div_up(n, TPB), TPB, s, c, fluid, Ad, W0, W1, W2);
+    // not early: its CTAs should have the SMs to themselves, as evenly as they can
+    launch_after(false, k_mic0_tiles, ntiles, FTHREADS, 0, s, c, fluid, Ad, W0, W1, W2, E, ticket, err, spinLimit);
 }
 // E to inverse pivots, 0 off the system.
 void mic0_inverse_pivots(const uint8_t *fluid, long long n, double *E, cudaStream_t s) {
@@ -1226,8 +1238,8 @@ int pressure_project(const StepConsts &c, const PressureArgs &a, PressureBuffers
     std::memcpy(mail->levelRange, lr, sizeof(lr));
     PCK(cudaMemcpyAsync(pb.levelRange, mail->levelRange, sizeof(lr), cudaMemcpyHostToDevice, s));
     PCK(cudaMemsetAsync(pb.scal, 0, 8 * sizeof(double), s));
-    { FLIP_COUNT(1); k_flags<<<div_up(n, FLAG_CELLS), TPB, 0, s>>>(c, a.phi, pb.fluid, pb.levelRange); }
-    { FLIP_COUNT(1); k_build<<<nb, TPB, 0, s>>>(c, a.phi, a.wu, a.wv, a.ww, a.u, a.v, a.w, mf, pb); }
+    launch_next(k_flags, div_up(n, FLAG_CELLS), TPB, s, c, a.phi, pb.fluid, pb.levelRange);
+    launch_next(k_build, nb, TPB, s, c, a.phi, a.wu, a.wv, a.ww, a.u, a.v, a.w, mf, pb);
     PCK(cudaMemcpyAsync(mail->levelRange, pb.levelRange, 7 * sizeof(int), cudaMemcpyDeviceToHost, s));
     PCK(cudaMemcpyAsync(&mail->bmax, pb.scal + 2, sizeof(double), cudaMemcpyDeviceToHost, s));
     PCK(sync());
@@ -1264,7 +1276,7 @@ int pressure_project(const StepConsts &c, const PressureArgs &a, PressureBuffers
     const SweepLayout sl = pb.sl;
     const unsigned ib = (unsigned)std::max(1LL, std::min<long long>(sweep_items_max(c.I, c.J, c.K), RBLOCKS));   // item loops
     launch_sweep_ranges(c, sl, pb.fluid, sw, s);
-    { FLIP_COUNT(1); k_items<<<1, 1024, 0, s>>>(sl, sw.range, pb.items, pb.nItems); }
+    launch_next(k_items, 1, 1024, s, sl, sw.range, pb.items, pb.nItems);
 
     // MIC(0) factor; the pivot weights go to A's buffer, which is filled after
     // it: zero wherever no item of this solve writes a coupling

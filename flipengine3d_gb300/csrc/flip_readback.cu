@@ -12,11 +12,15 @@ namespace flip {
 namespace {
 
 __global__ void k_flag_ids(const unsigned int *ids, int n, int *flags) {
+    pdl_wait();
+    pdl_trigger();
     int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t < n) flags[ids[t]] = 1;
 }
 
 __global__ void k_scatter_xyz(ParticleSoA p, int n, float *pos, float *vel) {
+    pdl_wait();
+    pdl_trigger();
     int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= n) return;
     long long o = 3LL * p.id[t];
@@ -25,6 +29,8 @@ __global__ void k_scatter_xyz(ParticleSoA p, int n, float *pos, float *vel) {
 }
 
 __global__ void k_renumber_ids(unsigned int *ids, int n, const int *rank) {
+    pdl_wait();
+    pdl_trigger();
     int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t < n) ids[t] = (unsigned int)rank[ids[t]];
 }
@@ -36,14 +42,14 @@ __global__ void k_renumber_ids(unsigned int *ids, int n, const int *rank) {
 void launch_compact_ids(const ParticleSoA &p, int n, int idSpace, int *flags, int *rank, int *scratch, int *total,
                         cudaStream_t s) {
     cudaMemsetAsync(flags, 0, (size_t)(idSpace + 1) * sizeof(int), s);
-    if (n > 0) { FLIP_COUNT(1); k_flag_ids<<<div_up(n, 256), 256, 0, s>>>(p.id, n, flags); }
+    if (n > 0) launch_next(k_flag_ids, div_up(n, 256), 256, s, p.id, n, flags);
     launch_scan_cells(flags, idSpace, rank, scratch, total, s);
-    if (n > 0) { FLIP_COUNT(1); k_renumber_ids<<<div_up(n, 256), 256, 0, s>>>(p.id, n, rank); }
+    if (n > 0) launch_next(k_renumber_ids, div_up(n, 256), 256, s, p.id, n, rank);
 }
 
 // Where the ids are dense (0..n-1), they are the ranks.
 void launch_readback_order(const ParticleSoA &p, int n, float *pos, float *vel, cudaStream_t s) {
-    if (n > 0) { FLIP_COUNT(1); k_scatter_xyz<<<div_up(n, 256), 256, 0, s>>>(p, n, pos, vel); }
+    if (n > 0) launch_next(k_scatter_xyz, div_up(n, 256), 256, s, p, n, pos, vel);
 }
 
 }  // namespace flip

@@ -663,6 +663,8 @@ __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(NTHREADS) k_wavefro
 __global__ void k_sweep_prep(unsigned int *ticket) { sweep_prep(ticket); }
 
 __global__ void k_tile_range_init(int2 *range, int n) {
+    pdl_wait();
+    pdl_trigger();
     int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t < n) range[t] = make_int2(0x7fffffff, -1);
 }
@@ -670,6 +672,8 @@ __global__ void k_tile_range_init(int2 *range, int n) {
 // First and last forward step at which a tile meets a system cell
 // (lanes of a warp that fall into the same tile reduce before the atomics).
 __global__ void k_tile_range(const uint8_t *fluid, int I, int J, int K, SweepLayout g, int2 *range) {
+    pdl_wait();
+    pdl_trigger();
     long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     bool f = t < (long long)I * J * K && fluid[t];
     int tile = -1, step = 0;
@@ -709,9 +713,9 @@ long long sweep_exchange_words(int I, int J, int K) {
 void launch_sweep_ranges(const StepConsts &c, const SweepLayout &g, const uint8_t *fluid, SweepState &sw,
                          cudaStream_t s) {
     const int n = g.nta * g.ntb;
-    { FLIP_COUNT(1); k_tile_range_init<<<div_up(n, 256), 256, 0, s>>>(sw.range, n); }
+    launch_next(k_tile_range_init, div_up(n, 256), 256, s, sw.range, n);
     long long nc = (long long)c.I * c.J * c.K;
-    { FLIP_COUNT(1); k_tile_range<<<div_up(nc, 256), 256, 0, s>>>(fluid, c.I, c.J, c.K, g, sw.range); }
+    launch_next(k_tile_range, div_up(nc, 256), 256, s, fluid, c.I, c.J, c.K, g, sw.range);
 }
 
 void launch_sweeps(const StepConsts &c, const SweepLayout &g, const float4 *L, const float *rf, float *z,
