@@ -29,6 +29,8 @@ struct StepConsts {
     // the reference's blocks of 10 cells, for its particle lists: float edge, 1 / edge
     float blockdxf, invBlockf;
     float centre[10];   // a cell's centre in its block's frame, by its place there
+    // liquid level set: particle radius; 3 dx, the smallest float no less than dx / 2, -dx / 2, 0.005 dx
+    float radiusf, sdfMax, sdfHalf, sdfNeg, sdfEps;
     double invBlock;
     // near-solid coarse grid
     int nsi, nsj, nsk;
@@ -92,14 +94,23 @@ inline void launch_after(bool overlap, void (*k)(P...), unsigned grid, unsigned 
     cudaLaunchKernelEx(&cfg, k, static_cast<P>(args)...);
 }
 
-// For kernels that wait and trigger as their first steps: launched early where
-// they are small, and a launch's latency is most of what they take.  Larger ones
-// would take the place of CTAs of the kernel before them (32^3 frames: 1195 us
-// without, 1142 with; 48^3: 1982, 1870; early launches of all sizes cost 64^3
-// frames 2.4% and 128^3 frames 1.5%).
+// For kernels that begin with pdl_begin: launched early where they are small, and
+// a launch's latency is most of what they take (32^3 frames: 1195 us without, 1142
+// with; 48^3: 1982, 1870).  Larger ones would take the place of CTAs of the kernel
+// before them (early launches of all sizes cost 64^3 frames 2.4%, 128^3 frames
+// 1.5%), and the two instructions alone cost them (k_save_force at 128^3: 27 us
+// against 18), so they do without.
+__host__ __device__ __forceinline__ bool launched_early(unsigned grid, unsigned block) {
+    return (long long)grid * block <= 1 << 17;
+}
+__device__ __forceinline__ void pdl_begin() {
+    if (!launched_early(gridDim.x, blockDim.x)) return;
+    pdl_wait();
+    pdl_trigger();
+}
 template <class... P, class... Q>
 inline void launch_next(void (*k)(P...), unsigned grid, unsigned block, cudaStream_t s, Q... args) {
-    launch_after((long long)grid * block <= 1 << 17, k, grid, block, 0, s, args...);
+    launch_after(launched_early(grid, block), k, grid, block, 0, s, args...);
 }
 
 // -- seeding from fluid meshes (flip_seed.cu); mask: one 8-bit sub-cell

@@ -1107,6 +1107,12 @@ int flip_create(int isize, int jsize, int ksize, double dx, flip_ctx **out) {
     c.I = isize; c.J = jsize; c.K = ksize;
     c.dx = dx; c.invdx = 1.0 / dx; c.invdxf = (float)(1.0 / dx); c.dxf = (float)dx;
     c.radius = 0.5 * 1.0 * dx * std::sqrt(3.0);
+    c.radiusf = (float)c.radius;
+    c.sdfMax = (float)(3.0 * dx);
+    c.sdfHalf = (float)(0.5 * dx);   // (double)v < dx / 2 where v is below the smallest float that is no less
+    if ((double)c.sdfHalf < 0.5 * dx) c.sdfHalf = std::nextafter(c.sdfHalf, INFINITY);
+    c.sdfNeg = (float)(-0.5f * dx);
+    c.sdfEps = (float)(0.005 * dx);
     c.blockdxf = (float)(10 * dx);
     for (int a = 0; a < 10; a++) c.centre[a] = (float)((double)(float)a * dx + 0.5 * dx);
     c.invBlock = 1.0 / (double)c.blockdxf;

@@ -30,8 +30,7 @@ __device__ __forceinline__ F3 normalize3(F3 v) {
 
 // ------------------------------------------------------------------ binning
 __global__ void k_keys(ParticleSoA p, int n, StepConsts c, unsigned int *keys) {
-    pdl_wait();
-    pdl_trigger();
+    pdl_begin();
     int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= n) return;
     int i = exact_floor(p.px[t], c.invdx, c.invdxf);
@@ -42,8 +41,7 @@ __global__ void k_keys(ParticleSoA p, int n, StepConsts c, unsigned int *keys) {
 }
 
 __global__ void k_bin_count(const unsigned int *keys, int n, int *count) {
-    pdl_wait();
-    pdl_trigger();
+    pdl_begin();
     int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= n) return;
     unsigned int k = keys[t];
@@ -82,8 +80,7 @@ __device__ int block_scan_excl(int v, int *sh, int *total) {
 }
 
 __global__ void k_scan_tiles(const int *in, int n, int *out, int *tileSums) {
-    pdl_wait();
-    pdl_trigger();
+    pdl_begin();
     __shared__ int sh[32];
     long long base = (long long)blockIdx.x * SCAN_TILE + threadIdx.x * SCAN_PER;
     int v[SCAN_PER];
@@ -106,8 +103,7 @@ __global__ void k_scan_tiles(const int *in, int n, int *out, int *tileSums) {
 }
 
 __global__ void k_scan_sums(int *tileSums, int ntiles, int *grandTotal) {
-    pdl_wait();
-    pdl_trigger();
+    pdl_begin();
     __shared__ int sh[32];
     int v[SCAN_PER];
     int sum = 0;
@@ -129,16 +125,14 @@ __global__ void k_scan_sums(int *tileSums, int ntiles, int *grandTotal) {
 }
 
 __global__ void k_scan_add(int *out, int n, const int *tileSums, const int *grandTotal) {
-    pdl_wait();
-    pdl_trigger();
+    pdl_begin();
     long long g = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (g < n) out[g] += tileSums[g / SCAN_TILE];
     if (g == n) out[n] = *grandTotal;
 }
 
 __global__ void k_bin_scatter(const unsigned int *keys, int n, const int *start, int *cursor, int *slots) {
-    pdl_wait();
-    pdl_trigger();
+    pdl_begin();
     int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= n) return;
     unsigned int k = keys[t];
@@ -154,8 +148,7 @@ __global__ void k_bin_scatter(const unsigned int *keys, int n, const int *start,
 // Kept slots are compacted to the front of the cell's segment.
 __global__ void k_cell_sort_select(const int *start, int ncells, int *slots, const unsigned int *ids,
                                    const unsigned int *keys, int maxPerCell, int *survivors) {
-    pdl_wait();
-    pdl_trigger();
+    pdl_begin();
     int c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= ncells) return;
     int b = start[c], e = start[c + 1];
@@ -199,8 +192,7 @@ __device__ __forceinline__ float gather_one(const ParticleSoA &src, const Partic
 }
 __global__ void k_gather(ParticleSoA src, ParticleSoA dst, const int *start, const int *slots,
                          const int *newStart, int ncells, unsigned int *maxSpeedSqBits) {
-    pdl_wait();
-    pdl_trigger();
+    pdl_begin();
     const int t = blockIdx.x * blockDim.x + threadIdx.x, total = newStart[ncells];
     float best = 0.0f;
     if (total == start[ncells]) {
@@ -227,7 +219,7 @@ __global__ void k_gather(ParticleSoA src, ParticleSoA dst, const int *start, con
 // first, as long as a row can still hold a nearer one.  A cell inside the
 // liquid has a particle within half a cell and stops at its own, and the air
 // far from it knows from a look of the warp at the 25 rows around.  Bound by the
-// latency and the instructions of the cells near the surface: 223 us at 128^3
+// latency and the instructions of the cells near the surface: 225 us at 128^3
 // (4.1M particles), 68 at 64^3; scattering every particle
 // into the ~100 cells of its box through shared-memory atomics took 820, 370.
 // 64 registers a thread: with 128 the occupancy is too low, with 42 small grids
@@ -276,8 +268,7 @@ __constant__ signed char kRing[25][2] = {
 template <int SDF_TPB>
 __global__ void __launch_bounds__(SDF_TPB, 1024 / SDF_TPB) k_liquid_sdf(ParticleSoA ps, const int *cellStart, StepConsts c,
                                                      const uint8_t *solidCC, float *phi) {
-    pdl_wait();
-    pdl_trigger();
+    pdl_begin();
     const long long ci = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     Dims cells{c.I, c.J, c.K};
     const bool valid = ci < cells.size();
@@ -299,9 +290,7 @@ __global__ void __launch_bounds__(SDF_TPB, 1024 / SDF_TPB) k_liquid_sdf(Particle
         rows = __ballot_sync(0xffffffffu, any);
     }
     if (!valid) return;
-    const double dx = c.dx;
-    const float maxd = (float)(3.0 * dx);
-    const float r = (float)c.radius;
+    const float maxd = c.sdfMax, r = c.radiusf;
     const float sr = __fmul_rn(2.0f, r);
     const int bx = gi / BW, by = gj / BW, bz = gk / BW, a = gi - bx * BW, b = gj - by * BW, cc = gk - bz * BW;
     const float offx = c.blockPos[bx + 1], offy = c.blockPos[by + 1], offz = c.blockPos[bz + 1];
@@ -376,12 +365,9 @@ __global__ void __launch_bounds__(SDF_TPB, 1024 / SDF_TPB) k_liquid_sdf(Particle
             }
         }
     }
-    const float eps = (float)(0.005 * dx);
-    const double half = 0.5 * dx;
-    const float neg = (float)(-0.5f * dx);
     float val = __float_as_uint(best) == 0x7f800000u ? maxd : fminf(maxd, __fsub_rn(__fsqrt_rn(best), r));
-    if ((double)val < half && solidCC[ci]) val = neg;
-    if (fabsf(val) < eps) val = val > 0 ? eps : -eps;
+    if (val < c.sdfHalf && solidCC[ci]) val = c.sdfNeg;
+    if (fabsf(val) < c.sdfEps) val = val > 0 ? c.sdfEps : -c.sdfEps;
     phi[ci] = val;
 }
 
@@ -417,8 +403,7 @@ constexpr int P2G_TPB = 128;
 __global__ void __launch_bounds__(P2G_TPB, 1024 / P2G_TPB) k_p2g(ParticleSoA p, const int *cellStart, StepConsts c,
                                              float *U, float *V, float *W, uint8_t *vu, uint8_t *vv, uint8_t *vw,
                                              PairConsts k2) {
-    pdl_wait();
-    pdl_trigger();
+    pdl_begin();
     const int ni = c.I + 1, nj = c.J + 1, nk = c.K + 1;
     const long long f = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (f >= (long long)ni * nj * nk) return;
@@ -530,8 +515,7 @@ __device__ __forceinline__ void face_word(const FaceBits &b, long long t, int &d
 }
 __global__ void __launch_bounds__(TPB) k_extrap_init(FaceBits b, const uint8_t *vu, const uint8_t *vv, const uint8_t *vw,
                                                      unsigned *known) {
-    pdl_wait();
-    pdl_trigger();
+    pdl_begin();
     const int lane = threadIdx.x & 31;
     const long long first = ((long long)blockIdx.x * (TPB / 32) + (threadIdx.x >> 5)) * 8;   // eight words a warp
 #pragma unroll
@@ -626,8 +610,7 @@ __global__ void __launch_bounds__(TPB) k_extrap_layer(FaceBits b, const unsigned
 __global__ void k_save_force(long long nu, long long nv, long long nw, float *u, float *v, float *w, float *su,
                              float *sv, float *sw, float fx, float fy, float fz, int ax, int ay, int az,
                              const uint8_t *ex) {
-    pdl_wait();
-    pdl_trigger();
+    pdl_begin();
     long long f = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     const bool skip = ex && f < nu + nv + nw && ex[f];
     if (f < nu) {
@@ -647,8 +630,7 @@ __global__ void k_save_force(long long nu, long long nv, long long nw, float *u,
 __global__ void k_constrain(long long nu, long long nv, long long nw, float *u, float *v, float *w, float *su,
                             float *sv, float *sw, const float *wu, const float *wv, const float *ww, const float *fu,
                             const float *fv, const float *fw) {
-    pdl_wait();
-    pdl_trigger();
+    pdl_begin();
     long long f = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     float *G, *S;
     const float *W, *F;
@@ -865,19 +847,27 @@ __device__ F3 resolve_collision(const StepConsts &c, const float *S, const uint8
     return res;
 }
 
+// What depends on the time step alone, worked out once: a thread that takes an
+// FP64 division of its own for each keeps the FP64 unit busy for most of the
+// kernel.
+struct AdvectSteps {
+    float half, threeQuarters, ninth;   // of the time step
+    float invSpeedStep;
+    double speedStep;
+};
+
 // Fused particle update: PIC/FLIP velocity (fluidsimulation.cpp:4082-4092),
 // Ralston RK3 (4191-4198), collision (4221-4296), then the removal tests and
 // the new cell key for the next binning.  Bound by instructions and the latency
-// of the 104 scattered corner reads a particle: a bounds test and a 64-bit
-// address per corner took 594 us at 128^3 (4.1M particles), one per cell 328
-// (256x128x128, 14.0M: 1720 -> 1111 us).
+// of the 104 scattered corner reads a particle, 269 us at 128^3 (4.1M particles),
+// 824 at 256x128x128 (14.0M).  A bounds test and a 64-bit address per corner took
+// 594, 1720; FP64 divisions of the time step by each thread 328, 1112.
 __global__ void __launch_bounds__(TPB) k_advect(ParticleSoA p, int n, StepConsts c, const float *u, const float *v,
                                                 const float *w, const float *su, const float *sv, const float *sw,
                                                 const float *S, const uint8_t *ns, float picRatio, float flipRatio,
-                                                double dt, unsigned int *keys, unsigned int *hist, double speedStep,
+                                                const AdvectSteps k, unsigned int *keys, unsigned int *hist,
                                                 const InflowConstraint ic) {
-    pdl_wait();
-    pdl_trigger();
+    pdl_begin();
     __shared__ unsigned int shist[8];
     if (threadIdx.x < 8) shist[threadIdx.x] = 0;
     __syncthreads();
@@ -904,19 +894,19 @@ __global__ void __launch_bounds__(TPB) k_advect(ParticleSoA p, int n, StepConsts
                     vn = f3(ic.vx[q], ic.vy[q], ic.vz[q]);
         }
         F3 k1 = vpic;
-        F3 k2 = eval_vel(c, u, v, w, add(p0, mul((float)(0.5 * dt), k1)));
-        F3 k3 = eval_vel(c, u, v, w, add(p0, mul((float)(0.75 * dt), k2)));
+        F3 k2 = eval_vel(c, u, v, w, add(p0, mul(k.half, k1)));
+        F3 k3 = eval_vel(c, u, v, w, add(p0, mul(k.threeQuarters, k2)));
         F3 sum = add(add(mul(2.0f, k1), mul(3.0f, k2)), mul(4.0f, k3));
-        F3 p1 = add(p0, mul((float)(dt / 9.0f), sum));
+        F3 p1 = add(p0, mul(k.ninth, sum));
         p1 = resolve_collision(c, S, ns, p0, p1);
         p.px[t] = p1.x; p.py[t] = p1.y; p.pz[t] = p1.z;
         p.vx[t] = vn.x; p.vy[t] = vn.y; p.vz[t] = vn.z;
         float speed = len3(vn);
         // floor(speed / step) as the reference's FP64 division gives it
-        float qf = __fmul_rn(speed, (float)(1.0 / speedStep));
+        float qf = __fmul_rn(speed, k.invSpeedStep);
         float fl = floorf(qf);
         int bin = (qf - fl > 1e-3f && qf - fl < 1.0f - 1e-3f) ? (int)fminf(fl, 5.0f)
-                                                               : (int)fmin(floor((double)speed / speedStep), 5.0);
+                                                               : (int)fmin(floor((double)speed / k.speedStep), 5.0);
         if (speed != speed) bin = 5;
         atomicAdd(&shist[bin], 1u);
         unsigned int key;
@@ -937,8 +927,7 @@ __global__ void __launch_bounds__(TPB) k_advect(ParticleSoA p, int n, StepConsts
 // _getMarkerParticleSpeedLimit (fluidsimulation.cpp:4298-4322), one thread
 __global__ void k_speed_limit(const unsigned int *hist, int n, int bins, double step, double maxPct, int maxAbs,
                               float *maxSpeedSq) {
-    pdl_wait();
-    pdl_trigger();
+    pdl_begin();
     int maxRemoval = (int)fmin((double)(int)((double)n * maxPct), (double)maxAbs);
     double maxspeed = bins * step;
     int cur = 0;
@@ -952,8 +941,7 @@ __global__ void k_speed_limit(const unsigned int *hist, int n, int bins, double 
 }
 
 __global__ void k_mark_fast(ParticleSoA p, int n, const float *maxSpeedSq, unsigned int *keys) {
-    pdl_wait();
-    pdl_trigger();
+    pdl_begin();
     int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= n) return;
     unsigned int k = keys[t];
@@ -1051,8 +1039,9 @@ void launch_advect(ParticleSoA p, int n, const StepConsts &c, const float *u, co
                    const uint8_t *nearSolid, float picRatio, float flipRatio, double dt, unsigned int *keys,
                    unsigned int *speedHist, double speedStep, const InflowConstraint &ic, cudaStream_t s) {
     if (n <= 0) return;
-    launch_next(k_advect, div_up(n, TPB), TPB, s, p, n, c, u, v, w, su, sv, sw, solidPhi, nearSolid, picRatio,
-                                            flipRatio, dt, keys, speedHist, speedStep, ic);
+    const AdvectSteps k{(float)(0.5 * dt), (float)(0.75 * dt), (float)(dt / 9.0f), (float)(1.0 / speedStep), speedStep};
+    launch_next(k_advect, div_up(n, TPB), TPB, s, p, n, c, u, v, w, su, sv, sw, solidPhi, nearSolid, picRatio, flipRatio, k,
+                keys, speedHist, ic);
 }
 void launch_speed_limit(const unsigned int *hist, int n, int bins, double speedStep, double maxPct, int maxAbs,
                         float *maxSpeedSq, cudaStream_t s) {

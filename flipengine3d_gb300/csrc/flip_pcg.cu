@@ -47,8 +47,7 @@ __device__ __forceinline__ bool sys_cell(const StepConsts &c, const float *phi, 
 // cells was bound by them, all on the same addresses (107 us at 128^3).
 constexpr int FLAG_CELLS = 4096;
 __global__ void __launch_bounds__(TPB) k_flags(StepConsts c, const float *phi, uint8_t *fluid, int *levelRange) {
-    pdl_wait();
-    pdl_trigger();
+    pdl_begin();
     __shared__ int sh[7][TPB / 32];
     const long long base = (long long)blockIdx.x * FLAG_CELLS, n = (long long)c.I * c.J * c.K;
     int v[7] = {0x7fffffff, -1, 0, 0x7fffffff, -1, 0x7fffffff, -1};
@@ -131,16 +130,20 @@ __device__ double4_32a row_coeffs(const StepConsts &c, const float *phi, const f
 // With nanAsInf a NaN reads as +inf (a residual norm that never passes for
 // converged); otherwise NaNs are ignored, as fmax ignores them.
 __device__ __forceinline__ void block_max_to(double v, unsigned long long *out, bool nanAsInf = true) {
-    __shared__ double sh[32];
+    __shared__ long long sh[32];
     if (v != v) v = nanAsInf ? __longlong_as_double(0x7ff0000000000000ll) : 0.0;
-    for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(0xffffffffu, v, o));
+    // as integers, which order non-negative doubles the same way and spare the
+    // scarce FP64
+    long long m = __double_as_longlong(v);
+    if (__any_sync(0xffffffffu, m > 0))
+        for (int o = 16; o > 0; o >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    if (lane == 0) sh[warp] = v;
+    if (lane == 0) sh[warp] = m;
     __syncthreads();
     if (warp == 0) {
-        v = lane < (int)(blockDim.x >> 5) ? sh[lane] : 0.0;
-        for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(0xffffffffu, v, o));
-        if (lane == 0 && v > 0.0) atomicMax(out, (unsigned long long)__double_as_longlong(v));
+        m = lane < (int)(blockDim.x >> 5) ? sh[lane] : 0;
+        for (int o = 16; o > 0; o >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
+        if (lane == 0 && m > 0) atomicMax(out, (unsigned long long)m);
     }
 }
 
@@ -149,8 +152,7 @@ constexpr long long NOT_YET = -1LL;   // the bits of a pivot's reciprocal before
 // RHS (pressuresolver.cpp:580-669; the domain walls do not move) and the rows.
 __global__ void k_build(StepConsts c, const float *phi, const float *wu, const float *wv, const float *ww,
                         const float *u, const float *v, const float *w, double mf, PressureBuffers pb) {
-    pdl_wait();
-    pdl_trigger();
+    pdl_begin();
     long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     Dims d{c.I, c.J, c.K};
     double bmag = 0.0;
@@ -165,7 +167,7 @@ __global__ void k_build(StepConsts c, const float *phi, const float *wu, const f
             double vR = wu[du.idx(i + 1, j, k)], vL = wu[du.idx(i, j, k)];
             double vT = wv[dv.idx(i, j + 1, k)], vB = wv[dv.idx(i, j, k)];
             double vF = ww[dw.idx(i, j, k + 1)], vK = ww[dw.idx(i, j, k)];
-            double factor = 1.0 / c.dx;
+            const double factor = c.invdx;
             double div = 0.0;
             div += -factor * vR * (double)u[du.idx(i + 1, j, k)];
             div += factor * vL * (double)u[du.idx(i, j, k)];
@@ -195,8 +197,7 @@ __global__ void k_build(StepConsts c, const float *phi, const float *wu, const f
 // elimination's order in the last bits; the factor is used rounded to FP32.
 __global__ void k_mic0_weights(StepConsts c, const uint8_t *fluid, const double4_32a *Ad, double *W0, double *W1,
                                double *W2) {
-    pdl_wait();
-    pdl_trigger();
+    pdl_begin();
     const long long n = (long long)c.I * c.J * c.K;
     const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= n) return;
@@ -306,8 +307,7 @@ struct FactorChunk {
 __global__ void __launch_bounds__(FTHREADS) k_mic0_tiles(StepConsts c, const uint8_t *fluid, const double4_32a *Ad,
                                                          const double *W0, const double *W1, const double *W2, double *E,
                                                          unsigned int *ticket, int *err, unsigned int spinLimit) {
-    pdl_wait();
-    pdl_trigger();
+    pdl_begin();
     __shared__ double prev[2][FT + 1][FT + 1];   // of the level before; row and column 0 stand for the edges
     __shared__ int tileSh, lvLo, lvHi;
     const int ntj = (c.J - 2 + FT - 1) / FT, ntk = (c.K - 2 + FT - 1) / FT;
@@ -451,8 +451,7 @@ __global__ void k_mic0_inverse(const uint8_t *fluid, long long n, double *E) {
 // the sweep layout) that the sweeps pass over, tile by tile.  An item is
 // tile * (T / SWEEP_CH) + chunk.  One CTA.
 __global__ void __launch_bounds__(1024) k_items(SweepLayout g, const int2 *range, int *items, int *nItems) {
-    pdl_wait();
-    pdl_trigger();
+    pdl_begin();
     __shared__ int sh[32], base;
     const int nt = g.nta * g.ntb, nch = g.T / SWEEP_CH, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     if (threadIdx.x == 0) base = 0;
@@ -1113,8 +1112,7 @@ __global__ void __launch_bounds__(TPB) k_x_to_cells(StepConsts c, SweepLayout g,
 __global__ void k_apply_pressure(StepConsts c, const float *phi, const float *wu, const float *wv, const float *ww,
                                  const float *P, float factor, float *u, float *v, float *w, uint8_t *vu,
                                  uint8_t *vv, uint8_t *vw) {
-    pdl_wait();
-    pdl_trigger();
+    pdl_begin();
     long long nu = (long long)(c.I + 1) * c.J * c.K, nv = (long long)c.I * (c.J + 1) * c.K;
     long long nw = (long long)c.I * c.J * (c.K + 1);
     long long f = (long long)blockIdx.x * blockDim.x + threadIdx.x;

@@ -12,15 +12,13 @@ namespace flip {
 namespace {
 
 __global__ void k_flag_ids(const unsigned int *ids, int n, int *flags) {
-    pdl_wait();
-    pdl_trigger();
+    pdl_begin();
     int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t < n) flags[ids[t]] = 1;
 }
 
 __global__ void k_scatter_xyz(ParticleSoA p, int n, float *pos, float *vel) {
-    pdl_wait();
-    pdl_trigger();
+    pdl_begin();
     int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= n) return;
     long long o = 3LL * p.id[t];
@@ -29,8 +27,7 @@ __global__ void k_scatter_xyz(ParticleSoA p, int n, float *pos, float *vel) {
 }
 
 __global__ void k_renumber_ids(unsigned int *ids, int n, const int *rank) {
-    pdl_wait();
-    pdl_trigger();
+    pdl_begin();
     int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t < n) ids[t] = (unsigned int)rank[ids[t]];
 }

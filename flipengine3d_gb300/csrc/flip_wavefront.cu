@@ -663,8 +663,7 @@ __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(NTHREADS) k_wavefro
 __global__ void k_sweep_prep(unsigned int *ticket) { sweep_prep(ticket); }
 
 __global__ void k_tile_range_init(int2 *range, int n) {
-    pdl_wait();
-    pdl_trigger();
+    pdl_begin();
     int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t < n) range[t] = make_int2(0x7fffffff, -1);
 }
@@ -672,8 +671,7 @@ __global__ void k_tile_range_init(int2 *range, int n) {
 // First and last forward step at which a tile meets a system cell
 // (lanes of a warp that fall into the same tile reduce before the atomics).
 __global__ void k_tile_range(const uint8_t *fluid, int I, int J, int K, SweepLayout g, int2 *range) {
-    pdl_wait();
-    pdl_trigger();
+    pdl_begin();
     long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     bool f = t < (long long)I * J * K && fluid[t];
     int tile = -1, step = 0;
