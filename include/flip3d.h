@@ -494,7 +494,7 @@ int flip_runtime_pending(flip_runtime *rt, int *queued, int *running);
  * (m = n when every id is in range).  id_space may be at most
  * FLIP_NOALLOC_MAX_IDS; a larger one is rejected with FLIP_E_OUT_OF_RANGE.
  * The work runs on `stream` (a cudaStream_t; NULL for the default stream) in
- * a device array of about 4 MiB that the library holds until exit on every
+ * a device array of 256 KiB that the library holds until exit on every
  * device that uses it.  The array's address is looked up in the current
  * context on every call (no allocation once the module is loaded); under
  * lazy module loading the first call in a context loads the module, so make
