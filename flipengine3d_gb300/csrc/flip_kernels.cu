@@ -1,7 +1,9 @@
 // FLIP step kernels for GB300 (sm_103a): particle binning, liquid SDF, P2G,
 // extrapolation, body force, constrain, and the fused PIC/FLIP + RK3 +
-// collision particle update.  Every kernel is an HBM-bound gather/stencil;
-// nothing here is a dense contraction, so no tensor cores are involved.
+// collision particle update.  Gathers and stencils: the searches, the splat and
+// the update are bound by the instructions and the latency of scattered reads,
+// the rest by HBM or, on small grids, by launches.  Nothing here is a dense
+// contraction, so no tensor cores are involved.
 #include <cstdio>
 #include <type_traits>
 

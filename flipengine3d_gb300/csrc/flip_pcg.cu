@@ -19,8 +19,6 @@
 // decided on it, with the reference's test |r|inf <= tol * |b|inf.
 #include <algorithm>
 #include <cmath>
-
-#include <cooperative_groups.h>
 #include <cstring>
 #include <string>
 
@@ -28,8 +26,6 @@
 #include "flip_device.cuh"
 
 namespace flip {
-
-namespace cg = cooperative_groups;
 
 namespace {
 
@@ -43,7 +39,7 @@ __device__ __forceinline__ bool sys_cell(const StepConsts &c, const float *phi, 
 
 // The rows' flags, and the extent of their levels i + j + k, their number and
 // their extent in j and k (for the sweep tile orientation).  A CTA reduces
-// over CELLS_PER_CTA cells before its seven atomics: one set per warp of 32
+// over FLAG_CELLS cells before its seven atomics: one set per warp of 32
 // cells was bound by them, all on the same addresses (107 us at 128^3).
 constexpr int FLAG_CELLS = 4096;
 __global__ void __launch_bounds__(TPB) k_flags(StepConsts c, const float *phi, uint8_t *fluid, int *levelRange) {

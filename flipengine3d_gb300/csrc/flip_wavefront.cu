@@ -57,8 +57,14 @@
 // gives up stays until the other CTAs of its cluster are done, since they may
 // still store into its shared memory.
 //
-// Measured per launch (events around a pair, one box): 128^3 dam break (518k
-// rows) 41.8 us, 64^3 19.6 us, 256 x 128 x 128 tank (1.8M rows) 56.6 us; the
+// A group of four steps tests its edge words on a vote: the words are loaded two
+// steps ahead and the vote taken one step ahead, inside the latency of the step
+// before (as the group's first act it cost 170 cycles, two steps' worth), and the
+// shuffles a step waits for are issued before the last one's stores.
+//
+// Measured per launch (events around a pair, in the frames): 128^3 dam break (518k
+// rows) 38.5 us, 64^3 17.0 us, 256 x 128 x 128 tank (1.8M rows) 51.2 us, without
+// the look ahead 41.0, 18.2 and 54.5; the
 // form before it (tiles of 32 x 8 pencils, four warps in lockstep with a
 // barrier a step, every edge through L2) took 50.5, 23.0 and 71.3 us.
 #include <atomic>
