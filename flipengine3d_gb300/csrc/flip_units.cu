@@ -1,10 +1,13 @@
-// The MIC(0) preconditioner on its own, through the C ABI: the factor
+// Steps of the solvers on their own, through the C ABI, so that each can be
+// checked apart from a frame.  The same kernels and launch sequences as inside
+// one; only the data comes from host arrays in flat order.
+//
+// The MIC(0) preconditioner: the factor
 // (factorModifiedIncompleteColesky0, pcgsolver.h:70-185) and the two
 // triangular sweeps (solveLower / solveLowerTransposeInPlace,
 // pcgsolver.h:192-221) that the pressure solve runs, on rows the caller
-// gives, so that each can be checked against the reference's own routines
-// on arbitrary 7-point matrices.  The same kernels and launch sequence as
-// inside a solve; only the data comes from host arrays in flat cell order.
+// gives: arbitrary 7-point matrices.  The viscosity step: the field that it
+// makes of any level sets and velocities.
 #include <algorithm>
 #include <cstring>
 #include <string>
@@ -153,5 +156,51 @@ extern "C" int flip_mic0_precondition(int I, int J, int K, const uint8_t *fluid,
                 const size_t t = i + (size_t)I * (j + (size_t)J * k);
                 if (fluid[t]) z[t] = hz[sweep_index(g, i, j, k)];
             }
+    return FLIP_OK;
+}
+
+extern "C" int flip_viscosity_step(int I, int J, int K, double dx, const float *liquid_phi, const float *solid_phi, float *u,
+                                   float *v, float *w, double viscosity, double dt, long long *rows, int *iterations,
+                                   double *residual) {
+    if (!liquid_phi || !solid_phi || !u || !v || !w) return record_error(FLIP_E_NULL, "null pointer");
+    if (I < 3 || J < 3 || K < 3) return record_error(FLIP_E_DOMAIN, "grid must be at least 3 cells on each axis");
+    if ((long long)I * J * K >= (1LL << 28)) return record_error(FLIP_E_DOMAIN, "grid too large");
+    if (!(dx > 0.0) || !(viscosity >= 0.0) || !(dt >= 0.0)) return record_error(FLIP_E_DOMAIN, "cell size, viscosity or time step");
+    const size_t nodes = (size_t)(I + 1) * (J + 1) * (K + 1), cells = (size_t)I * J * K;
+    for (int k = 0; k <= K; k++)
+        for (int j = 0; j <= J; j++)
+            for (int i = 0; i <= I; i++) {
+                const bool wall = i <= 1 || j <= 1 || k <= 1 || i >= I - 1 || j >= J - 1 || k >= K - 1;
+                if (wall && !(solid_phi[i + (size_t)(I + 1) * (j + (size_t)(J + 1) * k)] < 0.0f))
+                    return record_error(FLIP_E_DOMAIN, "a cell on the grid border is not solid");
+            }
+    long long nf, nn, ncorner, vol[7], rowBlocks, slotWords;
+    viscosity_buffer_sizes(I, J, K, &nf, &nn, &ncorner, vol, &rowBlocks, &slotWords);
+    const size_t n[3] = {(size_t)(I + 1) * J * K, (size_t)I * (J + 1) * K, (size_t)I * J * (K + 1)};
+    Scratch sc;
+    ViscosityBuffers b{};
+    float *phi, *solid, *f[3], *host[3] = {u, v, w};
+    bool ok = sc.get(&b.fluidFace, nf) && sc.get(&b.valid, nn) && sc.get(&b.valid2, nn) && sc.get(&b.inSys, nf) &&
+              sc.get(&b.coefs, 8 * nf) && sc.get(&b.x, nf) && sc.get(&b.r, nf) && sc.get(&b.zp, nf) && sc.get(&b.p, nf) &&
+              sc.get(&b.q, nf) && sc.get(&b.list, nf) && sc.get(&b.blockRows, rowBlocks) && sc.get(&b.slots, slotWords) &&
+              sc.get(&b.scal, 8) && sc.get(&phi, cells) && sc.get(&solid, nodes);
+    for (int g = 0; g < 7; g++) ok = ok && sc.get(&b.vol[g], vol[g]) && sc.get(&b.node[g], ncorner);
+    for (int d = 0; d < 3; d++) ok = ok && sc.get(&f[d], n[d]);
+    if (!ok) return record_error(FLIP_E_NOMEM, "cudaMalloc failed");
+    int rc;
+    if ((rc = cuda_status(cudaMemcpy(phi, liquid_phi, cells * 4, cudaMemcpyHostToDevice), "copy level set")) ||
+        (rc = cuda_status(cudaMemcpy(solid, solid_phi, nodes * 4, cudaMemcpyHostToDevice), "copy level set")))
+        return rc;
+    for (int d = 0; d < 3; d++)
+        if ((rc = cuda_status(cudaMemcpy(f[d], host[d], n[d] * 4, cudaMemcpyHostToDevice), "copy velocities"))) return rc;
+    StepConsts c = grid_consts(I, J, K);
+    c.dx = dx;
+    ViscosityResult res{};
+    if ((rc = viscosity_apply(c, b, phi, solid, f[0], f[1], f[2], viscosity, dt, &res, nullptr))) return rc;
+    for (int d = 0; d < 3; d++)
+        if ((rc = cuda_status(cudaMemcpy(host[d], f[d], n[d] * 4, cudaMemcpyDeviceToHost), "read velocities"))) return rc;
+    if (rows) *rows = res.rows;
+    if (iterations) *iterations = res.iterations;
+    if (residual) *residual = res.residual;
     return FLIP_OK;
 }

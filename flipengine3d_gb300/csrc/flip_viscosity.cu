@@ -446,7 +446,6 @@ __device__ bool cg_all(const CgArgs &a, unsigned epoch, double &a0, double &a1) 
         s0[warp] = a0;
         s1[warp] = m;
     }
-    __threadfence();
     __syncthreads();
     if (warp == 0) {
         a0 = lane < WARPS ? s0[lane] : 0.0;
@@ -456,6 +455,10 @@ __device__ bool cg_all(const CgArgs &a, unsigned epoch, double &a0, double &a1) 
         // number, so that a word is new or not as a whole.  Two sets in turn: a
         // CTA writes one again only after every CTA has read it.
         unsigned long long *set = a.slots + (size_t)(epoch & 1) * CG_CTAS * 4;
+        // Release: the lanes that write the slot have met the CTA's other threads at
+        // the barrier above, and their fence after it puts all that those wrote
+        // before the slot.  Acquire: below, after the slots have been seen.
+        asm volatile("fence.acq_rel.gpu;" ::: "memory");
         if (lane < 4) {
             const unsigned long long v = (unsigned long long)(lane < 2 ? __double_as_longlong(a0) : m);
             asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(set + 4 * blockIdx.x + lane),
@@ -496,7 +499,7 @@ __device__ bool cg_all(const CgArgs &a, unsigned epoch, double &a0, double &a1) 
                     m = max(m, (long long)((w[h][2] & 0xffffffffull) | w[h][3] << 32));
                 }
         }
-        __threadfence();
+        asm volatile("fence.acq_rel.gpu;" ::: "memory");
         if (!ok) *(volatile double *)&a.scal[7] = 1.0;
         ok = __all_sync(0xffffffffu, ok);
         lanes();

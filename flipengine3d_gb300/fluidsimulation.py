@@ -147,6 +147,8 @@ SIGNATURES = {
     "flip_order_particles_by_id_noalloc": [_P, _P, _P, _P, _I, _I, _P, _P],
     "flip_mic0_factor": [_I, _I, _I, _P, _P, _P],
     "flip_mic0_precondition": [_I, _I, _I, _P, _P, _P, _P, _I],
+    "flip_viscosity_step": [_I, _I, _I, _D, _P, _P, _P, _P, _P, _D, _D, C.POINTER(C.c_longlong), C.POINTER(C.c_int),
+                            C.POINTER(C.c_double)],
     "flip_get_device_bytes": [_P, C.POINTER(C.c_longlong)],
     "flip_estimate_device_bytes": [_I, _I, _I, _I, C.POINTER(C.c_longlong)],
     "flip_runtime_create": [_I, C.c_longlong, C.POINTER(C.c_void_p)],
@@ -374,6 +376,24 @@ def mic0_precondition(fluid: np.ndarray, factor: np.ndarray, r: np.ndarray, orie
     z = np.zeros((K, J, I), np.float32)
     _check(lib, lib.flip_mic0_precondition(I, J, K, _ptr(f), _ptr(L), _ptr(rr), _ptr(z), int(orientation)))
     return z
+
+
+def viscosity_step(liquid_phi: np.ndarray, solid_phi: np.ndarray, u: np.ndarray, v: np.ndarray, w: np.ndarray, dx: float,
+                   viscosity: float, dt: float):
+    """The viscosity step (setViscosity) alone, on the GPU: the field u, v, w
+    after it, and (rows, iterations, relative residual).  liquid_phi (K, J, I)
+    float32, solid_phi (K+1, J+1, I+1) float32 with its two outer layers solid."""
+    lib = load_library()
+    K, J, I = liquid_phi.shape
+    phi, solid = np.ascontiguousarray(liquid_phi, np.float32), np.ascontiguousarray(solid_phi, np.float32)
+    shapes = (K, J, I + 1), (K, J + 1, I), (K + 1, J, I)
+    if solid.shape != (K + 1, J + 1, I + 1) or tuple(np.shape(g) for g in (u, v, w)) != shapes:
+        raise ValueError("the arrays are not of one grid")
+    field = [np.array(g, np.float32, order="C") for g in (u, v, w)]
+    rows, it, res = C.c_longlong(), C.c_int(), C.c_double()
+    _check(lib, lib.flip_viscosity_step(I, J, K, float(dx), _ptr(phi), _ptr(solid), *map(_ptr, field), float(viscosity),
+                                        float(dt), C.byref(rows), C.byref(it), C.byref(res)))
+    return field, (rows.value, it.value, res.value)
 
 
 def estimate_device_bytes(isize: int, jsize: int, ksize: int, particles: int) -> int:

@@ -286,6 +286,16 @@ int flip_mic0_factor(int isize, int jsize, int ksize, const uint8_t *fluid, cons
 int flip_mic0_precondition(int isize, int jsize, int ksize, const uint8_t *fluid, const float *factor,
                            const float *r, float *z, int orientation);
 
+/* The viscosity step alone (unit interface, as above): the field u, v, w (K x J x
+ * (I+1), K x (J+1) x I, (K+1) x J x I floats, updated in place) after the step
+ * of flip_set_viscosity below, for a cell-centred liquid level set and a nodal
+ * solid one whose two outer layers of nodes are solid, as the domain's walls
+ * make them (FLIP_E_DOMAIN otherwise).  rows, iterations, residual (each may be
+ * NULL): as flip_get_viscosity_solve. */
+int flip_viscosity_step(int isize, int jsize, int ksize, double dx, const float *liquid_phi, const float *solid_phi,
+                        float *u, float *v, float *w, double viscosity, double dt, long long *rows, int *iterations,
+                        double *residual);
+
 /* Number of this library's kernel launches issued so far on the context. */
 int flip_get_launch_count(flip_ctx *ctx, long long *count);
 
