@@ -339,8 +339,8 @@ struct SweepState {
     unsigned int *ticket;    // [0] forward tile tickets, [1] the sweep pair's epoch, [2] backward tile tickets
     int *err;                // set when a bounded wait gave up
     unsigned int epoch;      // host count of the epochs issued (wrap guard)
-    unsigned int spinLimit = 0;   // poll rounds of the factor's and sweeps' waits (0: DEFAULT_SPIN_LIMIT)
-    int stall = 0;           // fault injection: the sweeps' edge waits await an epoch never published
+    unsigned int spinLimit = 0;   // poll rounds of the factor's, sweeps' and viscous solver's waits (0: DEFAULT_SPIN_LIMIT)
+    int stall = 0;           // fault injection: the sweeps' edge waits and the viscous solver's sums await an epoch never published
 };
 int sweep_tiles_max(int I, int J, int K);           // tiles of the larger orientation
 long long sweep_exchange_words(int I, int J, int K);   // for the larger orientation
@@ -399,7 +399,8 @@ struct ViscosityResult {
 void viscosity_buffer_sizes(int I, int J, int K, long long *nf, long long *nn, long long *ncorner,
                             long long vol[7], long long *rowBlocks, long long *slotWords);
 int viscosity_apply(const StepConsts &c, const ViscosityBuffers &vb, const float *liquidPhi, const float *solidPhi,
-                    float *u, float *v, float *w, double visc, double dt, ViscosityResult *res, cudaStream_t s);
+                    float *u, float *v, float *w, double visc, double dt, unsigned spinLimit, bool stall,
+                    ViscosityResult *res, cudaStream_t s);
 
 // -- surface reconstruction (flip_mesh.cu)
 // The frame of the mesher's one compute chunk: the subdivided grid, its

@@ -763,8 +763,8 @@ int apply_viscosity(flip_ctx *x, double dt) {
     const bool fr = x->box.anyFriction;
     launch_constrain(x->c, x->u, x->v, x->w, nullptr, nullptr, nullptr, x->wu, x->wv, x->ww, fr ? x->fu : nullptr,
                      fr ? x->fv : nullptr, fr ? x->fw : nullptr, x->stream);
-    return viscosity_apply(x->c, x->vb, x->phi, x->solidPhi, x->u, x->v, x->w, x->viscosity, dt, &x->viscResult,
-                           x->stream);
+    return viscosity_apply(x->c, x->vb, x->phi, x->solidPhi, x->u, x->v, x->w, x->viscosity, dt, x->sweep.spinLimit,
+                           x->sweep.stall != 0, &x->viscResult, x->stream);
 }
 
 // _stepFluid (fluidsimulation.cpp:5471-5508)

@@ -196,7 +196,8 @@ extern "C" int flip_viscosity_step(int I, int J, int K, double dx, const float *
     StepConsts c = grid_consts(I, J, K);
     c.dx = dx;
     ViscosityResult res{};
-    if ((rc = viscosity_apply(c, b, phi, solid, f[0], f[1], f[2], viscosity, dt, &res, nullptr))) return rc;
+    if ((rc = viscosity_apply(c, b, phi, solid, f[0], f[1], f[2], viscosity, dt, 0, false, &res, nullptr)))
+        return rc;
     for (int d = 0; d < 3; d++)
         if ((rc = cuda_status(cudaMemcpy(host[d], f[d], n[d] * 4, cudaMemcpyDeviceToHost), "read velocities"))) return rc;
     if (rows) *rows = res.rows;

@@ -324,17 +324,21 @@ __global__ void __launch_bounds__(TPB) k_visc_system(SysArgs a, long long nf, ui
     if (threadIdx.x == 0) blockRows[blockIdx.x] = rows;
 }
 
-// The system's faces, in order.
-__global__ void __launch_bounds__(TPB) k_visc_list(const uint8_t *inSys, long long nf, const int *start, int *list) {
+// The place of a face in the list of the system's faces, which is in order.
+__device__ __forceinline__ int row_place(bool in, const int *start) {
     __shared__ int warps[TPB / 32];
-    const long long f = (long long)blockIdx.x * TPB + threadIdx.x;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const bool in = f < nf && inSys[f];
     const unsigned m = __ballot_sync(0xffffffffu, in);
     if (lane == 0) warps[warp] = __popc(m);
     __syncthreads();
     int at = start[blockIdx.x] + __popc(m & ((1u << lane) - 1u));
     for (int w = 0; w < warp; w++) at += warps[w];
+    return at;
+}
+__global__ void __launch_bounds__(TPB) k_visc_list(const uint8_t *inSys, long long nf, const int *start, int *list) {
+    const long long f = (long long)blockIdx.x * TPB + threadIdx.x;
+    const bool in = f < nf && inSys[f];
+    const int at = row_place(in, start);
     if (in) list[at] = (int)f;
 }
 
@@ -382,14 +386,20 @@ __global__ void __launch_bounds__(TPB) k_visc_rows(SysArgs a, const int *list, c
     }
 }
 // _applySolutionToVelocityField (viscositysolver.cpp:856-891): the field is
-// cleared before the system's faces take the solution; without a system it is
-// left as it is (:55-58).
-__global__ void __launch_bounds__(TPB) k_visc_clear(SysArgs a, long long nf, const int *listed, float *u, float *v, float *w) {
+// cleared and the system's faces take the solution; without a system it is left
+// as it is (:55-58), as it is where a wait of the solver ran out.
+__global__ void __launch_bounds__(TPB) k_visc_write(FaceIdx fx, long long nf, const uint8_t *inSys, const int *start,
+                                                    const int *listed, const double *x, const double *scal, float *u, float *v,
+                                                    float *w) {
+    if (*listed == 0 || scal[7] != 0.0) return;
     const long long f = (long long)blockIdx.x * TPB + threadIdx.x;
-    if (f >= nf || *listed == 0) return;
-    if (f < a.fx.nu) u[f] = 0.0f;
-    else if (f < a.fx.nu + a.fx.nv) v[f - a.fx.nu] = 0.0f;
-    else w[f - a.fx.nu - a.fx.nv] = 0.0f;
+    const bool in = f < nf && inSys[f];
+    const int at = row_place(in, start);
+    if (f >= nf) return;
+    const float val = in ? (float)x[at] : 0.0f;
+    if (f < fx.nu) u[f] = val;
+    else if (f < fx.nu + fx.nv) v[f - fx.nu] = val;
+    else w[f - fx.nu - fx.nv] = val;
 }
 
 // ------------------------------------------------------------------- solve
@@ -411,7 +421,6 @@ __global__ void __launch_bounds__(TPB) k_visc_clear(SysArgs a, long long nf, con
 constexpr int CG_CTAS = 320, CG_TPB = 512;
 constexpr int CG_BATCH = 8;            // |r|inf is compared with the tolerance every so many iterations
 constexpr int CG_MAX_ITER = 2000;
-constexpr unsigned CG_SPINS = 1u << 24;   // of a wait, about 10 s
 
 struct CgArgs {
     FaceIdx fx;
@@ -421,7 +430,8 @@ struct CgArgs {
     double2 *zp;                // {z, p_old} by face
     unsigned long long *slots;  // [2][CG_CTAS][4]
     double *scal;
-    float *u, *v, *w;           // take the solution
+    unsigned spinLimit;         // looks of a wait before it gives up
+    unsigned skew;              // 0; nonzero only to make the waits run out (fault injection)
 };
 
 // Sums a0 and takes the maximum of a1 >= 0 over the grid, in a fixed order, and
@@ -485,9 +495,9 @@ __device__ bool cg_all(const CgArgs &a, unsigned epoch, double &a0, double &a1) 
 #pragma unroll
                 for (int h = 0; h < 4; h++)
 #pragma unroll
-                    for (int q = 0; q < 4; q++) all &= (unsigned)(w[h][q] >> 32) == epoch;
+                    for (int q = 0; q < 4; q++) all &= (unsigned)(w[h][q] >> 32) == epoch + a.skew;
                 if (all) break;
-                if (spin > CG_SPINS || ((spin & 1023u) == 1023u && *(volatile double *)&a.scal[7] != 0.0)) {
+                if (spin >= a.spinLimit || ((spin & 1023u) == 1023u && *(volatile double *)&a.scal[7] != 0.0)) {
                     ok = false;
                     break;
                 }
@@ -584,14 +594,6 @@ __global__ void __launch_bounds__(CG_TPB, 1) k_cg(CgArgs a) {
         rz = nrz;
         if (++it % CG_BATCH == 0) rmax = nmax;
     }
-    if (ok)
-        for (int n = first; n < rows; n += step) {
-            const long long f = a.list[n];
-            const float x = (float)a.x[n];
-            if (f < a.fx.nu) a.u[f] = x;
-            else if (f < a.fx.nu + a.fx.nv) a.v[f - a.fx.nu] = x;
-            else a.w[f - a.fx.nu - a.fx.nv] = x;
-        }
     if (first == 0) {
         a.scal[3] = rmax;
         a.scal[4] = bmax;
@@ -617,9 +619,11 @@ void viscosity_buffer_sizes(int I, int J, int K, long long *nf, long long *nn, l
 }
 
 // The viscosity step on the device (buffers from the caller, sized by
-// viscosity_buffer_sizes).  Returns FLIP_OK or FLIP_E_CUDA.
+// viscosity_buffer_sizes).  Returns FLIP_OK, FLIP_E_DEVICE_TIMEOUT (a wait ran
+// out: the field is as it was) or FLIP_E_CUDA.
 int viscosity_apply(const StepConsts &c, const ViscosityBuffers &vb, const float *liquidPhi, const float *solidPhi,
-                    float *u, float *v, float *w, double visc, double dt, ViscosityResult *res, cudaStream_t s) {
+                    float *u, float *v, float *w, double visc, double dt, unsigned spinLimit, bool stall,
+                    ViscosityResult *res, cudaStream_t s) {
     const long long nu = (long long)(c.I + 1) * c.J * c.K, nv = (long long)c.I * (c.J + 1) * c.K,
                     nw = (long long)c.I * c.J * (c.K + 1), nf = nu + nv + nw;
     const long long nn = (long long)(c.I + 1) * (c.J + 1) * (c.K + 1);
@@ -663,8 +667,9 @@ int viscosity_apply(const StepConsts &c, const ViscosityBuffers &vb, const float
     launch_scan_cells(vb.blockRows, blocks, start, total + 1, total, s);
     { FLIP_COUNT(1); k_visc_list<<<blocks, TPB, 0, s>>>(vb.inSys, nf, start, vb.list); }
     { FLIP_COUNT(1); k_visc_rows<<<std::min(blocks, 152 * 8), TPB, 0, s>>>(sa, vb.list, total, coefs); }
-    { FLIP_COUNT(1); k_visc_clear<<<blocks, TPB, 0, s>>>(sa, nf, total, u, v, w); }
-    const CgArgs a{sa.fx, coefs, vb.list, total, vb.x, vb.p, vb.q, vb.zp, vb.slots, vb.scal, u, v, w};
+    // an epoch half the numbers away is never written
+    const CgArgs a{sa.fx, coefs, vb.list, total, vb.x, vb.p, vb.q, vb.zp, vb.slots, vb.scal,
+                   spinLimit ? spinLimit : DEFAULT_SPIN_LIMIT, stall ? 1u << 31 : 0u};
     cudaError_t e = cudaMemsetAsync(vb.zp, 0, (size_t)nf * sizeof(double2), s);   // off the system
     if (e == cudaSuccess) e = cudaMemsetAsync(vb.slots, 0, sizeof(unsigned long long) * 8 * CG_CTAS, s);
     if (e == cudaSuccess) e = cudaMemsetAsync(vb.scal, 0, 8 * sizeof(double), s);
@@ -680,11 +685,12 @@ int viscosity_apply(const StepConsts &c, const ViscosityBuffers &vb, const float
         e = cudaLaunchCooperativeKernel((const void *)k_cg, dim3(ctas), dim3(CG_TPB), args, 0, s);
     }
     if (e != cudaSuccess) return record_error(FLIP_E_CUDA, std::string("viscosity: ") + cudaGetErrorString(e));
+    { FLIP_COUNT(1); k_visc_write<<<blocks, TPB, 0, s>>>(sa.fx, nf, vb.inSys, start, total, vb.x, vb.scal, u, v, w); }
     double hs[8];
     e = cudaMemcpyAsync(hs, vb.scal, sizeof(hs), cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess) { FLIP_SYNC_COUNT(); e = cudaStreamSynchronize(s); }
     if (e != cudaSuccess) return record_error(FLIP_E_CUDA, std::string("viscosity: ") + cudaGetErrorString(e));
-    if (hs[7] != 0.0) return record_error(FLIP_E_CUDA, "viscosity: a wait of the solver ran out");
+    if (hs[7] != 0.0) return record_error(FLIP_E_DEVICE_TIMEOUT, "viscosity: a wait of the solver ran out");
     res->rows = (long long)hs[5];
     res->iterations = (int)hs[6];
     res->residual = hs[4] > 0 && res->rows > 0 ? hs[3] / hs[4] : 0.0;

@@ -258,12 +258,14 @@ int flip_get_sweep_orientation(flip_ctx *ctx, int *last);
 int flip_get_binned_particles(flip_ctx *ctx, float *pos, unsigned int *ids, int *cell_start);
 
 /* Fault injection for the bounded device waits (test interface).  Every
- * wait of the factor's and the sweeps' wavefronts gives up after `polls`
- * poll rounds (0 restores the default, about a second) and the update
- * returns FLIP_E_DEVICE_TIMEOUT; the context stays usable.  With the stall
- * on, the sweeps' tiles await edge terms under an epoch no tile publishes,
- * so any tile with an upstream neighbour tile waits until its limit runs
- * out.  Nothing faults or hangs: each wait ends at its limit. */
+ * wait of the factor's and the sweeps' wavefronts and of the viscous solver's
+ * sums gives up after `polls` poll rounds (0 restores the default, one to a few
+ * seconds) and the update returns FLIP_E_DEVICE_TIMEOUT; the context stays
+ * usable.  With the stall on, the sweeps' tiles await edge terms, and the
+ * viscous solver's CTAs shares of their sums, under an epoch that none
+ * publishes, so any tile with an upstream neighbour tile, and every viscous
+ * solve, waits until its limit runs out.  Nothing faults or hangs: each wait
+ * ends at its limit. */
 int flip_set_device_wait_limit(flip_ctx *ctx, unsigned int polls);
 int flip_inject_sweep_stall(flip_ctx *ctx, int on);
 
