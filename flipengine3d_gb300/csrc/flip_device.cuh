@@ -47,11 +47,15 @@ struct StepConsts {
     const float *blockPosF;
 };
 
-// Pairs of floats in one 64-bit register (two cells): each operation rounds
-// each half as the scalar one does.  Sums and products are written as fused
-// multiply-adds that are exact up to that one rounding (a b + 0, a 1 + b), so
-// the compiler cannot contract two operations into one.
+// Pairs of floats in one 64-bit register: each operation rounds each half as the
+// scalar one does.  Sums and products are fused multiply-adds that are exact up
+// to that one rounding (a 1 + b, a b - 0).  A product's zero comes as a kernel
+// argument: the compiler folds a visible one away, and is then free to contract
+// the product with the sum after it, which rounds once where the two round twice
+// (it did in particle to grid).  A sum has nothing to contract with, so its 1 is
+// plain.
 using F2 = unsigned long long;
+__host__ __device__ constexpr F2 f2_bits(unsigned x, unsigned y) { return x | (F2)y << 32; }
 __device__ __forceinline__ F2 f2(float x, float y) {
     F2 r;
     asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(x), "f"(y));
@@ -64,10 +68,14 @@ __device__ __forceinline__ F2 f2_fma(F2 a, F2 b, F2 c) {
     asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
     return r;
 }
-constexpr F2 F2_ONE = 0x3f8000003f800000ull, F2_MINUS = 0xbf800000bf800000ull, F2_ZERO = 0x8000000080000000ull;   // -0
-__device__ __forceinline__ F2 f2_add(F2 a, F2 b) { return f2_fma(a, F2_ONE, b); }
-__device__ __forceinline__ F2 f2_sub(F2 a, F2 b) { return f2_fma(b, F2_MINUS, a); }
-__device__ __forceinline__ F2 f2_mul(F2 a, F2 b) { return f2_fma(a, b, F2_ZERO); }
+struct PairOps {
+    static constexpr F2 ONE = f2_bits(0x3f800000u, 0x3f800000u), MINUS = f2_bits(0xbf800000u, 0xbf800000u);
+    F2 zero = f2_bits(0x80000000u, 0x80000000u);   // (-0, -0)
+    __device__ F2 mul(F2 a, F2 b) const { return f2_fma(a, b, zero); }
+    __device__ F2 add(F2 a, F2 b) const { return f2_fma(a, ONE, b); }
+    __device__ F2 sub(F2 a, F2 b) const { return f2_fma(b, MINUS, a); }
+    __device__ F2 neg(F2 a) const { return a ^ f2_bits(0x80000000u, 0x80000000u); }
+};
 
 // Programmatic dependent launch: a kernel launched with launch_after may start
 // while the kernel before it in the stream still runs; what it reads or
@@ -372,6 +380,10 @@ void mic0_inverse_pivots(const uint8_t *fluid, long long n, double *E, cudaStrea
 // cells (a tuning knob, default 4096), at most PCG_MAX_PARTIALS.
 constexpr int PCG_MAX_PARTIALS = 152 * 8;
 int pressure_partials_for(int I, int J, int K, int cellsPerCta = 4096);
+// Steps of the solve: its items, its vectors' layout, one product (flip_pcg.cu)
+void launch_items(const StepConsts &c, PressureBuffers &pb, SweepState &sw, cudaStream_t s);
+void launch_layout(const StepConsts &c, const PressureBuffers &pb, SweepState &sw, cudaStream_t s);
+void launch_spmv(const PressureBuffers &pb, const float *sIn, float *sOut, SweepState &sw, cudaStream_t s);
 // PressureSolver::solve (pressuresolver.cpp:44-76) on the device.  Returns
 // FLIP_OK (velocities updated, or nothing to solve), FLIP_E_SOLVER_NOCONV
 // (left unchanged), FLIP_E_DEVICE_TIMEOUT or FLIP_E_CUDA.

@@ -392,19 +392,10 @@ __global__ void __launch_bounds__(SDF_TPB, 1024 / SDF_TPB) k_liquid_sdf(Particle
 // sr = r + 1e-6.  A particle within r of the face meets both: every coordinate
 // of the face is within r of the particle, and the 1e-6 margin is far above
 // the rounding of these float expressions (ulp(1) ~ 1.2e-7).
-// Packed sums and products as fused multiply-adds that are exact up to the one
-// rounding, with constants that the compiler does not see: it folds a visible 1
-// or 0 away and then contracts a product with the sum after it.
-struct PairConsts {
-    F2 one, minus, zero;   // (1, 1), (-1, -1), (-0, -0)
-    __device__ F2 mul(F2 a, F2 b) const { return f2_fma(a, b, zero); }
-    __device__ F2 add(F2 a, F2 b) const { return f2_fma(a, one, b); }
-    __device__ F2 sub(F2 a, F2 b) const { return f2_fma(b, minus, a); }
-};
 constexpr int P2G_TPB = 128;
 __global__ void __launch_bounds__(P2G_TPB, 1024 / P2G_TPB) k_p2g(ParticleSoA p, const int *cellStart, StepConsts c,
                                              float *U, float *V, float *W, uint8_t *vu, uint8_t *vv, uint8_t *vw,
-                                             PairConsts k2) {
+                                             PairOps k2) {
     pdl_begin();
     const int ni = c.I + 1, nj = c.J + 1, nk = c.K + 1;
     const long long f = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -428,7 +419,7 @@ __global__ void __launch_bounds__(P2G_TPB, 1024 / P2G_TPB) k_p2g(ParticleSoA p, 
     Dims cells{c.I, c.J, c.K};
     const F2 nox = f2(-offx, -offx), noy = f2(-offy, -offy), noz = f2(-offz, -offz), nh = f2(-h, -h);
     const F2 pgx = f2(gx, gx), pgy = f2(gy, gy), pgz = f2(gz, gz);
-    const F2 c1 = f2(coef1, coef1), c2 = f2(coef2, coef2), c3 = f2(coef3, coef3), one = k2.one;
+    const F2 c1 = f2(coef1, coef1), c2 = f2(coef2, coef2), c3 = f2(coef3, coef3), one = PairOps::ONE;
     float sc[3] = {0.0f, 0.0f, 0.0f}, wt[3] = {0.0f, 0.0f, 0.0f};
     // Two particles' shares of a face: weights of the two together, then the
     // sums in the particles' order.
@@ -994,7 +985,7 @@ void launch_liquid_sdf(const ParticleSoA &p, const int *cellStart, const StepCon
 void launch_p2g(const ParticleSoA &p, const int *cellStart, const StepConsts &c, float *u, float *v,
                 float *w, uint8_t *vu, uint8_t *vv, uint8_t *vw, cudaStream_t s) {
     launch_next(k_p2g, div_up((long long)(c.I + 1) * (c.J + 1) * (c.K + 1), P2G_TPB), P2G_TPB, s, p, cellStart, c, u, v, w, vu, vv, vw,
-                                                                                                  PairConsts{F2_ONE, F2_MINUS, F2_ZERO});
+                                                                                                  PairOps{});
 }
 FaceBits face_bits(int I, int J, int K) {
     FaceBits b;

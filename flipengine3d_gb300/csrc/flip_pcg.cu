@@ -663,29 +663,29 @@ __device__ __forceinline__ float2 df_scale(float f, float2 v) {
 // (sh, sl) += (ah, al) s for two cells, ns = -s: the leading product exact as
 // its rounded value plus its FMA-recovered error, the sum's rounding error by
 // Knuth's TwoSum
-__device__ __forceinline__ void df2_mul_add(F2 ah, F2 al, F2 sv, F2 ns, F2 &sh, F2 &sl) {
-    const F2 nph = f2_mul(ah, ns);                        // -(ah s) rounded
+__device__ __forceinline__ void df2_mul_add(const PairOps &k, F2 ah, F2 al, F2 sv, F2 ns, F2 &sh, F2 &sl) {
+    const F2 nph = k.mul(ah, ns);                         // -(ah s) rounded
     const F2 pl = f2_fma(al, sv, f2_fma(ah, sv, nph));   // its error, plus al s
-    const F2 t = f2_sub(sh, nph);
-    const F2 bb = f2_sub(t, sh);
-    const F2 err = f2_sub(f2_sub(sh, f2_sub(t, bb)), f2_add(nph, bb));   // exact error of the sum
-    sl = f2_add(sl, f2_add(err, pl));
+    const F2 t = k.sub(sh, nph);
+    const F2 bb = k.sub(t, sh);
+    const F2 err = k.sub(k.sub(sh, k.sub(t, bb)), k.add(nph, bb));   // exact error of the sum
+    sl = k.add(sl, k.add(err, pl));
     sh = t;
 }
 // df_norm, df_add and df_scale for two cells
-__device__ __forceinline__ void df2_norm(F2 h, F2 l, F2 &oh, F2 &ol) {
-    oh = f2_add(h, l);
-    ol = f2_sub(l, f2_sub(oh, h));
+__device__ __forceinline__ void df2_norm(const PairOps &k, F2 h, F2 l, F2 &oh, F2 &ol) {
+    oh = k.add(h, l);
+    ol = k.sub(l, k.sub(oh, h));
 }
-__device__ __forceinline__ void df2_add(F2 ah, F2 al, F2 bh, F2 bl, F2 &oh, F2 &ol) {
-    const F2 t = f2_add(ah, bh);
-    const F2 bb = f2_sub(t, ah);
-    const F2 err = f2_add(f2_sub(ah, f2_sub(t, bb)), f2_sub(bh, bb));
-    df2_norm(t, f2_add(err, f2_add(al, bl)), oh, ol);
+__device__ __forceinline__ void df2_add(const PairOps &k, F2 ah, F2 al, F2 bh, F2 bl, F2 &oh, F2 &ol) {
+    const F2 t = k.add(ah, bh);
+    const F2 bb = k.sub(t, ah);
+    const F2 err = k.add(k.sub(ah, k.sub(t, bb)), k.sub(bh, bb));
+    df2_norm(k, t, k.add(err, k.add(al, bl)), oh, ol);
 }
-__device__ __forceinline__ void df2_scale(F2 f, F2 nf, F2 vh, F2 vl, F2 &oh, F2 &ol) {   // nf = -f
-    oh = f2_mul(f, vh);
-    ol = f2_fma(f, vl, f2_sub(F2_ZERO, f2_fma(nf, vh, oh)));
+__device__ __forceinline__ void df2_scale(const PairOps &k, F2 f, F2 nf, F2 vh, F2 vl, F2 &oh, F2 &ol) {   // nf = -f
+    oh = k.mul(f, vh);
+    ol = f2_fma(f, vl, k.neg(f2_fma(nf, vh, oh)));
 }
 __device__ __forceinline__ void ld2x2(const float *p, F2 (&v)[2]) {
     const ulonglong2 q = *reinterpret_cast<const ulonglong2 *>(p);
@@ -736,7 +736,7 @@ __global__ void __launch_bounds__(TPB, 3)
     k_spmv_s(SweepLayout g, long long nsl, const int *__restrict__ items, const int *__restrict__ nItems,
              const float *__restrict__ A, const float *__restrict__ z, const float *__restrict__ sIn,
              float *__restrict__ sOut, float *__restrict__ qh, float *__restrict__ ql, const double *zrPartials,
-             double *partials, double *scal, PcgCtl *ctl, int *err) {
+             double *partials, double *scal, PcgCtl *ctl, int *err, PairOps k2) {
     __shared__ __align__(128) SpmvSmem sm;
     __shared__ double sh[TPB];
     const int n = *nItems, T = g.T, nch = T / SWEEP_CH, ctas = min((int)gridDim.x, n);
@@ -785,7 +785,7 @@ __global__ void __launch_bounds__(TPB, 3)
     const F2 beta = f2(betaf, betaf);
     const int u = threadIdx.x >> 5, p0 = (threadIdx.x & 31) * 4, la0 = p0 & 7, lb = (p0 >> 3) & 3, wa = (p0 >> 5) & 1,
               wb = p0 >> 6;
-    F2 dotH = F2_ZERO, dotL = F2_ZERO;
+    F2 dotH = k2.zero, dotL = k2.zero;
     unsigned phase = 0;
     for (int it = blockIdx.x; it < n; it += gridDim.x) {
         if (threadIdx.x == 0 && it != (int)blockIdx.x) issue(it, true, true);
@@ -840,10 +840,10 @@ __global__ void __launch_bounds__(TPB, 3)
             v[1] = f2_fma(beta, ss[1], zz[1]);
         };
         auto snew1 = [&](int r, int p) { return __fmaf_rn(betaf, sm.S[r][p], sm.Z[r][p]); };
-        F2 accH[2] = {F2_ZERO, F2_ZERO}, accL[2] = {F2_ZERO, F2_ZERO};
+        F2 accH[2] = {k2.zero, k2.zero}, accL[2] = {k2.zero, k2.zero};
         auto couple = [&](const F2 (&h)[2], const F2 (&l)[2], const F2 (&v)[2]) {
 #pragma unroll
-            for (int q = 0; q < 2; q++) df2_mul_add(h[q], l[q], v[q], f2_mul(v[q], F2_MINUS), accH[q], accL[q]);
+            for (int q = 0; q < 2; q++) df2_mul_add(k2, h[q], l[q], v[q], k2.neg(v[q]), accH[q], accL[q]);
         };
         // sU, sD: the steps after and before; nothing beyond the tile's ends
         F2 s0[2], sU[2] = {0, 0}, sD[2] = {0, 0}, h[2], l[2], v[2];
@@ -907,10 +907,10 @@ __global__ void __launch_bounds__(TPB, 3)
         F2 oh[2], ol[2];
 #pragma unroll
         for (int q = 0; q < 2; q++) {
-            df2_norm(accH[q], accL[q], oh[q], ol[q]);
+            df2_norm(k2, accH[q], accL[q], oh[q], ol[q]);
             F2 ph, pl;
-            df2_scale(s0[q], f2_mul(s0[q], F2_MINUS), oh[q], ol[q], ph, pl);
-            df2_add(dotH, dotL, ph, pl, dotH, dotL);
+            df2_scale(k2, s0[q], k2.neg(s0[q]), oh[q], ol[q], ph, pl);
+            df2_add(k2, dotH, dotL, ph, pl, dotH, dotL);
         }
         st2x2(sOut + e, s0);
         st2x2(qh + e, oh);
@@ -1202,6 +1202,26 @@ void mic0_inverse_pivots(const uint8_t *fluid, long long n, double *E, cudaStrea
     k_mic0_inverse<<<div_up(n, TPB), TPB, 0, s>>>(fluid, n, E);
 }
 
+// The chunks of the sweep layout that the sweeps pass over, and the system's
+// vectors there.
+static unsigned item_ctas(const StepConsts &c) {
+    return (unsigned)std::max(1LL, std::min<long long>(sweep_items_max(c.I, c.J, c.K), RBLOCKS));
+}
+void launch_items(const StepConsts &c, PressureBuffers &pb, SweepState &sw, cudaStream_t s) {
+    launch_sweep_ranges(c, pb.sl, pb.fluid, sw, s);
+    launch_next(k_items, 1, 1024, s, pb.sl, sw.range, pb.items, pb.nItems);
+}
+void launch_layout(const StepConsts &c, const PressureBuffers &pb, SweepState &sw, cudaStream_t s) {
+    FLIP_COUNT(1);
+    k_layout<<<item_ctas(c), TPB, 0, s>>>(c, pb.sl, pb.items, pb.nItems, pb, sw.ticket);
+}
+// sOut = z + beta sIn, q = A sOut and the partial sums of sOut.q
+void launch_spmv(const PressureBuffers &pb, const float *sIn, float *sOut, SweepState &sw, cudaStream_t s) {
+    launch_after(true, pb.sl.swap ? k_spmv_s<true> : k_spmv_s<false>, (unsigned)pb.nPartials, TPB, 0, s, pb.sl, pb.nsl, pb.items,
+                 pb.nItems, pb.A, pb.z, sIn, sOut, pb.qh, pb.ql, pb.partials + PCG_MAX_PARTIALS, pb.partials, pb.scal, pb.ctl,
+                 sw.err, PairOps{});
+}
+
 // The condition of the device-side loop over batches of PCG iterations: one
 // more batch while the solve has not converged, no wavefront has given up
 // and fewer than maxBatches batches have run (so the loop always ends).
@@ -1268,9 +1288,7 @@ int pressure_project(const StepConsts &c, const PressureArgs &a, PressureBuffers
         if (want != pb.sl.swap) pb.sl = sweep_layout(c.I, c.J, c.K, want);
     }
     const SweepLayout sl = pb.sl;
-    const unsigned ib = (unsigned)std::max(1LL, std::min<long long>(sweep_items_max(c.I, c.J, c.K), RBLOCKS));   // item loops
-    launch_sweep_ranges(c, sl, pb.fluid, sw, s);
-    launch_next(k_items, 1, 1024, s, sl, sw.range, pb.items, pb.nItems);
+    launch_items(c, pb, sw, s);
 
     // MIC(0) factor; the pivot weights go to A's buffer, which is filled after
     // it: zero wherever no item of this solve writes a coupling
@@ -1284,7 +1302,7 @@ int pressure_project(const StepConsts &c, const PressureArgs &a, PressureBuffers
         PCK(cudaMemsetAsync(pb.s2, 0, (pb.nsl + SWEEP_NP) * sizeof(float), s));
     }
     pb.stale = true;   // until this solve has converged
-    { FLIP_COUNT(1); k_layout<<<ib, TPB, 0, s>>>(c, sl, pb.items, pb.nItems, pb, sw.ticket); }
+    launch_layout(c, pb, sw, s);
 
     unsigned long long *rmax = pb.rmaxBits;
     double *zrPartials = pb.partials + PCG_MAX_PARTIALS;
@@ -1323,8 +1341,7 @@ int pressure_project(const StepConsts &c, const PressureArgs &a, PressureBuffers
     int sPar = 0;
     auto iteration = [&](int k, bool timed) {
         float *sIn = sPar ? pb.s2 : pb.s, *sOut = sPar ? pb.s : pb.s2;
-        launch_after(true, sl.swap ? k_spmv_s<true> : k_spmv_s<false>, rb, TPB, 0, s, sl, pb.nsl, pb.items, pb.nItems, pb.A,
-                     pb.z, sIn, sOut, pb.qh, pb.ql, zrPartials, pb.partials, pb.scal, pb.ctl, sw.err);
+        launch_spmv(pb, sIn, sOut, sw, s);
         launch_after(true, k_update_xr, rb, TPB, 0, s, pb.items, pb.nItems, pb.xh, pb.xl, pb.rh, pb.rl, sOut, pb.qh, pb.ql,
                      pb.partials, pb.scal, rmax, pb.ctl, sw.ticket);
         launch_after(true, k_true_residual, rb, TPB, 0, s, c, sl, pb.items, pb.nItems, pb.fluid, pb.Ad, pb.b, pb.xh, pb.xl,
@@ -1482,7 +1499,7 @@ int pressure_project(const StepConsts &c, const PressureArgs &a, PressureBuffers
     pb.stale = !ok;
     const bool accept = ok || (iterations == a.maxIter && resid < a.accTol);   // pressuresolver.cpp:810-840
     PCK(cudaMemsetAsync(pb.pressure, 0, n * sizeof(float), s));
-    { FLIP_COUNT(1); k_x_to_cells<<<ib, TPB, 0, s>>>(c, sl, pb.items, pb.nItems, pb.fluid, pb.xh, pb.xl, pb.pressure); }
+    { FLIP_COUNT(1); k_x_to_cells<<<item_ctas(c), TPB, 0, s>>>(c, sl, pb.items, pb.nItems, pb.fluid, pb.xh, pb.xl, pb.pressure); }
     if (a.dumpPressure) {
         PCK(sync());
         PCK(cudaMemcpy(a.dumpPressure, pb.pressure, n * sizeof(float), cudaMemcpyDeviceToHost));

@@ -6,7 +6,8 @@
 // (factorModifiedIncompleteColesky0, pcgsolver.h:70-185) and the two
 // triangular sweeps (solveLower / solveLowerTransposeInPlace,
 // pcgsolver.h:192-221) that the pressure solve runs, on rows the caller
-// gives: arbitrary 7-point matrices.  The viscosity step: the field that it
+// gives: arbitrary 7-point matrices.  The product A s of the solve's loop, on such
+// rows.  The viscosity step: the field that it
 // makes of any level sets and velocities.
 #include <algorithm>
 #include <cstring>
@@ -156,6 +157,84 @@ extern "C" int flip_mic0_precondition(int I, int J, int K, const uint8_t *fluid,
                 const size_t t = i + (size_t)I * (j + (size_t)J * k);
                 if (fluid[t]) z[t] = hz[sweep_index(g, i, j, k)];
             }
+    return FLIP_OK;
+}
+
+extern "C" int flip_pressure_apply(int I, int J, int K, const uint8_t *fluid, const double *rows, const float *z,
+                                   const float *s, float beta, int orientation, float *s_out, double *q, double *dot) {
+    if (!fluid || !rows || !z || !s || !s_out || !q || !dot) return record_error(FLIP_E_NULL, "null pointer");
+    if (orientation < 0 || orientation > 1) return record_error(FLIP_E_OUT_OF_RANGE, "orientation must be 0 or 1");
+    int rc = check_system(I, J, K, fluid);
+    if (rc) return rc;
+    const size_t n = (size_t)I * J * K;
+    const SweepLayout g = sweep_layout(I, J, K, orientation);
+    const size_t nsl = (size_t)sweep_layout_size(I, J, K), pad = nsl + SWEEP_NP;
+    std::vector<float> hz(pad, 0.0f), hs(pad, 0.0f), hq(2 * nsl);
+    bool any = false;
+    auto rows_of = [&](auto f) {
+        for (int k = 1; k <= K - 2; k++)
+            for (int j = 1; j <= J - 2; j++)
+                for (int i = 1; i <= I - 2; i++) {
+                    const size_t t = i + (size_t)I * (j + (size_t)J * k);
+                    if (fluid[t]) f(t, (size_t)sweep_index(g, i, j, k));
+                }
+    };
+    rows_of([&](size_t t, size_t e) {
+        hz[e] = z[t];
+        hs[e] = s[t];
+        any = true;
+    });
+    std::memset(s_out, 0, n * sizeof(float));
+    std::memset(q, 0, n * sizeof(double));
+    *dot = 0.0;
+    if (!any) return FLIP_OK;
+    Scratch sc;
+    PressureBuffers pb{};
+    pb.sl = g;
+    pb.nsl = (long long)nsl;
+    pb.nPartials = pressure_partials_for(I, J, K);
+    SweepState sw{};
+    const std::vector<double> ones(n, 1.0);
+    if (!sc.get(&pb.fluid, n) || !sc.get(&pb.items, sweep_items_max(I, J, K)) || !sc.get(&pb.nItems, 4) || !sc.get(&pb.Ad, n) ||
+        !sc.get(&pb.b, n) || !sc.get(&pb.pivotInv, n) || !sc.get(&pb.L, nsl) || !sc.get(&pb.A, 8 * pad) || !sc.get(&pb.xh, nsl) ||
+        !sc.get(&pb.xl, nsl) || !sc.get(&pb.rh, nsl) || !sc.get(&pb.rl, nsl) || !sc.get(&pb.qh, nsl) || !sc.get(&pb.ql, nsl) ||
+        !sc.get(&pb.z, pad) || !sc.get(&pb.s, pad) || !sc.get(&pb.s2, pad) || !sc.get(&pb.partials, 2 * PCG_MAX_PARTIALS) ||
+        !sc.get(&pb.scal, 8) || !sc.get(&pb.ctl, 1) || !sc.get(&sw.range, sweep_tiles_max(I, J, K)) || !sc.get(&sw.ticket, 4) ||
+        !sc.get(&sw.err, 4))
+        return record_error(FLIP_E_NOMEM, "cudaMalloc failed");
+    auto put = [&](void *to, const void *from, size_t bytes) { return cuda_status(cudaMemcpy(to, from, bytes, cudaMemcpyHostToDevice), "copy"); };
+    auto clear = [&](void *p, size_t bytes) { return cuda_status(cudaMemset(p, 0, bytes), "clear"); };
+    if ((rc = put(pb.fluid, fluid, n)) || (rc = put(pb.Ad, rows, n * sizeof(double4_32a))) ||
+        (rc = put(pb.pivotInv, ones.data(), n * sizeof(double))) || (rc = clear(pb.b, n * sizeof(double))) ||
+        (rc = clear(pb.A, 8 * pad * sizeof(float))) || (rc = clear(sw.ticket, 4 * sizeof(unsigned))) || (rc = clear(sw.err, 4 * sizeof(int))))
+        return rc;
+    StepConsts c = grid_consts(I, J, K);
+    cudaStream_t st = nullptr;
+    launch_items(c, pb, sw, st);
+    launch_layout(c, pb, sw, st);
+    // the second iteration of a solve whose z.r was 1 and is beta
+    PcgCtl ctl{};
+    ctl.it = 1;
+    std::vector<double> zr(PCG_MAX_PARTIALS, 0.0), scal(8, 0.0), sums(pb.nPartials);
+    zr[0] = beta;
+    scal[3] = 1.0;
+    if ((rc = put(pb.z, hz.data(), pad * 4)) || (rc = put(pb.s, hs.data(), pad * 4)) || (rc = put(pb.ctl, &ctl, sizeof(ctl))) ||
+        (rc = put(pb.partials + PCG_MAX_PARTIALS, zr.data(), zr.size() * 8)) || (rc = put(pb.scal, scal.data(), 64)))
+        return rc;
+    launch_spmv(pb, pb.s, pb.s2, sw, st);
+    if ((rc = cuda_status(cudaDeviceSynchronize(), "product"))) return rc;
+    int nItems = 0, err = 0;
+    auto get = [&](void *to, const void *from, size_t bytes) { return cuda_status(cudaMemcpy(to, from, bytes, cudaMemcpyDeviceToHost), "read"); };
+    if ((rc = get(&nItems, pb.nItems, sizeof(int))) || (rc = get(&err, sw.err, sizeof(int))) || (rc = get(hs.data(), pb.s2, nsl * 4)) ||
+        (rc = get(hq.data(), pb.qh, nsl * 4)) || (rc = get(hq.data() + nsl, pb.ql, nsl * 4)) ||
+        (rc = get(sums.data(), pb.partials, sums.size() * 8)))
+        return rc;
+    if (err) return record_error(FLIP_E_DEVICE_TIMEOUT, "a copy into shared memory did not arrive");
+    rows_of([&](size_t t, size_t e) {
+        s_out[t] = hs[e];
+        q[t] = (double)hq[e] + (double)hq[nsl + e];
+    });
+    for (int b = 0; b < std::min(pb.nPartials, nItems); b++) *dot += sums[b];
     return FLIP_OK;
 }
 

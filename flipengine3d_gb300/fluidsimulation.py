@@ -147,6 +147,7 @@ SIGNATURES = {
     "flip_order_particles_by_id_noalloc": [_P, _P, _P, _P, _I, _I, _P, _P],
     "flip_mic0_factor": [_I, _I, _I, _P, _P, _P],
     "flip_mic0_precondition": [_I, _I, _I, _P, _P, _P, _P, _I],
+    "flip_pressure_apply": [_I, _I, _I, _P, _P, _P, _P, C.c_float, _I, _P, _P, C.POINTER(C.c_double)],
     "flip_viscosity_step": [_I, _I, _I, _D, _P, _P, _P, _P, _P, _D, _D, C.POINTER(C.c_longlong), C.POINTER(C.c_int),
                             C.POINTER(C.c_double)],
     "flip_get_device_bytes": [_P, C.POINTER(C.c_longlong)],
@@ -376,6 +377,20 @@ def mic0_precondition(fluid: np.ndarray, factor: np.ndarray, r: np.ndarray, orie
     z = np.zeros((K, J, I), np.float32)
     _check(lib, lib.flip_mic0_precondition(I, J, K, _ptr(f), _ptr(L), _ptr(rr), _ptr(z), int(orientation)))
     return z
+
+
+def pressure_apply(fluid: np.ndarray, rows7: np.ndarray, z: np.ndarray, s: np.ndarray, beta: float, orientation: int = 0):
+    """One product of the pressure solve's loop on the GPU: (s, q, s.q) with
+    s = z + beta s (float32) and q = A s (kept as a pair of floats, returned as
+    float64), for rows as mic0_factor takes them."""
+    lib = load_library()
+    K, J, I = fluid.shape
+    f, rows = np.ascontiguousarray(fluid, np.uint8), np.ascontiguousarray(rows7, np.float64)
+    zz, ss = np.ascontiguousarray(z, np.float32), np.ascontiguousarray(s, np.float32)
+    out, q, dot = np.zeros((K, J, I), np.float32), np.zeros((K, J, I), np.float64), C.c_double()
+    _check(lib, lib.flip_pressure_apply(I, J, K, _ptr(f), _ptr(rows), _ptr(zz), _ptr(ss), float(beta), int(orientation), _ptr(out),
+                                        _ptr(q), C.byref(dot)))
+    return out, q, dot.value
 
 
 def viscosity_step(liquid_phi: np.ndarray, solid_phi: np.ndarray, u: np.ndarray, v: np.ndarray, w: np.ndarray, dx: float,

@@ -288,6 +288,13 @@ int flip_mic0_factor(int isize, int jsize, int ksize, const uint8_t *fluid, cons
 int flip_mic0_precondition(int isize, int jsize, int ksize, const uint8_t *fluid, const float *factor,
                            const float *r, float *z, int orientation);
 
+/* One product of the pressure solve's loop alone (unit interface, rows as above):
+ * s_out = z + beta s, q = A s_out and *dot = s_out.q over the flagged cells,
+ * by the solve's kernel: s_out in FP32, q as a pair of floats (here their sum).
+ * s_out and q are 0 off the system.  Errors as above. */
+int flip_pressure_apply(int isize, int jsize, int ksize, const uint8_t *fluid, const double *rows, const float *z,
+                        const float *s, float beta, int orientation, float *s_out, double *q, double *dot);
+
 /* The viscosity step alone (unit interface, as above): the field u, v, w (K x J x
  * (I+1), K x (J+1) x I, (K+1) x J x I floats, updated in place) after the step
  * of flip_set_viscosity below, for a cell-centred liquid level set and a nodal
