@@ -140,9 +140,9 @@ int scan_scratch_ints(int ncells);
 void launch_bin_scatter(const unsigned int *keys, int n, const int *cellStart, int *cursor, int *slots, cudaStream_t s);
 void launch_cell_sort_select(const int *cellStart, int ncells, int *slots, const unsigned int *ids,
                              const unsigned int *keys, int maxPerCell, int *survivorCount, cudaStream_t s);
-void launch_gather_particles(const ParticleSoA &src, ParticleSoA dst, int n,
-                             const int *cellStart, const int *slots, const int *newStart, int ncells,
-                             unsigned int *maxSpeedSqBits, cudaStream_t s);
+void launch_gather_particles(const ParticleSoA &src, ParticleSoA dst, int n, const int *cellStart, const int *slots,
+                             const unsigned int *keys, const int *newStart, int ncells, unsigned int *maxSpeedSqBits,
+                             cudaStream_t s);
 
 // -- grid stages
 // threads: the CTA size, 256, 512 (default) or 1024

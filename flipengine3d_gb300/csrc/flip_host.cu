@@ -602,7 +602,7 @@ int rebin(flip_ctx *x) {
     launch_bin_scatter(x->keys, x->n, x->cellStart, x->cursor, x->slots, s);
     launch_cell_sort_select(x->cellStart, nc, x->slots, x->pa.id, x->keys, x->maxPerCell, x->survivors, s);
     launch_scan_cells(x->survivors, nc, x->newStart, x->scanScratch, x->scanTotal, s);
-    launch_gather_particles(x->pa, x->pb, x->n, x->cellStart, x->slots, x->newStart, nc, x->maxVelSqBits, s);
+    launch_gather_particles(x->pa, x->pb, x->n, x->cellStart, x->slots, x->keys, x->newStart, nc, x->maxVelSqBits, s);
     CK(cudaMemcpyAsync(&x->mail->total, x->scanTotal, sizeof(int), cudaMemcpyDeviceToHost, s));
     CK(cudaMemcpyAsync(&x->mail->velSqBits, x->maxVelSqBits, sizeof(unsigned int), cudaMemcpyDeviceToHost, s));
     if (x->endMarkPending) {

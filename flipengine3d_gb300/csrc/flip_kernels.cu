@@ -176,11 +176,14 @@ __global__ void k_cell_sort_select(const int *start, int ncells, int *slots, con
     survivors[c] = kept;
 }
 
-// The kept particles in (cell, id) order.  Where no particle was removed, which
-// the totals of the two scans tell, particle o of the result is slots[o] and a
-// thread takes one particle: writes are coalesced, and reads nearly so, since
-// particles move few cells.  Otherwise a thread takes a cell, the only form
-// before (stage "binning" 818 -> 588 us with 14.0M particles).
+// The kept particles in (cell, id) order, a thread per binned particle: writes are
+// coalesced, and reads nearly so, since particles move few cells (a thread per
+// cell took 818 us with 14.0M particles, stage "binning", this 588).  Where none was
+// removed, which the totals of the two scans tell, particle t of the result is
+// slots[t].  Otherwise slots[t] is of the cell whose segment t lies in, kept if its
+// place there is among the first ones (300 particles of 256 x 128 x 128 cells, 50 of
+// them removed from one: the stage takes 1.25 ms, most of it that cell's sort; a
+// thread per cell, as many as there are particles, took 3.3 ms).
 __device__ __forceinline__ float gather_one(const ParticleSoA &src, const ParticleSoA &dst, int s, int o) {
     const float vx = src.vx[s], vy = src.vy[s], vz = src.vz[s];
     dst.px[o] = src.px[s];
@@ -192,19 +195,21 @@ __device__ __forceinline__ float gather_one(const ParticleSoA &src, const Partic
     dst.id[o] = src.id[s];
     return __fadd_rn(__fadd_rn(__fmul_rn(vx, vx), __fmul_rn(vy, vy)), __fmul_rn(vz, vz));
 }
-__global__ void k_gather(ParticleSoA src, ParticleSoA dst, const int *start, const int *slots,
+__global__ void k_gather(ParticleSoA src, ParticleSoA dst, const int *start, const int *slots, const unsigned int *keys,
                          const int *newStart, int ncells, unsigned int *maxSpeedSqBits) {
     pdl_begin();
-    const int t = blockIdx.x * blockDim.x + threadIdx.x, total = newStart[ncells];
+    const int binned = start[ncells];
+    const bool all = newStart[ncells] == binned;
     float best = 0.0f;
-    if (total == start[ncells]) {
-        for (int o = t; o < total; o += gridDim.x * blockDim.x)
-            best = fmaxf(best, gather_one(src, dst, slots[o], o));
-    } else {
-        for (int c = t; c < ncells; c += gridDim.x * blockDim.x) {
-            const int b = start[c], o = newStart[c], e = newStart[c + 1];
-            for (int q = 0; q < e - o; q++) best = fmaxf(best, gather_one(src, dst, slots[b + q], o + q));
+    for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < binned; t += gridDim.x * blockDim.x) {
+        const int s = slots[t];
+        int o = t;
+        if (!all) {
+            const int c = (int)(keys[s] & KEY_CELL_MASK), place = t - start[c], first = newStart[c];
+            if (place >= newStart[c + 1] - first) continue;
+            o = first + place;
         }
+        best = fmaxf(best, gather_one(src, dst, s, o));
     }
     for (int o = 16; o > 0; o >>= 1) best = fmaxf(best, __shfl_xor_sync(0xffffffffu, best, o));
     if ((threadIdx.x & 31) == 0 && best > 0.0f) atomicMax(maxSpeedSqBits, __float_as_uint(best));
@@ -966,12 +971,12 @@ void launch_cell_sort_select(const int *cellStart, int ncells, int *slots, const
                              const unsigned int *keys, int maxPerCell, int *survivorCount, cudaStream_t s) {
     launch_next(k_cell_sort_select, div_up(ncells, TPB), TPB, s, cellStart, ncells, slots, ids, keys, maxPerCell, survivorCount);
 }
-void launch_gather_particles(const ParticleSoA &src, ParticleSoA dst, int n,
-                             const int *cellStart, const int *slots, const int *newStart, int ncells,
-                             unsigned int *maxSpeedSqBits, cudaStream_t s) {
+void launch_gather_particles(const ParticleSoA &src, ParticleSoA dst, int n, const int *cellStart, const int *slots,
+                             const unsigned int *keys, const int *newStart, int ncells, unsigned int *maxSpeedSqBits,
+                             cudaStream_t s) {
     if (n <= 0) return;
-    launch_next(k_gather, std::min(div_up(n, TPB), 152u * 16u), TPB, s, src, dst, cellStart, slots, newStart, ncells,
-                                                               maxSpeedSqBits);
+    launch_next(k_gather, std::min(div_up(n, TPB), 152u * 16u), TPB, s, src, dst, cellStart, slots, keys, newStart, ncells,
+                maxSpeedSqBits);
 }
 void launch_liquid_sdf(const ParticleSoA &p, const int *cellStart, const StepConsts &c, const uint8_t *solidCC,
                        float *phi, int threads, cudaStream_t s) {
