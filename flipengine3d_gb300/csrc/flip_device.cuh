@@ -376,6 +376,7 @@ void sweep_epoch_guard(const StepConsts &c, SweepState &sw, long long upcoming, 
 void mic0_factor(const StepConsts &c, const uint8_t *fluid, const double4_32a *Ad, double *E, double *W0, double *W1,
                  double *W2, unsigned int *ticket, int *err, unsigned int spinLimit, cudaStream_t s);
 void mic0_inverse_pivots(const uint8_t *fluid, long long n, double *E, cudaStream_t s);
+void launch_pivot_functions(int n, const double *d, const float *off, double *recip, double *root, cudaStream_t s);
 // The reduction grid of the PCG row kernels: one CTA per `cellsPerCta` grid
 // cells (a tuning knob, default 4096), at most PCG_MAX_PARTIALS.
 constexpr int PCG_MAX_PARTIALS = 152 * 8;

@@ -234,8 +234,10 @@ __device__ __forceinline__ double widen(float f) {
     return __hiloint2double((b & 0x80000000) | (((b & 0x7fffffff) >> 3) + (896 << 20)), b << 29);
 }
 __device__ __forceinline__ float narrow_or_0(double d) { return in_fp32(d) ? narrow(d) : 0.0f; }
-// 1 / d from a guess g: one third-order step, e (1 + r + r^2) with r = 1 - d e,
-// which leaves r^3 < 2^-57; the division for a guess with fewer than 19 bits.
+// 1 / d from a guess g: one step of the third-order hyperpower iteration (Schulz's
+// iteration with the next term of the geometric series), e (1 + r + r^2) with
+// r = 1 - d e, which leaves r^3 < 2^-57; the division for a guess with fewer than
+// 19 bits.
 __device__ __forceinline__ double reciprocal(double d, float g) {
     const double e = widen(g), r = __fma_rn(-d, e, 1.0);
     if ((__double2hiint(r) >> 20 & 0x7ff) >= 1023 - 19) return 1.0 / d;
@@ -247,7 +249,8 @@ __device__ __forceinline__ float guess_reciprocal(float f) {
     return g;
 }
 // sqrt(e), e the reciprocal of a pivot: the inverse pivot.  The same way: a
-// guess from the FP32 unit, then two Newton steps.
+// guess from the FP32 unit, then two steps of Newton's iteration for x^2 = e with
+// the slope 1 / 2x kept from the guess.
 __device__ __forceinline__ double inverse_pivot(double e) {
     if (!(e > 0.0) || !in_fp32(e)) return sqrt(e);
     const float f = narrow(e);
@@ -436,6 +439,14 @@ __global__ void __launch_bounds__(FTHREADS) k_mic0_tiles(StepConsts c, const uin
         }
         now = next;
     }
+}
+// The two functions above on their own: 1 / d from the unit's guess times `off`,
+// and sqrt(d).
+__global__ void k_pivot_functions(int n, const double *d, const float *off, double *recip, double *root) {
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= n) return;
+    recip[t] = reciprocal(d[t], guess_reciprocal(narrow_or_0(d[t])) * off[t]);
+    root[t] = inverse_pivot(d[t]);
 }
 // Pivots' reciprocals to inverse pivots, 0 off the system.
 __global__ void k_mic0_inverse(const uint8_t *fluid, long long n, double *E) {
@@ -1200,6 +1211,11 @@ void mic0_factor(const StepConsts &c, const uint8_t *fluid, const double4_32a *A
 void mic0_inverse_pivots(const uint8_t *fluid, long long n, double *E, cudaStream_t s) {
     FLIP_COUNT(1);
     k_mic0_inverse<<<div_up(n, TPB), TPB, 0, s>>>(fluid, n, E);
+}
+
+void launch_pivot_functions(int n, const double *d, const float *off, double *recip, double *root, cudaStream_t s) {
+    FLIP_COUNT(1);
+    k_pivot_functions<<<div_up(n, TPB), TPB, 0, s>>>(n, d, off, recip, root);
 }
 
 // The chunks of the sweep layout that the sweeps pass over, and the system's

@@ -99,6 +99,25 @@ extern "C" int flip_mic0_factor(int I, int J, int K, const uint8_t *fluid, const
     return cuda_status(cudaMemcpy(invdiag, dInv, n * sizeof(double), cudaMemcpyDeviceToHost), "read pivots");
 }
 
+extern "C" int flip_mic0_pivot_functions(int n, const double *d, const float *guess_off, double *reciprocal, double *root) {
+    if (n < 0) return record_error(FLIP_E_DOMAIN, "negative count");
+    if (n == 0) return FLIP_OK;
+    if (!d || !guess_off || !reciprocal || !root) return record_error(FLIP_E_NULL, "null pointer");
+    Scratch sc;
+    double *dd, *dr, *ds;
+    float *doff;
+    const size_t bytes = (size_t)n * sizeof(double);
+    if (!sc.get(&dd, n) || !sc.get(&dr, n) || !sc.get(&ds, n) || !sc.get(&doff, n))
+        return record_error(FLIP_E_NOMEM, "cudaMalloc failed");
+    int rc;
+    if ((rc = cuda_status(cudaMemcpy(dd, d, bytes, cudaMemcpyHostToDevice), "copy")) ||
+        (rc = cuda_status(cudaMemcpy(doff, guess_off, (size_t)n * sizeof(float), cudaMemcpyHostToDevice), "copy")))
+        return rc;
+    launch_pivot_functions(n, dd, doff, dr, ds, nullptr);
+    if ((rc = cuda_status(cudaMemcpy(reciprocal, dr, bytes, cudaMemcpyDeviceToHost), "pivot functions"))) return rc;
+    return cuda_status(cudaMemcpy(root, ds, bytes, cudaMemcpyDeviceToHost), "read");
+}
+
 extern "C" int flip_mic0_precondition(int I, int J, int K, const uint8_t *fluid, const float *factor, const float *r,
                                       float *z, int orientation) {
     if (!fluid || !factor || !r || !z) return record_error(FLIP_E_NULL, "null pointer");

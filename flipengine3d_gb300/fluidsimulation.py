@@ -146,6 +146,7 @@ SIGNATURES = {
     "flip_get_sweep_orientation": [_P, C.POINTER(C.c_int)],
     "flip_order_particles_by_id_noalloc": [_P, _P, _P, _P, _I, _I, _P, _P],
     "flip_mic0_factor": [_I, _I, _I, _P, _P, _P],
+    "flip_mic0_pivot_functions": [_I, _P, _P, _P, _P],
     "flip_mic0_precondition": [_I, _I, _I, _P, _P, _P, _P, _I],
     "flip_pressure_apply": [_I, _I, _I, _P, _P, _P, _P, C.c_float, _I, _P, _P, C.POINTER(C.c_double)],
     "flip_viscosity_step": [_I, _I, _I, _D, _P, _P, _P, _P, _P, _D, _D, C.POINTER(C.c_longlong), C.POINTER(C.c_int),
@@ -362,6 +363,18 @@ def mic0_factor(fluid: np.ndarray, rows7: np.ndarray) -> np.ndarray:
     inv = np.zeros((K, J, I), np.float64)
     _check(lib, lib.flip_mic0_factor(I, J, K, _ptr(f), _ptr(rows), _ptr(inv)))
     return inv
+
+
+def mic0_pivot_functions(d: np.ndarray, guess_off: np.ndarray):
+    """(1 / d, sqrt(d)) as the MIC(0) factor works them out on the GPU; its guess
+    of each reciprocal is multiplied by guess_off (float32)."""
+    lib = load_library()
+    d, off = np.ascontiguousarray(d, np.float64), np.ascontiguousarray(guess_off, np.float32)
+    if d.ndim != 1 or off.shape != d.shape:
+        raise ValueError("two vectors of one length")
+    recip, root = np.zeros_like(d), np.zeros_like(d)
+    _check(lib, lib.flip_mic0_pivot_functions(len(d), _ptr(d), _ptr(off), _ptr(recip), _ptr(root)))
+    return recip, root
 
 
 def mic0_precondition(fluid: np.ndarray, factor: np.ndarray, r: np.ndarray, orientation: int = 0) -> np.ndarray:

@@ -282,8 +282,12 @@ int flip_inject_sweep_stall(flip_ctx *ctx, int on);
  *     solveLower then solveLowerTransposeInPlace (pcgsolver.h:192-221), with
  *     the factor given as {invdiag, L to +x, L to +y, L to +z} floats per cell;
  *     orientation 0 or 1 picks the sweep tiles' lane axis (j or k).
+ *   flip_mic0_pivot_functions: what the factor takes for 1 / d and sqrt(d) of n
+ *     doubles; its guess of each reciprocal is multiplied by guess_off (1 where
+ *     nothing is tried).
  * FLIP_E_DOMAIN for a flagged cell on the border, FLIP_E_DEVICE_TIMEOUT if a
  * bounded wait gave up. */
+int flip_mic0_pivot_functions(int n, const double *d, const float *guess_off, double *reciprocal, double *root);
 int flip_mic0_factor(int isize, int jsize, int ksize, const uint8_t *fluid, const double *rows, double *invdiag);
 int flip_mic0_precondition(int isize, int jsize, int ksize, const uint8_t *fluid, const float *factor,
                            const float *r, float *z, int orientation);
