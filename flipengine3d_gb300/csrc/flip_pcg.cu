@@ -425,8 +425,10 @@ __global__ void __launch_bounds__(FTHREADS) k_mic0_tiles(StepConsts c, const uin
                 d = __fma_rn(-now.w0[m], ez, d);
                 d = __fma_rn(-now.w1[m], ey, d);
                 const double least = 0.25 * ad;
-                // positive doubles compare as integers
-                const bool low = ad > 0.0 ? __double_as_longlong(d) < __double_as_longlong(least) : d < least;
+                // positive doubles compare as integers, and a quiet NaN, whatever its sign, is not below
+                const bool low = ad > 0.0 ? __double_as_longlong(d) < __double_as_longlong(least) &&
+                                                (unsigned)__double2hiint(d) <= 0xfff00000u
+                                          : d < least;
                 if (low) e = 1.0 / ad;
                 else if (ad != 0.0) e = reciprocal(d, g);
                 if (__double_as_longlong(e) == NOT_YET) e = __longlong_as_double(NOT_YET - 1);

@@ -1,7 +1,9 @@
 """What the MIC(0) factor takes for 1 / d and sqrt(d), against IEEE division and
 square root over the whole exponent range: subnormal, huge, negative, zero,
 infinite and NaN inputs, the ends of the range in which FP32 supplies the guess,
-and guesses that are off by more and by less than the step can mend.
+and guesses that are off by more and by less than the step can mend.  And a row
+that is not a number: what depends on it is not one either, as in the
+reference's elimination, and nothing else changes.
 
 Bound: the remainder of either iteration is below 2^-56 of the result, so it is
 within half a unit in the last place and a sixteenth of the exact value, and at
@@ -11,6 +13,8 @@ from __future__ import annotations
 
 import numpy as np
 import pytest
+
+from oracle import refsim
 
 
 def inputs():
@@ -43,3 +47,21 @@ def test_pivot_functions(gpu, off):
     plain = ~np.isfinite(want) | (d == 0) | ~np.isfinite(d)
     assert np.array_equal(recip[plain], want[plain], equal_nan=True)
     assert np.array_equal(root[plain], want_root[plain], equal_nan=True)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("what", [np.nan, -np.nan, np.inf])
+@pytest.mark.parametrize("entry", [0, 1, 2, 3])   # diagonal, couplings to +x, +y, +z
+def test_a_row_that_is_no_number(gpu, what, entry):
+    import flipengine3d_gb300.fluidsimulation as fs
+    fluid, rows = refsim.random_mic0_system((11, 13, 20), 3)
+    at = tuple(np.argwhere((fluid > 0) & (rows[..., 1] != 0) & (rows[..., 2] != 0) & (rows[..., 3] != 0))[40])
+    rows[at + (entry,)] = what
+    got = fs.mic0_factor(fluid, rows)
+    with np.errstate(all="ignore"):
+        want, _ = refsim.mic0_factor(fluid, rows, "orc")
+    m = (fluid > 0) & (rows[..., 0] != 0)   # a row of zeros has no pivot: 0 here, whatever is around it
+    assert not got[~m].any()
+    assert np.array_equal(np.isnan(got[m]), np.isnan(want[m])), (np.isnan(got[m]).sum(), np.isnan(want[m]).sum())
+    ok = m & ~np.isnan(want)
+    assert np.allclose(got[ok], want[ok], rtol=1e-12, atol=0)
