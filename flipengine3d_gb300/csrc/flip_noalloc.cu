@@ -29,8 +29,10 @@ constexpr int TPB = 256, SCAN_TPB = 1024;
 
 // Ids as bits, 32 to a word, and for each word how many ids lie below it: an id's
 // rank is that and the bits below its own.  Four launches of a few microseconds
-// each, every one started while the one before it ends; with a word per id,
-// scanned in three steps, there were six (300k ids: 29.7 us a call, now 20.5).
+// each, every one started while the one before it ends.  A call on ids in random
+// order takes 15.5 us for 1000, 17 for 300k and 42 for 2^20; with a word per id,
+// scanned in three steps, there were six launches (23, 31 and 50), and with the
+// words scanned by one CTA 300k took 21 and 2^20 95.
 __global__ void __launch_bounds__(TPB) k_na_clear(unsigned *bits, int words) {
     flip::pdl_trigger();
     const int t = blockIdx.x * TPB + threadIdx.x;
@@ -45,14 +47,17 @@ __global__ void __launch_bounds__(TPB) k_na_flag(const unsigned int *ids, int n,
     if (id < (unsigned int)idSpace) atomicOr(&bits[id >> 5], 1u << (id & 31));
 }
 
-// One CTA: each thread takes `per` words in a row.
-__global__ void __launch_bounds__(SCAN_TPB) k_na_scan(const unsigned *bits, int words, int per, int *below) {
-    __shared__ int warpSums[SCAN_TPB / 32];
+// A word a thread.  A CTA adds up the words before its own itself (at most 31 loads a
+// thread, side by side), so that there is nothing to wait for and no launch more.
+__global__ void __launch_bounds__(SCAN_TPB) k_na_scan(const unsigned *bits, int words, int *below) {
+    __shared__ int warpSums[SCAN_TPB / 32], warpBefore[SCAN_TPB / 32];
     flip::pdl_wait();
     flip::pdl_trigger();
-    const int first = threadIdx.x * per, last = min(first + per, words);
-    int own = 0;
-    for (int w = first; w < last; w++) own += __popc(bits[w]);
+    const int first = blockIdx.x * SCAN_TPB, w = first + threadIdx.x;
+    int before = 0;
+#pragma unroll 8
+    for (int v = threadIdx.x; v < first; v += SCAN_TPB) before += __popc(bits[v]);
+    const int own = w < words ? __popc(bits[w]) : 0;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     int inc = own;
 #pragma unroll
@@ -60,15 +65,15 @@ __global__ void __launch_bounds__(SCAN_TPB) k_na_scan(const unsigned *bits, int 
         const int y = __shfl_up_sync(0xffffffffu, inc, o);
         if (lane >= o) inc += y;
     }
-    if (lane == 31) warpSums[warp] = inc;
-    __syncthreads();
-    int sum = warpSums[lane];   // every warp adds up the warps before it
-    sum = __reduce_add_sync(0xffffffffu, lane < warp ? sum : 0);
-    int run = sum + inc - own;
-    for (int w = first; w < last; w++) {
-        below[w] = run;
-        run += __popc(bits[w]);
+    before = __reduce_add_sync(0xffffffffu, before);
+    if (lane == 31) {
+        warpSums[warp] = inc;
+        warpBefore[warp] = before;
     }
+    __syncthreads();
+    // every warp adds up the warps before it, and all of the earlier CTAs' words
+    const int sum = __reduce_add_sync(0xffffffffu, warpBefore[lane] + (lane < warp ? warpSums[lane] : 0));
+    if (w < words) below[w] = sum + inc - own;
 }
 
 __global__ void __launch_bounds__(TPB) k_na_scatter(const float *px, const float *py, const float *pz, const unsigned int *ids,
@@ -116,13 +121,13 @@ extern "C" int flip_order_particles_by_id_noalloc(const float *d_px, const float
     int rc = scratch_for_current_context(&scratch);
     if (rc) return rc;
     cudaStream_t s = (cudaStream_t)stream;
-    const int words = (id_space + 31) / 32, per = (words + SCAN_TPB - 1) / SCAN_TPB;
+    const int words = (id_space + 31) / 32;
     unsigned *bits = reinterpret_cast<unsigned *>(scratch);
     int *below = scratch + words;
     // the first one after all of the caller's work, the others overlapping the one before
     flip::launch_after(false, k_na_clear, flip::div_up(words, TPB), TPB, 0, s, bits, words);
     flip::launch_after(true, k_na_flag, flip::div_up(n, TPB), TPB, 0, s, d_ids, n, id_space, bits);
-    flip::launch_after(true, k_na_scan, 1, SCAN_TPB, 0, s, bits, words, per, below);
+    flip::launch_after(true, k_na_scan, flip::div_up(words, SCAN_TPB), SCAN_TPB, 0, s, bits, words, below);
     flip::launch_after(true, k_na_scatter, flip::div_up(n, TPB), TPB, 0, s, d_px, d_py, d_pz, d_ids, n, id_space, bits, below,
                        d_out_xyz);
     cudaError_t e = cudaGetLastError();
