@@ -74,7 +74,7 @@ struct PairOps {
     __device__ F2 mul(F2 a, F2 b) const { return f2_fma(a, b, zero); }
     __device__ F2 add(F2 a, F2 b) const { return f2_fma(a, ONE, b); }
     __device__ F2 sub(F2 a, F2 b) const { return f2_fma(b, MINUS, a); }
-    __device__ F2 neg(F2 a) const { return a ^ f2_bits(0x80000000u, 0x80000000u); }
+    __device__ F2 neg(F2 a) const { return f2_fma(a, MINUS, f2_bits(0x80000000u, 0x80000000u)); }   // exact
 };
 
 // Programmatic dependent launch: a kernel launched with launch_after may start
