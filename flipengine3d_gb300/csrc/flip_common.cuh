@@ -41,24 +41,12 @@ __device__ __forceinline__ int exact_floor(float p, double inv, float invf) {
     return floor_fp64(p, inv);
 }
 
-__device__ __forceinline__ float idx_to_pos(int i, double dx) { return (float)((double)(float)i * dx); }
 __device__ __forceinline__ float cell_centre(int i, double dx) { return (float)((double)(float)i * dx + 0.5 * dx); }
-
-// order-preserving float <-> uint32 encoding for deterministic atomicMin
-__device__ __forceinline__ unsigned int f2ord(float f) {
-    unsigned int b = __float_as_uint(f);
-    return (b & 0x80000000u) ? ~b : (b | 0x80000000u);
-}
-__device__ __forceinline__ float ord2f(unsigned int u) {
-    unsigned int b = (u & 0x80000000u) ? (u & 0x7fffffffu) : ~u;
-    return __uint_as_float(b);
-}
 
 // Particle key flags (bits above the 28-bit cell index).
 constexpr unsigned int KEY_CELL_MASK = 0x0fffffffu;
 constexpr unsigned int KEY_SOLID = 0x80000000u;    // removed: inside the solid
 constexpr unsigned int KEY_FAST = 0x40000000u;     // over the extreme-speed limit
-constexpr unsigned int KEY_NONE = 0xffffffffu;     // no particle
 
 inline unsigned int div_up(long long a, int b) { return (unsigned int)((a + b - 1) / b); }
 // Grid coordinates of a flat index i + ni*(j + nj*k).  Grids hold fewer than

@@ -212,7 +212,10 @@ void launch_mark_fast(const ParticleSoA &p, int n, const float *maxSpeedSq, unsi
 // (tile * T + tf) * SWEEP_NP + warp * 32 + lane.
 // T = I - 2 + (SWEEP_WA - 1) + (SWEEP_WB - 1) up to a multiple of SWEEP_CH, so that
 // a chunk of SWEEP_CH steps is one contiguous block in either sweep direction.
-// Entries that hold no interior cell stay zero.
+// In the chunks that a solve passes over (its items), the factor rows, the rows of
+// the matrix and the right-hand side are zero at entries without a cell of the
+// system.  Elsewhere the matrix is zero, the factor rows are not read, and z and s
+// hold finite values that an earlier solve left, which only ever meet a zero.
 constexpr int SWEEP_WA = 16, SWEEP_WB = 8, SWEEP_NP = SWEEP_WA * SWEEP_WB, SWEEP_CH = 8;
 constexpr int SWEEP_VA = 8, SWEEP_VB = 4;
 constexpr int SWEEP_CA = 2, SWEEP_CB = 4;   // tiles of a thread-block cluster along a and b
@@ -481,10 +484,11 @@ int mesh_surface(const MeshJob &job, MeshBuffers &mb, cudaStream_t s);
 void mesh_release(MeshBuffers &mb);
 int record_error(int code, const std::string &msg);   // sets flip_last_error()
 
-// Packed xyz positions/velocities (either may be null) of the n particles in
-// the reference's order; flags/rank hold idSpace+1 ints, scratch
-// scan_scratch_ints(idSpace) ints.
+// Packed xyz positions/velocities (either may be null) of the n particles, whose
+// ids are dense (0..n-1), in the reference's order.
 void launch_readback_order(const ParticleSoA &p, int n, float *pos, float *vel, cudaStream_t s);
+// Ids to their ranks 0..n-1: flags and rank hold idSpace+1 ints, scratch
+// scan_scratch_ints(idSpace).
 void launch_compact_ids(const ParticleSoA &p, int n, int idSpace, int *flags, int *rank, int *scratch, int *total,
                         cudaStream_t s);
 }  // namespace flip

@@ -156,7 +156,6 @@ struct flip_ctx {
     // device buffers
     ParticleSoA pa{}, pb{};
     unsigned int *keys = nullptr;
-    int idSpace = 0;   // ids are ranks in the load order, below idSpace
     int *idFlags = nullptr, *idRank = nullptr, *idScratch = nullptr, *idTotal = nullptr;
     int *cellCount = nullptr, *cellStart = nullptr, *cursor = nullptr, *slots = nullptr;
     int *survivors = nullptr, *newStart = nullptr, *scanScratch = nullptr, *scanTotal = nullptr;
@@ -346,7 +345,6 @@ int alloc_particles(flip_ctx *x, int cap) {
     int rc;
     cap += cap & 1;   // planes of pairs of floats
     x->capacity = cap;
-    x->idSpace = cap;
     ParticleSoA *bufs[2] = {&x->pa, &x->pb};
     for (ParticleSoA *b : bufs) {   // one block per buffer: 6 float planes then the ids
         float *base;
@@ -1563,7 +1561,7 @@ int flip_estimate_device_bytes(int isize, int jsize, int ksize, int particles, l
     long long b = 0;
     b += 5 * (nc + 1) * 4 + (scan_scratch_ints((int)nc) + 4) * 4 + 16;   // binning
     b += nc * 4 + (I + 1) * (J + 1) * (K + 1) * 4 + nc;                  // phi, solid phi, solid cells
-    b += faces * (4 * 3 + 1) + 8 * face_bits(isize, jsize, ksize).words;                                        // weights, velocity, saved, valid, status
+    b += faces * (4 * 3 + 1) + 8 * face_bits(isize, jsize, ksize).words;   // weights, velocity, saved, valid; known
     b += nc * (1 + 32 + 8 * 2 + 4) + nsl * (16 + 4 * 9) + 12 * SWEEP_NP + 4 * std::max(8 * (nsl + SWEEP_NP), 6 * nc);   // pressure system
     b += 4 * (sweep_items_max(isize, jsize, ksize) + 8) + 16;              // its items
     b += 2 * PCG_MAX_PARTIALS * 8 + 64 + 16 + 32;

@@ -178,7 +178,7 @@ __global__ void k_cell_sort_select(const int *start, int ncells, int *slots, con
 
 // The kept particles in (cell, id) order, a thread per binned particle: writes are
 // coalesced, and reads nearly so, since particles move few cells (a thread per
-// cell took 818 us with 14.0M particles, stage "binning", this 588).  Where none was
+// cell took 813 us with 14.0M particles, stage "binning", this 537).  Where none was
 // removed, which the totals of the two scans tell, particle t of the result is
 // slots[t].  Otherwise slots[t] is of the cell whose segment t lies in, kept if its
 // place there is among the first ones (300 particles of 256 x 128 x 128 cells, 50 of
@@ -226,12 +226,12 @@ __global__ void k_gather(ParticleSoA src, ParticleSoA dst, const int *start, con
 // first, as long as a row can still hold a nearer one.  A cell inside the
 // liquid has a particle within half a cell and stops at its own, and the air
 // far from it knows from a look of the warp at the 25 rows around.  Bound by the
-// latency and the instructions of the cells near the surface: 225 us at 128^3
-// (4.1M particles), 68 at 64^3; scattering every particle
-// into the ~100 cells of its box through shared-memory atomics took 820, 370.
-// 64 registers a thread: with 128 the occupancy is too low, with 42 small grids
-// lose what large ones gain (in CTAs of 512: 313, 456 and 274 us at 128^3, 68, 94
-// and 74 at 64^3).
+// latency and the instructions of the cells near the surface.  The stage in
+// frames: 253 us at 128^3 (4.1M particles), 69 at 64^3, 251 at 256x128x128 (14.0M);
+// scattering every particle into the ~100 cells of its box through shared-memory
+// atomics took 857, 375 and 1947.  64 registers a thread: with 128 the occupancy is
+// too low, with 42 small grids lose what large ones gain (the kernel alone, in CTAs
+// of 512: 313, 456 and 274 us at 128^3, 68, 94 and 74 at 64^3).
 // Then the solid post-process (particlelevelset.cpp:172-196).
 constexpr int BW = 10;
 
@@ -389,9 +389,10 @@ __global__ void __launch_bounds__(SDF_TPB, 1024 / SDF_TPB) k_liquid_sdf(Particle
 // at a time, in packed arithmetic (each half rounds as the scalar operation),
 // and of each row of cells only the faces it can reach.  The lanes of a warp
 // visit different cells, so a load touches 32 lines; positions and velocities
-// load in pairs.  P2G at 128^3 (4.1M particles), at 256x128x128 (14.0M): a kernel
-// per direction 740, 2000 us; one for the three 640, 1160; now 433, 730.  16-byte
-// vectors of a particle's coordinates touch four times the lines: slower.
+// load in pairs.  The stage in frames, with the extrapolation's seven layers: 587 us
+// at 128^3 (4.1M particles), 889 at 256x128x128 (14.0M), the kernel 476 at 128^3
+// (cold, in a profile); with a kernel per direction 875 and 2389.  16-byte vectors of
+// a particle's coordinates touch four times the lines: slower.
 // The reference also requires the face to lie in the particle's local box and
 // the particle to be in the block's list, both taken with the support radius
 // sr = r + 1e-6.  A particle within r of the face meets both: every coordinate
@@ -506,7 +507,7 @@ __global__ void __launch_bounds__(P2G_TPB, 1024 / P2G_TPB) k_p2g(ParticleSoA p, 
 // fill are looked at face by face, a lane per face.  A status byte and a
 // thread per face and layer took 31 us a layer at 128^3, nearly all of it on
 // faces with nothing to do (stage "constrain", 7 layers and two passes: 233 ->
-// 129 us at 128^3, 335 -> 171 us at 256 x 128 x 128).
+// 138 us at 128^3, 335 -> 172 us at 256 x 128 x 128).
 __device__ __forceinline__ void face_word(const FaceBits &b, long long t, int &dir, int &wx, int &j, int &k) {
     dir = t < b.base[1] ? 0 : (t < b.base[2] ? 1 : 2);
     unflatten(t - b.base[dir], b.wpr[dir], b.nj[dir], wx, j, k);
@@ -857,9 +858,9 @@ struct AdvectSteps {
 // Fused particle update: PIC/FLIP velocity (fluidsimulation.cpp:4082-4092),
 // Ralston RK3 (4191-4198), collision (4221-4296), then the removal tests and
 // the new cell key for the next binning.  Bound by instructions and the latency
-// of the 104 scattered corner reads a particle, 269 us at 128^3 (4.1M particles),
-// 824 at 256x128x128 (14.0M).  A bounds test and a 64-bit address per corner took
-// 594, 1720; FP64 divisions of the time step by each thread 328, 1112.
+// of the 104 scattered corner reads a particle: the stage takes 278 us at 128^3 (4.1M
+// particles), 817 at 256x128x128 (14.0M).  A bounds test and a 64-bit address per
+// corner took 614, 1705; FP64 divisions of the time step by each thread 328, 1112.
 __global__ void __launch_bounds__(TPB) k_advect(ParticleSoA p, int n, StepConsts c, const float *u, const float *v,
                                                 const float *w, const float *su, const float *sv, const float *sw,
                                                 const float *S, const uint8_t *ns, float picRatio, float flipRatio,
@@ -982,7 +983,8 @@ void launch_liquid_sdf(const ParticleSoA &p, const int *cellStart, const StepCon
                        float *phi, int threads, cudaStream_t s) {
     FLIP_COUNT(1);
     // CTAs of half the knob's threads: a CTA lasts as long as its slowest warp
-    // (128^3: 223 us with CTAs of 256 threads, 299 with 512, 370 with 1024)
+    // (the kernel alone at 128^3: 223 us with CTAs of 256 threads, 299 with 512, 370
+    // with 1024)
     const int cta = threads / 2;
     auto *kernel = cta == 128 ? k_liquid_sdf<128> : cta == 512 ? k_liquid_sdf<512> : k_liquid_sdf<256>;
     kernel<<<div_up((long long)c.I * c.J * c.K, cta), cta, 0, s>>>(p, cellStart, c, solidCC, phi);

@@ -506,7 +506,11 @@ __device__ __forceinline__ bool near_particles(const MeshFrame &m, const unsigne
 // k_mesh_walls, which works on full warps.
 // Bound by the searches near the surface and their latency: 345 us at 128^3,
 // subdivision 2 (17M nodes), where scattering every particle over its box took
-// 2250 us for all values; 21 us at 71x59x83, subdivision 1.
+// 2250 us for all values; 21 us at 71x59x83, subdivision 1.  The searches grow with the
+// particles' radius, but less than the boxes did: whole meshes of a 64^3 dam,
+// subdivision 2, took 876 us where the scatter took 1462 at marker particle scale 1,
+// 345 (943) at 3, 393 (3256) at 8 and 463 (7465) at 12; of 20000 lone particles in
+// 128^3 cells 2.2 ms (10.5) at 3 and 8.1 (15.8) at 12.
 __global__ void __launch_bounds__(SEARCH_TPB, 1024 / SEARCH_TPB) k_mesh_inside(ParticleSoA p, const int *cellStart, MeshFrame m,
                                                                                const uint8_t *active, const unsigned *around,
                                                                                const float *solidPhi, unsigned *inside,

@@ -633,15 +633,15 @@ __device__ __forceinline__ double bits_to_resid(const unsigned long long *p) {
 }
 
 // The row kernels below run over the items of the solve on a fixed grid per
-// context (pressure_row_grid CTAs): each thread sums its entries in a fixed
-// order, each CTA writes one partial, and the last CTA adds the partials in a
-// fixed order, so every sum is deterministic.  Entries without a row hold
+// context (pressure_partials_for CTAs): each thread sums its entries in a fixed
+// order, each CTA writes one partial, and whoever needs the sum adds the partials
+// in a fixed order, so every sum is deterministic.  Entries without a row hold
 // zeros.  The vectors live in the sweep layout: a warp takes one step of a
 // tile, whose entries are contiguous, and a row's six neighbours are entries
 // of the steps before and after it, so loads are 16-byte and coalesced (a row
-// list in cell order gathered every neighbour on its own).  Warm times of the
-// SpMV, the update and z.r: 17.3, 8.9 and 5.0 us at 518k rows (16.4, 12.4 and
-// 12.5 us with the row list), 8.2, 4.9 and 3.8 us at 59k rows (11.1, 9.2, 8.8).
+// list in cell order gathered every neighbour on its own).  The SpMV, the update
+// and z.r, cold in a launch list: 17.7, 11.6 and 6.6 us at 518k rows (18.5, 14.8 and
+// 13.9 with the row list).
 
 // Double-float arithmetic on the FP32 pipe (this GPU's FP64 rate is ~1/64
 // of FP32): a coefficient a = hi + lo (floats, exact to 48 bits) times an

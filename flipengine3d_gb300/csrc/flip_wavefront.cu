@@ -20,9 +20,9 @@
 // a or b (two shuffles a step).  The warps of a tile share the step numbers
 // and run on four schedulers without a barrier; each waits only for the terms
 // of its own edge pencils.  A step is bound by the latencies of one warp's
-// instructions (about 75 cycles, plus 60 for the group's and the chunk's
-// waits); bundles of 2 x 2 pencils per lane, one warp a tile, took 205 cycles
-// a step and saved fewer hops than that costs.  128 pencils
+// instructions (about 85 cycles, and some 30 more for its part of the group's and
+// the chunk's waits); bundles of 2 x 2 pencils per lane, one warp a tile, took 205
+// cycles a step and saved fewer hops than that costs.  128 pencils
 // per CTA rather than more: a step reads 20 and writes 4 bytes per pencil, and
 // 3 KB a step is what one SM can draw from L2 in the time of a step.  In the
 // forward sweep a cell hands its neighbours the finished products L_c * y_c
@@ -63,10 +63,10 @@
 // shuffles a step waits for are issued before the last one's stores.
 //
 // Measured per launch (events around a pair, in the frames): 128^3 dam break (518k
-// rows) 38.5 us, 64^3 17.0 us, 256 x 128 x 128 tank (1.8M rows) 51.2 us, without
-// the look ahead 41.0, 18.2 and 54.5; the
-// form before it (tiles of 32 x 8 pencils, four warps in lockstep with a
-// barrier a step, every edge through L2) took 50.5, 23.0 and 71.3 us.
+// rows) 39.0 us, 64^3 (58k rows) 19.6 us, 256 x 128 x 128 tank (1.8M rows) 50.7 us;
+// the form before it (tiles of 32 x 8 pencils, four warps in lockstep with a barrier
+// a step, every edge through L2) took 53.2, 25.6 and 71.4 us on the same box, and the
+// look ahead saved 2.5, 1.2 and 3.4.
 #include <atomic>
 #include <type_traits>
 
